@@ -471,11 +471,11 @@ static int knn_device_tc(int mode, int nq, int nc, int d, int k, const float *Xq
     const double ctas = (double)P.qtiles * P.S, warps = ctas * TC_EPI_WARPS;
     std::fprintf(stderr,
                  "gsknn tc: mode=%d n=%d m=%d d=%d k=%d S=%d N=%d NST=%d: logged/query=%.1f "
-                 "inserts/query=%.1f loop-iters/warp=%.1f slow-chunks/warp=%.1f "
+                 "flushes/warp=%.1f slow-chunks/warp=%.1f "
                  "chunks/warp=%.1f rerank-scanned/query=%.1f exact/query=%.1f fallback=%d | "
                  "cycles/CTA: mma-loop=%.0f mma-wait-tma=%.0f mma-wait-epilogue=%.0f | "
                  "cycles/warp: epi-loop=%.0f epi-wait-mma=%.0f\n",
-                 mode, nq, nc, d, k, P.S, P.N, P.NST, (double)h[0] / nq, (double)h[1] / nq,
+                 mode, nq, nc, d, k, P.S, P.N, P.NST, (double)h[0] / nq,
                  (double)h[2] / warps, (double)h[3] / warps, (double)h[4] / warps,
                  (double)h[5] / nq, (double)h[6] / nq, nfb, (double)h[10] / ctas,
                  (double)h[7] / ctas, (double)h[8] / ctas, (double)h[11] / warps,

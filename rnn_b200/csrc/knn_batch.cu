@@ -919,10 +919,10 @@ int gsknn_batch_sync(gsknn_batch_t *job) {
     BCU(cudaMemset(b->tc_counters, 0, sizeof(h)));
     const double rows = (double)b->tc_cnt_rows, warps = (double)b->tc_cnt_ctas * 8;
     std::fprintf(stderr,
-                 "gsknn batch tc: panel rows=%lld logged/row=%.1f inserts/row=%.1f "
+                 "gsknn batch tc: panel rows=%lld logged/row=%.1f "
                  "slow-chunks/warp=%.1f chunks/warp=%.1f rerank-scanned/row=%.1f "
                  "exact/row=%.1f\n",
-                 b->tc_cnt_rows, (double)h[0] / rows, (double)h[1] / rows, (double)h[3] / warps,
+                 b->tc_cnt_rows, (double)h[0] / rows, (double)h[3] / warps,
                  (double)h[4] / warps, (double)h[5] / rows, (double)h[6] / rows);
     b->tc_cnt_rows = b->tc_cnt_ctas = 0;
   }

@@ -112,7 +112,7 @@ void batch_set_global_ids(void *job, const uint32_t *gid);
 
 struct TcPlan {
   bool ok;
-  int fmt, elem, d_pad, nkc, a_terms, b_terms, kp;
+  int fmt, elem, d_pad, nkc, a_terms, kp;
   int N, NST, qtiles, rtiles, q_pad, r_pad, S, tiles_per_split, logcap;
   unsigned smem;
   float coefA, coefB;
@@ -127,7 +127,7 @@ struct TcPlan {
   size_t cand_bytes;  // prepared-candidate area at the start of the workspace (0: separate)
   // Escalation: queries whose band log overflowed in this format run again in a narrower one
   // (esc_mode, 0 = none: they go straight to the FP64 brute force). Its query-side workspace
-  // starts at o_esc; o_ecand holds its candidate panels when the prepared candidates carry
+  // starts at o_esc, over the logs that the re-rank is done with; o_ecand holds its candidate panels when the prepared candidates carry
   // none (packed only when some query overflowed).
   int esc_mode;
   size_t o_esc, o_ecand, esc_bytes, ecand_bytes;

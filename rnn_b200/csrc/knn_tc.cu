@@ -19,12 +19,12 @@
 //                 ceil(k/2) smallest d' of its own columns in shared memory; any two such heaps
 //                 hold k candidates, so the second smallest root a row can see (its own, the
 //                 other part's, and the roots up to three other splits published) bounds the
-//                 k-th from above (threshold = that + 2E); a per-query log in HBM of every
-//                 candidate under the threshold
-//   tc_rerank     one warp per query: exact FP64 distances of the logged band, sorted merge with
-//                 the incoming heap row, descending write-back (a valid max-heap);
-//                 tc_rerank_hold (BF16, k <= 64) holds the band above the approximate k-th back,
-//                 tc_rerank_leaf (batching form) sorts and writes a row only if it changes
+//                 k-th from above (threshold = that + 2E); per-query logs in HBM of every group of
+//                 four adjacent candidates with one under the threshold
+//   tc_rerank     one warp per query (tc_rerank_cta: one CTA per query, for few queries): exact
+//                 FP64 distances of the logged band, sorted merge with the incoming heap row,
+//                 descending write-back (a valid max-heap); tc_rerank_leaf (batching form) sorts
+//                 and writes a row only if it changes
 //   tc_fallback   queries whose log overflowed: exact FP64 brute force over all candidates
 //
 // Error bound (per query q, all candidates c; u = unit roundoff of the MMA input format,
@@ -58,6 +58,7 @@ constexpr int NTHREADS = 32 * (2 + NEPI);
 // accumulator columns per TMEM wait: 64 (two loads) while the registers allow, else 32
 constexpr int EPI_STEP = NPART <= 2 ? 64 : 32;
 constexpr uint32_t LOG_OVF = 1u << 30;
+constexpr size_t LOG_ENTRY = sizeof(float4) + sizeof(uint32_t);  // a logged quad and its position
 // The epilogue frees a TMEM accumulator as soon as its reads have landed, while it still uses
 // the tile's candidate norms; the norms therefore get one slot more than the two accumulators
 // (the slot the MMA warp refills belongs to a tile every epilogue warp has finished).
@@ -298,7 +299,8 @@ static inline unsigned tc_pack_grid(long long rows) {
 // ------------------------------------------------------------------------------------------
 struct TcParams {
   int Q, k, nkc, ntiles_r, N, NST, logcap;
-  int a_terms, b_terms, fmt;
+  int a_terms, fmt;
+  int fold;  // norm column in use (set by launch_tc_knn)
   uint32_t idesc;
   const float *cn;
   const uint32_t *cid;
@@ -308,11 +310,14 @@ struct TcParams {
   const float *Din;
   int ldD;
   float coefA, coefB, coefC;
-  uint2 *log;
+  // Band logs: entry e of a log is a quad, four adjacent columns of the accumulator as the epilogue
+  // filtered them (v, or w = -v/2 with the norm column), and the packed position of the first.
+  float4 *log;
+  uint32_t *logpos;
   int *logcnt;
   // Partition bound. A query's candidates fall into P = NPART * S partitions (split, part). Each
-  // keeps a heap of the hk = ceil(k / NPART) smallest approximate distances among its own
-  // candidates seen so far, and publishes its root at proot[query * P + split * NPART + part]
+  // keeps a heap of the hk = ceil(k / NPART) smallest approximate distances among the quad minima
+  // of its own candidates seen so far (each a real candidate of its own), and publishes its root at proot[query * P + split * NPART + part]
   // (bits of max(root, 0); all bits set while the heap is not full). Any NPART heaps hold at
   // least k real candidates, so the NPART-th smallest root among any partitions of the query --
   // those of its own CTA, and of up to W - 1 other splits as far as they have run -- bounds the
@@ -339,7 +344,7 @@ struct TcParams {
 };
 
 struct SmemLayout {
-  uint32_t a_off, b_off, an_off, bn_off, heap_off, cn_off, bar_off, tmem_off, total;
+  uint32_t a_off, b_off, an_off, bn_off, heap_off, ring_off, cn_off, bar_off, tmem_off, total;
 };
 
 // Norm column (fold): an all-ones A tile and two slots of candidate norm tiles, 32-byte rows.
@@ -348,26 +353,38 @@ constexpr int NORM_ROW = 32;
 // Partition bound (see TcParams::proot): heap entries per row and part, and the splits whose
 // published roots a row reads (its own and up to three more).
 __host__ __device__ inline int tc_heap_k(int k) { return (k + NPART - 1) / NPART; }
+// Partition lists are kept in whole blocks of LIST_BLOCK values (list_insert). The extreme values
+// of the quads a lane has logged but not yet offered to its list wait in a ring in shared memory:
+// a warp offers them once any lane has FLUSH_AT (a chunk may add eight), INSERT_BATCH at a time.
+constexpr int LIST_BLOCK = 8;
+constexpr int FLUSH_AT = 6;
+constexpr int RING = FLUSH_AT - 1 + 8;
+constexpr int INSERT_BATCH = (RING + 1) / 2;
+__host__ __device__ inline int list_slots(int hk) {
+  return (hk + LIST_BLOCK - 1) / LIST_BLOCK * LIST_BLOCK;
+}
 __host__ __device__ inline int tc_window(int S) { return S < 4 ? S : 4; }
 
 // heap_row: heap entries per row over all epilogue parts; fold: the norm column areas
-__host__ __device__ inline SmemLayout tc_smem_layout(int nkc, int a_terms, int b_terms, int N,
-                                                     int NST, int heap_row, bool fold = false) {
+__host__ __device__ inline SmemLayout tc_smem_layout(int nkc, int a_terms, int N, int NST,
+                                                     int heap_row, bool fold = false) {
   SmemLayout L;
   uint32_t off = 0;
   L.a_off = off;
   off += (uint32_t)a_terms * nkc * A_CHUNK;
   L.b_off = off;
-  off += (uint32_t)NST * b_terms * N * CHUNK_BYTES;
+  off += (uint32_t)NST * N * CHUNK_BYTES;
   L.an_off = off;  // 1024-aligned: every area above is a multiple of 1 KB
   off += fold ? (uint32_t)TC_M * NORM_ROW : 0u;
   L.bn_off = off;
   off += fold ? 2u * N * NORM_ROW : 0u;
   L.heap_off = off;
   off += (uint32_t)heap_row * TC_M * 4;
+  L.ring_off = off;
+  off += (uint32_t)NPART * RING * TC_M * 4;
   off = (off + 15) & ~15u;
   L.cn_off = off;  // candidate norms of the tiles in flight, copied by the MMA warp
-  off += (uint32_t)CN_SLOTS * N * 4;
+  off += fold ? 0u : (uint32_t)CN_SLOTS * N * 4;
   off = (off + 7) & ~7u;
   L.bar_off = off;
   // full, empty, tfull[2], tempty[2], afull, cnfull, nfull[2], nempty[2]
@@ -383,11 +400,11 @@ struct EpiState {
   // the row reads (as last published); pub: what this part last published
   // Tv: the filter bound on v = d' - qn'; Tw = -Tv/2 the same bound on w = -v/2 (norm column)
   float qn, E2, thr0, root, o1, o2, pub, thr, Tv, Tw;
-  int cnt;
+  int cnt;   // logged quads
+  int done;  // of them, already offered to the heap
   int ovf;
-  // optional diagnostics: logged candidates, heap inserts, convergent-loop iterations, chunks
-  // that took the slow path
-  unsigned n_ev, n_ins, n_it, n_sc;
+  // optional diagnostics: flushes, chunks that took the slow path
+  unsigned n_fl, n_sc;
 };
 
 // Any two partitions' heaps hold at least k real candidates, so the second smallest root among
@@ -408,79 +425,66 @@ __device__ __forceinline__ void refresh_threshold(EpiState &s) {
   s.Tw = -0.5f * s.Tv;  // exact: v <= Tv  <=>  w >= Tw
 }
 
-// Replace the heap root by x (< root) and sift down; returns the new root. Heap of k floats,
-// element i of this thread's query at heap[i * TC_M + row] (bank-conflict free across a warp).
-__device__ __forceinline__ float heap_replace_root(float *heap, int row, int k, float x) {
-  int s = 0;
-  while (true) {
-    int c = 2 * s + 1;
-    if (c >= k) break;
-    float cv = heap[c * TC_M + row];
-    if (c + 1 < k) {
-      const float c2 = heap[(c + 1) * TC_M + row];
-      if (c2 > cv) { cv = c2; c = c + 1; }
+// Partition lists: every row and part keeps its hk smallest values ascending in shared memory,
+// element i of this thread's row at list[i * TC_M + row] (bank-conflict free across a warp), hk
+// rounded up to whole blocks of LIST_BLOCK. The "root" is element hk - 1. A batch of values goes
+// through one block of registers after the other: with a sorted block a, inserting x gives
+// a'[i] = min(max(a[i-1], x), a[i]) for every i at once, and the block's largest moves on to the
+// next block. A binary heap's sift-down is a chain of shared-memory round trips per value (7,700
+// cycles a flush at hk = 16); this is arithmetic without one.
+__device__ __forceinline__ void list_insert(float *list, int row, int hk, float (&x)[INSERT_BATCH]) {
+  for (int b = 0; b < hk; b += LIST_BLOCK) {
+    float a[LIST_BLOCK];
+    float *const blk = list + b * TC_M + row;
+#pragma unroll
+    for (int i = 0; i < LIST_BLOCK; i++) a[i] = blk[i * TC_M];
+#pragma unroll
+    for (int j = 0; j < INSERT_BATCH; j++) {
+      const float v = x[j];
+      x[j] = fmaxf(a[LIST_BLOCK - 1], v);  // moves on to the next block
+#pragma unroll
+      for (int i = LIST_BLOCK - 1; i > 0; i--) a[i] = fminf(fmaxf(a[i - 1], v), a[i]);
+      a[0] = fminf(a[0], v);
     }
-    if (!(cv > x)) break;
-    heap[s * TC_M + row] = cv;
-    s = c;
+#pragma unroll
+    for (int i = 0; i < LIST_BLOCK; i++) blk[i * TC_M] = a[i];
   }
-  heap[s * TC_M + row] = x;
-  return heap[row];
 }
 
-// Drops log entries above the current threshold; returns the new count. Reads in batches of
-// 16 before writing (writes never pass the read position), so the loads overlap.
-__device__ __noinline__ int log_compact(uint2 *lg, int cnt, float thr) {
-  int w = 0;
-  for (int e = 0; e < cnt; e += 16) {
-    uint2 buf[16];
+// Whether the extreme value of a quad or chunk (largest w with the norm column, else smallest v)
+// admits it under the row's filter bound.
+template <bool FOLD>
+__device__ __forceinline__ bool epi_hit(const EpiState &s, float m) {
+  return FOLD ? m >= s.Tw : m <= s.Tv;
+}
+template <bool FOLD>
+__device__ __forceinline__ float quad_extreme(float a, float b, float c, float d) {
+  return FOLD ? fmaxf(fmax3(a, b, c), d) : fminf(fmin3(a, b, c), d);
+}
+// approximate distance d' of a filtered value: v + qn, with v = -2w (exact)
+template <bool FOLD>
+__device__ __forceinline__ float epi_dist(float x, float qn) {
+  return FOLD ? fmaf(-2.0f, x, qn) : x + qn;
+}
+
+// Offer the quads logged since the last flush to the row's list, by their extreme values in the
+// ring (all lanes of the warp together), publish the new root to the other partitions and tighten
+// the threshold. (Reading the quads back from their log instead costs a round trip to L2 per
+// flush.)
+template <bool FOLD>
+__device__ __forceinline__ void epi_flush(EpiState &s, float *heap, const float *ring, int row,
+                                          int hk, unsigned *pslot) {
+  s.n_fl++;
+  const int np = s.cnt - s.done;
+  for (int e = 0; __any_sync(FULL_MASK, e < np); e += INSERT_BATCH) {
+    float x[INSERT_BATCH];
 #pragma unroll
-    for (int j = 0; j < 16; j++) buf[j] = e + j < cnt ? lg[e + j] : make_uint2(0x7f800000u, 0u);
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-      if (__uint_as_float(buf[j].x) <= thr) lg[w++] = buf[j];
+    for (int j = 0; j < INSERT_BATCH; j++)
+      x[j] = e + j < np ? epi_dist<FOLD>(ring[(e + j) * TC_M + row], s.qn) : Num<float>::inf();
+    list_insert(heap, row, hk, x);
   }
-  return w;
-}
-
-constexpr int PEND = 8;  // heap inserts a lane may defer before the warp flushes them
-
-// Defer the heap insert of `dp` (when `ins`) into a small register ring, filled through
-// compile-time indices so it stays in registers.
-__device__ __forceinline__ void epi_defer(float dp, bool ins, float (&pend)[PEND], int &np) {
-#pragma unroll
-  for (int j = 0; j < PEND; j++) pend[j] = (ins && j == np) ? dp : pend[j];
-  np += ins ? 1 : 0;
-}
-
-// One candidate of the exact slow path: log it (when `act` and under the threshold) and defer
-// its heap insert. Branch-free: every lane of the warp runs it, with predicates instead of
-// divergent branches.
-__device__ __forceinline__ void epi_candidate(EpiState &s, float v, uint32_t id, bool act,
-                                              uint2 *lg, int logcap, float (&pend)[PEND],
-                                              int &np) {
-  const float dp = v + s.qn;
-  const bool take = act && dp <= s.thr;
-  s.n_ev += take ? 1u : 0u;
-  const bool room = s.cnt < logcap;
-  if (take && !s.ovf && room) lg[s.cnt] = make_uint2(__float_as_uint(dp), id);
-  s.cnt += (take && !s.ovf && room) ? 1 : 0;
-  s.ovf |= (take && !room) ? 1 : 0;
-  epi_defer(dp, take && dp < s.root, pend, np);
-}
-
-// Apply the deferred inserts (all lanes of the warp together, so their sift-downs overlap),
-// publish the new root to the other partitions and tighten the threshold.
-__device__ __forceinline__ void epi_flush(EpiState &s, float *heap, int row, int k,
-                                          float (&pend)[PEND], int &np, unsigned *pslot) {
-#pragma unroll
-  for (int j = 0; j < PEND; j++) {
-    if (j < np && pend[j] < s.root) {
-      s.n_ins++;
-      s.root = heap_replace_root(heap, row, k, pend[j]);
-    }
-  }
-  np = 0;
+  s.root = heap[(hk - 1) * TC_M + row];
+  s.done = s.cnt;
   // published as non-negative float bits (a larger value bounds as well), which order like
   // unsigned integers; only this partition writes its slot
   const float pv = fmaxf(s.root, 0.0f);
@@ -489,6 +493,22 @@ __device__ __forceinline__ void epi_flush(EpiState &s, float *heap, int row, int
     s.pub = pv;
   }
   refresh_threshold(s);
+}
+
+// Drops log entries above the current threshold (all of them already offered to the heap);
+// returns the new count.
+template <bool FOLD>
+__device__ __noinline__ int log_compact(float4 *lg, uint32_t *lp, int cnt, const EpiState &s) {
+  int w = 0;
+  for (int e = 0; e < cnt; e++) {
+    const float4 v = __ldcg(lg + e);
+    const uint32_t pos = __ldcg(lp + e);
+    if (epi_hit<FOLD>(s, quad_extreme<FOLD>(v.x, v.y, v.z, v.w))) {
+      lg[w] = v;
+      lp[w++] = pos;
+    }
+  }
+  return w;
 }
 
 // FOLD: the candidate norms enter through the MMA (the norm column, write_norm_row), so the
@@ -500,6 +520,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
            const __grid_constant__ CUtensorMap tB, const __grid_constant__ CUtensorMap tBlo,
            const __grid_constant__ CUtensorMap tBn, const TcParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
+  constexpr int TERMS = FMT == 2 ? 2 : 1;  // B tiles per K chunk
   // escalation pass: launched for the largest possible query count, the tiles past the count
   // on the device exit before any set-up
   const int Qn = p.dQ ? *p.dQ : p.Q;
@@ -510,12 +531,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const uint32_t raw = su32(smem_raw);
   unsigned char *smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   const SmemLayout L =
-      tc_smem_layout(p.nkc, p.a_terms, p.b_terms, p.N, p.NST, NPART * p.hk, FOLD);
+      tc_smem_layout(p.nkc, p.a_terms, p.N, p.NST, NPART * list_slots(p.hk), FOLD);
   unsigned char *sA = smem + L.a_off;
   unsigned char *sB = smem + L.b_off;
   unsigned char *sAn = smem + L.an_off;
   unsigned char *sBn = smem + L.bn_off;
   float *heap = reinterpret_cast<float *>(smem + L.heap_off);
+  float *ring = reinterpret_cast<float *>(smem + L.ring_off);
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bar_off);
   uint64_t *full = bars;
   uint64_t *empty = bars + p.NST;
@@ -544,7 +566,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (t_end > p.ntiles_r) t_end = p.ntiles_r;
   const int ntile = t_end > t_begin ? t_end - t_begin : 0;
   const int N = p.N;
-  const uint32_t b_stage_bytes = (uint32_t)p.b_terms * N * CHUNK_BYTES;
+  const uint32_t b_stage_bytes = (uint32_t)N * CHUNK_BYTES;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.NST; s++) {
@@ -569,7 +591,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
   // the per-row heaps start at +inf before any epilogue warp reads a root (each part of a lane
   // quarter reads the other's root as part of its bound)
-  for (int i = threadIdx.x; i < NPART * p.hk * TC_M; i += NTHREADS) heap[i] = Num<float>::inf();
+  for (int i = threadIdx.x; i < NPART * list_slots(p.hk) * TC_M; i += NTHREADS) heap[i] = Num<float>::inf();
   if (FOLD) {
     // the all-ones A side of the norm column (every 16-byte chunk alike, so any swizzle of it is
     // the same bytes), made visible to the tensor core's operand reads
@@ -607,15 +629,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           mbar_expect_tx(&nfull[nb], (uint32_t)(N * NORM_ROW));
           tma_load_2d(sBn + (uint32_t)nb * N * NORM_ROW, &tBn, 0, tile * N, &nfull[nb]);
         }
-        for (int kc = 0; kc < p.nkc; kc++, it++) {
+        // a stage is one K chunk of one term: in split BF16 the hi and lo tiles take stages in
+        // turn, which the pipeline refills one by one
+        for (int i = 0; i < TERMS * p.nkc; i++, it++) {
           const int s = it % p.NST;
           const uint32_t round = (uint32_t)(it / p.NST);
           if (!mbar_wait(&empty[s], (round & 1u) ^ 1u)) { failed = true; break; }
           mbar_expect_tx(&full[s], b_stage_bytes);
-          unsigned char *dst = sB + (uint32_t)s * b_stage_bytes;
-          tma_load_2d(dst, &tB, kc * celems, tile * N, &full[s]);
-          if (FMT == 2)
-            tma_load_2d(dst + N * CHUNK_BYTES, &tBlo, kc * celems, tile * N, &full[s]);
+          tma_load_2d(sB + (uint32_t)s * b_stage_bytes, i % TERMS ? &tBlo : &tB,
+                      i / TERMS * celems, tile * N, &full[s]);
         }
       }
     }
@@ -652,8 +674,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                    &cnfull[c]);
           tc_fence_after();
         }
-        for (int kc = 0; kc < p.nkc; kc++, it++) {
-          const int s = it % p.NST;
+        for (int i = 0; i < TERMS * p.nkc; i++, it++) {
+          const int s = it % p.NST, kc = i / TERMS;
+          const bool lo = i % TERMS != 0;
           const uint32_t round = (uint32_t)(it / p.NST);
           t0 = p.counters ? clock64() : 0;
           if (!mbar_wait(&full[s], round & 1u)) { failed = true; break; }
@@ -666,17 +689,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             const uint32_t off = (uint32_t)ks * 32u;
             const uint64_t ad = sdesc_k_sw128(a_chunk + off);
             const uint64_t bd = sdesc_k_sw128(b_chunk + off);
-            const uint32_t first = (!FOLD && kc == 0 && ks == 0) ? 0u : 1u;
+            const uint32_t first = (!FOLD && i == 0 && ks == 0) ? 0u : 1u;
             if (FMT == 0) {
               mma_tf32(tmem_d, ad, bd, p.idesc, first);
             } else {
               mma_f16(tmem_d, ad, bd, p.idesc, first);
-              if (FMT == 2) {
-                const uint64_t alo = sdesc_k_sw128(a_chunk + (uint32_t)p.nkc * A_CHUNK + off);
-                const uint64_t blo = sdesc_k_sw128(b_chunk + (uint32_t)N * CHUNK_BYTES + off);
-                mma_f16(tmem_d, ad, blo, p.idesc, 1u);
-                mma_f16(tmem_d, alo, bd, p.idesc, 1u);
-              }
+              // hi stage: the query's lo part too; lo stage: the query's hi part alone
+              if (FMT == 2 && !lo)
+                mma_f16(tmem_d, sdesc_k_sw128(a_chunk + (uint32_t)p.nkc * A_CHUNK + off), bd,
+                        p.idesc, 1u);
             }
           }
           mma_commit(&empty[s]);
@@ -699,22 +720,20 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const int row = lq * 32 + lane;
     const int gq = qt * TC_M + row;
     const bool valid = gq < Qn && (!p.rowmap || p.rowmap[gq] >= 0);
-    float *const myheap = heap + part * p.hk * TC_M;
-    const float *const otherheap = heap + (NPART - 1 - part) * p.hk * TC_M;
+    float *const myheap = heap + part * list_slots(p.hk) * TC_M;
+    const float *const otherheap = heap + (NPART - 1 - part) * list_slots(p.hk) * TC_M;
+    float *const myring = ring + part * RING * TC_M;
     const int P = NPART * p.S;  // partitions of a query
     EpiState s;
     s.cnt = 0;
+    s.done = 0;
     s.ovf = 0;
     s.o1 = Num<float>::inf();
     s.o2 = Num<float>::inf();
     s.pub = Num<float>::inf();
-    s.n_ev = s.n_ins = s.n_it = s.n_sc = 0;
+    s.n_fl = s.n_sc = 0;
     unsigned *const pslot = p.proot + (size_t)(valid ? gq : 0) * P + NPART * split + part;
     const unsigned *const prow = p.proot + (size_t)(valid ? gq : 0) * P;
-    float pend[PEND];
-    int np = 0;
-#pragma unroll
-    for (int j = 0; j < PEND; j++) pend[j] = Num<float>::inf();
     s.root = Num<float>::inf();
     s.qn = 0.0f;
     s.E2 = 0.0f;
@@ -744,54 +763,40 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       s.Tw = Num<float>::inf();
     }
     const int lslot = NPART * split + part;  // this warp's log among the NPART*S logs of the query
-    uint2 *lg = p.log + ((size_t)lslot * p.Q + (valid ? gq : 0)) * p.logcap;
-    // One 32-column chunk: approximate distances, a cheap min-filter, and for the rare chunks
-    // with survivors a warp-convergent pass in which every lane with pending candidates handles
-    // one of them per iteration (selected from its registers by index).
-    // Fast part of a 32-column chunk: d' - qn' (the v space) over the accumulator values in
-    // place, and their minimum (a tree of depth 5). Two chunks' fast parts run back to back in
+    float4 *const lg = p.log + ((size_t)lslot * p.Q + (valid ? gq : 0)) * p.logcap;
+    uint32_t *const lp = p.logpos + ((size_t)lslot * p.Q + (valid ? gq : 0)) * p.logcap;
+    // Fast part of a 32-column chunk: v = d' - qn' over the accumulator values in place (with the
+    // norm column the registers already hold w = -v/2), the extreme value of every quad of four
+    // columns and of the chunk, in three-input steps. Two chunks' fast parts run back to back in
     // one basic block so their independent arithmetic overlaps.
-    // With the norm column (FOLD) the registers already hold w = -v/2 and the fast part is the
-    // maximum alone.
-    auto fast = [&](uint32_t (&r)[32], const float *cnt, int c0) -> float {
-      if constexpr (FOLD) {
-        float m11[11];
+    auto fast = [&](uint32_t (&r)[32], float (&g)[8], const float *cnt, int c0) -> float {
+      if constexpr (!FOLD) {
+        const float4 *cn4 = reinterpret_cast<const float4 *>(cnt + c0);
 #pragma unroll
-        for (int j = 0; j < 10; j++)
-          m11[j] = fmax3(__uint_as_float(r[3 * j]), __uint_as_float(r[3 * j + 1]),
-                         __uint_as_float(r[3 * j + 2]));
-        m11[10] = fmaxf(__uint_as_float(r[30]), __uint_as_float(r[31]));
-        const float n0 = fmax3(m11[0], m11[1], m11[2]), n1 = fmax3(m11[3], m11[4], m11[5]);
-        const float n2 = fmax3(m11[6], m11[7], m11[8]), n3 = fmaxf(m11[9], m11[10]);
-        return fmaxf(fmax3(n0, n1, n2), n3);
+        for (int j = 0; j < 8; j++) {
+          const float4 c4 = cn4[j];
+          float v0, v1, v2, v3;
+          fma2(v0, v1, __uint_as_float(r[4 * j + 0]), __uint_as_float(r[4 * j + 1]), -2.0f, c4.x,
+               c4.y);
+          fma2(v2, v3, __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]), -2.0f, c4.z,
+               c4.w);
+          r[4 * j + 0] = __float_as_uint(v0);
+          r[4 * j + 1] = __float_as_uint(v1);
+          r[4 * j + 2] = __float_as_uint(v2);
+          r[4 * j + 3] = __float_as_uint(v3);
+        }
       }
-      const float4 *cn4 = reinterpret_cast<const float4 *>(cnt + c0);
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const float4 c4 = cn4[j];
-        float v0, v1, v2, v3;
-        fma2(v0, v1, __uint_as_float(r[4 * j + 0]), __uint_as_float(r[4 * j + 1]), -2.0f, c4.x,
-             c4.y);
-        fma2(v2, v3, __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]), -2.0f, c4.z,
-             c4.w);
-        r[4 * j + 0] = __float_as_uint(v0);
-        r[4 * j + 1] = __float_as_uint(v1);
-        r[4 * j + 2] = __float_as_uint(v2);
-        r[4 * j + 3] = __float_as_uint(v3);
-      }
-      // minimum: three-input tree of depth 4 (32 -> 11 -> 4 -> 1)
-      float m11[11];
-#pragma unroll
-      for (int j = 0; j < 10; j++)
-        m11[j] = fmin3(__uint_as_float(r[3 * j]), __uint_as_float(r[3 * j + 1]),
-                       __uint_as_float(r[3 * j + 2]));
-      m11[10] = fminf(__uint_as_float(r[30]), __uint_as_float(r[31]));
-      const float n0 = fmin3(m11[0], m11[1], m11[2]), n1 = fmin3(m11[3], m11[4], m11[5]);
-      const float n2 = fmin3(m11[6], m11[7], m11[8]), n3 = fminf(m11[9], m11[10]);
-      return fminf(fmin3(n0, n1, n2), n3);
+      for (int j = 0; j < 8; j++)
+        g[j] = quad_extreme<FOLD>(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                  __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+      if constexpr (FOLD)
+        return fmax3(fmax3(g[0], g[1], g[2]), fmax3(g[3], g[4], g[5]), fmaxf(g[6], g[7]));
+      else
+        return fmin3(fmin3(g[0], g[1], g[2]), fmin3(g[3], g[4], g[5]), fminf(g[6], g[7]));
     };
-    // whether a chunk's extreme value (minimum v, or maximum w with the norm column) admits
-    auto hit = [&](float m) { return FOLD ? m >= s.Tw : m <= s.Tv; };
+    // whether a chunk's extreme value admits it
+    auto hit = [&](float m) { return epi_hit<FOLD>(s, m); };
     auto dbg_write = [&](const uint32_t (&r)[32], size_t cbase, int c0) {
       for (int i = 0; i < 32; i++) {
         const long long col = (long long)cbase + c0 + i;
@@ -799,85 +804,109 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (col < p.dbg_ncols) p.dbg[(size_t)gq * p.dbg_ld + col] = v + s.qn;
       }
     };
-    // Slow part, for a chunk in which some lane has a candidate under its threshold: a
-    // warp-convergent pass in which every lane with pending candidates logs one of them per
-    // iteration (selected from its registers by index) and defers its heap insert.
-    auto slow = [&](const uint32_t (&r)[32], size_t cbase, int c0) {
+    // Slow part, for a chunk in which some lane has a candidate under its threshold: every lane
+    // logs its quads that have one, whole (four registers that lie side by side, one 16-byte store
+    // and one 4-byte store, both predicated; no value is selected by index and no loop runs over
+    // the survivors). What it costs is the eight predicated stores' issue; logging single
+    // candidates, each found by a mask and selected by a 31-instruction tree, took about 1,150
+    // cycles a chunk, this about 250. With the partition lists in registers during a flush and the
+    // other splits' roots first touched a tile after their loads: tc_knn on 65,536 x 262,144,
+    // d = 64, k = 32 8,283 -> 5,853 us; 32,768 x 262,144, d = 256, k = 64 6,790 -> 4,466 us;
+    // 2,003 x 30,011, d = 20 105 -> 64 us; 16 x 4,096 42 -> 10 us; 8 trees over 262,144 points
+    // 6.1 -> 3.1 ms.
+    auto slow = [&](const uint32_t (&r)[32], const float (&g)[8], uint32_t pos) {
       // (a compaction that frees less than half of the log marks it overflowed: repeated
       // compactions that each free a few entries would cost a full read of the log per chunk)
-      if (__any_sync(FULL_MASK, s.cnt > p.logcap - 32)) {
-        if (s.cnt > p.logcap - 32 && !s.ovf) {
-          if (!p.no_compact) s.cnt = log_compact(lg, s.cnt, s.thr);
+      if (__any_sync(FULL_MASK, s.cnt > p.logcap - 8)) {
+        epi_flush<FOLD>(s, myheap, myring, row, p.hk, pslot);
+        if (s.cnt > p.logcap - 8 && !s.ovf) {
+          if (!p.no_compact) s.cnt = s.done = log_compact<FOLD>(lg, lp, s.cnt, s);
           if (s.cnt > p.logcap / 2) {
             s.ovf = 1;
             refresh_threshold(s);
           }
         }
       }
-      // pass mask as an OR tree (depth 5), built by every lane
-      uint32_t m16[16];
-#pragma unroll
-      for (int j = 0; j < 16; j++) {
-        if constexpr (FOLD)
-          m16[j] = (__uint_as_float(r[2 * j]) >= s.Tw ? 1u << (2 * j) : 0u) |
-                   (__uint_as_float(r[2 * j + 1]) >= s.Tw ? 1u << (2 * j + 1) : 0u);
-        else
-          m16[j] = (__uint_as_float(r[2 * j]) <= s.Tv ? 1u << (2 * j) : 0u) |
-                   (__uint_as_float(r[2 * j + 1]) <= s.Tv ? 1u << (2 * j + 1) : 0u);
-      }
-#pragma unroll
-      for (int w = 8; w >= 1; w >>= 1)
-#pragma unroll
-        for (int j = 0; j < w; j++) m16[j] = m16[2 * j] | m16[2 * j + 1];
-      uint32_t mask = m16[0];
       s.n_sc++;
-      while (__any_sync(FULL_MASK, mask != 0)) {
-        s.n_it++;
-        const bool act = mask != 0;
-        const int i = (__ffs(mask) - 1) & 31;
-        mask &= mask - 1;
-        // v[i] for a runtime i: a 5-level select tree on the bits of i
-        float t16[16];
+      const uint32_t rbase = su32(myring + row);
 #pragma unroll
-        for (int j = 0; j < 16; j++) t16[j] = __uint_as_float((i & 16) ? r[j + 16] : r[j]);
+      for (int j = 0; j < 8; j++) {
+        const float4 *const at = lg + s.cnt;
+        const uint32_t *const pt = lp + s.cnt;
+        const uint32_t rp = rbase + (uint32_t)(s.cnt - s.done) * (TC_M * 4);
+        if constexpr (FOLD)
+          asm volatile(
+              "{\n\t.reg .pred p;\n\t"
+              "setp.ge.f32 p, %1, %2;\n\t"
+              "@p st.global.v4.b32 [%3], {%4, %5, %6, %7};\n\t"
+              "@p st.global.b32 [%8], %9;\n\t"
+              "@p st.shared.f32 [%10], %1;\n\t"
+              "@p add.s32 %0, %0, 1;\n\t}\n"
+              : "+r"(s.cnt)
+              : "f"(g[j]), "f"(s.Tw), "l"(at), "r"(r[4 * j]), "r"(r[4 * j + 1]),
+                "r"(r[4 * j + 2]), "r"(r[4 * j + 3]), "l"(pt), "r"(pos + 4 * j), "r"(rp)
+              : "memory");
+        else
+          asm volatile(
+              "{\n\t.reg .pred p;\n\t"
+              "setp.le.f32 p, %1, %2;\n\t"
+              "@p st.global.v4.b32 [%3], {%4, %5, %6, %7};\n\t"
+              "@p st.global.b32 [%8], %9;\n\t"
+              "@p st.shared.f32 [%10], %1;\n\t"
+              "@p add.s32 %0, %0, 1;\n\t}\n"
+              : "+r"(s.cnt)
+              : "f"(g[j]), "f"(s.Tv), "l"(at), "r"(r[4 * j]), "r"(r[4 * j + 1]),
+                "r"(r[4 * j + 2]), "r"(r[4 * j + 3]), "l"(pt), "r"(pos + 4 * j), "r"(rp)
+              : "memory");
+      }
+      if (__any_sync(FULL_MASK, s.cnt - s.done >= FLUSH_AT))
+        epi_flush<FOLD>(s, myheap, myring, row, p.hk, pslot);
+    };
+    // the roots up to three other splits have published (all bits set, which orders last: a list
+    // not full yet). The loads for the next tile are issued a tile ahead and their values are
+    // first touched there, so that their latency hides behind the tile's work
+    uint2 win[3];
+    auto load_window = [&]() {
 #pragma unroll
-        for (int w = 8, bit = 8; w >= 1; w >>= 1, bit >>= 1)
-#pragma unroll
-          for (int j = 0; j < w; j++) t16[j] = (i & bit) ? t16[j + w] : t16[j];
-        const float vsel = FOLD ? -2.0f * t16[0] : t16[0];
-        epi_candidate(s, vsel, (uint32_t)(cbase + c0 + i), act && valid, lg, p.logcap, pend, np);
-        if (__any_sync(FULL_MASK, np == PEND)) epi_flush(s, myheap, row, p.hk, pend, np, pslot);
+      for (int w = 0; w < 3; w++) {
+        win[w] = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+        if (w + 1 < p.W) {
+          int sp = split + w + 1;
+          if (sp >= p.S) sp -= p.S;
+          win[w] = __ldcg(reinterpret_cast<const uint2 *>(prow + NPART * sp));
+        }
       }
     };
-    // the two smallest roots up to W - 1 other splits have published (all bits set, which
-    // orders last: a heap not full yet); the loads for the next tile are issued a tile ahead
-    // so their latency hides behind the tile's work
+    // their two smallest
     auto read_window = [&](unsigned &m1, unsigned &m2) {
       m1 = m2 = 0xFFFFFFFFu;
-      for (int w = 1; w < p.W; w++) {
-        int sp = split + w;
-        if (sp >= p.S) sp -= p.S;
-        const uint2 v = __ldcg(reinterpret_cast<const uint2 *>(prow + NPART * sp));
-        m2 = min(m2, max(m1, v.x));
-        m1 = min(m1, v.x);
-        m2 = min(m2, max(m1, v.y));
-        m1 = min(m1, v.y);
+#pragma unroll
+      for (int w = 0; w < 3; w++) {
+        m2 = min(m2, max(m1, win[w].x));
+        m1 = min(m1, win[w].x);
+        m2 = min(m2, max(m1, win[w].y));
+        m1 = min(m1, win[w].y);
       }
     };
     auto as_bound = [](unsigned u) {
       return u == 0xFFFFFFFFu ? Num<float>::inf() : __uint_as_float(u);
     };
-    unsigned win1 = 0xFFFFFFFFu, win2 = 0xFFFFFFFFu;
-    if (valid) read_window(win1, win2);
+    load_window();
     const long long t_start = p.counters ? clock64() : 0;
     long long w_tfull = 0;
     for (int lt = 0; lt < ntile && !failed; lt++) {
       const int b = lt & 1, c = lt % CN_SLOTS;
       const uint32_t use = (uint32_t)(lt >> 1), cuse = (uint32_t)(lt / CN_SLOTS);
-      if (valid) {
-        // the other part of this lane quarter (same rows, other columns) keeps its heap in
+      // (every tile while the bound still falls fast, then every fourth: the update takes about
+      // 420 of a tile's 3,000 cycles)
+      const bool look = lt < 16 || (lt & 3) == 0;
+      if (valid && look) {
+        unsigned win1, win2;
+        read_window(win1, win2);
+        // the other part of this lane quarter (same rows, other columns) keeps its list in
         // shared memory: its root is read directly (one 4-byte word, written whole)
-        const float a = *reinterpret_cast<volatile const float *>(&otherheap[row]);
+        const float a =
+            *reinterpret_cast<volatile const float *>(&otherheap[(p.hk - 1) * TC_M + row]);
         const float w1 = as_bound(win1), w2 = as_bound(win2);
         const float o1 = fminf(a, w1), o2 = fminf(fmaxf(a, w1), w2);
         if (o1 < s.o1 || o2 < s.o2) {
@@ -885,8 +914,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           s.o2 = fminf(s.o2, o2);
           refresh_threshold(s);
         }
-        read_window(win1, win2);
       }
+      if (look) load_window();
       const long long t0 = p.counters ? clock64() : 0;
       if (!mbar_wait(&tfull[b], use & 1u)) { failed = true; break; }
       if (!FOLD && !mbar_wait(&cnfull[c], cuse & 1u)) { failed = true; break; }
@@ -923,14 +952,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[b]);
           }
-          const float ma = fast(ra, cnt, c0);
-          const float mb = fast(rb, cnt, c0 + 32);
+          float ga[8], gb[8];
+          const float ma = fast(ra, ga, cnt, c0);
+          const float mb = fast(rb, gb, cnt, c0 + 32);
           if (p.dbg && valid) {
             dbg_write(ra, cbase, c0);
             dbg_write(rb, cbase, c0 + 32);
           }
-          if (__any_sync(FULL_MASK, hit(ma))) slow(ra, cbase, c0);
-          if (__any_sync(FULL_MASK, hit(mb))) slow(rb, cbase, c0 + 32);
+          if (__any_sync(FULL_MASK, hit(ma))) slow(ra, ga, (uint32_t)(cbase + c0));
+          if (__any_sync(FULL_MASK, hit(mb))) slow(rb, gb, (uint32_t)(cbase + c0 + 32));
         } else {
           uint32_t ra[32];
           __syncwarp();
@@ -942,19 +972,19 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[b]);
           }
-          const float ma = fast(ra, cnt, c0);
+          float ga[8];
+          const float ma = fast(ra, ga, cnt, c0);
           if (p.dbg && valid) dbg_write(ra, cbase, c0);
-          if (__any_sync(FULL_MASK, hit(ma))) slow(ra, cbase, c0);
+          if (__any_sync(FULL_MASK, hit(ma))) slow(ra, ga, (uint32_t)(cbase + c0));
         }
       }
     }
-    epi_flush(s, myheap, row, p.hk, pend, np, pslot);
+    epi_flush<FOLD>(s, myheap, myring, row, p.hk, pslot);
     if (valid) p.logcnt[(size_t)lslot * p.Q + gq] = s.cnt | (s.ovf ? (int)LOG_OVF : 0);
     if (p.counters) {
-      atomicAdd(&p.counters[0], (unsigned long long)s.n_ev);
-      atomicAdd(&p.counters[1], (unsigned long long)s.n_ins);
+      atomicAdd(&p.counters[0], (unsigned long long)s.cnt);
       if (lane == 0) {
-        atomicAdd(&p.counters[2], (unsigned long long)s.n_it);
+        atomicAdd(&p.counters[2], (unsigned long long)s.n_fl);
         atomicAdd(&p.counters[3], (unsigned long long)s.n_sc);
         atomicAdd(&p.counters[4], (unsigned long long)ntile * (N / 64));
         atomicAdd(&p.counters[9], (unsigned long long)w_tfull);
@@ -972,10 +1002,26 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // ------------------------------------------------------------------------------------------
 // FP64 re-rank of the logged band
 // ------------------------------------------------------------------------------------------
+// What bounds it: latency and, in the batching form, issue. A query's band sits in NPART * S short logs, so a warp that walks them
+// one after another waits for a count, then for a few entries, then for the next count. Here the
+// counts are read at once and scanned, and the logs are read as one concatenated list.
+//   1. entries at or under the partition bound + 2E go into a list in shared memory;
+//   2. a bisection over the listed d' gives a bound on the approximate k-th close to it;
+//   3. exact FP64 distances of the entries at or under that bound (about k of them), merged into
+//      the sorted row; then of the entries above it, as far as they lie under the k-th of the
+//      exact list + E.
+// One warp per query (tc_rerank, tc_rerank_leaf), or one CTA per query when the queries are too
+// few to fill the chip with warps (tc_rerank_cta).
+// Measured against a warp that walked log after log with one lane per exact distance: 65,536 x
+// 262,144, d = 64, k = 32: 751 -> 485 us; 32,768 x 262,144, d = 256, k = 64: 2,743 -> 1,246 us;
+// 2,003 x 30,011: 119 -> 31 us; 16 x 4,096: 144 -> 15 us; 8 trees over 262,144 points: 9.4 -> 5.8 ms.
 struct RerankParams {
   int Q, k, S, logcap, d;
-  const uint2 *log;
+  const float4 *log;        // quads as the epilogue filtered them, d' = qmul * value + qn
+  const uint32_t *logpos;   // packed position of each quad's first candidate
   const int *logcnt;
+  const float *qn;
+  float qmul;
   const unsigned *proot;  // partition roots of tc_knn ([query][S]; S counts NPART per split)
   const float *margin;
   const float *Xq, *Xq2, *Xc, *Xc2;
@@ -994,10 +1040,45 @@ struct RerankParams {
   int dedup;
 };
 
-// Exact squared distance of the oracle: (-2 <q,c> + |c|^2) + |q|^2 in FP64 from float inputs,
-// clamped at zero; the dot product is split across the warp.
-// The same distance computed by one thread: the FP64 dot product accumulates the (exact)
-// float x float products in dimension order, as the oracle does (frame/dgsknn_ref_impl.h).
+// (-2 <q,c> + |c|^2) + |q|^2, clamped at zero
+__device__ __forceinline__ double exact_dist(double dot, double cc, double qq) {
+  const double v = fma(-2.0, dot, cc) + qq;
+  return v < 0.0 ? 0.0 : v;
+}
+
+// FP64 dot product of two float rows by four adjacent lanes (sub = lane & 3): lane `sub` sums the
+// (exact) float x float products of every fourth group of four dimensions, then the four sums are
+// added as a tree, so every candidate's value comes out of the same order of operations. Four lanes
+// per row read 64 bytes of it side by side (a lane per row touches 32 lines with every load) and
+// the FP64 chain is a quarter as long. All 32 lanes call it; every lane of the four gets the value.
+__device__ __forceinline__ double exact_dot4(const float *q, const float *c, int d, int sub) {
+  double acc = 0.0;
+  const uintptr_t qc = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(c);
+  if ((d & 3) == 0 && (qc & 15) == 0) {
+    const float4 *q4 = reinterpret_cast<const float4 *>(q);
+    const float4 *c4 = reinterpret_cast<const float4 *>(c);
+#pragma unroll 4
+    for (int i = sub; i < (d >> 2); i += 4) {
+      const float4 a = __ldg(q4 + i), b = __ldg(c4 + i);
+      acc = fma((double)a.x, (double)b.x, acc);
+      acc = fma((double)a.y, (double)b.y, acc);
+      acc = fma((double)a.z, (double)b.z, acc);
+      acc = fma((double)a.w, (double)b.w, acc);
+    }
+  } else {
+    for (int i = 4 * sub; i < d; i += 16)
+      for (int pp = i; pp < min(i + 4, d); pp++) acc = fma((double)q[pp], (double)c[pp], acc);
+  }
+  return acc;
+}
+__device__ __forceinline__ double sum4(double acc) {
+  acc += __shfl_xor_sync(FULL_MASK, acc, 1);
+  acc += __shfl_xor_sync(FULL_MASK, acc, 2);
+  return acc;
+}
+
+// The same distance by one thread, summed in dimension order (the brute-force passes, which compute
+// all of a query's distances themselves).
 __device__ __forceinline__ double exact_dist_lane(const float *q, const float *c, int d,
                                                   double cc, double qq) {
   double acc = 0.0;
@@ -1015,18 +1096,7 @@ __device__ __forceinline__ double exact_dist_lane(const float *q, const float *c
   } else {
     for (int pp = 0; pp < d; pp++) acc = fma((double)q[pp], (double)c[pp], acc);
   }
-  const double v = fma(-2.0, acc, cc) + qq;
-  return v < 0.0 ? 0.0 : v;
-}
-
-__device__ __forceinline__ double exact_dist_warp(const float *q, const float *c, int d,
-                                                  double cc, double qq, int lane) {
-  double acc = 0.0;
-  for (int pp = lane; pp < d; pp += 32) acc = fma((double)q[pp], (double)c[pp], acc);
-#pragma unroll
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(FULL_MASK, acc, o);
-  double v = fma(-2.0, acc, cc) + qq;
-  return v < 0.0 ? 0.0 : v;
+  return exact_dist(acc, cc, qq);
 }
 
 template <int E>
@@ -1043,280 +1113,495 @@ __device__ __forceinline__ void write_heap_row(float *D, int *I, int ldD, int q,
   }
 }
 
-// (sort = false leaves the list in the row's own order; sort it before merging into it)
+// The heap row as it lies (reversed, so that the library's own descending rows come out
+// ascending); the places past k hold (inf, NO_ID).
 template <int E>
 __device__ __forceinline__ void load_heap_row(const float *D, const int *I, int ldD, int q, int k,
-                                              double (&ld)[E], uint32_t (&li)[E], int lane,
-                                              bool sort = true) {
+                                              double (&ld)[E], uint32_t (&li)[E], int lane) {
 #pragma unroll
   for (int e = 0; e < E; e++) {
     const int t = e * 32 + lane;
     if (t < k) {
-      ld[e] = (double)D[(size_t)q * ldD + t];
-      li[e] = (uint32_t)I[(size_t)q * ldD + t];
+      ld[e] = (double)D[(size_t)q * ldD + (k - 1 - t)];
+      li[e] = (uint32_t)I[(size_t)q * ldD + (k - 1 - t)];
     } else {
       ld[e] = Num<double>::inf();
       li[e] = NO_ID;
     }
   }
-  if (sort) warp_sort<double, E>(ld, li, lane);
 }
 
-// thr <- min(thr, k-th of the ascending exact list + E), rounded up: a candidate with d' above it
-// has d > that k-th and cannot enter the list.
+// Sorts the row ascending; a row that already is (an earlier call wrote it, or it is fresh) costs
+// one comparison with each neighbour.
 template <int E>
-__device__ __forceinline__ void tighten_thr(const double (&ld)[E], int k, float Eq, float &thr) {
+__device__ __forceinline__ void sort_heap_row(double (&ld)[E], uint32_t (&li)[E], int lane) {
+  bool bad = false;
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    double nd = __shfl_down_sync(FULL_MASK, ld[e], 1);
+    uint32_t ni = __shfl_down_sync(FULL_MASK, li[e], 1);
+    if (e + 1 < E) {
+      const double fd = __shfl_sync(FULL_MASK, ld[e + 1 < E ? e + 1 : e], 0);
+      const uint32_t fi = __shfl_sync(FULL_MASK, li[e + 1 < E ? e + 1 : e], 0);
+      if (lane == 31) { nd = fd; ni = fi; }
+    }
+    // (a NaN is not in order with anything: the row is sorted)
+    if (lane < 31 || e + 1 < E) bad |= !(ld[e] < nd || (ld[e] == nd && li[e] <= ni));
+  }
+  if (__any_sync(FULL_MASK, bad)) warp_sort<double, E>(ld, li, lane);
+}
+
+// k-th smallest (0-based index k - 1) of the ascending list the warp holds
+template <int E>
+__device__ __forceinline__ double list_kth(const double (&ld)[E], int k) {
   double t = ld[0];
 #pragma unroll
-  for (int e2 = 0; e2 < E; e2++)
-    if (e2 == (k - 1) / 32) t = ld[e2];
-  const double dk = __shfl_sync(FULL_MASK, t, (k - 1) & 31);
-  if (dk < 1e38) thr = fminf(thr, __fadd_ru(__double2float_ru(dk), Eq));
-}
-
-// Whether `id` (NO_ID: never) is one of the ids the warp holds in `li` (E per lane).
-template <int E>
-__device__ __forceinline__ bool id_in_row(uint32_t id, const uint32_t (&li)[E]) {
-  bool hit = false;
-#pragma unroll
   for (int e = 0; e < E; e++)
-    for (int src = 0; src < 32; src++) hit |= __shfl_sync(FULL_MASK, li[e], src) == id;
-  return hit && id != NO_ID;
+    if (e == (k - 1) / 32) t = ld[e];
+  return __shfl_sync(FULL_MASK, t, (k - 1) & 31);
 }
 
-constexpr int RR_BAND = 128;  // band entries (d' above the approximate k-th) a warp holds back
+// Largest value of the row (its k-th distance once it is full), -inf when all are NaN.
+__device__ __forceinline__ float row_max(const float *row, int k, int lane) {
+  float mx = -Num<float>::inf();
+  for (int j = lane; j < k; j += 32) mx = fmaxf(mx, row[j]);
+  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL_MASK, mx, o));
+  return mx;
+}
 
-// HOLD: entries above the approximate k-th are held back and filtered against the threshold the
-// nearly final exact k-th gives (pays where the band is wide: BF16); else one pass in log order.
-// LAZY (the batching form's leaf pass): the incoming row stays unsorted until a candidate can
-// enter it, and a row nothing entered is not written back.
-template <int E, bool HOLD, bool LAZY>
-__device__ __forceinline__ void rerank_body(const RerankParams &p) {
-  __shared__ uint32_t rr_stage[8][64];
-  __shared__ uint2 rr_band[8][HOLD ? RR_BAND : 1];
+// Whether `id` (NO_ID: never) is one of the n ids in shared memory.
+__device__ __forceinline__ bool id_in_row(uint32_t id, const uint32_t *ids, int n4) {
+  const uint4 *v = reinterpret_cast<const uint4 *>(ids);
+  bool a = false, b = false;
+  for (int j = 0; j < n4; j++) {
+    const uint4 x = v[j];
+    a |= x.x == id || x.y == id;
+    b |= x.z == id || x.w == id;
+  }
+  return (a || b) && id != NO_ID;
+}
+
+// A bound on the k-th smallest of the n >= k values list[i].x (as floats) with at most k + k/8 of
+// them under it, or at most 1/4096 of their range above it; one warp.
+__device__ __forceinline__ float list_bound(const uint2 *list, int n, int k, int lane) {
+  float lo = Num<float>::inf(), hi = -Num<float>::inf();
+  for (int i = lane; i < n; i += 32) {
+    const float v = __uint_as_float(list[i].x);
+    lo = fminf(lo, v);
+    hi = fmaxf(hi, v);
+  }
+  for (int o = 16; o; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(FULL_MASK, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(FULL_MASK, hi, o));
+  }
+  for (int it = 0; it < 12; it++) {
+    const float mid = lo + 0.5f * (hi - lo);
+    int c = 0;
+    for (int i = lane; i < n; i += 32) c += __uint_as_float(list[i].x) <= mid ? 1 : 0;
+    c = __reduce_add_sync(FULL_MASK, c);
+    if (c >= k) {
+      hi = mid;
+      if (c <= k + (k >> 3)) break;
+    } else {
+      lo = mid;
+    }
+  }
+  return hi;
+}
+
+// Smallest and second smallest of the published partition roots over the warp's lanes.
+__device__ __forceinline__ void two_smallest(unsigned &m1, unsigned &m2) {
+  for (int o = 16; o; o >>= 1) {
+    const unsigned a1 = __shfl_xor_sync(FULL_MASK, m1, o);
+    const unsigned a2 = __shfl_xor_sync(FULL_MASK, m2, o);
+    m2 = min(max(m1, a1), min(m2, a2));
+    m1 = min(m1, a1);
+  }
+}
+
+// the band: d' <= (bound on the approximate k-th) + 2E, and <= lim (a NaN bound admits nothing)
+__device__ __forceinline__ float band_thr(float T, float E2, float lim) {
+  const float t = __fadd_ru(T, E2);
+  return lim < t ? lim : t;
+}
+
+// a row's largest distance + E bounds d' of any candidate that can still enter it
+__device__ __forceinline__ float band_limit(float mx, float Eq) {
+  return mx > -Num<float>::inf() && mx < 1e38f ? __fadd_ru(mx, Eq) : Num<float>::inf();
+}
+
+constexpr int RR_WARPS = 8;
+// CTAs per SM the registers are held to: 64 registers up to 64 neighbours
+template <int E>
+constexpr int RR_OCC = E <= 2 ? 4 : 2;
+template <int E>
+constexpr int rr_cap() { return E == 1 ? 384 : 512; }  // listed entries per warp (k <= 32 E)
+
+template <int E>
+struct RerankSmem {
+  uint2 list[rr_cap<E>()];     // (d', packed position)
+  uint32_t stage[64];          // positions whose exact distances are next
+  uint32_t fresh[32];          // batching form: the ids of a batch that are not in the row
+  __align__(16) uint32_t ids[32 * E];  // batching form: the incoming row's ids
+};
+
+// One query by one warp. LEAF (the batching form): ids already in the row are not entered again,
+// the incoming row stays unsorted until a candidate can enter it, and a row nothing entered is
+// not written back.
+template <int E, bool LEAF>
+__device__ __forceinline__ void rerank_warp(const RerankParams &p, int q, RerankSmem<E> &sm) {
+  constexpr int CAP = rr_cap<E>();
   const int lane = threadIdx.x & 31;
-  const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (q >= (p.dQ ? *p.dQ : p.Q)) return;
   const int hr = p.rowmap ? p.rowmap[q] : q;  // heap row and query position
   if (hr < 0) return;                          // a padding row of a leaf panel
-  // overflowed logs: the query goes to the next pass (a narrower format, or brute force)
-  bool ovf = false;
-  for (int s = 0; s < p.S; s++) ovf |= (p.logcnt[(size_t)s * p.Q + q] & (int)LOG_OVF) != 0;
-  // the second smallest final root over the query's partitions (any two heaps hold k entries;
-  // all bits set, ordering last: a heap that never filled)
-  float T;
-  {
-    const unsigned *pr = p.proot + (size_t)q * p.S;
-    unsigned m1 = 0xFFFFFFFFu, m2 = 0xFFFFFFFFu;
-    for (int s = 0; s < p.S; s++) {
-      const unsigned u = pr[s];
-      m2 = min(m2, max(m1, u));
-      m1 = min(m1, u);
-    }
-    T = m2 == 0xFFFFFFFFu ? Num<float>::inf() : __uint_as_float(m2);
-  }
-  if (ovf) {
-    if (lane == 0) p.fallback_list[atomicAdd(p.fallback_count, 1)] = p.dedup ? q : hr;
-    return;
-  }
-  const float E2 = p.margin[q];
-  // Pass 1: the exact k-th smallest approximate distance over all of the query's logs. Every
-  // candidate among the k smallest approximate distances was logged (its d' was below every
-  // threshold in force), so this is the global approximate k-th, usually far below the bound T
-  // the splits ended with. When all the logs together hold at most 32 entries (short lists:
-  // leaves of the batching form), pass 2 takes them in one batch of exact distances whatever
-  // the bound, so pass 1 is skipped and T stays the partition bound.
-  int total = 0;
-  for (int s = 0; s < p.S; s++) total += p.logcnt[(size_t)s * p.Q + q];
-  if (total > 32) {
-    float kd[E];
-    uint32_t ki[E];
-#pragma unroll
-    for (int e = 0; e < E; e++) { kd[e] = Num<float>::inf(); ki[e] = NO_ID; }
-    float kth = T;
-    for (int s = 0; s < p.S; s++) {
-      const int cnt = p.logcnt[(size_t)s * p.Q + q];
-      const uint2 *lg = p.log + ((size_t)s * p.Q + q) * p.logcap;
-      // one batch of log entries is loaded ahead, so that its latency overlaps the vote and
-      // merge of the current batch
-      float dv_next = lane < cnt ? __uint_as_float(lg[lane].x) : Num<float>::inf();
-      for (int base = 0; base < cnt; base += 32) {
-        const int e = base + lane;
-        const float dv = dv_next;
-        dv_next = e + 32 < cnt ? __uint_as_float(lg[e + 32].x) : Num<float>::inf();
-        if (!__any_sync(FULL_MASK, dv <= kth)) continue;
-        float b1[1] = {dv};
-        uint32_t i1[1] = {(uint32_t)e};
-        warp_sort<float, 1>(b1, i1, lane);
-        warp_merge_32<float, E>(kd, ki, b1[0], i1[0], lane);
-        float t = kd[0];
-#pragma unroll
-        for (int e2 = 0; e2 < E; e2++)
-          if (e2 == (p.k - 1) / 32) t = kd[e2];
-        kth = fminf(kth, __shfl_sync(FULL_MASK, t, (p.k - 1) & 31));
-      }
-    }
-    T = kth;
-  }
-  // A candidate in the final top-k has d' <= d_k + E <= T + 2E. Its exact distance is also at
-  // most the k-th of any k real candidates with exact distances (the incoming row and those
-  // computed so far), so d' <= that k-th + E: the threshold tightens as the exact list fills.
-  float thr = T + E2;
-  const float Eq = 0.5f * E2;
+  const int k = p.k;
   double ld[E];
   uint32_t li[E];
-  // LAZY: the incoming row stays unsorted until some candidate can enter it: a batch whose
-  // exact distances all exceed the list's k-th (the row's largest distance, until the first
-  // merge) changes nothing, and a row nothing entered is not written back.
-  load_heap_row<E>(p.D, p.I, p.ldD, hr, p.k, ld, li, lane, !LAZY);
-  bool sorted = !LAZY;
-  double lim = Num<double>::inf();
-  if (HOLD) {
-    tighten_thr<E>(ld, p.k, Eq, thr);
-  } else {
-    // the incoming row's largest distance bounds the k-th (as the list's k-th would)
-    float mx = -Num<float>::inf();
-    for (int j = lane; j < p.k; j += 32) mx = fmaxf(mx, p.D[(size_t)hr * p.ldD + j]);
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL_MASK, mx, o));
-    if (mx > -Num<float>::inf() && mx < 1e38f) thr = fminf(thr, __fadd_ru(mx, Eq));
-    lim = (double)mx;
+  load_heap_row<E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+  bool ovf = false;
+  unsigned m1 = 0xFFFFFFFFu, m2 = 0xFFFFFFFFu;
+  for (int s = lane; s < p.S; s += 32) {
+    ovf |= (p.logcnt[(size_t)s * p.Q + q] & (int)LOG_OVF) != 0;
+    const unsigned u = p.proot[(size_t)q * p.S + s];
+    m2 = min(m2, max(m1, u));
+    m1 = min(m1, u);
   }
-  uint32_t li0[E];  // the incoming row's ids (the batching form's duplicate check)
+  // overflowed logs: the query goes to the next pass (a narrower format, or brute force)
+  if (__any_sync(FULL_MASK, ovf)) {
+    if (lane == 0) p.fallback_list[atomicAdd(p.fallback_count, 1)] = LEAF ? q : hr;
+    return;
+  }
+  // Any two heaps hold k candidates, so the second smallest final root bounds the approximate
+  // k-th (all bits set: a heap that never filled). A candidate in the final top-k has d' <= the
+  // approximate k-th + 2E, and d' <= (the k-th of any k exact distances) + E.
+  two_smallest(m1, m2);
+  float T = m2 == 0xFFFFFFFFu ? Num<float>::inf() : __uint_as_float(m2);
+  const float E2 = p.margin[q], Eq = 0.5f * E2, qn = p.qn[q];
+  float mx = -Num<float>::inf();
 #pragma unroll
-  for (int e = 0; e < E; e++) li0[e] = li[e];
+  for (int e = 0; e < E; e++)
+    if (e * 32 + lane < k) mx = fmaxf(mx, (float)ld[e]);
+  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL_MASK, mx, o));
+  float lim = band_limit(mx, Eq);
+  float thr = band_thr(T, E2, lim);
+  double kth = (double)mx;  // of the exact list so far
+  bool sorted = false;
+  if (LEAF) {
+#pragma unroll
+    for (int e = 0; e < E; e++) sm.ids[e * 32 + lane] = li[e];
+    __syncwarp();
+  } else {
+    sort_heap_row<E>(ld, li, lane);
+    sorted = true;
+  }
   const long long qrow = p.qidx[hr];
   const float *qv = p.Xq + qrow * p.d;
   const double qq = (double)p.Xq2[qrow];
-  // Pass 2: entries under the threshold are compacted into a per-warp staging list; every 32 of
-  // them each lane computes one exact distance (independent row gathers across the lanes), then
-  // the batch is sorted and merged into the exact list. With HOLD, entries at or under T (the k
-  // smallest d') go first; those above T are held back in shared memory (as far as it holds
-  // them) and filtered afterwards against the threshold the nearly final exact k-th gives.
-  uint32_t *stg = rr_stage[threadIdx.x >> 5];
-  int nb = 0;
-  auto flush = [&](int count) {
-    double dist = Num<double>::inf();
-    uint32_t id = NO_ID;
-    if (lane < count) id = p.cid[stg[lane]];
-    // batching form: an id already in the incoming row is not entered again, and costs no
-    // row gather
-    if (p.dedup && id_in_row<E>(id, li0)) id = NO_ID;
-    if (id != NO_ID)
-      dist = exact_dist_lane(qv, p.Xc + (long long)id * p.d, p.d, (double)p.Xc2[id], qq);
-    if (p.counters && lane == 0) atomicAdd(&p.counters[6], (unsigned long long)count);
-    if (LAZY) {
-      // nothing in this batch can enter (ties are settled by the merge itself)
-      if (!__any_sync(FULL_MASK, id != NO_ID && dist <= lim)) return;
-      if (!sorted) {
-        warp_sort<double, E>(ld, li, lane);
-        sorted = true;
-      }
-    }
-    double b1[1] = {dist};
-    uint32_t i1[1] = {id};
-    warp_sort<double, 1>(b1, i1, lane);
-    warp_merge_32<double, E>(ld, li, b1[0], i1[0], lane);
-    if (LAZY) {
-      double t = ld[0];
+  int n = 0;  // listed entries
+
+  // The logs, 32 at a time, as one concatenated list: lane s holds where log g + s starts. Entries
+  // under the threshold fill the list; a full list is first cut down to what the bound from its
+  // own entries admits, and if that is still most of it, or the logs are at their end, the exact
+  // distances of the listed entries follow: those at or under the bound first (pass 0), then
+  // those above it that the k-th of the exact list still admits.
+  int g = -32, base = 0, total = 0, excl = 0;
+  while (true) {
+    bool done = false;
+    while (n <= CAP - 128) {
+      while (base >= total) {
+        g += 32;
+        if (g >= p.S) {
+          done = true;
+          break;
+        }
+        const int cnt = g + lane < p.S ? p.logcnt[(size_t)(g + lane) * p.Q + q] : 0;
+        int incl = cnt;
 #pragma unroll
-      for (int e2 = 0; e2 < E; e2++)
-        if (e2 == (p.k - 1) / 32) t = ld[e2];
-      lim = __shfl_sync(FULL_MASK, t, (p.k - 1) & 31);
-    }
-  };
-  if constexpr (!HOLD) {
-    for (int s = 0; s < p.S; s++) {
-      const int cnt = p.logcnt[(size_t)s * p.Q + q];
-      const uint2 *lg = p.log + ((size_t)s * p.Q + q) * p.logcap;
-      if (p.counters && lane == 0) atomicAdd(&p.counters[5], (unsigned long long)cnt);
-      for (int base = 0; base < cnt; base += 32) {
-        const int e = base + lane;
-        uint2 ent = make_uint2(0u, NO_ID);
-        bool take = false;
-        if (e < cnt) {
-          ent = lg[e];
-          take = __uint_as_float(ent.x) <= thr;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(FULL_MASK, incl, o);
+          if (lane >= o) incl += v;
         }
+        excl = incl - cnt;
+        total = __shfl_sync(FULL_MASK, incl, 31);
+        base = 0;
+        if (p.counters && lane == 0) atomicAdd(&p.counters[5], (unsigned long long)total);
+      }
+      if (done) break;
+      const int e = base + lane;
+      int s = 0;  // the last log that starts at or before e
+#pragma unroll
+      for (int st = 16; st; st >>= 1) {
+        const int v = __shfl_sync(FULL_MASK, excl, s + st);
+        if (v <= e) s += st;
+      }
+      const int off = e - __shfl_sync(FULL_MASK, excl, s);
+      float dv[4];
+      uint32_t pos = 0u;
+      {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (e < total) {
+          const size_t at = ((size_t)(g + s) * p.Q + q) * p.logcap + off;
+          v = p.log[at];
+          pos = p.logpos[at];
+        }
+        dv[0] = fmaf(p.qmul, v.x, qn);
+        dv[1] = fmaf(p.qmul, v.y, qn);
+        dv[2] = fmaf(p.qmul, v.z, qn);
+        dv[3] = fmaf(p.qmul, v.w, qn);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const bool take = e < total && dv[u] <= thr;
         const unsigned m = __ballot_sync(FULL_MASK, take);
-        if (take) stg[nb + __popc(m & ((1u << lane) - 1u))] = ent.y;
-        nb += __popc(m);
+        if (take)
+          sm.list[n + __popc(m & ((1u << lane) - 1u))] =
+              make_uint2(__float_as_uint(dv[u]), pos + u);
+        n += __popc(m);
+      }
+      base += 32;
+    }
+    __syncwarp();
+    if (n > 32 && n >= k) T = fminf(T, list_bound(sm.list, n, k, lane));
+    thr = band_thr(T, E2, lim);
+    const float split = n > 32 ? T : Num<float>::inf();  // one batch takes a short list whole
+    if (!done) {
+      int w = 0;
+      for (int b0 = 0; b0 < n; b0 += 32) {
+        const int e = b0 + lane;
+        const uint2 ent = e < n ? sm.list[e] : make_uint2(0u, 0u);
+        const bool keep = e < n && __uint_as_float(ent.x) <= thr;
+        const unsigned m = __ballot_sync(FULL_MASK, keep);
+        if (keep) sm.list[w + __popc(m & ((1u << lane) - 1u))] = ent;
+        w += __popc(m);
         __syncwarp();
-        if (nb >= 32) {
-          flush(32);
+      }
+      n = w;
+      if (n <= CAP / 2) continue;
+    }
+    int nb = 0;  // staged positions
+    const int nblk = (n + 31) / 32;
+    for (int i = 0; i < (n > 32 ? 2 * nblk : nblk); i++) {
+      const bool pass1 = i >= nblk;
+      const int e = (pass1 ? i - nblk : i) * 32 + lane;
+      uint2 ent = make_uint2(0u, 0u);
+      bool take = false;
+      if (e < n) {
+        ent = sm.list[e];
+        const float dv = __uint_as_float(ent.x);
+        take = dv <= thr && (dv > split) == pass1;
+      }
+      const unsigned m = __ballot_sync(FULL_MASK, take);
+      if (take) sm.stage[nb + __popc(m & ((1u << lane) - 1u))] = ent.y;
+      nb += __popc(m);
+      __syncwarp();
+      const bool end = i == nblk - 1 || i == 2 * nblk - 1;
+      while (nb >= 32 || (end && nb > 0)) {
+        const int count = nb < 32 ? nb : 32;
+        const uint32_t pos = sm.stage[lane < count ? lane : 0];
+        const uint32_t rest = sm.stage[32 + lane];
+        __syncwarp();
+        sm.stage[lane] = rest;
+        nb -= count;
+        __syncwarp();
+        // exact distances of these positions, merged into the list: lane i takes candidate i's
+        // id and norm, four lanes its dot product
+        uint32_t id = NO_ID;
+        if (lane < count) id = p.cid[pos];
+        // an id already in the incoming row costs no row gather: the others move together
+        int cnt = count;
+        if (LEAF) {
+          const bool fresh = !id_in_row(id, sm.ids, 8 * E) && id != NO_ID;
+          const unsigned m = __ballot_sync(FULL_MASK, fresh);
+          if (m == 0) continue;
+          cnt = __popc(m);
+          if (fresh) sm.fresh[__popc(m & ((1u << lane) - 1u))] = id;
           __syncwarp();
-          const uint32_t rest = lane < nb - 32 ? stg[32 + lane] : 0u;
+          id = lane < cnt ? sm.fresh[lane] : NO_ID;
           __syncwarp();
-          if (lane < nb - 32) stg[lane] = rest;
-          nb -= 32;
-          __syncwarp();
+        }
+        const double cc = id != NO_ID ? (double)p.Xc2[id] : 0.0;
+        double dot = 0.0;
+        for (int r = 0; r < cnt; r += 8) {
+          const uint32_t cid = __shfl_sync(FULL_MASK, id, r + (lane >> 2));
+          double part = 0.0;
+          if (cid != NO_ID)
+            part = exact_dot4(qv, p.Xc + (long long)cid * p.d, p.d, lane & 3);
+          part = __shfl_sync(FULL_MASK, sum4(part), (lane & 7) * 4);
+          if ((lane >> 3) == (r >> 3)) dot = part;
+        }
+        const double dist = id != NO_ID ? exact_dist(dot, cc, qq) : Num<double>::inf();
+        if (p.counters && lane == 0) atomicAdd(&p.counters[6], (unsigned long long)cnt);
+        if (LEAF) {
+          // nothing in this batch can enter (ties are settled by the merge itself)
+          if (!__any_sync(FULL_MASK, id != NO_ID && dist <= kth)) continue;
+          if (!sorted) {
+            sort_heap_row<E>(ld, li, lane);
+            sorted = true;
+          }
+        }
+        double b1[1] = {dist};
+        uint32_t i1[1] = {id};
+        warp_sort<double, 1>(b1, i1, lane);
+        warp_merge_32<double, E>(ld, li, b1[0], i1[0], lane);
+        kth = list_kth<E>(ld, k);
+        if (kth < 1e38) {
+          lim = fminf(lim, __fadd_ru(__double2float_ru(kth), Eq));
+          if (lim < thr) thr = lim;
         }
       }
     }
-  } else {
-    uint2 *bnd = rr_band[threadIdx.x >> 5];
-    int nbd = 0;
-    // sources in order: the NPART * S logs, then (HOLD) the held band; one flush site
-    for (int s = 0; s < p.S + (HOLD ? 1 : 0); s++) {
-      const bool from_log = s < p.S;
-      const int cnt = from_log ? p.logcnt[(size_t)s * p.Q + q] : nbd;
-      const uint2 *lg = from_log ? p.log + ((size_t)s * p.Q + q) * p.logcap : bnd;
-      if (p.counters && lane == 0 && from_log)
-        atomicAdd(&p.counters[5], (unsigned long long)cnt);
-      for (int base = 0; base < cnt; base += 32) {
-        const int e = base + lane;
-        uint2 ent = make_uint2(0u, NO_ID);
-        bool take = false, band = false;
-        if (e < cnt) {
-          ent = lg[e];
-          const float dv = __uint_as_float(ent.x);
-          take = dv <= thr;
-          band = HOLD && from_log && take && dv > T;
-        }
-        if (HOLD && from_log) {
-          const unsigned mb = __ballot_sync(FULL_MASK, band);
-          if (nbd + __popc(mb) <= RR_BAND) {
-            if (band) bnd[nbd + __popc(mb & ((1u << lane) - 1u))] = ent;
-            nbd += __popc(mb);
-            take = take && !band;
-          }
-          __syncwarp();
-        }
-        const unsigned m = __ballot_sync(FULL_MASK, take);
-        if (take) stg[nb + __popc(m & ((1u << lane) - 1u))] = ent.y;
-        nb += __popc(m);
-        __syncwarp();
-        if (nb >= 32) {
-          flush(32);
-          if (HOLD) tighten_thr<E>(ld, p.k, Eq, thr);
-          __syncwarp();
-          const uint32_t rest = lane < nb - 32 ? stg[32 + lane] : 0u;
-          __syncwarp();
-          if (lane < nb - 32) stg[lane] = rest;
-          nb -= 32;
-          __syncwarp();
-        }
+    if (done) break;
+    n = 0;
+    __syncwarp();
+  }
+  if (sorted) write_heap_row<E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+}
+
+template <int E>
+__global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank(RerankParams p) {
+  __shared__ RerankSmem<E> sm[RR_WARPS];
+  const int q = blockIdx.x * RR_WARPS + (threadIdx.x >> 5);
+  if (q >= (p.dQ ? *p.dQ : p.Q)) return;
+  rerank_warp<E, false>(p, q, sm[threadIdx.x >> 5]);
+}
+
+template <int E>
+__global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_leaf(RerankParams p) {
+  __shared__ RerankSmem<E> sm[RR_WARPS];
+  const int q = blockIdx.x * RR_WARPS + (threadIdx.x >> 5);
+  if (q >= p.Q) return;
+  rerank_warp<E, true>(p, q, sm[threadIdx.x >> 5]);
+}
+
+// One query by one CTA: all warps read the logs into one list and share the exact distances; warp
+// 0 merges. A query whose list does not fit is left to warp 0 alone (rerank_warp).
+constexpr int RC_CAP = 1024;  // listed entries per CTA
+constexpr int RC_LOGS = 512;  // logs (NPART * S) the prefix array holds
+
+template <int E>
+__global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(RerankParams p) {
+  __shared__ uint2 list[RC_CAP];
+  __shared__ double xd[RC_CAP];
+  __shared__ uint32_t xi[RC_CAP];
+  __shared__ int pre[RC_LOGS + 1];
+  __shared__ float s_T, s_thr;
+  __shared__ int s_n, s_state;
+  __shared__ RerankSmem<E> sm;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int q = blockIdx.x;
+  if (q >= (p.dQ ? *p.dQ : p.Q)) return;
+  const int hr = p.rowmap ? p.rowmap[q] : q;
+  if (hr < 0) return;
+  const int k = p.k;
+  const float E2 = p.margin[q], Eq = 0.5f * E2, qn = p.qn[q];
+  if (warp == 0) {
+    // prefix sums of the counts, the overflow flag and the partition bound
+    bool ovf = false;
+    unsigned m1 = 0xFFFFFFFFu, m2 = 0xFFFFFFFFu;
+    int carry = 0;
+    for (int g = 0; g < p.S; g += 32) {
+      int c = 0;
+      if (g + lane < p.S) {
+        c = p.logcnt[(size_t)(g + lane) * p.Q + q];
+        ovf |= (c & (int)LOG_OVF) != 0;
+        const unsigned u = p.proot[(size_t)q * p.S + g + lane];
+        m2 = min(m2, max(m1, u));
+        m1 = min(m1, u);
+      }
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(FULL_MASK, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (g + lane < p.S) pre[g + lane + 1] = carry + incl;
+      carry += __shfl_sync(FULL_MASK, incl, 31);
+    }
+    ovf = __any_sync(FULL_MASK, ovf);
+    two_smallest(m1, m2);
+    const float T = m2 == 0xFFFFFFFFu ? Num<float>::inf() : __uint_as_float(m2);
+    const float lim = band_limit(row_max(p.D + (size_t)hr * p.ldD, k, lane), Eq);
+    if (lane == 0) {
+      pre[0] = 0;
+      s_T = T;
+      s_thr = band_thr(T, E2, lim);
+      s_n = 0;
+      s_state = ovf ? 1 : 0;
+      if (ovf) p.fallback_list[atomicAdd(p.fallback_count, 1)] = hr;
+      if (p.counters) atomicAdd(&p.counters[5], (unsigned long long)carry);
+    }
+  }
+  __syncthreads();
+  if (s_state) return;
+  const int total = pre[p.S];
+  float thr = s_thr;
+  for (int e = tid; e < total; e += 32 * RR_WARPS) {
+    int a = 0, b = p.S;  // the last log that starts at or before e
+    while (b - a > 1) {
+      const int m = (a + b) >> 1;
+      if (pre[m] <= e) a = m;
+      else b = m;
+    }
+    const size_t at = ((size_t)a * p.Q + q) * p.logcap + (e - pre[a]);
+    const float4 v4 = p.log[at];
+    const uint32_t pos = p.logpos[at];
+    const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const float dv = fmaf(p.qmul, v[u], qn);
+      if (dv <= thr) {
+        const int to = atomicAdd(&s_n, 1);
+        if (to < RC_CAP) list[to] = make_uint2(__float_as_uint(dv), pos + u);
       }
     }
   }
-  if (nb > 0) flush(nb);
-  if (sorted) write_heap_row<E>(p.D, p.I, p.ldD, hr, p.k, ld, li, lane);
-}
-
-template <int E>
-__global__ void __launch_bounds__(256) tc_rerank(RerankParams p) {
-  rerank_body<E, false, false>(p);
-}
-
-template <int E>
-__global__ void __launch_bounds__(256) tc_rerank_leaf(RerankParams p) {
-  rerank_body<E, false, true>(p);
-}
-
-// The held variant is capped at 64 registers (four CTAs per SM): this latency-bound kernel loses
-// more to fewer resident warps than to a few spills.
-template <int E>
-__global__ void __launch_bounds__(256, 4) tc_rerank_hold(RerankParams p) {
-  rerank_body<E, true, false>(p);
+  __syncthreads();
+  const int n = s_n;
+  if (n > RC_CAP) {
+    if (warp == 0) rerank_warp<E, false>(p, q, sm);
+    return;
+  }
+  if (n > 32 && n >= k) {
+    if (warp == 0) {
+      const float T = fminf(s_T, list_bound(list, n, k, lane));
+      if (lane == 0) s_thr = band_thr(T, E2, thr);
+    }
+    __syncthreads();
+    thr = s_thr;
+  }
+  const long long qrow = p.qidx[hr];
+  const float *qv = p.Xq + qrow * p.d;
+  const double qq = (double)p.Xq2[qrow];
+  for (int base = warp * 8; base < n; base += 8 * RR_WARPS) {
+    const int i = base + (lane >> 2);  // four lanes per candidate
+    uint32_t id = NO_ID;
+    if (i < n && __uint_as_float(list[i].x) <= thr) id = p.cid[list[i].y];
+    double dot = 0.0;
+    if (id != NO_ID) dot = exact_dot4(qv, p.Xc + (long long)id * p.d, p.d, lane & 3);
+    dot = sum4(dot);
+    if (i < n && (lane & 3) == 0) {
+      xd[i] = id != NO_ID ? exact_dist(dot, (double)p.Xc2[id], qq) : Num<double>::inf();
+      xi[i] = id;
+      if (p.counters && id != NO_ID) atomicAdd(&p.counters[6], 1ull);
+    }
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  double ld[E];
+  uint32_t li[E];
+  load_heap_row<E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+  sort_heap_row<E>(ld, li, lane);
+  double kth = list_kth<E>(ld, k);
+  for (int base = 0; base < n; base += 32) {
+    const int i = base + lane;
+    double b1[1] = {i < n ? xd[i] : Num<double>::inf()};
+    uint32_t i1[1] = {i < n ? xi[i] : NO_ID};
+    if (!__any_sync(FULL_MASK, i1[0] != NO_ID && !(b1[0] > kth))) continue;
+    warp_sort<double, 1>(b1, i1, lane);
+    warp_merge_32<double, E>(ld, li, b1[0], i1[0], lane);
+    kth = list_kth<E>(ld, k);
+  }
+  write_heap_row<E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1388,6 +1673,7 @@ __global__ void __launch_bounds__(256) tc_fallback(FallbackParams p) {
       double md[E];
       uint32_t mi[E];
       load_heap_row<E>(p.D, p.I, p.ldD, q, p.k, md, mi, lane);
+      sort_heap_row<E>(md, mi, lane);
       for (int w2 = 0; w2 < 8; w2++) {
         double bd[E];
         uint32_t bi[E];
@@ -1435,9 +1721,13 @@ __global__ void __launch_bounds__(256) tc_fallback_leaf(LeafFallbackParams p) {
     double ld[E];
     uint32_t li[E];
     load_heap_row<E>(p.D, p.I, p.ldD, hr, p.k, ld, li, lane);
-    uint32_t li0[E];
+    sort_heap_row<E>(ld, li, lane);
+    __shared__ __align__(16) uint32_t ids[8][32 * E];  // the incoming row's ids
+    uint32_t *const li0 = ids[threadIdx.x >> 5];
+    __syncwarp();
 #pragma unroll
-    for (int e = 0; e < E; e++) li0[e] = li[e];
+    for (int e = 0; e < E; e++) li0[e * 32 + lane] = li[e];
+    __syncwarp();
     for (int base = r.x * p.N; base < r.y * p.N; base += 32) {  // warp-uniform trip count
       const int c = base + lane;
       uint32_t id = NO_ID;
@@ -1447,7 +1737,7 @@ __global__ void __launch_bounds__(256) tc_fallback_leaf(LeafFallbackParams p) {
         if (id != NO_ID)
           dist = exact_dist_lane(qv, p.X + (long long)id * p.d, p.d, (double)p.X2[id], qq);
       }
-      if (id_in_row<E>(id, li0)) {
+      if (id_in_row(id, li0, 8 * E)) {
         dist = Num<double>::inf();
         id = NO_ID;
       }
@@ -1526,6 +1816,7 @@ static cudaError_t launch_tc_knn(const TcPlan &P, void *npanel, int npanel_rows,
     const cudaError_t e = make_norm_map(&mBn, npanel, P.elem, npanel_rows, P.N);
     if (e != cudaSuccess) return e;
   }
+  tp.fold = fold ? 1 : 0;
   tp.coefA = fold ? P.coefA_fold : P.coefA;
   tp.coefB = P.coefB;
   tp.coefC = fold ? P.coefC_fold : P.coefC;
@@ -1617,6 +1908,14 @@ cudaError_t tc_cand_prepare(TcCand *C, void *mem, int nc, int d, int mode, const
   return cudaGetLastError();
 }
 
+// Quads per log: `want`, or as many as keep all `logs` logs under 16 GB, but not fewer than fit the
+// 8 * want bytes that a log of `want` single candidates takes.
+static int log_entries(int want, size_t logs) {
+  const size_t fit = ((size_t)16 << 30) / (std::max(logs, (size_t)1) * tc::LOG_ENTRY);
+  if (fit >= (size_t)want) return want;
+  return (int)std::max(fit, (size_t)want * 8 / tc::LOG_ENTRY);
+}
+
 static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool with_cand,
                           int max_splits) {
   using namespace tc;
@@ -1630,20 +1929,38 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   P.elem = elem;
   P.d_pad = ((d + celems - 1) / celems) * celems;
   P.nkc = P.d_pad / celems;
-  P.a_terms = P.b_terms = P.fmt == 2 ? 2 : 1;
+  P.a_terms = P.fmt == 2 ? 2 : 1;
   P.kp = 32;
   while (P.kp < k) P.kp <<= 1;
   if (k > 256) return P;
-  // candidate tile width and pipeline depth that fit in shared memory
+  // Candidate tile width and pipeline depth that fit in shared memory, and whether the norm column
+  // fits beside them: in split BF16, and in BF16 from two K chunks (measured: config 2 split BF16
+  // -4% in tc_knn, BF16 at d = 256 -1.6%, but BF16 at d = 64 +5%). Three stages of the pipeline
+  // are worth less than the norm column's areas.
   const uint32_t smem_max = 227 * 1024;
+  const int lists = NPART * list_slots(tc_heap_k(k));
+  bool fold = P.fmt == 2 || (P.fmt == 1 && P.nkc >= 2);
+  if (const char *v = getenv("GSKNN_TC_FOLD"))
+    if (atoi(v) == 0) fold = false;
   int best_N = 0, best_NST = 0;
+  uint32_t smem_fold = 0;
   const int Ns[2] = {256, 128};
   for (int ni = 0; ni < 2 && !best_N; ni++) {
     const int N = Ns[ni];
     if (P.fmt == 0 && N == 256 && P.nkc > 4) continue;  // keep the TF32 A tile room
-    for (int NST = 6; NST >= 2; NST--) {
-      SmemLayout L = tc_smem_layout(P.nkc, P.a_terms, P.b_terms, N, NST, NPART * tc_heap_k(k));
-      if (L.total <= smem_max) { best_N = N; best_NST = NST; break; }
+    for (int NST = 6; NST >= 2 && !best_N; NST--) {
+      const uint32_t with = tc_smem_layout(P.nkc, P.a_terms, N, NST, lists, true).total;
+      if (fold && with <= smem_max && NST >= 3) {
+        best_N = N;
+        best_NST = NST;
+        smem_fold = with;
+      }
+    }
+    for (int NST = 6; NST >= 2 && !best_N; NST--) {
+      if (tc_smem_layout(P.nkc, P.a_terms, N, NST, lists).total <= smem_max) {
+        best_N = N;
+        best_NST = NST;
+      }
     }
   }
   if (!best_N) return P;
@@ -1666,19 +1983,12 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   P.S = best_s;
   P.tiles_per_split = (P.rtiles + P.S - 1) / P.S;
   P.hk = tc_heap_k(k);
-  P.smem = tc_smem_layout(P.nkc, P.a_terms, P.b_terms, P.N, P.NST, NPART * P.hk).total;
-  // the norm column where its areas fit beside the same tiles: in split BF16, and in BF16 from
-  // two K chunks (measured: config 2 split BF16 -4% in tc_knn, BF16 at d = 256 -1.6%, but
-  // BF16 at d = 64 +5%)
-  {
-    const uint32_t sf =
-        tc_smem_layout(P.nkc, P.a_terms, P.b_terms, P.N, P.NST, NPART * P.hk, true).total;
-    const bool wanted = P.fmt == 2 || (P.fmt == 1 && P.nkc >= 2);
-    P.smem_fold = wanted && sf <= smem_max ? sf : 0u;
-    if (const char *v = getenv("GSKNN_TC_FOLD"))
-      if (atoi(v) == 0) P.smem_fold = 0u;
-  }
-  P.logcap = std::max(8 * P.kp, 1024);
+  P.smem = tc_smem_layout(P.nkc, P.a_terms, P.N, P.NST, lists).total;
+  P.smem_fold = smem_fold;
+  // (no log needs more than the quads its part of a split holds, and the room that a chunk's eight
+  // want)
+  P.logcap = std::min(log_entries(std::max(8 * P.kp, 1024), (size_t)NPART * best_s * nq),
+                      P.tiles_per_split * (P.N / NPART / 4) + 8);
   // workspace: [prepared candidates | query side]
   P.cand_bytes = with_cand ? al256(tc_cand_bytes(nc, d, mode)) : 0;
   size_t off = P.cand_bytes;
@@ -1688,12 +1998,13 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   P.o_qn = take((size_t)P.q_pad * 4);
   P.o_qnrm = take((size_t)P.q_pad * 4);
   // NPART logs per (query, split): one per epilogue warp of a lane quarter
-  P.o_log = take((size_t)NPART * P.S * nq * P.logcap * 8);
   P.o_logcnt = take((size_t)NPART * P.S * nq * 4);
   P.o_proot = take((size_t)NPART * P.S * nq * 4);
   P.o_margin = take((size_t)nq * 4);
   P.o_fbl = take((size_t)nq * 4);
   P.o_fbc = take(16);
+  // last: once the re-rank has read the logs, the escalation pass takes their place
+  P.o_log = take((size_t)NPART * P.S * nq * P.logcap * LOG_ENTRY);
   P.bytes = off;
   // error-bound coefficients
   const double D = (double)P.d_pad;
@@ -1753,9 +2064,9 @@ TcPlan tc_plan(int nq, int nc, int d, int k, int mode, int sms, bool with_cand,
   P.esc_mode = tc_escalation_mode(nq, nc, d, k, mode, sms);
   if (P.esc_mode) {
     const TcPlan EP = tc_plan_base(nq, nc, d, k, P.esc_mode, sms, false, max_splits);
-    P.o_esc = al256(P.bytes);
+    P.o_esc = P.o_log;
     P.esc_bytes = EP.bytes;
-    size_t off = al256(P.o_esc + EP.bytes);
+    size_t off = al256(std::max(P.bytes, P.o_esc + EP.bytes));
     if (with_cand) {  // per-call candidates: their escalation panels live in the workspace
       P.o_ecand = off;
       P.ecand_bytes = panel_bytes(EP.r_pad, EP.d_pad, EP.fmt);
@@ -1833,11 +2144,12 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, void *cand_pb, void
   TcParams tp{};
   tp.Q = nq; tp.k = k; tp.nkc = P.nkc; tp.ntiles_r = P.rtiles;
   tp.N = P.N; tp.NST = P.NST; tp.logcap = P.logcap;
-  tp.a_terms = P.a_terms; tp.b_terms = P.b_terms; tp.fmt = P.fmt;
+  tp.a_terms = P.a_terms; tp.fmt = P.fmt;
   tp.idesc = idesc_f32acc(P.fmt == 0 ? 2u : 1u, TC_M, P.N);
   tp.cn = C.cn; tp.cid = C.cid; tp.qn = qn; tp.qnrm = qnrm; tp.stats = C.stats;
   tp.Din = D; tp.ldD = ldD;
-  tp.log = reinterpret_cast<uint2 *>(base + P.o_log);
+  tp.log = reinterpret_cast<float4 *>(base + P.o_log);
+  tp.logpos = reinterpret_cast<uint32_t *>(tp.log + (size_t)NPART * P.S * nq * P.logcap);
   tp.logcnt = reinterpret_cast<int *>(base + P.o_logcnt);
   tp.proot = reinterpret_cast<unsigned *>(base + P.o_proot);
   tp.hk = P.hk;
@@ -1860,7 +2172,8 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, void *cand_pb, void
 
   RerankParams rp{};
   rp.Q = nq; rp.k = k; rp.S = NPART * P.S; rp.logcap = P.logcap; rp.d = d;
-  rp.log = tp.log; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
+  rp.log = tp.log; rp.logpos = tp.logpos; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
+  rp.qn = tp.qn; rp.qmul = tp.fold ? -2.0f : 1.0f;
   rp.proot = tp.proot;
   rp.Xq = Xq; rp.Xq2 = Xq2; rp.Xc = C.Xc; rp.Xc2 = C.Xc2; rp.qidx = qidx; rp.cid = C.cid;
   rp.D = D; rp.I = I; rp.ldD = ldD;
@@ -1869,18 +2182,20 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, void *cand_pb, void
   rp.counters = counters;
   rp.dQ = dQ;
   rp.rowmap = rowmap;
-  const int rb = (nq + 7) / 8;
-  // one BF16 MMA per product leaves the widest band: hold it back behind the core entries
-  // (k <= 64: larger lists would spill the held variant's registers)
-  const bool hold = P.fmt == 1 && P.kp <= 64;
+  const int rb = (nq + RR_WARPS - 1) / RR_WARPS;
+  // one CTA per query up to four waves of one CTA per SM: 16 queries x 4,096 took 21 us against
+  // 40 us with a warp each; at 2,003 queries the warps fill the chip (37 us against 67 us)
+  const bool cta = nq <= 4 * 148 && rp.S <= RC_LOGS;
   mark(n_rr, true);
   switch (P.kp) {
-    case 32: hold ? tc_rerank_hold<1><<<rb, 256, 0, st>>>(rp)
-                  : tc_rerank<1><<<rb, 256, 0, st>>>(rp); break;
-    case 64: hold ? tc_rerank_hold<2><<<rb, 256, 0, st>>>(rp)
-                  : tc_rerank<2><<<rb, 256, 0, st>>>(rp); break;
-    case 128: tc_rerank<4><<<rb, 256, 0, st>>>(rp); break;
-    case 256: tc_rerank<8><<<rb, 256, 0, st>>>(rp); break;
+    case 32: cta ? tc_rerank_cta<1><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
+                 : tc_rerank<1><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
+    case 64: cta ? tc_rerank_cta<2><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
+                 : tc_rerank<2><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
+    case 128: cta ? tc_rerank_cta<4><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
+                  : tc_rerank<4><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
+    case 256: cta ? tc_rerank_cta<8><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
+                  : tc_rerank<8><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
     default: return cudaErrorInvalidValue;
   }
   e = cudaGetLastError();
@@ -2015,7 +2330,7 @@ TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms) {
   L.rows_cap = rows_cap;
   // per-query area for rows_cap rows, one split; smaller logs than the per-call path (a leaf
   // offers at most a few thousand candidates; a full log overflows to the leaf brute force)
-  P.logcap = std::max(2 * P.kp, 256);
+  P.logcap = log_entries(std::max(2 * P.kp, 256), (size_t)NPART * rows_cap);
   P.S = 1;
   P.qtiles = L.rows_cap / TC_M;
   P.q_pad = L.rows_cap;
@@ -2037,7 +2352,7 @@ TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms) {
   P.o_pa_lo = L.o_pb_lo;
   P.o_qn = L.o_cn;
   P.o_qnrm = L.o_cnrm;
-  P.o_log = take((size_t)NPART * R * P.logcap * 8);
+  P.o_log = take((size_t)NPART * R * P.logcap * LOG_ENTRY);
   P.o_logcnt = take((size_t)NPART * R * 4);
   P.o_proot = take((size_t)NPART * R * 4);
   P.o_margin = take(R * 4);
@@ -2100,11 +2415,12 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   TcParams tp{};
   tp.Q = rows; tp.k = k; tp.nkc = P.nkc; tp.ntiles_r = rows / P.N;
   tp.N = P.N; tp.NST = P.NST; tp.logcap = P.logcap;
-  tp.a_terms = P.a_terms; tp.b_terms = P.b_terms; tp.fmt = P.fmt;
+  tp.a_terms = P.a_terms; tp.fmt = P.fmt;
   tp.idesc = idesc_f32acc(1u, TC_M, P.N);
   tp.cn = cn; tp.cid = cid; tp.qn = cn; tp.qnrm = cnrm; tp.stats = stats;
   tp.Din = D; tp.ldD = ldD;
-  tp.log = reinterpret_cast<uint2 *>(base + P.o_log);
+  tp.log = reinterpret_cast<float4 *>(base + P.o_log);
+  tp.logpos = reinterpret_cast<uint32_t *>(tp.log + (size_t)NPART * P.S * rows * P.logcap);
   tp.logcnt = reinterpret_cast<int *>(base + P.o_logcnt);
   tp.proot = reinterpret_cast<unsigned *>(base + P.o_proot);
   tp.hk = P.hk;
@@ -2119,7 +2435,8 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   if (e != cudaSuccess) return e;
   RerankParams rp{};
   rp.Q = rows; rp.k = k; rp.S = NPART; rp.logcap = P.logcap; rp.d = d;
-  rp.log = tp.log; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
+  rp.log = tp.log; rp.logpos = tp.logpos; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
+  rp.qn = tp.qn; rp.qmul = tp.fold ? -2.0f : 1.0f;
   rp.proot = tp.proot;
   rp.Xq = X; rp.Xq2 = X2; rp.Xc = X; rp.Xc2 = X2; rp.qidx = iota; rp.cid = cid;
   rp.D = D; rp.I = I; rp.ldD = ldD;
@@ -2132,7 +2449,7 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   fp.k = k; fp.d = d; fp.N = P.N; fp.X = X; fp.X2 = X2; fp.rowmap = pidx; fp.ids = cid;
   fp.rtab = rtab; fp.D = D; fp.I = I; fp.ldD = ldD; fp.list = rp.fallback_list;
   fp.count = fbc;
-  const int rb = (rows + 7) / 8;
+  const int rb = (rows + RR_WARPS - 1) / RR_WARPS;
   switch (P.kp) {
     case 32:
       tc_rerank_leaf<1><<<rb, 256, 0, st>>>(rp);
