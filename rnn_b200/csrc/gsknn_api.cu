@@ -448,8 +448,7 @@ static int knn_device_tc(int mode, int nq, int nc, int d, int k, const float *Xq
   void *ws = nullptr, *stv = nullptr;
   CU(scratch(SLOT_KERNEL, P.bytes, st, &ws));
   CU(scratch(SLOT_STATUS, 256, st, &stv));
-  int *status = static_cast<int *>(stv);
-  CU(cudaMemsetAsync(status, 0, sizeof(int), st));
+  int *status = static_cast<int *>(stv);  // cleared by the first kernel
   // GSKNN_TC_COUNTERS=1: per-call diagnostics of the tensor-core epilogue on stderr
   static const bool want_counters = std::getenv("GSKNN_TC_COUNTERS") != nullptr;
   unsigned long long *counters = nullptr;

@@ -115,14 +115,14 @@ struct TcPlan {
   int fmt, elem, d_pad, nkc, a_terms, kp;
   int N, NST, qtiles, rtiles, q_pad, r_pad, S, tiles_per_split, logcap;
   unsigned smem;
-  float coefA, coefB;
-  // norm column (the candidate norms enter through the MMA): shared memory of that form (0: it
-  // does not fit), and its error-bound coefficients (coefB is shared; coefC multiplies CN)
+  // error-bound coefficients (tc_plan_base)
+  float kA, kB, kC_fold, kS;
+  // shared memory of the form with the norm column (the candidate norms enter through the MMA; 0:
+  // it does not fit)
   unsigned smem_fold;
-  float coefA_fold, coefC_fold, coefC;
   // query-side workspace offsets (absolute within the workspace; they start after the
   // prepared-candidate area when the plan includes it)
-  size_t o_pa, o_pa_lo, o_qn, o_qnrm, o_log, o_logcnt, o_proot, o_margin, o_fbl, o_fbc;
+  size_t o_pa, o_pa_lo, o_qn, o_qe, o_qmx, o_log, o_logcnt, o_proot, o_margin, o_fbl, o_fbc;
   int hk;  // partition bound: heap entries per row and epilogue part
   size_t cand_bytes;  // prepared-candidate area at the start of the workspace (0: separate)
   // Escalation: queries whose band log overflowed in this format run again in a narrower one
@@ -136,20 +136,22 @@ struct TcPlan {
 };
 
 // Candidates packed once in the MMA input format, with everything a query batch needs from
-// them: shift mu, |mu|^2, bound statistics (max centred norm, max |effective norm|), packed
-// panels [r_pad][d_pad] (r_pad a multiple of 256), effective norms, centred norm bounds, ids,
+// them: shift mu, |mu|^2, bound statistics (maxima over the candidates), packed panels
+// [r_pad][d_pad] (r_pad a multiple of 256), effective norms, ids,
 // and the caller's table for the FP64 re-rank. A resident reference set is prepared once and
 // serves any number of query batches.
 struct TcCand {
   int fmt, elem, d, d_pad, nc, r_pad;
   float *mu;
   double *mu2;
-  unsigned *stats;
+  double *part;  // tc_center's partial sums and row counts
+  int *part_n;
+  unsigned *stats, *estats;  // bound statistics of the main and of the escalation format
   void *pb, *pb_lo;
   void *pn;  // norm panel (the MMA's norm column), null when absent
-  float *cn, *cnrm;
+  float *cn;
   uint32_t *cid;
-  const float *Xc, *Xc2;
+  const void *Xc, *Xc2;  // float or double, as the caller's table
   long long nrows_c;
   const int *cidx;
   // optional panels of the same candidates in a second format (escalation pass; shift, norms,
@@ -191,7 +193,7 @@ struct TcLeafPlan {
   bool ok;
   TcPlan P;        // the split-BF16 tile plan (one split), per-query area for rows_cap rows
   int rows_cap;    // panel rows one tree may need
-  size_t o_mu, o_mu2, o_cpart, o_stats, o_pb, o_pb_lo, o_pn, o_cn, o_cnrm, o_cid, o_iota, bytes;
+  size_t o_mu, o_mu2, o_cpart, o_stats, o_pb, o_pb_lo, o_pn, o_cn, o_cid, o_iota, bytes;
 };
 // npts: points of the table; rows_cap: panel rows one tree may use (a multiple of 128).
 TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms);

@@ -472,6 +472,7 @@ static gsknn::TcCand escalation_as_main(const gsknn::TcCand &C, int esc_mode) {
   S.pb = C.epb;
   S.pb_lo = C.epb_lo;
   S.pn = C.epn;
+  S.stats = C.estats;
   S.efmt = -1;
   S.epb = S.epb_lo = S.epn = nullptr;
   return S;
@@ -501,7 +502,8 @@ static bool probe_modes(Engine *E, int esc) {
       const long long n = (long long)rows * kb;
       gs::fill_heap<<<(unsigned)((n + 255) / 256), 256, 0, s.st>>>(s.Db, s.Ib, n);
       ok = cudaEventRecord(a, s.st) == cudaSuccess &&
-           tc_run_prepared(P, *cands[m], rows, E->d, kb, E->C.Xc, E->C.Xc2, E->nref, s.qidx,
+           tc_run_prepared(P, *cands[m], rows, E->d, kb, static_cast<const float *>(E->C.Xc),
+                           static_cast<const float *>(E->C.Xc2), E->nref, s.qidx,
                            s.Db, s.Ib, kb, s.ws, s.status, nullptr, 0, nullptr, s.st, nullptr,
                            nullptr) == cudaSuccess &&
            cudaEventRecord(b, s.st) == cudaSuccess &&

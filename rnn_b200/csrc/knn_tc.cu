@@ -5,12 +5,11 @@
 // the lower id) of the caller's float inputs, merged into the caller's heaps.
 //
 // Kernels (one call):
-//   tc_center,    shift vector mu = mean of a strided sample of candidate rows (partial sums
-//   tc_center_fin per slice, then their fixed-order total and mu.mu)
-//   tc_pack       one warp per row: gather, centre, round to the MMA format into a row-major
-//                 [rows][d_pad] panel (TMA source), effective norm X2 - 2 mu.x + mu.mu (the
-//                 centred norm, built on the caller's norm) in FP64, centred norm bound, ids;
-//                 running maxima for the bound
+//   tc_center     partial sums of the shift vector mu = mean of a strided sample of candidate rows
+//   tc_pack       candidates and queries: add the partial sums, gather, centre, round to the MMA
+//                 format into a row-major [rows][d_pad] panel (TMA source), effective norm
+//                 X2 - 2 mu.x + mu.mu (the centred norm, built on the caller's norm) in FP64,
+//                 the terms of the error bound, ids; running maxima over the candidates
 //   tc_knn        warp 0 TMA producer, warp 1 MMA issuer (TMEM owner), warps 2-9 epilogue (two
 //                 per TMEM lane quarter, each taking half of every tile's columns) with one
 //                 query row per thread: approximate d' = qn' + cn' - 2<q~,c~> (with the norm
@@ -27,13 +26,17 @@
 //                 and writes a row only if it changes
 //   tc_fallback   queries whose log overflowed: exact FP64 brute force over all candidates
 //
-// Error bound (per query q, all candidates c; u = unit roundoff of the MMA input format,
-// M = max |c~|, CN = max |cn'|, D = padded dimension):
-//   |d'(q,c) - d(q,c)| <= E_q = 1.25 * [ 2 (2u + u^2 + D 2^-23 (1+u)^2) |q~| M
-//                                         + 3 * 2^-24 (CN + |qn'| + 2 |q~| M) ]
-// For the split format the input term 2u + u^2 is replaced by 3.2 u^2 (u = 2^-8) and the
-// accumulation term counts 3D products. With the norm column the accumulation counts 3 more
-// terms, and E gains 1.25 (n 2^-23 + 2^-24) CN for the norm parts it sums (n accumulated terms).
+// Error bound (per query q, all candidates c; r(x) = |x - fmt(x)|, the norm of a row's rounding
+// residual, measured per row; M = max |c~|, R = max r(c~), CN = max |cn'|, D = padded dimension,
+// n = D + 3 accumulated terms, u = unit roundoff of the MMA input format):
+//   |d'(q,c) - d(q,c)| <= E_q = 1.25 * [ 2 (r(q~) M + (|q~| + r(q~)) R)          input rounding
+//                                  + 2 (n 2^-23 (1+u)^2 + 2^-22) |q~| M          accumulation
+//                                  + 3 * 2^-24 (CN + |qn'| + 2 |q~| M) ] + noise
+// For the split format r(q~) M + ... is replaced by 3.2 u^2 |q~| M (u = 2^-8; it covers the omitted
+// lo x lo product) and n = 3D + 3. With the norm column E gains 1.25 (n 2^-23 + 2^-24) CN for the
+// norm parts it sums. `noise` covers the rounding of the FP64 distance itself, (4d + 32) 2^-53 of
+// the squared norms' scale. Measuring r takes the input term to about 0.4 of its worst case
+// (2u + u^2) |q~| M.
 #include "knn_common.cuh"
 #include "knn_internal.h"
 #include "tc_ptx.cuh"
@@ -67,42 +70,47 @@ constexpr int CN_SLOTS = 3;
 // ------------------------------------------------------------------------------------------
 // shift vector
 // ------------------------------------------------------------------------------------------
-// The shift is the mean of a strided sample of the candidate rows, summed in a fixed order in
-// two steps so that it is the same bits on every run:
-//   tc_center   grid (dimension groups of 32, CENTER_SLICES slices of the sample), 32 warps per
-//               block: lane = dimension, warps stride over the slice's rows (coalesced 128-byte
-//               row segments), a block reduction in warp order, one partial sum per (slice,
-//               dimension) and one row count per slice;
-//   tc_center_fin  one block: mu = (sum of the partials in slice order) / rows, and mu.mu in FP64.
+// The shift is the mean of a strided sample of the candidate rows, summed in a fixed order so that
+// it is the same bits on every run: tc_center, on a grid of (dimension groups of 32, CENTER_SLICES
+// slices of the sample), 16 warps per block, lane = dimension, warps striding over the slice's rows
+// (coalesced row segments), writes one partial sum per (slice, dimension) and one row count per
+// slice; tc_pack adds the partials in slice order. Being the first kernel of a call it also clears
+// the call's status word and the candidates' bound statistics.
 constexpr int CENTER_SLICES = 16;
+constexpr int CENTER_ROWS = 1024;  // sampled rows (any shift is valid; it only narrows the bound)
+constexpr int CENTER_WARPS = 16;
 
-__global__ void __launch_bounds__(1024) tc_center(const float *__restrict__ X, int d,
-                                                  long long nrows, const int *__restrict__ idx,
-                                                  int count, int nsample,
-                                                  double *__restrict__ part,
-                                                  int *__restrict__ part_n) {
-  __shared__ double ps[32][33];
-  __shared__ int pc[32];
+template <typename T>
+__global__ void __launch_bounds__(32 * CENTER_WARPS) tc_center(
+    const T *__restrict__ X, int d, long long nrows, const int *__restrict__ idx, int count,
+    int nsample, double *__restrict__ part, int *__restrict__ part_n, unsigned *stats,
+    int nstats, int *clear) {
+  __shared__ double ps[CENTER_WARPS][33];
+  __shared__ int pc[CENTER_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.x == 0 && blockIdx.y == 0) {
+    if (stats && (int)threadIdx.x < nstats) stats[threadIdx.x] = 0u;
+    if (clear && threadIdx.x == 0) *clear = 0;
+  }
   const int p = blockIdx.x * 32 + lane;
   const int t_lo = (int)((long long)nsample * blockIdx.y / CENTER_SLICES);
   const int t_hi = (int)((long long)nsample * (blockIdx.y + 1) / CENTER_SLICES);
   double s = 0.0;
   int used = 0;
-  // eight sample rows per round: their index and row loads are independent and issue together
-  for (int t0 = t_lo + warp; t0 < t_hi; t0 += 32 * 8) {
-    float v[8];
-    bool ok[8];
+  // four sample rows per round: their index and row loads are independent and issue together
+  for (int t0 = t_lo + warp; t0 < t_hi; t0 += CENTER_WARPS * 4) {
+    T v[4];
+    bool ok[4];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int t = t0 + 32 * u;
+    for (int u = 0; u < 4; u++) {
+      const int t = t0 + CENTER_WARPS * u;
       long long row = -1;
       if (t < t_hi) row = idx[(long long)t * count / nsample];
       ok[u] = row >= 0 && row < nrows;
-      v[u] = ok[u] && p < d ? X[row * d + p] : 0.0f;
+      v[u] = ok[u] && p < d ? X[row * d + p] : T(0);
     }
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
+    for (int u = 0; u < 4; u++) {
       if (ok[u]) {
         if (p < d) s += (double)v[u];
         used++;
@@ -115,37 +123,12 @@ __global__ void __launch_bounds__(1024) tc_center(const float *__restrict__ X, i
   if (warp == 0) {
     double tot = 0.0;
     int n = 0;
-    for (int w = 0; w < 32; w++) {
+    for (int w = 0; w < CENTER_WARPS; w++) {
       tot += ps[w][lane];
       n += pc[w];
     }
     if (p < d) part[(size_t)blockIdx.y * d + p] = tot;
     if (blockIdx.x == 0 && lane == 0) part_n[blockIdx.y] = n;
-  }
-}
-
-__global__ void __launch_bounds__(256) tc_center_fin(const double *__restrict__ part,
-                                                     const int *__restrict__ part_n, int d,
-                                                     float *__restrict__ mu,
-                                                     double *__restrict__ mu2) {
-  __shared__ double red[8];
-  int n = 0;
-  for (int sl = 0; sl < CENTER_SLICES; sl++) n += part_n[sl];
-  double s2 = 0.0;
-  for (int p = threadIdx.x; p < d; p += blockDim.x) {
-    double tot = 0.0;
-    for (int sl = 0; sl < CENTER_SLICES; sl++) tot += part[(size_t)sl * d + p];
-    const float m = n ? (float)(tot / n) : 0.0f;
-    mu[p] = m;
-    s2 += (double)m * (double)m;
-  }
-  for (int o = 16; o; o >>= 1) s2 += __shfl_xor_sync(FULL_MASK, s2, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s2;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-    *mu2 = t;
   }
 }
 
@@ -194,104 +177,246 @@ __device__ __forceinline__ void write_norm_row(int fmt, void *npanel, int r, boo
 }
 
 // fmt: 0 = TF32 (4-byte panel), 1 = BF16, 2 = split BF16 (hi and lo panels)
-// Optional forms: `dcount` (device) replaces `count` and limits the panel to the tiles it needs;
-// `rowmap` packs point idx[rowmap[r]] as row r; `gate` (device) skips all work when it reads 0;
-// a null `enorm` writes the panels only (norms, bounds, ids and statistics are left alone);
-// `pad_ok` packs index -1 as an empty padding row instead of reporting it; `npanel` (candidates)
-// receives each row's norm column (write_norm_row).
-__global__ void __launch_bounds__(256) tc_pack(
-    int fmt, const float *__restrict__ X, const float *__restrict__ X2, int d, int d_pad,
-    long long nrows, const int *__restrict__ idx, int count, int rows_pad,
-    const float *__restrict__ mu, const double *__restrict__ mu2, int is_cand, void *panel,
-    void *panel_lo, float *__restrict__ enorm, float *__restrict__ cnrm,
-    uint32_t *__restrict__ ids, unsigned *__restrict__ stats, int *__restrict__ status,
-    const int *__restrict__ dcount = nullptr, const int *__restrict__ rowmap = nullptr,
-    const int *__restrict__ gate = nullptr, int pad_ok = 0, void *npanel = nullptr) {
-  const int lane = threadIdx.x & 31;
-  if (gate && *gate == 0) return;
-  if (dcount) {
-    count = *dcount;
-    const int used = ((count + TC_M - 1) / TC_M) * TC_M;
-    if (used < rows_pad) rows_pad = used;
-  }
-  // one row per warp, grid-stride; the candidate bound statistics are kept per warp and reach
-  // the global maxima once per warp (not once per row: same-address atomics serialize)
-  unsigned mx_nrm = 0u, mx_en = 0u;
-  const int wstride = gridDim.x * (blockDim.x >> 5);
-  for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows_pad;
-       r += wstride) {
-    long long row = -1;
-    if (r < count) {
-      row = idx[rowmap ? rowmap[r] : r];
-      if (pad_ok && row == -1) {
-        // a padding row of a leaf panel (the batching form): silently empty
-      } else if (row < 0 || row >= nrows) {
-        if (lane == 0) atomicExch(status, GSKNN_ERR_INDEX);
-        row = -1;
-      }
+//
+// One side of a packing launch: `rows_pad` panel rows, of which the first `count` are points
+// idx[r] (idx[rowmap[r]] with a row map) of table X. `dcount` (device) replaces `count` and limits
+// the panel to the tiles it needs; `gate` (device) skips the side when it reads 0; `pad_ok` packs
+// index -1 as an empty padding row instead of reporting it, and takes the point as its heap row.
+template <typename T>
+struct PackSide {
+  const T *X, *X2;
+  long long nrows;
+  const int *idx, *rowmap, *dcount, *gate;
+  int count, rows_pad, pad_ok;
+  void *panel, *panel_lo;
+  void *npanel;     // candidates: each row's norm column (write_norm_row)
+  float *enorm;     // effective norm X2 - 2 mu.x + mu.mu; null: panels and statistics only
+  uint32_t *ids;
+  unsigned *stats;  // candidates: maxima of the bound (PackStats)
+  // queries: the terms of the error bound, the row's largest incoming distance, and the
+  // initialisation of its partition roots and of the overflow count
+  float4 *qe;
+  float *qmx;
+  const T *Din;
+  int ldD, k, nroots, nproot;  // proot holds nproot rows of nroots
+  unsigned *proot;
+  int *zero;
+};
+
+// Maxima over the candidates (bits of non-negative floats, which order like unsigned integers):
+// centred norm |c~|, |effective norm|, norm of the rounding residual |c~ - fmt(c~)|, and the scale
+// of the FP64 distance's own rounding.
+enum PackStats { ST_M = 0, ST_CN, ST_RES, ST_SCALE };
+
+template <typename T>
+struct PackArgs {
+  int fmt, d, d_pad;
+  PackSide<T> a, b;
+  // the shift: from tc_center's partial sums (and written to mu / mu2 for later launches), or, with
+  // part null, read from mu / mu2
+  const double *part;
+  const int *part_n;
+  float *mu;
+  double *mu2;
+  float kA, kB, kS;  // bound coefficients (TcPlan)
+  int *status;
+};
+
+template <typename T>
+__device__ __forceinline__ void pack_load4(const T *x, int n, bool vec, T (&v)[4]) {
+  if (vec) {
+    if constexpr (sizeof(T) == 4) {
+      const float4 t = __ldg(reinterpret_cast<const float4 *>(x));
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+      const double2 t = __ldg(reinterpret_cast<const double2 *>(x));
+      const double2 u = __ldg(reinterpret_cast<const double2 *>(x) + 1);
+      v[0] = t.x; v[1] = t.y; v[2] = u.x; v[3] = u.y;
     }
-    double s2 = 0.0, smx = 0.0;
-    for (int p = lane; p < d_pad; p += 32) {
-      float y = 0.0f;
-      if (row >= 0 && p < d) {
-        const float x = X[row * d + p];
-        const float m = mu[p];
-        y = x - m;
-        smx += (double)m * (double)x;
-        s2 += (double)y * (double)y;
-      }
-      const size_t o = (size_t)r * d_pad + p;
-      if (fmt == 0) {
-        reinterpret_cast<uint32_t *>(panel)[o] = to_tf32(y);
-      } else if (fmt == 1) {
-        reinterpret_cast<__nv_bfloat16 *>(panel)[o] = __float2bfloat16_rn(y);
-      } else {
-        const __nv_bfloat16 hi = __float2bfloat16_rn(y);
-        const __nv_bfloat16 lo = __float2bfloat16_rn(y - __bfloat162float(hi));
-        reinterpret_cast<__nv_bfloat16 *>(panel)[o] = hi;
-        reinterpret_cast<__nv_bfloat16 *>(panel_lo)[o] = lo;
-      }
-    }
-    for (int o = 16; o; o >>= 1) {
-      s2 += __shfl_xor_sync(FULL_MASK, s2, o);
-      smx += __shfl_xor_sync(FULL_MASK, smx, o);
-    }
-    if (lane == 0 && npanel) {
-      // the same effective norm as below (the epilogue's cn), as the MMA's norm column
-      const float enf = row >= 0 ? (float)((double)X2[row] - 2.0 * smx + *mu2) : 0.0f;
-      write_norm_row(fmt, npanel, r, row >= 0, enf);
-    }
-    if (lane == 0 && enorm) {
-      if (row >= 0) {
-        // |x - mu|^2 expressed through the caller's norm: X2 - 2 mu.x + mu.mu
-        const double en = (double)X2[row] - 2.0 * smx + *mu2;
-        const float enf = (float)en;
-        // centred norm of the stored (FP32-rounded) shift, rounded up
-        const float nrm = (float)(sqrt(s2) * (1.0 + 1e-6)) * (1.0f + 1e-6f);
-        enorm[r] = enf;
-        cnrm[r] = nrm;
-        if (ids) ids[r] = (uint32_t)row;
-        // non-negative floats order like their bit patterns
-        mx_nrm = max(mx_nrm, __float_as_uint(nrm));
-        mx_en = max(mx_en, __float_as_uint(fabsf(enf) * (1.0f + 1e-6f)));
-      } else {
-        enorm[r] = Num<float>::nan();
-        cnrm[r] = 0.0f;
-        if (ids) ids[r] = NO_ID;
-      }
-    }
-  }
-  if (lane == 0 && enorm && is_cand && (mx_nrm | mx_en)) {
-    atomicMax(&stats[0], mx_nrm);
-    atomicMax(&stats[1], mx_en);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; j++) v[j] = j < n ? x[j] : T(0);
   }
 }
 
-// Blocks of a tc_pack launch over `rows` panel rows: one warp per row up to 16 CTAs of 8 warps
-// per SM, grid-stride beyond.
+__device__ __forceinline__ float up_f(float x) { return x; }
+__device__ __forceinline__ float up_f(double x) { return __double2float_ru(x); }
+
+// Eight lanes per row, four dimensions per lane at a time: coalesced 16-byte loads of 128 bytes of a
+// row, and reductions over eight lanes for four rows at once (a warp per row spent most of its
+// instructions on 32-lane FP64 reductions). Candidates and queries of a call share one launch, and
+// every block sums the shift from tc_center's partials itself, in one fixed order, instead of
+// waiting for a kernel of one block. Bound: HBM reads of the gathered rows.
+template <typename T>
+__global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
+  extern __shared__ double pack_mu[];  // [d] shift, as doubles
+  __shared__ double red[8];
+  __shared__ unsigned bmx[4];
+  const int tid = threadIdx.x, lane = tid & 31, sub = lane & 7;
+  if (tid < 4) bmx[tid] = 0u;
+  int a_rows = g.a.rows_pad, b_rows = g.b.rows_pad;
+  if (g.a.gate && *g.a.gate == 0) a_rows = 0;
+  if (g.b.gate && *g.b.gate == 0) b_rows = 0;
+  int b_count = g.b.count;
+  if (g.b.dcount) {
+    b_count = *g.b.dcount;
+    b_rows = min(b_rows, (b_count + TC_M - 1) / TC_M * TC_M);
+  }
+  if (blockIdx.x == 0 && tid < 4 && g.b.zero) g.b.zero[tid] = 0;
+  if (a_rows + b_rows == 0) return;
+  double mu2;
+  {
+    double s2 = 0.0;
+    int n = 0;
+    if (g.part)
+      for (int sl = 0; sl < CENTER_SLICES; sl++) n += g.part_n[sl];
+    for (int p = tid; p < g.d; p += 256) {
+      float m;
+      if (g.part) {
+        double tot = 0.0;
+        for (int sl = 0; sl < CENTER_SLICES; sl++) tot += g.part[(size_t)sl * g.d + p];
+        m = n ? (float)(tot / n) : 0.0f;
+        if (blockIdx.x == 0) g.mu[p] = m;
+      } else {
+        m = g.mu[p];
+      }
+      pack_mu[p] = (double)m;
+      s2 += (double)m * (double)m;
+    }
+    for (int o = 16; o; o >>= 1) s2 += __shfl_xor_sync(FULL_MASK, s2, o);
+    if (lane == 0) red[tid >> 5] = s2;
+    __syncthreads();
+    mu2 = 0.0;
+    for (int w = 0; w < 8; w++) mu2 += red[w];
+    if (g.part && blockIdx.x == 0 && tid == 0) *g.mu2 = mu2;
+  }
+  unsigned mx[4] = {0u, 0u, 0u, 0u};
+  const int step = gridDim.x * 32;
+  // (four rows per warp; a side's rows are whole tiles, so a warp's rows lie on one side)
+  for (int r4 = blockIdx.x * 32 + (tid >> 5) * 4; r4 < a_rows + b_rows; r4 += step) {
+    const bool is_a = r4 < a_rows;
+    const PackSide<T> &s = is_a ? g.a : g.b;
+    const int r = (is_a ? r4 : r4 - a_rows) + (lane >> 3);
+    const int count = is_a ? s.count : b_count;
+    long long row = -1;
+    int hr = r;  // heap row (queries)
+    if (r < count) {
+      if (s.rowmap) hr = s.rowmap[r];
+      row = s.idx[hr];
+      if (s.pad_ok) hr = (int)row;
+      if (s.pad_ok && row == -1) {
+        // a padding row of a leaf panel (the batching form): silently empty
+      } else if (row < 0 || row >= s.nrows) {
+        if (sub == 0) atomicExch(g.status, GSKNN_ERR_INDEX);
+        row = -1;
+      }
+    }
+    double s2 = 0.0, smx = 0.0, r2 = 0.0;
+    const T *x = s.X + (row >= 0 ? row : 0) * g.d;
+    const bool vec = (g.d & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    for (int p = 4 * sub; p < g.d_pad; p += 32) {
+      T v[4] = {T(0), T(0), T(0), T(0)};
+      if (row >= 0 && p < g.d) pack_load4<T>(x + p, g.d - p, vec, v);
+      float y[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        y[j] = 0.0f;
+        if (row >= 0 && p + j < g.d) {
+          const double m = pack_mu[p + j], yd = (double)v[j] - m;
+          y[j] = (float)yd;
+          smx = fma(m, (double)v[j], smx);
+          s2 = fma(yd, yd, s2);
+        }
+      }
+      const size_t o = (size_t)r * g.d_pad + p;
+      if (g.fmt == 0) {
+        uint32_t t[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          t[j] = to_tf32(y[j]);
+          const double res = (double)(y[j] - __uint_as_float(t[j]));
+          r2 = fma(res, res, r2);
+        }
+        *reinterpret_cast<uint4 *>(reinterpret_cast<uint32_t *>(s.panel) + o) =
+            make_uint4(t[0], t[1], t[2], t[3]);
+      } else {
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const __nv_bfloat16 hi = __float2bfloat16_rn(y[j]);
+          const float rest = y[j] - __bfloat162float(hi);
+          h[j] = __bfloat16_as_ushort(hi);
+          l[j] = __bfloat16_as_ushort(__float2bfloat16_rn(rest));
+          if (g.fmt == 1) r2 = fma((double)rest, (double)rest, r2);
+        }
+        *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(s.panel) + o) =
+            make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+        if (g.fmt == 2)
+          *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(s.panel_lo) + o) =
+              make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+      }
+    }
+    float qmx = -Num<float>::inf();
+    if (s.qmx && row >= 0 && s.Din)
+      for (int j = sub; j < s.k; j += 8) qmx = fmaxf(qmx, up_f(s.Din[(size_t)hr * s.ldD + j]));
+    if (s.proot && r < s.nproot)
+      for (int j = sub; j < s.nroots; j += 8) s.proot[(size_t)r * s.nroots + j] = 0xFFFFFFFFu;
+#pragma unroll
+    for (int o = 4; o; o >>= 1) {
+      s2 += __shfl_xor_sync(FULL_MASK, s2, o);
+      smx += __shfl_xor_sync(FULL_MASK, smx, o);
+      if (g.fmt < 2) r2 += __shfl_xor_sync(FULL_MASK, r2, o);
+      qmx = fmaxf(qmx, __shfl_xor_sync(FULL_MASK, qmx, o));
+    }
+    if (sub == 0) {
+      // |x - mu|^2 expressed through the caller's norm: X2 - 2 mu.x + mu.mu
+      const double x2 = row >= 0 ? (double)s.X2[row] : 0.0;
+      const float enf = row >= 0 ? (float)(x2 - 2.0 * smx + mu2) : Num<float>::nan();
+      if (s.npanel) write_norm_row(g.fmt, s.npanel, r, row >= 0, row >= 0 ? enf : 0.0f);
+      // norms of the centred row and of its rounding residual (in split BF16 a bound on it, 3.2 u^2
+      // of the norm, that covers the omitted lo x lo product too), rounded up; and the scale of the
+      // FP64 distance's own rounding: the caller's norm, and |x|^2 <= 2 (|x - mu|^2 + |mu|^2)
+      const float nrm = row >= 0 ? up_f(sqrt(s2) * (1.0 + 1e-6)) : 0.0f;
+      const float res = row < 0 ? 0.0f
+                        : g.fmt == 2 ? nrm * (3.2f / 65536.0f)
+                                     : up_f(sqrt(r2) * (1.0 + 1e-6));
+      const float scale = row >= 0 ? up_f(fmax(fabs(x2), 2.0 * (s2 + mu2))) : 0.0f;
+      if (s.enorm) {
+        s.enorm[r] = enf;
+        if (s.ids) s.ids[r] = row >= 0 ? (uint32_t)row : NO_ID;
+      }
+      if (s.qe) {
+        const float eM = 2.5f * (res + g.kA * nrm) + 2.0f * g.kB * nrm;
+        const float eR = g.fmt == 2 ? 0.0f : 2.5f * (nrm + res);
+        s.qe[r] = make_float4(eM, eR, g.kB * fabsf(enf) + g.kS * scale, 0.0f);
+        s.qmx[r] = qmx;
+      }
+      if (s.stats && row >= 0) {
+        mx[ST_M] = max(mx[ST_M], __float_as_uint(nrm));
+        mx[ST_CN] = max(mx[ST_CN], __float_as_uint(fabsf(enf) * (1.0f + 1e-6f)));
+        mx[ST_RES] = max(mx[ST_RES], __float_as_uint(g.fmt == 2 ? 0.0f : res));
+        mx[ST_SCALE] = max(mx[ST_SCALE], __float_as_uint(scale));
+      }
+    }
+  }
+  // the maxima reach the global words once per block (same-address atomics serialize: once per
+  // warp took 20 us of a 32,000-row launch)
+  unsigned *stats = g.a.stats ? g.a.stats : g.b.stats;
+  if (!stats) return;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const unsigned v = __reduce_max_sync(FULL_MASK, mx[i]);
+    if (lane == 0 && v) atomicMax(&bmx[i], v);
+  }
+  __syncthreads();
+  if (tid < 4 && bmx[tid]) atomicMax(&stats[tid], bmx[tid]);
+}
+
+// Blocks of a tc_pack launch over `rows` panel rows: 32 rows a block, up to eight blocks per SM,
+// grid-stride beyond.
 static inline unsigned tc_pack_grid(long long rows) {
-  const long long want = (rows + 7) / 8;
-  return (unsigned)std::max(1LL, std::min(want, 148LL * 16));
+  const long long want = (rows + 31) / 32;
+  return (unsigned)std::max(1LL, std::min(want, 148LL * 8));
 }
 
 // ------------------------------------------------------------------------------------------
@@ -305,11 +430,10 @@ struct TcParams {
   const float *cn;
   const uint32_t *cid;
   const float *qn;
-  const float *qnrm;
-  const unsigned *stats;
-  const float *Din;
-  int ldD;
-  float coefA, coefB, coefC;
+  const float4 *qe;       // per-query terms of the error bound (tc_pack)
+  const float *qmx;       // largest incoming distance of each query's heap row (-inf: none)
+  const unsigned *stats;  // candidate maxima (PackStats)
+  float kC, kS;           // bound coefficients of CN and of the distances' own scale
   // Band logs: entry e of a log is a quad, four adjacent columns of the accumulator as the epilogue
   // filtered them (v, or w = -v/2 with the norm column), and the packed position of the first.
   float4 *log;
@@ -740,18 +864,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     s.thr0 = Num<float>::inf();
     if (valid) {
       s.qn = p.qn[gq];
-      const float M = __uint_as_float(p.stats[0]);
-      const float CN = __uint_as_float(p.stats[1]);
-      const float qa = p.qnrm[gq];
-      const float E =
-          p.coefA * qa * M + p.coefB * (CN + fabsf(s.qn) + 2.0f * qa * M) + p.coefC * CN;
+      const float4 e = p.qe[gq];
+      const float E = e.x * __uint_as_float(p.stats[ST_M]) +
+                      e.y * __uint_as_float(p.stats[ST_RES]) + e.z +
+                      p.kC * __uint_as_float(p.stats[ST_CN]) +
+                      p.kS * __uint_as_float(p.stats[ST_SCALE]);
       s.E2 = 2.0f * E;
-      if (p.Din) {
-        float mx = -Num<float>::inf();
-        const float *rowD = p.Din + (size_t)(p.rowmap ? p.rowmap[gq] : gq) * p.ldD;
-        for (int j = 0; j < p.k; j++) mx = fmaxf(mx, rowD[j]);
-        if (mx > -Num<float>::inf()) s.thr0 = mx + s.E2;
-      }
+      const float mx = p.qmx[gq];
+      if (mx > -Num<float>::inf()) s.thr0 = mx + s.E2;
       refresh_threshold(s);
       if (split == 0 && part == 0) p.margin[gq] = s.E2;
     } else {
@@ -1015,6 +1135,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // Measured against a warp that walked log after log with one lane per exact distance: 65,536 x
 // 262,144, d = 64, k = 32: 751 -> 485 us; 32,768 x 262,144, d = 256, k = 64: 2,743 -> 1,246 us;
 // 2,003 x 30,011: 119 -> 31 us; 16 x 4,096: 144 -> 15 us; 8 trees over 262,144 points: 9.4 -> 5.8 ms.
+template <typename T>
 struct RerankParams {
   int Q, k, S, logcap, d;
   const float4 *log;        // quads as the epilogue filtered them, d' = qmul * value + qn
@@ -1024,10 +1145,11 @@ struct RerankParams {
   float qmul;
   const unsigned *proot;  // partition roots of tc_knn ([query][S]; S counts NPART per split)
   const float *margin;
-  const float *Xq, *Xq2, *Xc, *Xc2;
+  const T *Xq, *Xq2, *Xc, *Xc2;
+  long long nrows_q;
   const int *qidx;
   const uint32_t *cid;  // packed candidate position -> point id
-  float *D;
+  T *D;
   int *I;
   int ldD;
   int *fallback_list;
@@ -1077,10 +1199,10 @@ __device__ __forceinline__ double sum4(double acc) {
   return acc;
 }
 
-// The same distance by one thread, summed in dimension order (the brute-force passes, which compute
-// all of a query's distances themselves).
-__device__ __forceinline__ double exact_dist_lane(const float *q, const float *c, int d,
-                                                  double cc, double qq) {
+// FP64 dot product by one thread, summed in dimension order: the brute-force passes, which compute
+// all of a query's distances themselves, and double tables, whose distances come out of the
+// CUDA-core kernel's order of operations bit for bit.
+__device__ __forceinline__ double dot_lane(const float *q, const float *c, int d) {
   double acc = 0.0;
   const uintptr_t qc = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(c);
   if ((d & 3) == 0 && (qc & 15) == 0) {
@@ -1096,18 +1218,40 @@ __device__ __forceinline__ double exact_dist_lane(const float *q, const float *c
   } else {
     for (int pp = 0; pp < d; pp++) acc = fma((double)q[pp], (double)c[pp], acc);
   }
-  return exact_dist(acc, cc, qq);
+  return acc;
+}
+__device__ __forceinline__ double dot_lane(const double *q, const double *c, int d) {
+  double acc = 0.0;
+  const uintptr_t qc = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(c);
+  if ((d & 1) == 0 && (qc & 15) == 0) {
+    const double2 *q2 = reinterpret_cast<const double2 *>(q);
+    const double2 *c2 = reinterpret_cast<const double2 *>(c);
+#pragma unroll 4
+    for (int i = 0; i < (d >> 1); i++) {
+      const double2 a = __ldg(q2 + i), b = __ldg(c2 + i);
+      acc = fma(a.x, b.x, acc);
+      acc = fma(a.y, b.y, acc);
+    }
+  } else {
+#pragma unroll 4
+    for (int pp = 0; pp < d; pp++) acc = fma(__ldg(q + pp), __ldg(c + pp), acc);
+  }
+  return acc;
+}
+__device__ __forceinline__ double exact_dist_lane(const float *q, const float *c, int d,
+                                                  double cc, double qq) {
+  return exact_dist(dot_lane(q, c, d), cc, qq);
 }
 
-template <int E>
-__device__ __forceinline__ void write_heap_row(float *D, int *I, int ldD, int q, int k,
+template <typename T, int E>
+__device__ __forceinline__ void write_heap_row(T *D, int *I, int ldD, int q, int k,
                                                const double (&ld)[E], const uint32_t (&li)[E],
                                                int lane) {
 #pragma unroll
   for (int e = 0; e < E; e++) {
     const int t = e * 32 + lane;
     if (t < k) {
-      D[(size_t)q * ldD + (k - 1 - t)] = (float)ld[e];
+      D[(size_t)q * ldD + (k - 1 - t)] = (T)ld[e];
       I[(size_t)q * ldD + (k - 1 - t)] = (int)li[e];
     }
   }
@@ -1115,8 +1259,8 @@ __device__ __forceinline__ void write_heap_row(float *D, int *I, int ldD, int q,
 
 // The heap row as it lies (reversed, so that the library's own descending rows come out
 // ascending); the places past k hold (inf, NO_ID).
-template <int E>
-__device__ __forceinline__ void load_heap_row(const float *D, const int *I, int ldD, int q, int k,
+template <typename T, int E>
+__device__ __forceinline__ void load_heap_row(const T *D, const int *I, int ldD, int q, int k,
                                               double (&ld)[E], uint32_t (&li)[E], int lane) {
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -1161,10 +1305,12 @@ __device__ __forceinline__ double list_kth(const double (&ld)[E], int k) {
   return __shfl_sync(FULL_MASK, t, (k - 1) & 31);
 }
 
-// Largest value of the row (its k-th distance once it is full), -inf when all are NaN.
-__device__ __forceinline__ float row_max(const float *row, int k, int lane) {
+// Largest value of the row (its k-th distance once it is full), as a float rounded up; -inf when
+// all are NaN.
+template <typename T>
+__device__ __forceinline__ float row_max(const T *row, int k, int lane) {
   float mx = -Num<float>::inf();
-  for (int j = lane; j < k; j += 32) mx = fmaxf(mx, row[j]);
+  for (int j = lane; j < k; j += 32) mx = fmaxf(mx, up_f(row[j]));
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL_MASK, mx, o));
   return mx;
 }
@@ -1248,8 +1394,8 @@ struct RerankSmem {
 // One query by one warp. LEAF (the batching form): ids already in the row are not entered again,
 // the incoming row stays unsorted until a candidate can enter it, and a row nothing entered is
 // not written back.
-template <int E, bool LEAF>
-__device__ __forceinline__ void rerank_warp(const RerankParams &p, int q, RerankSmem<E> &sm) {
+template <typename Tab, int E, bool LEAF>
+__device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, RerankSmem<E> &sm) {
   constexpr int CAP = rr_cap<E>();
   const int lane = threadIdx.x & 31;
   const int hr = p.rowmap ? p.rowmap[q] : q;  // heap row and query position
@@ -1257,7 +1403,7 @@ __device__ __forceinline__ void rerank_warp(const RerankParams &p, int q, Rerank
   const int k = p.k;
   double ld[E];
   uint32_t li[E];
-  load_heap_row<E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+  load_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
   bool ovf = false;
   unsigned m1 = 0xFFFFFFFFu, m2 = 0xFFFFFFFFu;
   for (int s = lane; s < p.S; s += 32) {
@@ -1266,7 +1412,10 @@ __device__ __forceinline__ void rerank_warp(const RerankParams &p, int q, Rerank
     m2 = min(m2, max(m1, u));
     m1 = min(m1, u);
   }
-  // overflowed logs: the query goes to the next pass (a narrower format, or brute force)
+  const float E2 = p.margin[q], Eq = 0.5f * E2, qn = p.qn[q];
+  // overflowed logs: the query goes to the next pass (a narrower format, or brute force); so does a
+  // double query whose bound left the floats' range
+  if (sizeof(Tab) == 8 && !(E2 < 1e38f)) ovf = true;
   if (__any_sync(FULL_MASK, ovf)) {
     if (lane == 0) p.fallback_list[atomicAdd(p.fallback_count, 1)] = LEAF ? q : hr;
     return;
@@ -1276,11 +1425,10 @@ __device__ __forceinline__ void rerank_warp(const RerankParams &p, int q, Rerank
   // approximate k-th + 2E, and d' <= (the k-th of any k exact distances) + E.
   two_smallest(m1, m2);
   float T = m2 == 0xFFFFFFFFu ? Num<float>::inf() : __uint_as_float(m2);
-  const float E2 = p.margin[q], Eq = 0.5f * E2, qn = p.qn[q];
   float mx = -Num<float>::inf();
 #pragma unroll
   for (int e = 0; e < E; e++)
-    if (e * 32 + lane < k) mx = fmaxf(mx, (float)ld[e]);
+    if (e * 32 + lane < k) mx = fmaxf(mx, up_f((Tab)ld[e]));
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL_MASK, mx, o));
   float lim = band_limit(mx, Eq);
   float thr = band_thr(T, E2, lim);
@@ -1295,7 +1443,8 @@ __device__ __forceinline__ void rerank_warp(const RerankParams &p, int q, Rerank
     sorted = true;
   }
   const long long qrow = p.qidx[hr];
-  const float *qv = p.Xq + qrow * p.d;
+  if (qrow < 0 || qrow >= p.nrows_q) return;  // reported by tc_pack
+  const Tab *qv = p.Xq + qrow * p.d;
   const double qq = (double)p.Xq2[qrow];
   int n = 0;  // listed entries
 
@@ -1421,7 +1570,9 @@ __device__ __forceinline__ void rerank_warp(const RerankParams &p, int q, Rerank
         }
         const double cc = id != NO_ID ? (double)p.Xc2[id] : 0.0;
         double dot = 0.0;
-        for (int r = 0; r < cnt; r += 8) {
+        if constexpr (sizeof(Tab) == 8) {
+          if (id != NO_ID) dot = dot_lane(qv, p.Xc + (long long)id * p.d, p.d);
+        } else for (int r = 0; r < cnt; r += 8) {
           const uint32_t cid = __shfl_sync(FULL_MASK, id, r + (lane >> 2));
           double part = 0.0;
           if (cid != NO_ID)
@@ -1454,23 +1605,23 @@ __device__ __forceinline__ void rerank_warp(const RerankParams &p, int q, Rerank
     n = 0;
     __syncwarp();
   }
-  if (sorted) write_heap_row<E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+  if (sorted) write_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
 }
 
-template <int E>
-__global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank(RerankParams p) {
+template <typename Tab, int E>
+__global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank(RerankParams<Tab> p) {
   __shared__ RerankSmem<E> sm[RR_WARPS];
   const int q = blockIdx.x * RR_WARPS + (threadIdx.x >> 5);
   if (q >= (p.dQ ? *p.dQ : p.Q)) return;
-  rerank_warp<E, false>(p, q, sm[threadIdx.x >> 5]);
+  rerank_warp<Tab, E, false>(p, q, sm[threadIdx.x >> 5]);
 }
 
 template <int E>
-__global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_leaf(RerankParams p) {
+__global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_leaf(RerankParams<float> p) {
   __shared__ RerankSmem<E> sm[RR_WARPS];
   const int q = blockIdx.x * RR_WARPS + (threadIdx.x >> 5);
   if (q >= p.Q) return;
-  rerank_warp<E, true>(p, q, sm[threadIdx.x >> 5]);
+  rerank_warp<float, E, true>(p, q, sm[threadIdx.x >> 5]);
 }
 
 // One query by one CTA: all warps read the logs into one list and share the exact distances; warp
@@ -1478,8 +1629,8 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_leaf(Reran
 constexpr int RC_CAP = 1024;  // listed entries per CTA
 constexpr int RC_LOGS = 512;  // logs (NPART * S) the prefix array holds
 
-template <int E>
-__global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(RerankParams p) {
+template <typename Tab, int E>
+__global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(RerankParams<Tab> p) {
   __shared__ uint2 list[RC_CAP];
   __shared__ double xd[RC_CAP];
   __shared__ uint32_t xi[RC_CAP];
@@ -1517,7 +1668,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
       if (g + lane < p.S) pre[g + lane + 1] = carry + incl;
       carry += __shfl_sync(FULL_MASK, incl, 31);
     }
-    ovf = __any_sync(FULL_MASK, ovf);
+    ovf = __any_sync(FULL_MASK, ovf) || (sizeof(Tab) == 8 && !(E2 < 1e38f));
     two_smallest(m1, m2);
     const float T = m2 == 0xFFFFFFFFu ? Num<float>::inf() : __uint_as_float(m2);
     const float lim = band_limit(row_max(p.D + (size_t)hr * p.ldD, k, lane), Eq);
@@ -1558,7 +1709,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
   __syncthreads();
   const int n = s_n;
   if (n > RC_CAP) {
-    if (warp == 0) rerank_warp<E, false>(p, q, sm);
+    if (warp == 0) rerank_warp<Tab, E, false>(p, q, sm);
     return;
   }
   if (n > 32 && n >= k) {
@@ -1570,16 +1721,22 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
     thr = s_thr;
   }
   const long long qrow = p.qidx[hr];
-  const float *qv = p.Xq + qrow * p.d;
+  if (qrow < 0 || qrow >= p.nrows_q) return;  // reported by tc_pack
+  const Tab *qv = p.Xq + qrow * p.d;
   const double qq = (double)p.Xq2[qrow];
-  for (int base = warp * 8; base < n; base += 8 * RR_WARPS) {
-    const int i = base + (lane >> 2);  // four lanes per candidate
+  constexpr int LPC = sizeof(Tab) == 8 ? 1 : 4;  // lanes per candidate
+  for (int base = warp * (32 / LPC); base < n; base += 32 / LPC * RR_WARPS) {
+    const int i = base + lane / LPC;
     uint32_t id = NO_ID;
     if (i < n && __uint_as_float(list[i].x) <= thr) id = p.cid[list[i].y];
     double dot = 0.0;
-    if (id != NO_ID) dot = exact_dot4(qv, p.Xc + (long long)id * p.d, p.d, lane & 3);
-    dot = sum4(dot);
-    if (i < n && (lane & 3) == 0) {
+    if constexpr (LPC == 1) {
+      if (id != NO_ID) dot = dot_lane(qv, p.Xc + (long long)id * p.d, p.d);
+    } else {
+      if (id != NO_ID) dot = exact_dot4(qv, p.Xc + (long long)id * p.d, p.d, lane & 3);
+      dot = sum4(dot);
+    }
+    if (i < n && lane % LPC == 0) {
       xd[i] = id != NO_ID ? exact_dist(dot, (double)p.Xc2[id], qq) : Num<double>::inf();
       xi[i] = id;
       if (p.counters && id != NO_ID) atomicAdd(&p.counters[6], 1ull);
@@ -1589,7 +1746,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
   if (warp != 0) return;
   double ld[E];
   uint32_t li[E];
-  load_heap_row<E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+  load_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
   sort_heap_row<E>(ld, li, lane);
   double kth = list_kth<E>(ld, k);
   for (int base = 0; base < n; base += 32) {
@@ -1601,7 +1758,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
     warp_merge_32<double, E>(ld, li, b1[0], i1[0], lane);
     kth = list_kth<E>(ld, k);
   }
-  write_heap_row<E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+  write_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1672,7 +1829,7 @@ __global__ void __launch_bounds__(256) tc_fallback(FallbackParams p) {
     if (warp == 0) {
       double md[E];
       uint32_t mi[E];
-      load_heap_row<E>(p.D, p.I, p.ldD, q, p.k, md, mi, lane);
+      load_heap_row<float, E>(p.D, p.I, p.ldD, q, p.k, md, mi, lane);
       sort_heap_row<E>(md, mi, lane);
       for (int w2 = 0; w2 < 8; w2++) {
         double bd[E];
@@ -1684,7 +1841,7 @@ __global__ void __launch_bounds__(256) tc_fallback(FallbackParams p) {
         }
         warp_merge_lists<double, E>(md, mi, bd, bi, lane);
       }
-      write_heap_row<E>(p.D, p.I, p.ldD, q, p.k, md, mi, lane);
+      write_heap_row<float, E>(p.D, p.I, p.ldD, q, p.k, md, mi, lane);
     }
     __syncthreads();
   }
@@ -1720,7 +1877,7 @@ __global__ void __launch_bounds__(256) tc_fallback_leaf(LeafFallbackParams p) {
     const double qq = (double)p.X2[hr];
     double ld[E];
     uint32_t li[E];
-    load_heap_row<E>(p.D, p.I, p.ldD, hr, p.k, ld, li, lane);
+    load_heap_row<float, E>(p.D, p.I, p.ldD, hr, p.k, ld, li, lane);
     sort_heap_row<E>(ld, li, lane);
     __shared__ __align__(16) uint32_t ids[8][32 * E];  // the incoming row's ids
     uint32_t *const li0 = ids[threadIdx.x >> 5];
@@ -1746,7 +1903,7 @@ __global__ void __launch_bounds__(256) tc_fallback_leaf(LeafFallbackParams p) {
       warp_sort<double, 1>(b1, i1, lane);
       warp_merge_32<double, E>(ld, li, b1[0], i1[0], lane);
     }
-    write_heap_row<E>(p.D, p.I, p.ldD, hr, p.k, ld, li, lane);
+    write_heap_row<float, E>(p.D, p.I, p.ldD, hr, p.k, ld, li, lane);
   }
 }
 
@@ -1817,9 +1974,8 @@ static cudaError_t launch_tc_knn(const TcPlan &P, void *npanel, int npanel_rows,
     if (e != cudaSuccess) return e;
   }
   tp.fold = fold ? 1 : 0;
-  tp.coefA = fold ? P.coefA_fold : P.coefA;
-  tp.coefB = P.coefB;
-  tp.coefC = fold ? P.coefC_fold : P.coefC;
+  tp.kC = P.kB + (fold ? P.kC_fold : 0.0f);
+  tp.kS = P.kS;
   const unsigned smem = fold ? P.smem_fold : P.smem;
   cudaError_t e = cudaSuccess;
   auto go = [&](auto kern) {
@@ -1843,7 +1999,7 @@ int tc_format_of_mode(int mode) {
 
 // Prepared-candidate area: mu, mu2, stats, panel(s), norms, norm bounds, ids.
 struct CandLayout {
-  size_t o_mu, o_mu2, o_cpart, o_stats, o_pb, o_pb_lo, o_pn, o_cn, o_cnrm, o_cid, bytes;
+  size_t o_mu, o_mu2, o_cpart, o_stats, o_pb, o_pb_lo, o_pn, o_cn, o_cid, bytes;
   int fmt, elem, d_pad, r_pad;
 };
 
@@ -1860,52 +2016,100 @@ static CandLayout cand_layout(int nc, int d, int mode) {
   L.o_mu = take((size_t)d * 4);
   L.o_mu2 = take(8);
   L.o_cpart = take((size_t)CENTER_SLICES * d * 8 + CENTER_SLICES * 4);
-  L.o_stats = take(16);
+  L.o_stats = take(32);
   L.o_pb = take((size_t)L.r_pad * L.d_pad * L.elem);
   L.o_pb_lo = L.fmt == 2 ? take((size_t)L.r_pad * L.d_pad * L.elem) : 0;
   L.o_pn = take((size_t)L.r_pad * NORM_ROW);
   L.o_cn = take((size_t)L.r_pad * 4);
-  L.o_cnrm = take((size_t)L.r_pad * 4);
   L.o_cid = take((size_t)L.r_pad * 4);
   L.bytes = off;
   return L;
 }
 
+static int tc_mode_of_format(int fmt) {
+  return fmt == 1 ? GSKNN_TC_BF16 : fmt == 2 ? GSKNN_TC_BF16X3 : GSKNN_TC_TF32;
+}
+
 size_t tc_cand_bytes(int nc, int d, int mode) { return cand_layout(nc, d, mode).bytes; }
 
-cudaError_t tc_cand_prepare(TcCand *C, void *mem, int nc, int d, int mode, const float *Xc,
-                            const float *Xc2, long long nrows_c, const int *cidx, int *status,
-                            cudaStream_t st) {
+// Lays out candidates in `mem` (cand_layout) and enqueues their shift.
+template <typename T>
+static cudaError_t cand_begin(TcCand *C, void *mem, int nc, int d, int mode, const T *Xc,
+                              const T *Xc2, long long nrows_c, const int *cidx, int *clear,
+                              cudaStream_t st) {
   using namespace tc;
   const CandLayout L = cand_layout(nc, d, mode);
   char *base = static_cast<char *>(mem);
   C->fmt = L.fmt; C->elem = L.elem; C->d = d; C->d_pad = L.d_pad; C->nc = nc; C->r_pad = L.r_pad;
   C->mu = reinterpret_cast<float *>(base + L.o_mu);
   C->mu2 = reinterpret_cast<double *>(base + L.o_mu2);
+  C->part = reinterpret_cast<double *>(base + L.o_cpart);
+  C->part_n = reinterpret_cast<int *>(base + L.o_cpart + (size_t)CENTER_SLICES * d * 8);
   C->stats = reinterpret_cast<unsigned *>(base + L.o_stats);
+  C->estats = C->stats + 4;
   C->pb = base + L.o_pb;
   C->pb_lo = L.fmt == 2 ? base + L.o_pb_lo : nullptr;
   C->pn = base + L.o_pn;
   C->cn = reinterpret_cast<float *>(base + L.o_cn);
-  C->cnrm = reinterpret_cast<float *>(base + L.o_cnrm);
   C->cid = reinterpret_cast<uint32_t *>(base + L.o_cid);
   C->Xc = Xc; C->Xc2 = Xc2; C->nrows_c = nrows_c; C->cidx = cidx;
   C->efmt = -1; C->epb = nullptr; C->epb_lo = nullptr; C->epn = nullptr;
-  cudaError_t e = cudaMemsetAsync(C->stats, 0, 16, st);
-  if (e != cudaSuccess) return e;
-  const int nsample = std::min(nc, 4096);
-  {
-    double *part = reinterpret_cast<double *>(base + L.o_cpart);
-    int *part_n = reinterpret_cast<int *>(base + L.o_cpart + (size_t)CENTER_SLICES * d * 8);
-    tc_center<<<dim3((d + 31) / 32, CENTER_SLICES), 1024, 0, st>>>(Xc, d, nrows_c, cidx, nc,
-                                                                    nsample, part, part_n);
-    tc_center_fin<<<1, 256, 0, st>>>(part, part_n, d, C->mu, C->mu2);
-  }
-  tc_pack<<<tc_pack_grid(L.r_pad), 256, 0, st>>>(L.fmt, Xc, Xc2, d, L.d_pad, nrows_c, cidx, nc,
-                                            L.r_pad, C->mu, C->mu2, 1, C->pb, C->pb_lo, C->cn,
-                                            C->cnrm, C->cid, C->stats, status, nullptr, nullptr,
-                                            nullptr, 0, C->pn);
+  tc_center<T><<<dim3((d + 31) / 32, CENTER_SLICES), 32 * CENTER_WARPS, 0, st>>>(
+      Xc, d, nrows_c, cidx, nc, std::min(nc, CENTER_ROWS), C->part, C->part_n, C->stats, 8, clear);
   return cudaGetLastError();
+}
+
+// The candidates' side of a packing launch, in their main format.
+template <typename T>
+static tc::PackSide<T> cand_side(const TcCand &C) {
+  tc::PackSide<T> s{};
+  s.X = static_cast<const T *>(C.Xc);
+  s.X2 = static_cast<const T *>(C.Xc2);
+  s.nrows = C.nrows_c;
+  s.idx = C.cidx;
+  s.count = C.nc;
+  s.rows_pad = C.r_pad;
+  s.panel = C.pb;
+  s.panel_lo = C.pb_lo;
+  s.npanel = C.pn;
+  s.enorm = C.cn;
+  s.ids = C.cid;
+  s.stats = C.stats;
+  return s;
+}
+
+// Packs one side or both; with `sums` the shift comes from the partial sums of tc_center.
+template <typename T>
+static cudaError_t launch_tc_pack(const tc::PackSide<T> &a, const tc::PackSide<T> &b,
+                                  const TcCand &C, int fmt, int d_pad, bool sums, float kA,
+                                  float kB, float kS, int *status, cudaStream_t st) {
+  tc::PackArgs<T> g{};
+  g.fmt = fmt;
+  g.d = C.d;
+  g.d_pad = d_pad;
+  g.a = a;
+  g.b = b;
+  g.part = sums ? C.part : nullptr;
+  g.part_n = C.part_n;
+  g.mu = C.mu;
+  g.mu2 = C.mu2;
+  g.kA = kA;
+  g.kB = kB;
+  g.kS = kS;
+  g.status = status;
+  tc::tc_pack<T><<<tc::tc_pack_grid((long long)a.rows_pad + b.rows_pad), 256,
+                   (size_t)C.d * sizeof(double), st>>>(g);
+  return cudaGetLastError();
+}
+
+cudaError_t tc_cand_prepare(TcCand *C, void *mem, int nc, int d, int mode, const float *Xc,
+                            const float *Xc2, long long nrows_c, const int *cidx, int *status,
+                            cudaStream_t st) {
+  const cudaError_t e =
+      cand_begin<float>(C, mem, nc, d, mode, Xc, Xc2, nrows_c, cidx, nullptr, st);
+  if (e != cudaSuccess) return e;
+  return launch_tc_pack<float>(cand_side<float>(*C), tc::PackSide<float>{}, *C, C->fmt, C->d_pad,
+                               true, 0.0f, 0.0f, 0.0f, status, st);
 }
 
 // Quads per log: `want`, or as many as keep all `logs` logs under 16 GB, but not fewer than fit the
@@ -1996,7 +2200,8 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   P.o_pa = take((size_t)P.q_pad * P.d_pad * elem);
   P.o_pa_lo = P.fmt == 2 ? take((size_t)P.q_pad * P.d_pad * elem) : 0;
   P.o_qn = take((size_t)P.q_pad * 4);
-  P.o_qnrm = take((size_t)P.q_pad * 4);
+  P.o_qe = take((size_t)P.q_pad * 16);
+  P.o_qmx = take((size_t)P.q_pad * 4);
   // NPART logs per (query, split): one per epilogue warp of a lane quarter
   P.o_logcnt = take((size_t)NPART * P.S * nq * 4);
   P.o_proot = take((size_t)NPART * P.S * nq * 4);
@@ -2006,30 +2211,22 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   // last: once the re-rank has read the logs, the escalation pass takes their place
   P.o_log = take((size_t)NPART * P.S * nq * P.logcap * LOG_ENTRY);
   P.bytes = off;
-  // error-bound coefficients
-  const double D = (double)P.d_pad;
-  double inp, accum, u;
-  if (P.fmt == 2) {
-    u = 1.0 / 256.0;
-    inp = 3.2 * u * u;
-    accum = 3.0 * D * std::ldexp(1.0, -23);
-  } else {
-    u = P.fmt == 0 ? std::ldexp(1.0, -11) : std::ldexp(1.0, -8);
-    inp = 2.0 * u + u * u;
-    accum = D * std::ldexp(1.0, -23) * (1 + u) * (1 + u);
-  }
-  P.coefA = (float)(1.25 * 2.0 * (inp + accum + std::ldexp(1.0, -22)));
-  P.coefB = (float)(1.25 * 3.0 * std::ldexp(1.0, -24) + 1e-12);
-  P.coefC = 0.0f;
-  // With the norm column the accumulation also adds the three parts of -cn/2 (exact in the
-  // input format): n = (products) + 3 terms accumulate, charged as truncation on the sum of
-  // their magnitudes, |<q~, c~>| (1 + u)^2 + CN / 2; in v = -2w that is twice as much. The final
-  // d' = v + qn' rounds once, inside the coefB term.
+  // Error-bound coefficients. kA: accumulation, charged as truncation on the sum of the products'
+  // magnitudes, |q~| |c~| (1 + u)^2 (the rounded factors), over the products and the three parts
+  // of the norm column, and the FP32 rounding of both centred factors. kB: FP32 rounding of the
+  // norm terms. kS: the FP64 distance's own rounding (and the effective norms'). With the norm
+  // column the accumulation also adds the three parts of -cn/2 (exact in the input format), whose
+  // magnitudes sum to CN / 2; in v = -2w that is twice as much: kC_fold. The final d' = v + qn'
+  // rounds once, inside the kB term. The input rounding itself is measured (tc_pack).
   {
+    const double D = (double)P.d_pad;
+    const double u = P.fmt == 0 ? std::ldexp(1.0, -11) : std::ldexp(1.0, -8);
     const double n = (P.fmt == 2 ? 3.0 * D : D) + 3.0;
-    const double accf = n * std::ldexp(1.0, -23);
-    P.coefA_fold = (float)(1.25 * 2.0 * (inp + accf * (1 + u) * (1 + u) + std::ldexp(1.0, -22)));
-    P.coefC_fold = (float)(1.25 * (accf + std::ldexp(1.0, -24)) + 1e-12);
+    const double acc = n * std::ldexp(1.0, -23);
+    P.kA = (float)(acc * (1 + u) * (1 + u) + std::ldexp(1.0, -22));
+    P.kB = (float)(1.25 * 3.0 * std::ldexp(1.0, -24) + 1e-12);
+    P.kC_fold = (float)(1.25 * (acc + std::ldexp(1.0, -24)) + 1e-12);
+    P.kS = (float)(1.25 * (4.0 * d + 32.0) * std::ldexp(1.0, -53));
   }
   P.ok = true;
   return P;
@@ -2077,44 +2274,37 @@ TcPlan tc_plan(int nq, int nc, int d, int k, int mode, int sms, bool with_cand,
   return P;
 }
 
-cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *Xq,
-                   const float *Xq2, long long nrows_q, const int *qidx, const float *Xc,
-                   const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,
-                   int ldD, void *ws, int *status, float *dbg, long long dbg_ld,
-                   unsigned long long *counters, cudaStream_t st, TraceHook hook,
-                   void *hook_ctx) {
-  if (P.cand_bytes == 0) return cudaErrorInvalidValue;
-  // centre, mu.mu and the candidate pack share the tracer's packing bracket
-  if (hook) hook(hook_ctx, "tc_pack", true, st, 0);
-  TcCand C{};
-  const int mode = P.fmt == 1 ? GSKNN_TC_BF16 : P.fmt == 2 ? GSKNN_TC_BF16X3 : GSKNN_TC_TF32;
-  cudaError_t e = tc_cand_prepare(&C, ws, nc, d, mode, Xc, Xc2, nrows_c, cidx, status, st);
-  if (hook) hook(hook_ctx, "tc_pack", false, st, 3);
-  if (e != cudaSuccess) return e;
-  return tc_run_prepared(P, C, nq, d, k, Xq, Xq2, nrows_q, qidx, D, I, ldD, ws, status, dbg,
-                         dbg_ld, counters, st, hook, hook_ctx);
+// The escalation pass's candidates: panels, norms and statistics of the second format.
+static TcCand escalation_cand(const TcCand &C, const TcPlan &EP, void *pb, void *pb_lo, void *pn) {
+  TcCand E = C;
+  E.fmt = EP.fmt;
+  E.elem = EP.elem;
+  E.d_pad = EP.d_pad;
+  E.pb = pb;
+  E.pb_lo = pb_lo;
+  E.pn = pn;
+  E.stats = C.estats;
+  return E;
 }
 
 // One approximate pass + re-rank: pack the queries (all of them, or on an escalation pass the
-// `dQ` queries listed in `rowmap`), tc_knn in the plan's format, tc_rerank. Queries whose log
+// `dQ` queries listed in `rowmap`) and, with `pack_cand`, the candidates C (for the escalation pass
+// only if some query is listed); tc_knn in the plan's format; tc_rerank. Queries whose log
 // overflowed are appended (as heap rows) to the plan's fallback list, whose count sits at
 // base + P.o_fbc.
-static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, void *cand_pb, void *cand_pb_lo,
-                           void *cand_pn, int nq, int d, int k, const float *Xq, const float *Xq2,
-                           long long nrows_q, const int *qidx, const int *dQ, const int *rowmap,
-                           float *D, int *I, int ldD, char *base, int *status, float *dbg,
-                           long long dbg_ld, unsigned long long *counters, cudaStream_t st,
-                           TraceHook hook, void *hook_ctx, bool escalation) {
+template <typename T>
+static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, bool pack_cand, bool sums, int nq,
+                           int d, int k, const T *Xq, const T *Xq2, long long nrows_q,
+                           const int *qidx, const int *dQ, const int *rowmap, T *D, int *I,
+                           int ldD, char *base, int *status, float *dbg, long long dbg_ld,
+                           unsigned long long *counters, cudaStream_t st, TraceHook hook,
+                           void *hook_ctx) {
   using namespace tc;
+  const bool escalation = dQ != nullptr;
   void *pa = base + P.o_pa;
   void *pa_lo = P.fmt == 2 ? base + P.o_pa_lo : nullptr;
   float *qn = reinterpret_cast<float *>(base + P.o_qn);
-  float *qnrm = reinterpret_cast<float *>(base + P.o_qnrm);
   int *fbc = reinterpret_cast<int *>(base + P.o_fbc);
-  cudaError_t e = cudaMemsetAsync(fbc, 0, 16, st);
-  if (e == cudaSuccess)
-    e = cudaMemsetAsync(base + P.o_proot, 0xFF, (size_t)NPART * P.S * nq * 4, st);
-  if (e != cudaSuccess) return e;
   // tracer brackets; `nk` = kernels of this file launched inside the bracket
   auto mark = [&](const char *name, bool begin, int nk = 0) {
     if (hook) hook(hook_ctx, name, begin, st, nk);
@@ -2122,23 +2312,49 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, void *cand_pb, void
   const char *n_pack = escalation ? "tc_escalate" : "tc_pack";
   const char *n_knn = escalation ? "tc_escalate" : "tc_knn";
   const char *n_rr = escalation ? "tc_escalate" : "tc_rerank";
+  PackSide<T> qs{};
+  qs.X = Xq;
+  qs.X2 = Xq2;
+  qs.nrows = nrows_q;
+  qs.idx = qidx;
+  qs.rowmap = rowmap;
+  qs.dcount = dQ;
+  qs.count = nq;
+  qs.rows_pad = P.q_pad;
+  qs.panel = pa;
+  qs.panel_lo = pa_lo;
+  qs.enorm = qn;
+  qs.qe = reinterpret_cast<float4 *>(base + P.o_qe);
+  qs.qmx = reinterpret_cast<float *>(base + P.o_qmx);
+  qs.Din = D;
+  qs.ldD = ldD;
+  qs.k = k;
+  qs.nroots = NPART * P.S;
+  qs.nproot = nq;
+  qs.proot = reinterpret_cast<unsigned *>(base + P.o_proot);
+  qs.zero = fbc;
+  PackSide<T> cs{};
+  if (pack_cand) {
+    cs = cand_side<T>(C);
+    if (escalation) {
+      cs.enorm = nullptr;
+      cs.gate = dQ;
+    }
+  }
   mark(n_pack, true);
-  tc_pack<<<tc_pack_grid(P.q_pad), 256, 0, st>>>(P.fmt, Xq, Xq2, d, P.d_pad, nrows_q, qidx, nq,
-                                            P.q_pad, C.mu, C.mu2, 0, pa, pa_lo, qn, qnrm,
-                                            nullptr, C.stats, status, dQ, rowmap, nullptr);
-  e = cudaGetLastError();
-  mark(n_pack, false, 1);  // query pack
+  cudaError_t e = launch_tc_pack<T>(cs, qs, C, P.fmt, P.d_pad, sums, P.kA, P.kB, P.kS, status, st);
+  mark(n_pack, false, 1);
   if (e != cudaSuccess) return e;
 
   CUtensorMap mA, mAlo, mB, mBlo;
   e = make_panel_map(&mA, pa, P.elem, P.d_pad, P.q_pad, TC_M);
-  if (e == cudaSuccess) e = make_panel_map(&mB, cand_pb, P.elem, P.d_pad, P.r_pad, P.N);
+  if (e == cudaSuccess) e = make_panel_map(&mB, C.pb, P.elem, P.d_pad, P.r_pad, P.N);
   if (e != cudaSuccess) return e;
   mAlo = mA;
   mBlo = mB;
   if (P.fmt == 2) {
     e = make_panel_map(&mAlo, pa_lo, P.elem, P.d_pad, P.q_pad, TC_M);
-    if (e == cudaSuccess) e = make_panel_map(&mBlo, cand_pb_lo, P.elem, P.d_pad, P.r_pad, P.N);
+    if (e == cudaSuccess) e = make_panel_map(&mBlo, C.pb_lo, P.elem, P.d_pad, P.r_pad, P.N);
     if (e != cudaSuccess) return e;
   }
   TcParams tp{};
@@ -2146,12 +2362,11 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, void *cand_pb, void
   tp.N = P.N; tp.NST = P.NST; tp.logcap = P.logcap;
   tp.a_terms = P.a_terms; tp.fmt = P.fmt;
   tp.idesc = idesc_f32acc(P.fmt == 0 ? 2u : 1u, TC_M, P.N);
-  tp.cn = C.cn; tp.cid = C.cid; tp.qn = qn; tp.qnrm = qnrm; tp.stats = C.stats;
-  tp.Din = D; tp.ldD = ldD;
+  tp.cn = C.cn; tp.cid = C.cid; tp.qn = qn; tp.qe = qs.qe; tp.qmx = qs.qmx; tp.stats = C.stats;
   tp.log = reinterpret_cast<float4 *>(base + P.o_log);
   tp.logpos = reinterpret_cast<uint32_t *>(tp.log + (size_t)NPART * P.S * nq * P.logcap);
   tp.logcnt = reinterpret_cast<int *>(base + P.o_logcnt);
-  tp.proot = reinterpret_cast<unsigned *>(base + P.o_proot);
+  tp.proot = qs.proot;
   tp.hk = P.hk;
   tp.W = tc_window(P.S);
   tp.S = P.S;
@@ -2166,16 +2381,18 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, void *cand_pb, void
   tp.no_compact = P.esc_mode != 0;
   dim3 grid(P.qtiles, P.S);
   mark(n_knn, true);
-  e = launch_tc_knn(P, cand_pn, P.r_pad, grid, mA, mAlo, mB, mBlo, tp, st);
+  e = launch_tc_knn(P, C.pn, P.r_pad, grid, mA, mAlo, mB, mBlo, tp, st);
   mark(n_knn, false, 1);
   if (e != cudaSuccess) return e;
 
-  RerankParams rp{};
+  RerankParams<T> rp{};
   rp.Q = nq; rp.k = k; rp.S = NPART * P.S; rp.logcap = P.logcap; rp.d = d;
   rp.log = tp.log; rp.logpos = tp.logpos; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
   rp.qn = tp.qn; rp.qmul = tp.fold ? -2.0f : 1.0f;
   rp.proot = tp.proot;
-  rp.Xq = Xq; rp.Xq2 = Xq2; rp.Xc = C.Xc; rp.Xc2 = C.Xc2; rp.qidx = qidx; rp.cid = C.cid;
+  rp.Xq = Xq; rp.Xq2 = Xq2; rp.nrows_q = nrows_q;
+  rp.Xc = static_cast<const T *>(C.Xc); rp.Xc2 = static_cast<const T *>(C.Xc2);
+  rp.qidx = qidx; rp.cid = C.cid;
   rp.D = D; rp.I = I; rp.ldD = ldD;
   rp.fallback_list = reinterpret_cast<int *>(base + P.o_fbl);
   rp.fallback_count = fbc;
@@ -2188,14 +2405,14 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, void *cand_pb, void
   const bool cta = nq <= 4 * 148 && rp.S <= RC_LOGS;
   mark(n_rr, true);
   switch (P.kp) {
-    case 32: cta ? tc_rerank_cta<1><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
-                 : tc_rerank<1><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
-    case 64: cta ? tc_rerank_cta<2><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
-                 : tc_rerank<2><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
-    case 128: cta ? tc_rerank_cta<4><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
-                  : tc_rerank<4><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
-    case 256: cta ? tc_rerank_cta<8><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
-                  : tc_rerank<8><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
+    case 32: cta ? tc_rerank_cta<T, 1><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
+                 : tc_rerank<T, 1><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
+    case 64: cta ? tc_rerank_cta<T, 2><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
+                 : tc_rerank<T, 2><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
+    case 128: cta ? tc_rerank_cta<T, 4><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
+                  : tc_rerank<T, 4><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
+    case 256: cta ? tc_rerank_cta<T, 8><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
+                  : tc_rerank<T, 8><<<rb, 32 * RR_WARPS, 0, st>>>(rp); break;
     default: return cudaErrorInvalidValue;
   }
   e = cudaGetLastError();
@@ -2209,7 +2426,8 @@ static cudaError_t tc_brute(const TcPlan &P, const TcCand &C, int d, int k, cons
                             char *base, cudaStream_t st, TraceHook hook, void *hook_ctx) {
   using namespace tc;
   FallbackParams fp{};
-  fp.k = k; fp.d = d; fp.nc = C.nc; fp.Xq = Xq; fp.Xq2 = Xq2; fp.Xc = C.Xc; fp.Xc2 = C.Xc2;
+  fp.k = k; fp.d = d; fp.nc = C.nc; fp.Xq = Xq; fp.Xq2 = Xq2;
+  fp.Xc = static_cast<const float *>(C.Xc); fp.Xc2 = static_cast<const float *>(C.Xc2);
   fp.qidx = qidx; fp.cidx = C.cidx; fp.nrows_c = C.nrows_c; fp.D = D; fp.I = I; fp.ldD = ldD;
   fp.list = reinterpret_cast<const int *>(base + P.o_fbl);
   fp.count = reinterpret_cast<const int *>(base + P.o_fbc);
@@ -2226,26 +2444,29 @@ static cudaError_t tc_brute(const TcPlan &P, const TcCand &C, int d, int k, cons
   return e;
 }
 
-cudaError_t tc_run_prepared(const TcPlan &P, const TcCand &C, int nq, int d, int k,
-                            const float *Xq, const float *Xq2, long long nrows_q,
-                            const int *qidx, float *D, int *I, int ldD, void *ws, int *status,
-                            float *dbg, long long dbg_ld, unsigned long long *counters,
-                            cudaStream_t st, TraceHook hook, void *hook_ctx) {
-  using namespace tc;
+// The pass in the plan's format, then the escalation: the queries whose log overflowed run again in
+// the narrower format against the same candidates (their panels in that format: prepared with the
+// candidates, or packed here only when some query overflowed), as a pass over the list of
+// overflowed heap rows whose length stays on the device. *list / *count: the heap rows (and their
+// number) that overflowed in the last format too.
+template <typename T>
+static cudaError_t tc_passes(const TcPlan &P, const TcCand &C, bool per_call, int nq, int d, int k,
+                             const T *Xq, const T *Xq2, long long nrows_q, const int *qidx, T *D,
+                             int *I, int ldD, char *base, int *status, float *dbg,
+                             long long dbg_ld, unsigned long long *counters, cudaStream_t st,
+                             TraceHook hook, void *hook_ctx, const TcPlan **last, char **last_base,
+                             TcPlan *EPout) {
   if (C.fmt != P.fmt || C.d_pad != P.d_pad || C.r_pad != P.r_pad) return cudaErrorInvalidValue;
-  char *base = static_cast<char *>(ws);
-  cudaError_t e = tc_pass(P, C, C.pb, C.pb_lo, C.pn, nq, d, k, Xq, Xq2, nrows_q, qidx, nullptr,
-                          nullptr, D, I, ldD, base, status, dbg, dbg_ld, counters, st, hook,
-                          hook_ctx, false);
-  if (e != cudaSuccess) return e;
-  // Escalation: the queries whose log overflowed run again in the narrower format against the
-  // same candidates (their panels in that format: prepared with the candidates, or packed here
-  // only when some query overflowed), as a pass over the list of overflowed heap rows whose
-  // length stays on the device. What overflows there too goes to the FP64 brute force.
-  const TcPlan EP = P.esc_mode ? tc_plan_base(nq, C.nc, d, k, P.esc_mode, P.sms, false,
-                                              P.max_splits)
-                               : TcPlan{};
+  *last = &P;
+  *last_base = base;
+  cudaError_t e = tc_pass<T>(P, C, per_call, per_call, nq, d, k, Xq, Xq2, nrows_q, qidx, nullptr,
+                             nullptr, D, I, ldD, base, status, dbg, dbg_ld, counters, st, hook,
+                             hook_ctx);
+  if (e != cudaSuccess || !P.esc_mode) return e;
+  TcPlan &EP = *EPout;
+  EP = tc_plan_base(nq, C.nc, d, k, P.esc_mode, P.sms, false, P.max_splits);
   void *epb = nullptr, *epb_lo = nullptr, *epn = nullptr;
+  bool pack = false;
   if (EP.ok && C.efmt == EP.fmt) {
     epb = C.epb;
     epb_lo = C.epb_lo;
@@ -2256,38 +2477,60 @@ cudaError_t tc_run_prepared(const TcPlan &P, const TcCand &C, int nq, int d, int
     epb = base + P.o_ecand;
     epb_lo = EP.fmt == 2 ? base + P.o_ecand + one : nullptr;
     epn = base + P.o_ecand + (EP.fmt == 2 ? 2 * one : one);
-    if (hook) hook(hook_ctx, "tc_escalate", true, st, 0);
-    tc_pack<<<tc_pack_grid(C.r_pad), 256, 0, st>>>(EP.fmt, C.Xc, C.Xc2, d, EP.d_pad, C.nrows_c,
-                                              C.cidx, C.nc, C.r_pad, C.mu, C.mu2, 1, epb,
-                                              epb_lo, nullptr, nullptr, nullptr, nullptr,
-                                              status, nullptr, nullptr,
-                                              reinterpret_cast<int *>(base + P.o_fbc), 0, epn);
-    e = cudaGetLastError();
-    if (hook) hook(hook_ctx, "tc_escalate", false, st, 1);
-    if (e != cudaSuccess) return e;
+    pack = true;
   }
-  if (!epb) return tc_brute(P, C, d, k, Xq, Xq2, qidx, D, I, ldD, base, st, hook, hook_ctx);
-  TcCand C2 = C;
-  C2.fmt = EP.fmt;
-  C2.elem = EP.elem;
-  C2.d_pad = EP.d_pad;
-  C2.pb = epb;
-  C2.pb_lo = epb_lo;
-  C2.pn = epn;
-  char *ebase = base + P.o_esc;
-  e = tc_pass(EP, C2, epb, epb_lo, epn, nq, d, k, Xq, Xq2, nrows_q, qidx,
-              reinterpret_cast<const int *>(base + P.o_fbc),
-              reinterpret_cast<const int *>(base + P.o_fbl), D, I, ldD, ebase, status, nullptr,
-              0, nullptr, st, hook, hook_ctx, true);
+  if (!epb) return cudaSuccess;
+  const TcCand C2 = escalation_cand(C, EP, epb, epb_lo, epn);
+  *last = EPout;
+  *last_base = base + P.o_esc;
+  return tc_pass<T>(EP, C2, pack, false, nq, d, k, Xq, Xq2, nrows_q, qidx,
+                    reinterpret_cast<const int *>(base + P.o_fbc),
+                    reinterpret_cast<const int *>(base + P.o_fbl), D, I, ldD, *last_base, status,
+                    nullptr, 0, nullptr, st, hook, hook_ctx);
+}
+
+cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *Xq,
+                   const float *Xq2, long long nrows_q, const int *qidx, const float *Xc,
+                   const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,
+                   int ldD, void *ws, int *status, float *dbg, long long dbg_ld,
+                   unsigned long long *counters, cudaStream_t st, TraceHook hook,
+                   void *hook_ctx) {
+  if (P.cand_bytes == 0) return cudaErrorInvalidValue;
+  if (hook) hook(hook_ctx, "tc_pack", true, st, 0);
+  TcCand C{};
+  cudaError_t e = cand_begin<float>(&C, ws, nc, d, tc_mode_of_format(P.fmt), Xc, Xc2, nrows_c,
+                                    cidx, status, st);
+  if (hook) hook(hook_ctx, "tc_pack", false, st, 1);
   if (e != cudaSuccess) return e;
-  return tc_brute(EP, C2, d, k, Xq, Xq2, qidx, D, I, ldD, ebase, st, hook, hook_ctx);
+  const TcPlan *last;
+  char *lbase;
+  TcPlan EP;
+  e = tc_passes<float>(P, C, true, nq, d, k, Xq, Xq2, nrows_q, qidx, D, I, ldD,
+                       static_cast<char *>(ws), status, dbg, dbg_ld, counters, st, hook, hook_ctx,
+                       &last, &lbase, &EP);
+  if (e != cudaSuccess) return e;
+  return tc_brute(*last, C, d, k, Xq, Xq2, qidx, D, I, ldD, lbase, st, hook, hook_ctx);
+}
+
+cudaError_t tc_run_prepared(const TcPlan &P, const TcCand &C, int nq, int d, int k,
+                            const float *Xq, const float *Xq2, long long nrows_q,
+                            const int *qidx, float *D, int *I, int ldD, void *ws, int *status,
+                            float *dbg, long long dbg_ld, unsigned long long *counters,
+                            cudaStream_t st, TraceHook hook, void *hook_ctx) {
+  const TcPlan *last;
+  char *lbase;
+  TcPlan EP;
+  const cudaError_t e = tc_passes<float>(P, C, false, nq, d, k, Xq, Xq2, nrows_q, qidx, D, I, ldD,
+                                         static_cast<char *>(ws), status, dbg, dbg_ld, counters,
+                                         st, hook, hook_ctx, &last, &lbase, &EP);
+  if (e != cudaSuccess) return e;
+  return tc_brute(*last, C, d, k, Xq, Xq2, qidx, D, I, ldD, lbase, st, hook, hook_ctx);
 }
 
 // Escalation panels of a prepared candidate set (kept with it, e.g. a serving engine's
-// resident set): the same rows in `mode`'s format, sharing shift, norms, bounds and ids.
+// resident set): the same rows in `mode`'s format, sharing shift, norms and ids.
 cudaError_t tc_cand_prepare_escalation(TcCand *C, void *mem, int mode, int *status,
                                        cudaStream_t st) {
-  using namespace tc;
   const CandLayout L = cand_layout(C->nc, C->d, mode);
   if (L.r_pad != C->r_pad) return cudaErrorInvalidValue;
   char *b = static_cast<char *>(mem);
@@ -2296,12 +2539,14 @@ cudaError_t tc_cand_prepare_escalation(TcCand *C, void *mem, int mode, int *stat
   C->epb = b;
   C->epb_lo = L.fmt == 2 ? b + one : nullptr;
   C->epn = b + (L.fmt == 2 ? 2 * one : one);
-  tc_pack<<<tc_pack_grid(C->r_pad), 256, 0, st>>>(L.fmt, C->Xc, C->Xc2, C->d, L.d_pad,
-                                             C->nrows_c, C->cidx, C->nc, C->r_pad, C->mu, C->mu2, 1,
-                                             C->epb, C->epb_lo, nullptr, nullptr, nullptr,
-                                             nullptr, status, nullptr, nullptr, nullptr, 0,
-                                             C->epn);
-  return cudaGetLastError();
+  tc::PackSide<float> s = cand_side<float>(*C);
+  s.panel = C->epb;
+  s.panel_lo = C->epb_lo;
+  s.npanel = C->epn;
+  s.enorm = nullptr;
+  s.stats = C->estats;
+  return launch_tc_pack<float>(s, tc::PackSide<float>{}, *C, L.fmt, L.d_pad, false, 0.0f, 0.0f,
+                               0.0f, status, st);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2345,13 +2590,13 @@ TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms) {
   L.o_pb_lo = take(R * P.d_pad * 2);
   L.o_pn = take(R * NORM_ROW);
   L.o_cn = take(R * 4);
-  L.o_cnrm = take(R * 4);
   L.o_cid = take(R * 4);
   L.o_iota = take((size_t)npts * 4);
   P.o_pa = L.o_pb;  // the query panel is the candidate panel
   P.o_pa_lo = L.o_pb_lo;
   P.o_qn = L.o_cn;
-  P.o_qnrm = L.o_cnrm;
+  P.o_qe = take(R * 16);
+  P.o_qmx = take(R * 4);
   P.o_log = take((size_t)NPART * R * P.logcap * LOG_ENTRY);
   P.o_logcnt = take((size_t)NPART * R * 4);
   P.o_proot = take((size_t)NPART * R * 4);
@@ -2383,28 +2628,51 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   unsigned *stats = reinterpret_cast<unsigned *>(base + L.o_stats);
   void *pb = base + L.o_pb, *pb_lo = base + L.o_pb_lo, *pn = base + L.o_pn;
   float *cn = reinterpret_cast<float *>(base + L.o_cn);
-  float *cnrm = reinterpret_cast<float *>(base + L.o_cnrm);
   uint32_t *cid = reinterpret_cast<uint32_t *>(base + L.o_cid);
   int *iota = reinterpret_cast<int *>(base + L.o_iota);
   int *fbc = reinterpret_cast<int *>(base + P.o_fbc);
   cudaError_t e = cudaMemsetAsync(stats, 0, 16, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(fbc, 0, 16, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(base + P.o_proot, 0xFF, (size_t)NPART * rows * 4, st);
   if (e != cudaSuccess) return e;
+  TcCand C{};
+  C.d = d;
+  C.mu = mu;
+  C.mu2 = mu2;
+  C.part = reinterpret_cast<double *>(base + L.o_cpart);
+  C.part_n = reinterpret_cast<int *>(base + L.o_cpart + (size_t)CENTER_SLICES * d * 8);
   if (setup) {
     // once per workspace: the row index map, and the shift (mean of a strided sample of the
     // first panel's rows, padding skipped), which serves every later tree of the same table
     iota_kernel<<<296, 256, 0, st>>>(iota, npts);
-    double *part = reinterpret_cast<double *>(base + L.o_cpart);
-    int *part_n = reinterpret_cast<int *>(base + L.o_cpart + (size_t)CENTER_SLICES * d * 8);
-    tc_center<<<dim3((d + 31) / 32, CENTER_SLICES), 1024, 0, st>>>(
-        X, d, npts, pidx, rows, std::min(rows, 4096), part, part_n);
-    tc_center_fin<<<1, 256, 0, st>>>(part, part_n, d, mu, mu2);
+    tc_center<float><<<dim3((d + 31) / 32, CENTER_SLICES), 32 * CENTER_WARPS, 0, st>>>(
+        X, d, npts, pidx, rows, std::min(rows, CENTER_ROWS), C.part, C.part_n, nullptr, 0,
+        nullptr);
   }
-  tc_pack<<<tc_pack_grid(rows), 256, 0, st>>>(2, X, X2, d, P.d_pad, npts, pidx, rows, rows, mu, mu2,
-                                         1, pb, pb_lo, cn, cnrm, cid, stats, status, nullptr,
-                                         nullptr, nullptr, 1, pn);
-  e = cudaGetLastError();
+  // the panel's rows are candidates and queries at once
+  PackSide<float> ps{};
+  ps.X = X;
+  ps.X2 = X2;
+  ps.nrows = npts;
+  ps.idx = pidx;
+  ps.count = rows;
+  ps.rows_pad = rows;
+  ps.pad_ok = 1;
+  ps.panel = pb;
+  ps.panel_lo = pb_lo;
+  ps.npanel = pn;
+  ps.enorm = cn;
+  ps.ids = cid;
+  ps.stats = stats;
+  ps.qe = reinterpret_cast<float4 *>(base + P.o_qe);
+  ps.qmx = reinterpret_cast<float *>(base + P.o_qmx);
+  ps.Din = D;
+  ps.ldD = ldD;
+  ps.k = k;
+  ps.nroots = NPART;
+  ps.nproot = rows;
+  ps.proot = reinterpret_cast<unsigned *>(base + P.o_proot);
+  ps.zero = fbc;
+  e = launch_tc_pack<float>(PackSide<float>{}, ps, C, 2, P.d_pad, setup, P.kA, P.kB, P.kS, status,
+                            st);
   if (e != cudaSuccess) return e;
   CUtensorMap mA, mAlo, mB, mBlo;
   e = make_panel_map(&mA, pb, P.elem, P.d_pad, rows, TC_M);
@@ -2417,8 +2685,7 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   tp.N = P.N; tp.NST = P.NST; tp.logcap = P.logcap;
   tp.a_terms = P.a_terms; tp.fmt = P.fmt;
   tp.idesc = idesc_f32acc(1u, TC_M, P.N);
-  tp.cn = cn; tp.cid = cid; tp.qn = cn; tp.qnrm = cnrm; tp.stats = stats;
-  tp.Din = D; tp.ldD = ldD;
+  tp.cn = cn; tp.cid = cid; tp.qn = cn; tp.qe = ps.qe; tp.qmx = ps.qmx; tp.stats = stats;
   tp.log = reinterpret_cast<float4 *>(base + P.o_log);
   tp.logpos = reinterpret_cast<uint32_t *>(tp.log + (size_t)NPART * P.S * rows * P.logcap);
   tp.logcnt = reinterpret_cast<int *>(base + P.o_logcnt);
@@ -2433,12 +2700,13 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   tp.counters = counters;
   e = launch_tc_knn(P, pn, rows, nqt, mA, mAlo, mB, mBlo, tp, st);
   if (e != cudaSuccess) return e;
-  RerankParams rp{};
+  RerankParams<float> rp{};
   rp.Q = rows; rp.k = k; rp.S = NPART; rp.logcap = P.logcap; rp.d = d;
   rp.log = tp.log; rp.logpos = tp.logpos; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
   rp.qn = tp.qn; rp.qmul = tp.fold ? -2.0f : 1.0f;
   rp.proot = tp.proot;
-  rp.Xq = X; rp.Xq2 = X2; rp.Xc = X; rp.Xc2 = X2; rp.qidx = iota; rp.cid = cid;
+  rp.Xq = X; rp.Xq2 = X2; rp.nrows_q = npts; rp.Xc = X; rp.Xc2 = X2; rp.qidx = iota;
+  rp.cid = cid;
   rp.D = D; rp.I = I; rp.ldD = ldD;
   rp.fallback_list = reinterpret_cast<int *>(base + P.o_fbl);
   rp.fallback_count = fbc;
