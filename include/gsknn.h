@@ -153,7 +153,11 @@ void dgsknn_ref_stl(int m, int n, int k, int r, double *XA, double *XA2, int *al
 int gsknn_last_error(void);
 const char *gsknn_last_error_string(void);
 
-/* Arithmetic of the float path of sgsknn / sgsknn_var1 / gsknn_s_device:
+/* Double calls return FP64 distances in any mode. From 32,768 (query, candidate) pairs on, with
+ * k <= 256 and the 2-norm, a tensor-core pass with a rigorous error bound first narrows the
+ * candidates whose FP64 distances are formed; the results are the CUDA-core kernel's bit for bit.
+ *
+ * Arithmetic of the float path of sgsknn / sgsknn_var1 / gsknn_s_device:
  *   GSKNN_MODE_FP32 -- CUDA-core FP32 distances;
  *   GSKNN_MODE_TF32, GSKNN_MODE_BF16 -- tensor-core distances with an FP64 re-rank of every
  *     candidate within the rounding bound of the k-th distance (exact index sets);

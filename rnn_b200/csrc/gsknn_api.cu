@@ -347,6 +347,85 @@ static void trace_hook(void *, const char *name, bool begin, cudaStream_t st, in
 // ------------------------------------------------------------------------------------------
 // device pipeline: pack -> fused select -> finalize (queries = heap rows)
 // ------------------------------------------------------------------------------------------
+// Sizes and workspace of the CUDA-core pipeline (offsets from the start of its workspace).
+struct SimtPlan {
+  SimtGeom g;
+  int nkc, qtiles, rtiles, S, tps;
+  size_t oA, oB, oQN, oCN, oCI, oPD, oPI, bytes;
+};
+
+template <typename T>
+static SimtPlan simt_plan(int nq, int nc, int d, int k) {
+  SimtPlan P{};
+  P.g = simt_geometry<T>(k);
+  if (P.g.kp == 0) return P;
+  const SimtGeom &g = P.g;
+  P.nkc = (d + g.dk - 1) / g.dk;
+  P.qtiles = (nq + g.bq - 1) / g.bq;
+  P.rtiles = (nc + g.br - 1) / g.br;
+  P.S = choose_splits(P.qtiles, P.rtiles, sm_count() * std::max(1, g.minb));
+  P.tps = (P.rtiles + P.S - 1) / P.S;
+  size_t off = 0;
+  auto take = [&](size_t bytes) { size_t o = off; off = align256(off + bytes); return o; };
+  P.oA = take((size_t)P.qtiles * P.nkc * g.dk * g.bq * sizeof(T));
+  P.oB = take((size_t)P.rtiles * P.nkc * g.dk * g.br * sizeof(T));
+  P.oQN = take((size_t)P.qtiles * g.bq * sizeof(T));
+  P.oCN = take((size_t)P.rtiles * g.br * sizeof(T));
+  P.oCI = take((size_t)P.rtiles * g.br * 4);
+  P.oPD = take((size_t)P.S * nq * k * sizeof(T));
+  P.oPI = take((size_t)P.S * nq * k * 4);
+  P.bytes = off;
+  return P;
+}
+
+// The CUDA-core kernels of one call; with `rows` / `nrows` (device) only for those heap rows.
+template <typename T>
+static int simt_run(const SimtPlan &P, int nq, int nc, int d, int k, const T *Xq, const T *Xq2,
+                    long long nrows_q, const int *qidx, const T *Xc, const T *Xc2,
+                    long long nrows_c, const int *cidx, T *D, int *I, int ldD, char *base,
+                    int *status, cudaStream_t st, int metric, const int *rows = nullptr,
+                    const int *nrows = nullptr) {
+  const SimtGeom &g = P.g;
+  T *Apack = reinterpret_cast<T *>(base + P.oA);
+  T *Bpack = reinterpret_cast<T *>(base + P.oB);
+  T *qn = reinterpret_cast<T *>(base + P.oQN);
+  T *cn = reinterpret_cast<T *>(base + P.oCN);
+  uint32_t *cid = reinterpret_cast<uint32_t *>(base + P.oCI);
+  T *partD = reinterpret_cast<T *>(base + P.oPD);
+  uint32_t *partI = reinterpret_cast<uint32_t *>(base + P.oPI);
+  {
+    TraceScope ts(rows ? "tc_fallback" : "pack_panels", st);
+    CU(launch_pack<T>(Xq, Xq2, d, nrows_q, qidx, nq, g.bq, g.dk, P.nkc, Apack, qn, nullptr,
+                      status, st, nrows, rows));
+  }
+  {
+    TraceScope ts(rows ? "tc_fallback" : "pack_panels", st);
+    CU(launch_pack<T>(Xc, Xc2, d, nrows_c, cidx, nc, g.br, g.dk, P.nkc, Bpack, cn, cid, status,
+                      st, nrows));
+  }
+  SimtArgs<T> sa{};
+  sa.Apack = Apack; sa.Bpack = Bpack; sa.qn = qn; sa.cn = cn; sa.cid = cid;
+  sa.Din = D; sa.ldD = ldD; sa.Q = nq; sa.k = k; sa.nkc = P.nkc;
+  sa.ntiles_r = P.rtiles; sa.tiles_per_split = P.tps; sa.partD = partD; sa.partI = partI;
+  sa.metric = metric;
+  sa.dQ = nrows;
+  sa.rowmap = rows;
+  {
+    TraceScope ts(rows ? "tc_fallback" : "fused_knn_simt", st);
+    CU(launch_simt<T>(sa, g.kp, P.qtiles, P.S, st));
+  }
+  FinalizeArgs<T> fa{};
+  fa.Din = D; fa.Iin = I; fa.ldD = ldD; fa.Q = nq; fa.k = k; fa.S = P.S;
+  fa.partD = partD; fa.partI = partI; fa.Dout = D; fa.Iout = I;
+  fa.dQ = nrows;
+  fa.rowmap = rows;
+  {
+    TraceScope ts(rows ? "tc_fallback" : "finalize_heap", st);
+    CU(launch_finalize<T>(fa, g.kp, st));
+  }
+  return set_status(GSKNN_OK, nullptr);
+}
+
 template <typename T>
 int knn_device_simt(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, long long nrows_q,
                     const int *qidx, const T *Xc, const T *Xc2, long long nrows_c,
@@ -360,67 +439,16 @@ int knn_device_simt(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, lon
   if (!Xq || !qidx || !Xc || !cidx || !D || !I || (metric == 0 && (!Xq2 || !Xc2)))
     return set_status(GSKNN_ERR_ARG, "null pointer argument");
   if (metric) Xq2 = Xc2 = nullptr;
-  const SimtGeom g = simt_geometry<T>(k);
-  if (g.kp == 0)
+  const SimtPlan P = simt_plan<T>(nq, nc, d, k);
+  if (P.g.kp == 0)
     return set_status(GSKNN_ERR_UNSUPPORTED, "k=%d exceeds the fused kernel's list size", k);
-
-  const int nkc = (d + g.dk - 1) / g.dk;
-  const int qtiles = (nq + g.bq - 1) / g.bq;
-  const int rtiles = (nc + g.br - 1) / g.br;
-  const int S = choose_splits(qtiles, rtiles, sm_count() * std::max(1, g.minb));
-  const int tps = (rtiles + S - 1) / S;
-
-  size_t off = 0;
-  auto take = [&](size_t bytes) { size_t o = off; off = align256(off + bytes); return o; };
-  const size_t oA = take((size_t)qtiles * nkc * g.dk * g.bq * sizeof(T));
-  const size_t oB = take((size_t)rtiles * nkc * g.dk * g.br * sizeof(T));
-  const size_t oQN = take((size_t)qtiles * g.bq * sizeof(T));
-  const size_t oCN = take((size_t)rtiles * g.br * sizeof(T));
-  const size_t oCI = take((size_t)rtiles * g.br * 4);
-  const size_t oPD = take((size_t)S * nq * k * sizeof(T));
-  const size_t oPI = take((size_t)S * nq * k * 4);
   void *ws = nullptr, *stv = nullptr;
-  CU(scratch(SLOT_KERNEL, off, st, &ws));
+  CU(scratch(SLOT_KERNEL, P.bytes, st, &ws));
   CU(scratch(SLOT_STATUS, 256, st, &stv));
-  char *base = static_cast<char *>(ws);
   int *status = static_cast<int *>(stv);
   CU(cudaMemsetAsync(status, 0, sizeof(int), st));
-
-  T *Apack = reinterpret_cast<T *>(base + oA);
-  T *Bpack = reinterpret_cast<T *>(base + oB);
-  T *qn = reinterpret_cast<T *>(base + oQN);
-  T *cn = reinterpret_cast<T *>(base + oCN);
-  uint32_t *cid = reinterpret_cast<uint32_t *>(base + oCI);
-  T *partD = reinterpret_cast<T *>(base + oPD);
-  uint32_t *partI = reinterpret_cast<uint32_t *>(base + oPI);
-
-  {
-    TraceScope ts("pack_panels", st);
-    CU(launch_pack<T>(Xq, Xq2, d, nrows_q, qidx, nq, g.bq, g.dk, nkc, Apack, qn, nullptr,
-                      status, st));
-  }
-  {
-    TraceScope ts("pack_panels", st);
-    CU(launch_pack<T>(Xc, Xc2, d, nrows_c, cidx, nc, g.br, g.dk, nkc, Bpack, cn, cid, status,
-                      st));
-  }
-  SimtArgs<T> sa{};
-  sa.Apack = Apack; sa.Bpack = Bpack; sa.qn = qn; sa.cn = cn; sa.cid = cid;
-  sa.Din = D; sa.ldD = ldD; sa.Q = nq; sa.k = k; sa.nkc = nkc;
-  sa.ntiles_r = rtiles; sa.tiles_per_split = tps; sa.partD = partD; sa.partI = partI;
-  sa.metric = metric;
-  {
-    TraceScope ts("fused_knn_simt", st);
-    CU(launch_simt<T>(sa, g.kp, qtiles, S, st));
-  }
-  FinalizeArgs<T> fa{};
-  fa.Din = D; fa.Iin = I; fa.ldD = ldD; fa.Q = nq; fa.k = k; fa.S = S;
-  fa.partD = partD; fa.partI = partI; fa.Dout = D; fa.Iout = I;
-  {
-    TraceScope ts("finalize_heap", st);
-    CU(launch_finalize<T>(fa, g.kp, st));
-  }
-  return set_status(GSKNN_OK, nullptr);
+  return simt_run<T>(P, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I, ldD,
+                     static_cast<char *>(ws), status, st, metric);
 }
 
 static int g_mode = GSKNN_MODE_AUTO;
@@ -486,11 +514,8 @@ static int knn_device_tc(int mode, int nq, int nc, int d, int k, const float *Xq
   return set_status(GSKNN_OK, nullptr);
 }
 
-// The arithmetic used for a float call: explicit modes are honoured; AUTO takes the
-// tensor-core form with the exact FP64 re-rank where it fits (split BF16 below d = 128, BF16
-// from there, TF32 where neither fits), else the CUDA-core FP32 kernel.
-static int pick_mode(int nq, int nc, int d, int k) {
-  if (g_mode != GSKNN_MODE_AUTO) return g_mode;
+// The tensor-core mode AUTO takes for a shape (GSKNN_MODE_FP32: none fits).
+static int auto_mode(int nq, int nc, int d, int k) {
   // Split BF16 keeps the re-rank band narrowest (input error ~u^2): at d = 64 plain BF16's band
   // overflows the logs and most queries run again. From d = 128 one BF16 MMA per product was
   // measured fastest (d = 256: 10.8 ms against 13.9 ms in split BF16 for 32,768 x 262,144,
@@ -499,6 +524,45 @@ static int pick_mode(int nq, int nc, int d, int k) {
   if (tc_plan(nq, nc, d, k, GSKNN_TC_BF16X3, sm_count()).ok) return GSKNN_TC_BF16X3;
   if (tc_plan(nq, nc, d, k, GSKNN_TC_TF32, sm_count()).ok) return GSKNN_TC_TF32;
   return GSKNN_MODE_FP32;
+}
+
+// The arithmetic used for a float call: explicit modes are honoured; AUTO takes the
+// tensor-core form with the exact FP64 re-rank where it fits (split BF16 below d = 128, BF16
+// from there, TF32 where neither fits), else the CUDA-core FP32 kernel.
+static int pick_mode(int nq, int nc, int d, int k) {
+  return g_mode != GSKNN_MODE_AUTO ? g_mode : auto_mode(nq, nc, d, k);
+}
+
+// A double call through the tensor cores: approximate distances with a rigorous bound, exact FP64
+// distances of the band in the CUDA-core kernel's own order of operations, so the results are the
+// same bits. Queries that the passes could not bound (their band overflows in the narrowest
+// format; values beyond the floats' range; NaN) run through the CUDA-core kernels, which are
+// launched behind them over the list of such rows, mostly empty. Returns -1 when the form does not
+// apply (shared memory, k) or its scratch cannot be had: the caller takes the CUDA cores.
+static int knn_device_tc_double(int nq, int nc, int d, int k, const double *Xq, const double *Xq2,
+                                long long nrows_q, const int *qidx, const double *Xc,
+                                const double *Xc2, long long nrows_c, const int *cidx, double *D,
+                                int *I, int ldD, cudaStream_t st) {
+  if (nq <= 0 || nc <= 0 || d <= 0 || k <= 0 || ldD < k || !Xq || !Xq2 || !qidx || !Xc || !Xc2 ||
+      !cidx || !D || !I)
+    return -1;  // (the CUDA-core path reports)
+  const int mode = auto_mode(nq, nc, d, k);
+  if (mode == GSKNN_MODE_FP32) return -1;
+  const TcPlan P = tc_plan(nq, nc, d, k, mode, sm_count());
+  const SimtPlan F = simt_plan<double>(nq, nc, d, k);
+  if (!P.ok || F.g.kp == 0) return -1;
+  void *ws = nullptr, *stv = nullptr;
+  const size_t simt_off = align256(P.bytes);
+  const cudaError_t se = scratch(SLOT_KERNEL, simt_off + F.bytes, st, &ws);
+  if (se == cudaErrorMemoryAllocation) return -1;
+  CU(se);
+  CU(scratch(SLOT_STATUS, 256, st, &stv));
+  int *status = static_cast<int *>(stv);  // cleared by the first kernel
+  const int *left = nullptr, *nleft = nullptr;
+  CU(tc_run_double(P, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I, ldD, ws,
+                   status, &left, &nleft, st, trace_hook, nullptr));
+  return simt_run<double>(F, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I,
+                          ldD, static_cast<char *>(ws) + simt_off, status, st, 0, left, nleft);
 }
 
 template <typename T>
@@ -553,6 +617,17 @@ int knn_device(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, long lon
   if (simt_geometry<T>(k).kp == 0)
     return knn_device_large<T>(nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D,
                                I, ldD, 0, st);
+  if constexpr (std::is_same<T, double>::value) {
+    // From 32,768 pairs on the tensor-core form is the faster one (B200, us, CUDA cores -> tensor
+    // cores: 1 x 300, d = 3 91 -> 103; 16 x 4,096, d = 32 136 -> 113; 4,096 x 4,096, d = 32
+    // 426 -> 130; 1,000 x 20,000, k = 200 1,928 -> 476; 5,003 x 50,021, d = 100, k = 50
+    // 7,853 -> 565; 8,192 x 65,536, d = 3 2,584 -> 357).
+    if ((long long)nq * nc >= 32768) {
+      const int rc = knn_device_tc_double(nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c,
+                                          cidx, D, I, ldD, st);
+      if (rc != -1) return rc;
+    }
+  }
   return knn_device_simt<T>(nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I,
                             ldD, st);
 }

@@ -44,6 +44,10 @@ struct SimtArgs {
   T *partD;              // [S][Q][k] sorted ascending
   uint32_t *partI;
   int metric;            // 0: squared 2-norm, 1: 1-norm
+  // optional: only the heap rows rowmap[0 .. *dQ) (device; Q stays the stride of the lists), whose
+  // panels hold them in that order
+  const int *dQ;
+  const int *rowmap;
 };
 
 template <typename T>
@@ -56,12 +60,15 @@ struct FinalizeArgs {
   const uint32_t *partI;
   T *Dout;
   int *Iout;
+  const int *dQ;         // optional, as in SimtArgs
+  const int *rowmap;
 };
 
 template <typename T>
 cudaError_t launch_pack(const T *X, const T *X2, int d, long long nrows, const int *idx,
                         int count, int BT, int DK, int nkc, T *P, T *norms, uint32_t *ids,
-                        int *status, cudaStream_t st);
+                        int *status, cudaStream_t st, const int *dcount = nullptr,
+                        const int *rowmap = nullptr);
 template <typename T>
 SimtGeom simt_geometry(int k);
 template <typename T>
@@ -185,6 +192,16 @@ cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *X
                    int ldD, void *ws, int *status, float *dbg, long long dbg_ld,
                    unsigned long long *counters, cudaStream_t st, TraceHook hook,
                    void *hook_ctx);
+// The same for double tables: the approximate pass runs on the centred rows rounded to the MMA
+// format, the re-rank on the double rows, in the CUDA-core kernel's order of operations. Queries
+// that neither it nor the escalation could bound are left: their heap rows at *left, their number
+// at *nleft (both on the device).
+cudaError_t tc_run_double(const TcPlan &P, int nq, int nc, int d, int k, const double *Xq,
+                          const double *Xq2, long long nrows_q, const int *qidx,
+                          const double *Xc, const double *Xc2, long long nrows_c,
+                          const int *cidx, double *D, int *I, int ldD, void *ws, int *status,
+                          const int **left, const int **nleft, cudaStream_t st, TraceHook hook,
+                          void *hook_ctx);
 // Tensor-core form of the batching pass (all-NN within randomized-tree leaves): one tree's
 // leaves laid out in a panel, each leaf padded to whole candidate tiles; every query tile runs
 // against its own leaf's tiles only, and the exact re-rank merges into the heap rows in place,

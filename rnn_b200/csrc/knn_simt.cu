@@ -33,18 +33,24 @@ template <typename T>
 __global__ void __launch_bounds__(256) pack_panels(
     const T *__restrict__ X, const T *__restrict__ X2, int d, long long nrows,
     const int *__restrict__ idx, int count, int BT, int DK, int nkc, T *__restrict__ P,
-    T *__restrict__ norms, uint32_t *__restrict__ ids, int *__restrict__ status) {
+    T *__restrict__ norms, uint32_t *__restrict__ ids, int *__restrict__ status,
+    const int *__restrict__ dcount, const int *__restrict__ rowmap) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *s = reinterpret_cast<T *>(smem_raw);  // [DK][BT + 1]
   const int tile = blockIdx.x / nkc;
   const int kc = blockIdx.x % nkc;
   const int tid = threadIdx.x;
+  if (dcount) {
+    const int n = *dcount;  // rows of the row map; without one, all rows if there are any
+    if (n == 0 || (rowmap && tile * BT >= n)) return;
+    if (rowmap) count = n;
+  }
   for (int e = tid; e < BT * DK; e += blockDim.x) {
     const int r = e / DK, p = e % DK;
     const int gr = tile * BT + r, gp = kc * DK + p;
     T v = T(0);
     if (gr < count && gp < d) {
-      const long long row = idx[gr];
+      const long long row = idx[rowmap ? rowmap[gr] : gr];
       if (row >= 0 && row < nrows) v = X[row * d + gp];
     }
     s[p * (BT + 1) + r] = v;
@@ -61,7 +67,7 @@ __global__ void __launch_bounds__(256) pack_panels(
       T nv = Num<T>::nan();
       uint32_t id = NO_ID;
       if (gr < count) {
-        const long long row = idx[gr];
+        const long long row = idx[rowmap ? rowmap[gr] : gr];
         if (row >= 0 && row < nrows) {
           nv = X2 ? X2[row] : T(0);
           id = (uint32_t)row;
@@ -85,6 +91,8 @@ __global__ void __launch_bounds__(C::NTHR, C::MINB) fused_knn_simt(SimtArgs<type
   extern __shared__ __align__(128) unsigned char smem[];
   const int qt = blockIdx.x, split = blockIdx.y;
   const int q0 = qt * C::BQ;
+  const int Q = a.dQ ? *a.dQ : a.Q;
+  if (q0 >= Q) return;
   SimtBlock<T> b;
   b.Apan = a.Apack + (size_t)qt * a.nkc * C::DK * C::BQ;
   b.Bpack = a.Bpack;
@@ -96,8 +104,8 @@ __global__ void __launch_bounds__(C::NTHR, C::MINB) fused_knn_simt(SimtArgs<type
   b.t_begin = split * a.tiles_per_split;
   b.t_end = b.t_begin + a.tiles_per_split;
   if (b.t_end > a.ntiles_r) b.t_end = a.ntiles_r;
-  b.nrows = a.Q - q0 < C::BQ ? a.Q - q0 : C::BQ;
-  b.rowid = nullptr;
+  b.nrows = Q - q0 < C::BQ ? Q - q0 : C::BQ;
+  b.rowid = a.rowmap ? reinterpret_cast<const uint32_t *>(a.rowmap) + q0 : nullptr;
   b.row0 = q0;
   b.Din = a.Din;
   b.ldD = a.ldD;
@@ -113,8 +121,9 @@ __global__ void __launch_bounds__(C::NTHR, C::MINB) fused_knn_simt(SimtArgs<type
 template <typename T, int E>
 __global__ void __launch_bounds__(256) finalize_heap(FinalizeArgs<T> a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q = blockIdx.x * 8 + warp;
-  if (q >= a.Q) return;
+  const int i = blockIdx.x * 8 + warp;
+  if (i >= (a.dQ ? *a.dQ : a.Q)) return;
+  const int q = a.rowmap ? a.rowmap[i] : i;
   const int k = a.k;
   T ld[E];
   uint32_t li[E];
@@ -158,12 +167,12 @@ __global__ void __launch_bounds__(256) finalize_heap(FinalizeArgs<T> a) {
 template <typename T>
 cudaError_t launch_pack(const T *X, const T *X2, int d, long long nrows, const int *idx,
                         int count, int BT, int DK, int nkc, T *P, T *norms, uint32_t *ids,
-                        int *status, cudaStream_t st) {
+                        int *status, cudaStream_t st, const int *dcount, const int *rowmap) {
   const int ntiles = (count + BT - 1) / BT;
   if (ntiles == 0) return cudaSuccess;
   const size_t sm = (size_t)DK * (BT + 1) * sizeof(T);
   pack_panels<T><<<ntiles * nkc, 256, sm, st>>>(X, X2, d, nrows, idx, count, BT, DK, nkc, P,
-                                                norms, ids, status);
+                                                norms, ids, status, dcount, rowmap);
   return cudaGetLastError();
 }
 
@@ -244,7 +253,7 @@ cudaError_t launch_finalize(const FinalizeArgs<T> &a, int kp, cudaStream_t st) {
 #define GSKNN_INST(T)                                                                       \
   template cudaError_t launch_pack<T>(const T *, const T *, int, long long, const int *, int, \
                                       int, int, int, T *, T *, uint32_t *, int *,           \
-                                      cudaStream_t);                                        \
+                                      cudaStream_t, const int *, const int *);                                        \
   template SimtGeom simt_geometry<T>(int);                                                  \
   template cudaError_t launch_simt<T>(const SimtArgs<T> &, int, int, int, cudaStream_t);    \
   template cudaError_t launch_finalize<T>(const FinalizeArgs<T> &, int, cudaStream_t);

@@ -2,7 +2,9 @@
 // BF16 or split BF16 (hi*hi + hi*lo + lo*hi), with FP32 accumulation in TMEM, followed by an
 // FP64 re-rank of every candidate whose approximate distance lies within a rigorous rounding
 // bound of the query's k-th approximate distance. The result is the exact FP64 top-k (ties to
-// the lower id) of the caller's float inputs, merged into the caller's heaps.
+// the lower id) of the caller's inputs, merged into the caller's heaps. Tables are float or double:
+// double rows are centred in FP64 before they are rounded to the MMA format, and rows that leave
+// the floats' range go back to the caller's CUDA-core path.
 //
 // Kernels (one call):
 //   tc_center     partial sums of the shift vector mu = mean of a strided sample of candidate rows
@@ -388,7 +390,9 @@ __global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
       if (s.qe) {
         const float eM = 2.5f * (res + g.kA * nrm) + 2.0f * g.kB * nrm;
         const float eR = g.fmt == 2 ? 0.0f : 2.5f * (nrm + res);
-        s.qe[r] = make_float4(eM, eR, g.kB * fabsf(enf) + g.kS * scale, 0.0f);
+        // (double rows: distances under 1e-30 are left to FP64, floats cannot bound them)
+        const float e0 = g.kB * fabsf(enf) + g.kS * scale + (sizeof(T) == 8 ? 1e-30f : 0.0f);
+        s.qe[r] = make_float4(eM, eR, e0, 0.0f);
         s.qmx[r] = qmx;
       }
       if (s.stats && row >= 0) {
@@ -535,7 +539,8 @@ struct EpiState {
 // this part's and the others' bounds the query's k-th smallest approximate distance from above.
 __device__ __forceinline__ void refresh_threshold(EpiState &s) {
   static_assert(NPART == 2, "the bound takes the NPART-th smallest root");
-  float t = fminf(fmaxf(s.root, s.o1), s.o2) + s.E2;
+  // (exact distances are clamped at 0: a k-th bound below it admits every clamped candidate too)
+  float t = fmaxf(fminf(fmaxf(s.root, s.o1), s.o2), 0.0f) + s.E2;
   s.thr = t < s.thr0 ? t : s.thr0;
   // padding rows past the last query never admit; nor does a row whose log overflowed (the
   // query is finished by a later pass), so its chunks stop taking the slow path
@@ -1510,7 +1515,7 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
       base += 32;
     }
     __syncwarp();
-    if (n > 32 && n >= k) T = fminf(T, list_bound(sm.list, n, k, lane));
+    if (n > 32 && n >= k) T = fminf(T, fmaxf(list_bound(sm.list, n, k, lane), 0.0f));
     thr = band_thr(T, E2, lim);
     const float split = n > 32 ? T : Num<float>::inf();  // one batch takes a short list whole
     if (!done) {
@@ -1714,7 +1719,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
   }
   if (n > 32 && n >= k) {
     if (warp == 0) {
-      const float T = fminf(s_T, list_bound(list, n, k, lane));
+      const float T = fminf(s_T, fmaxf(list_bound(list, n, k, lane), 0.0f));
       if (lane == 0) s_thr = band_thr(T, E2, thr);
     }
     __syncthreads();
@@ -2489,27 +2494,59 @@ static cudaError_t tc_passes(const TcPlan &P, const TcCand &C, bool per_call, in
                     nullptr, 0, nullptr, st, hook, hook_ctx);
 }
 
+// The per-call passes: candidates prepared in the workspace, then tc_passes.
+template <typename T>
+static cudaError_t tc_call(const TcPlan &P, TcCand *C, int nq, int nc, int d, int k, const T *Xq,
+                           const T *Xq2, long long nrows_q, const int *qidx, const T *Xc,
+                           const T *Xc2, long long nrows_c, const int *cidx, T *D, int *I, int ldD,
+                           void *ws, int *status, float *dbg, long long dbg_ld,
+                           unsigned long long *counters, cudaStream_t st, TraceHook hook,
+                           void *hook_ctx, const TcPlan **last, char **last_base, TcPlan *EP) {
+  if (P.cand_bytes == 0) return cudaErrorInvalidValue;
+  if (hook) hook(hook_ctx, "tc_pack", true, st, 0);
+  const cudaError_t e = cand_begin<T>(C, ws, nc, d, tc_mode_of_format(P.fmt), Xc, Xc2, nrows_c,
+                                      cidx, status, st);
+  if (hook) hook(hook_ctx, "tc_pack", false, st, 1);
+  if (e != cudaSuccess) return e;
+  return tc_passes<T>(P, *C, true, nq, d, k, Xq, Xq2, nrows_q, qidx, D, I, ldD,
+                      static_cast<char *>(ws), status, dbg, dbg_ld, counters, st, hook, hook_ctx,
+                      last, last_base, EP);
+}
+
 cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *Xq,
                    const float *Xq2, long long nrows_q, const int *qidx, const float *Xc,
                    const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,
                    int ldD, void *ws, int *status, float *dbg, long long dbg_ld,
                    unsigned long long *counters, cudaStream_t st, TraceHook hook,
                    void *hook_ctx) {
-  if (P.cand_bytes == 0) return cudaErrorInvalidValue;
-  if (hook) hook(hook_ctx, "tc_pack", true, st, 0);
   TcCand C{};
-  cudaError_t e = cand_begin<float>(&C, ws, nc, d, tc_mode_of_format(P.fmt), Xc, Xc2, nrows_c,
-                                    cidx, status, st);
-  if (hook) hook(hook_ctx, "tc_pack", false, st, 1);
-  if (e != cudaSuccess) return e;
   const TcPlan *last;
   char *lbase;
   TcPlan EP;
-  e = tc_passes<float>(P, C, true, nq, d, k, Xq, Xq2, nrows_q, qidx, D, I, ldD,
-                       static_cast<char *>(ws), status, dbg, dbg_ld, counters, st, hook, hook_ctx,
-                       &last, &lbase, &EP);
+  const cudaError_t e = tc_call<float>(P, &C, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2,
+                                       nrows_c, cidx, D, I, ldD, ws, status, dbg, dbg_ld, counters,
+                                       st, hook, hook_ctx, &last, &lbase, &EP);
   if (e != cudaSuccess) return e;
   return tc_brute(*last, C, d, k, Xq, Xq2, qidx, D, I, ldD, lbase, st, hook, hook_ctx);
+}
+
+cudaError_t tc_run_double(const TcPlan &P, int nq, int nc, int d, int k, const double *Xq,
+                          const double *Xq2, long long nrows_q, const int *qidx,
+                          const double *Xc, const double *Xc2, long long nrows_c,
+                          const int *cidx, double *D, int *I, int ldD, void *ws, int *status,
+                          const int **left, const int **nleft, cudaStream_t st, TraceHook hook,
+                          void *hook_ctx) {
+  TcCand C{};
+  const TcPlan *last;
+  char *lbase;
+  TcPlan EP;
+  const cudaError_t e = tc_call<double>(P, &C, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2,
+                                        nrows_c, cidx, D, I, ldD, ws, status, nullptr, 0, nullptr,
+                                        st, hook, hook_ctx, &last, &lbase, &EP);
+  if (e != cudaSuccess) return e;
+  *left = reinterpret_cast<const int *>(lbase + last->o_fbl);
+  *nleft = reinterpret_cast<const int *>(lbase + last->o_fbc);
+  return cudaSuccess;
 }
 
 cudaError_t tc_run_prepared(const TcPlan &P, const TcCand &C, int nq, int d, int k,
