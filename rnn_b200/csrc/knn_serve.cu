@@ -459,9 +459,6 @@ static void completion_loop(Engine *E) {
   }
 }
 
-// Rows per batch that keep one batch near 3 ms of tensor work on one B200: the exact forms
-// measured about 1.5e12 evals/s at d = 64 and 8.6e11 at d = 128, i.e. about 3e11 eval-dims per
-// 3 ms. Whole query tiles (128 rows), at least one, at most max_batch_queries.
 // The resident set's escalation panels as a main-format candidate set of their own.
 static gsknn::TcCand escalation_as_main(const gsknn::TcCand &C, int esc_mode) {
   gsknn::TcCand S = C;
@@ -478,13 +475,24 @@ static gsknn::TcCand escalation_as_main(const gsknn::TcCand &C, int esc_mode) {
   return S;
 }
 
-// Times one probe batch (the first min(max_q, 1024) resident points as queries, k = max_k) in
-// the prepared mode with escalation and in the escalation mode alone; keeps the faster (second
-// of two runs each, on slot 0's buffers). Returns false when a probe call fails.
+// Rows per batch that keep one batch near 3 ms of tensor work on one B200: the exact forms
+// measured about 2.6e12 evals/s at d = 64 and 2.0e12 at d = 128, i.e. 5e11 to 7.7e11 eval-dims
+// per 3 ms. Whole query tiles (128 rows), at least one, at most max_batch_queries.
+static int auto_slice(const Engine *E) {
+  const double rows = 5.0e11 / ((double)E->nref * (double)E->d);
+  int s = (int)(rows / 128.0) * 128;
+  return std::min(E->max_q, std::max(128, s));
+}
+
+// Times one probe batch (the first resident points as queries, as many as a batch of requests
+// holds but at most 2,048, k = max_k) in the prepared mode with escalation and in the escalation mode alone; keeps
+// the faster (second of two runs each, on slot 0's buffers). Returns false when a probe call fails.
+// (Probes of 1,024 rows took the two forms to be level where batches of 2,176 ran 1.4 times
+// faster in BF16: 1,048,576 x 128, 5.4 against 7.7 ms for 9,753 mixed rows.)
 static bool probe_modes(Engine *E, int esc) {
   using namespace gsknn;
   gs::Slot &s = E->slots[0];
-  const int rows = std::min(E->max_q, 1024), kb = E->max_k;
+  const int rows = std::min(auto_slice(E), 2048), kb = E->max_k;
   const TcCand Cesc = escalation_as_main(E->C, esc);
   const int modes[2] = {E->mode, esc};
   const TcCand *cands[2] = {&E->C, &Cesc};
@@ -523,11 +531,6 @@ static bool probe_modes(Engine *E, int esc) {
   return ok;
 }
 
-static int auto_slice(const Engine *E) {
-  const double rows = 3.0e11 / ((double)E->nref * (double)E->d);
-  int s = (int)(rows / 128.0) * 128;
-  return std::min(E->max_q, std::max(128, s));
-}
 
 extern "C" {
 

@@ -60,8 +60,6 @@ constexpr int A_CHUNK = TC_M * CHUNK_BYTES;  // 16 KB
 constexpr int NEPI = TC_EPI_WARPS;
 constexpr int NPART = TC_EPI_PARTS;
 constexpr int NTHREADS = 32 * (2 + NEPI);
-// accumulator columns per TMEM wait: 64 (two loads) while the registers allow, else 32
-constexpr int EPI_STEP = NPART <= 2 ? 64 : 32;
 constexpr uint32_t LOG_OVF = 1u << 30;
 constexpr size_t LOG_ENTRY = sizeof(float4) + sizeof(uint32_t);  // a logged quad and its position
 // The epilogue frees a TMEM accumulator as soon as its reads have landed, while it still uses
@@ -561,14 +559,15 @@ __device__ __forceinline__ void refresh_threshold(EpiState &s) {
 // a'[i] = min(max(a[i-1], x), a[i]) for every i at once, and the block's largest moves on to the
 // next block. A binary heap's sift-down is a chain of shared-memory round trips per value (7,700
 // cycles a flush at hk = 16); this is arithmetic without one.
-__device__ __forceinline__ void list_insert(float *list, int row, int hk, float (&x)[INSERT_BATCH]) {
+template <int NB>
+__device__ __forceinline__ void list_insert(float *list, int row, int hk, float (&x)[NB]) {
   for (int b = 0; b < hk; b += LIST_BLOCK) {
     float a[LIST_BLOCK];
     float *const blk = list + b * TC_M + row;
 #pragma unroll
     for (int i = 0; i < LIST_BLOCK; i++) a[i] = blk[i * TC_M];
 #pragma unroll
-    for (int j = 0; j < INSERT_BATCH; j++) {
+    for (int j = 0; j < NB; j++) {
       const float v = x[j];
       x[j] = fmaxf(a[LIST_BLOCK - 1], v);  // moves on to the next block
 #pragma unroll
@@ -596,6 +595,34 @@ __device__ __forceinline__ float epi_dist(float x, float qn) {
   return FOLD ? fmaf(-2.0f, x, qn) : x + qn;
 }
 
+// Publish the list's root to the other partitions and tighten the threshold.
+__device__ __forceinline__ void epi_publish(EpiState &s, const float *heap, int row, int hk,
+                                            unsigned *pslot) {
+  s.root = heap[(hk - 1) * TC_M + row];
+  // published as non-negative float bits (a larger value bounds as well), which order like
+  // unsigned integers; only this partition writes its slot
+  const float pv = fmaxf(s.root, 0.0f);
+  if (pv < s.pub) {
+    __stcg(pslot, __float_as_uint(pv));
+    s.pub = pv;
+  }
+  refresh_threshold(s);
+}
+
+// Offer a chunk's eight quads to the row's list, by their extreme values.
+template <bool FOLD>
+__device__ __forceinline__ void epi_offer(const EpiState &s, float *heap, int row, int hk,
+                                          const float (&g)[8]) {
+  float x[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    x[j] = epi_dist<FOLD>(g[j], s.qn);
+    // padding columns; and padding rows, whose published root would be query 0's
+    if (!(x[j] < Num<float>::inf()) || s.thr0 == -Num<float>::inf()) x[j] = Num<float>::inf();
+  }
+  list_insert(heap, row, hk, x);
+}
+
 // Offer the quads logged since the last flush to the row's list, by their extreme values in the
 // ring (all lanes of the warp together), publish the new root to the other partitions and tighten
 // the threshold. (Reading the quads back from their log instead costs a round trip to L2 per
@@ -612,16 +639,8 @@ __device__ __forceinline__ void epi_flush(EpiState &s, float *heap, const float 
       x[j] = e + j < np ? epi_dist<FOLD>(ring[(e + j) * TC_M + row], s.qn) : Num<float>::inf();
     list_insert(heap, row, hk, x);
   }
-  s.root = heap[(hk - 1) * TC_M + row];
   s.done = s.cnt;
-  // published as non-negative float bits (a larger value bounds as well), which order like
-  // unsigned integers; only this partition writes its slot
-  const float pv = fmaxf(s.root, 0.0f);
-  if (pv < s.pub) {
-    __stcg(pslot, __float_as_uint(pv));
-    s.pub = pv;
-  }
-  refresh_threshold(s);
+  epi_publish(s, heap, row, hk, pslot);
 }
 
 // Drops log entries above the current threshold (all of them already offered to the heap);
@@ -939,7 +958,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // d = 64, k = 32 8,283 -> 5,853 us; 32,768 x 262,144, d = 256, k = 64 6,790 -> 4,466 us;
     // 2,003 x 30,011, d = 20 105 -> 64 us; 16 x 4,096 42 -> 10 us; 8 trees over 262,144 points
     // 6.1 -> 3.1 ms.
-    auto slow = [&](const uint32_t (&r)[32], const float (&g)[8], uint32_t pos) {
+    auto slow = [&](const uint32_t (&r)[32], const float (&g)[8], uint32_t pos, bool offered) {
       // (a compaction that frees less than half of the log marks it overflowed: repeated
       // compactions that each free a few entries would cost a full read of the log per chunk)
       if (__any_sync(FULL_MASK, s.cnt > p.logcap - 8)) {
@@ -984,6 +1003,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 "r"(r[4 * j + 2]), "r"(r[4 * j + 3]), "l"(pt), "r"(pos + 4 * j), "r"(rp)
               : "memory");
       }
+      if (offered) s.done = s.cnt;  // the lists have these already
       if (__any_sync(FULL_MASK, s.cnt - s.done >= FLUSH_AT))
         epi_flush<FOLD>(s, myheap, myring, row, p.hk, pslot);
     };
@@ -1017,6 +1037,26 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       return u == 0xFFFFFFFFu ? Num<float>::inf() : __uint_as_float(u);
     };
     load_window();
+    // the other part of this lane quarter (same rows, other columns) keeps its list in shared
+    // memory: its root is read directly (one 4-byte word, written whole)
+    auto other_root = [&]() {
+      return *reinterpret_cast<volatile const float *>(&otherheap[(p.hk - 1) * TC_M + row]);
+    };
+    // the two smallest roots among the other partitions, and the threshold they give
+    auto look_around = [&]() {
+      unsigned win1, win2;
+      read_window(win1, win2);
+      const float a = other_root(), w1 = as_bound(win1), w2 = as_bound(win2);
+      const float o1 = fminf(a, w1), o2 = fminf(fmaxf(a, w1), w2);
+      if (o1 < s.o1 || o2 < s.o2) {
+        s.o1 = fminf(s.o1, o1);
+        s.o2 = fminf(s.o2, o2);
+        refresh_threshold(s);
+      }
+    };
+    // rows with no bound yet, and lists that the first tile's quads fill
+    bool first = p.hk <= N / NPART / 4 &&
+                 __any_sync(FULL_MASK, valid && !(s.thr0 < Num<float>::inf()));
     const long long t_start = p.counters ? clock64() : 0;
     long long w_tfull = 0;
     for (int lt = 0; lt < ntile && !failed; lt++) {
@@ -1025,21 +1065,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // (every tile while the bound still falls fast, then every fourth: the update takes about
       // 420 of a tile's 3,000 cycles)
       const bool look = lt < 16 || (lt & 3) == 0;
-      if (valid && look) {
-        unsigned win1, win2;
-        read_window(win1, win2);
-        // the other part of this lane quarter (same rows, other columns) keeps its list in
-        // shared memory: its root is read directly (one 4-byte word, written whole)
-        const float a =
-            *reinterpret_cast<volatile const float *>(&otherheap[(p.hk - 1) * TC_M + row]);
-        const float w1 = as_bound(win1), w2 = as_bound(win2);
-        const float o1 = fminf(a, w1), o2 = fminf(fmaxf(a, w1), w2);
-        if (o1 < s.o1 || o2 < s.o2) {
-          s.o1 = fminf(s.o1, o1);
-          s.o2 = fminf(s.o2, o2);
-          refresh_threshold(s);
-        }
-      }
+      if (valid && look) look_around();
       if (look) load_window();
       const long long t0 = p.counters ? clock64() : 0;
       if (!mbar_wait(&tfull[b], use & 1u)) { failed = true; break; }
@@ -1050,9 +1076,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const float *cnt = cn_s + c * N;
       const int tile = t_begin + lt;
       const size_t cbase = (size_t)tile * N;
-      // this warp's N/NPART columns, EPI_STEP at a time (one or two 32-column chunks per TMEM
-      // wait); the accumulator is freed for the MMA warp once the tile's last loads of every
-      // epilogue warp have landed (the norms stay in their own slot)
+      // this warp's N/NPART columns, 64 at a time (two 32-column chunks per TMEM wait); the
+      // accumulator is freed for the MMA warp once the tile's last loads of every epilogue warp
+      // have landed (the norms stay in their own slot)
       const int cb = part * (N / NPART), ce = cb + N / NPART;
       if (!p.dbg && __all_sync(FULL_MASK, !valid || s.ovf)) {
         // every row of this warp is padding or finished by a later pass: release the
@@ -1063,45 +1089,54 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (lane == 0) mbar_arrive(&tempty[b]);
         continue;
       }
-      for (int c0 = cb; c0 < ce; c0 += EPI_STEP) {
-        if constexpr (EPI_STEP == 64) {
-          uint32_t ra[32], rb[32];
-          __syncwarp();
-          tmem_ld32(taddr + (uint32_t)c0, ra);
-          tmem_ld32(taddr + (uint32_t)c0 + 32u, rb);
-          tmem_wait_ld();
-          reg_fence32(ra);
-          reg_fence32(rb);
-          if (c0 + 64 >= ce) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[b]);
-          }
-          float ga[8], gb[8];
-          const float ma = fast(ra, ga, cnt, c0);
-          const float mb = fast(rb, gb, cnt, c0 + 32);
-          if (p.dbg && valid) {
-            dbg_write(ra, cbase, c0);
-            dbg_write(rb, cbase, c0 + 32);
-          }
-          if (__any_sync(FULL_MASK, hit(ma))) slow(ra, ga, (uint32_t)(cbase + c0));
-          if (__any_sync(FULL_MASK, hit(mb))) slow(rb, gb, (uint32_t)(cbase + c0 + 32));
-        } else {
+      // The first tile of rows without an incoming bound is read twice: once to offer its quads'
+      // extreme values to the lists, then to log what lies under the bound that gives. Logging as
+      // the lists fill took most of a short split's time: every lane stores every quad, 32 lines
+      // per store (2,003 x 30,011, d = 20, nine splits: 882 -> 395 quads a query, 66 -> 54 us).
+      const bool warm = first;
+      if (warm) {
+        first = false;
+        for (int c0 = cb; c0 < ce; c0 += 32) {
           uint32_t ra[32];
           __syncwarp();
           tmem_ld32(taddr + (uint32_t)c0, ra);
           tmem_wait_ld();
           reg_fence32(ra);
-          if (c0 + 32 >= ce) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[b]);
-          }
           float ga[8];
-          const float ma = fast(ra, ga, cnt, c0);
-          if (p.dbg && valid) dbg_write(ra, cbase, c0);
-          if (__any_sync(FULL_MASK, hit(ma))) slow(ra, ga, (uint32_t)(cbase + c0));
+          fast(ra, ga, cnt, c0);
+          epi_offer<FOLD>(s, myheap, row, p.hk, ga);
         }
+        epi_publish(s, myheap, row, p.hk, pslot);
+        // the other part fills its list at the same time: give it a moment
+        for (int i = 0; i < 64; i++) {
+          const bool there = other_root() < Num<float>::inf();
+          if (__all_sync(FULL_MASK, !valid || there)) break;
+          __nanosleep(32);
+        }
+        if (valid) look_around();
+      }
+      for (int c0 = cb; c0 < ce; c0 += 64) {
+        uint32_t ra[32], rb[32];
+        __syncwarp();
+        tmem_ld32(taddr + (uint32_t)c0, ra);
+        tmem_ld32(taddr + (uint32_t)c0 + 32u, rb);
+        tmem_wait_ld();
+        reg_fence32(ra);
+        reg_fence32(rb);
+        if (c0 + 64 >= ce) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty[b]);
+        }
+        float ga[8], gb[8];
+        const float ma = fast(ra, ga, cnt, c0);
+        const float mb = fast(rb, gb, cnt, c0 + 32);
+        if (p.dbg && valid) {
+          dbg_write(ra, cbase, c0);
+          dbg_write(rb, cbase, c0 + 32);
+        }
+        if (__any_sync(FULL_MASK, hit(ma))) slow(ra, ga, (uint32_t)(cbase + c0), warm);
+        if (__any_sync(FULL_MASK, hit(mb))) slow(rb, gb, (uint32_t)(cbase + c0 + 32), warm);
       }
     }
     epi_flush<FOLD>(s, myheap, myring, row, p.hk, pslot);
