@@ -1182,6 +1182,7 @@ struct RerankParams {
   const uint32_t *logpos;   // packed position of each quad's first candidate
   const int *logcnt;
   const float *qn;
+  const float *qmx;  // largest incoming distance of each query's heap row (tc_pack)
   float qmul;
   const unsigned *proot;  // partition roots of tc_knn ([query][S]; S counts NPART per split)
   const float *margin;
@@ -1283,15 +1284,28 @@ __device__ __forceinline__ double exact_dist_lane(const float *q, const float *c
   return exact_dist(dot_lane(q, c, d), cc, qq);
 }
 
+// Order-preserving integer image of a double (-0 as 0, NaN last): the lists are sorted and merged
+// by it, since a 64-bit integer comparison is two ALU instructions and an FP64 one goes through
+// the narrow FP64 pipe.
+typedef unsigned long long Ord;
+constexpr Ord ORD_INF = 0xFFF0000000000000ull;  // image of +inf
+__device__ __forceinline__ Ord to_ord(double x) {
+  const Ord b = (Ord)__double_as_longlong(x + 0.0);
+  return (b >> 63) ? (x != x ? ~0ull : ~b) : b | 0x8000000000000000ull;
+}
+__device__ __forceinline__ double from_ord(Ord o) {
+  return __longlong_as_double((long long)((o >> 63) ? o & 0x7FFFFFFFFFFFFFFFull : ~o));
+}
+
 template <typename T, int E>
 __device__ __forceinline__ void write_heap_row(T *D, int *I, int ldD, int q, int k,
-                                               const double (&ld)[E], const uint32_t (&li)[E],
+                                               const Ord (&ld)[E], const uint32_t (&li)[E],
                                                int lane) {
 #pragma unroll
   for (int e = 0; e < E; e++) {
     const int t = e * 32 + lane;
     if (t < k) {
-      D[(size_t)q * ldD + (k - 1 - t)] = (T)ld[e];
+      D[(size_t)q * ldD + (k - 1 - t)] = (T)from_ord(ld[e]);
       I[(size_t)q * ldD + (k - 1 - t)] = (int)li[e];
     }
   }
@@ -1301,15 +1315,15 @@ __device__ __forceinline__ void write_heap_row(T *D, int *I, int ldD, int q, int
 // ascending); the places past k hold (inf, NO_ID).
 template <typename T, int E>
 __device__ __forceinline__ void load_heap_row(const T *D, const int *I, int ldD, int q, int k,
-                                              double (&ld)[E], uint32_t (&li)[E], int lane) {
+                                              Ord (&ld)[E], uint32_t (&li)[E], int lane) {
 #pragma unroll
   for (int e = 0; e < E; e++) {
     const int t = e * 32 + lane;
     if (t < k) {
-      ld[e] = (double)D[(size_t)q * ldD + (k - 1 - t)];
+      ld[e] = to_ord((double)D[(size_t)q * ldD + (k - 1 - t)]);
       li[e] = (uint32_t)I[(size_t)q * ldD + (k - 1 - t)];
     } else {
-      ld[e] = Num<double>::inf();
+      ld[e] = ORD_INF;
       li[e] = NO_ID;
     }
   }
@@ -1318,27 +1332,38 @@ __device__ __forceinline__ void load_heap_row(const T *D, const int *I, int ldD,
 // Sorts the row ascending; a row that already is (an earlier call wrote it, or it is fresh) costs
 // one comparison with each neighbour.
 template <int E>
-__device__ __forceinline__ void sort_heap_row(double (&ld)[E], uint32_t (&li)[E], int lane) {
+__device__ __forceinline__ void sort_heap_row(Ord (&ld)[E], uint32_t (&li)[E], int lane) {
   bool bad = false;
 #pragma unroll
   for (int e = 0; e < E; e++) {
-    double nd = __shfl_down_sync(FULL_MASK, ld[e], 1);
+    Ord nd = __shfl_down_sync(FULL_MASK, ld[e], 1);
     uint32_t ni = __shfl_down_sync(FULL_MASK, li[e], 1);
     if (e + 1 < E) {
-      const double fd = __shfl_sync(FULL_MASK, ld[e + 1 < E ? e + 1 : e], 0);
+      const Ord fd = __shfl_sync(FULL_MASK, ld[e + 1 < E ? e + 1 : e], 0);
       const uint32_t fi = __shfl_sync(FULL_MASK, li[e + 1 < E ? e + 1 : e], 0);
       if (lane == 31) { nd = fd; ni = fi; }
     }
-    // (a NaN is not in order with anything: the row is sorted)
     if (lane < 31 || e + 1 < E) bad |= !(ld[e] < nd || (ld[e] == nd && li[e] <= ni));
   }
-  if (__any_sync(FULL_MASK, bad)) warp_sort<double, E>(ld, li, lane);
+  if (__any_sync(FULL_MASK, bad)) warp_sort<Ord, E>(ld, li, lane);
+}
+
+// Sorts the first n of the warp's 32 keys ascending, the others being (inf, NO_ID): the bitonic
+// network over the next power of two from eight on.
+__device__ __forceinline__ void warp_sort_first(Ord &d, uint32_t &id, int n, int lane) {
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1) {
+    if (size > 8 && n <= size / 2) break;
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1)
+      cx_shfl(d, id, stride, (lane & size) == 0, lane);
+  }
 }
 
 // k-th smallest (0-based index k - 1) of the ascending list the warp holds
 template <int E>
-__device__ __forceinline__ double list_kth(const double (&ld)[E], int k) {
-  double t = ld[0];
+__device__ __forceinline__ Ord list_kth(const Ord (&ld)[E], int k) {
+  Ord t = ld[0];
 #pragma unroll
   for (int e = 0; e < E; e++)
     if (e == (k - 1) / 32) t = ld[e];
@@ -1426,8 +1451,7 @@ constexpr int rr_cap() { return E == 1 ? 384 : 512; }  // listed entries per war
 template <int E>
 struct RerankSmem {
   uint2 list[rr_cap<E>()];     // (d', packed position)
-  uint32_t stage[64];          // positions whose exact distances are next
-  uint32_t fresh[32];          // batching form: the ids of a batch that are not in the row
+  uint32_t stage[64];          // positions (batching form: ids) whose exact distances are next
   __align__(16) uint32_t ids[32 * E];  // batching form: the incoming row's ids
 };
 
@@ -1441,7 +1465,7 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
   const int hr = p.rowmap ? p.rowmap[q] : q;  // heap row and query position
   if (hr < 0) return;                          // a padding row of a leaf panel
   const int k = p.k;
-  double ld[E];
+  Ord ld[E];
   uint32_t li[E];
   load_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
   bool ovf = false;
@@ -1463,16 +1487,13 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
   // Any two heaps hold k candidates, so the second smallest final root bounds the approximate
   // k-th (all bits set: a heap that never filled). A candidate in the final top-k has d' <= the
   // approximate k-th + 2E, and d' <= (the k-th of any k exact distances) + E.
-  two_smallest(m1, m2);
+  if (LEAF) m2 = max(__shfl_sync(FULL_MASK, m1, 0), __shfl_sync(FULL_MASK, m1, 1));
+  else two_smallest(m1, m2);
   float T = m2 == 0xFFFFFFFFu ? Num<float>::inf() : __uint_as_float(m2);
-  float mx = -Num<float>::inf();
-#pragma unroll
-  for (int e = 0; e < E; e++)
-    if (e * 32 + lane < k) mx = fmaxf(mx, up_f((Tab)ld[e]));
-  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL_MASK, mx, o));
+  const float mx = p.qmx[q];
   float lim = band_limit(mx, Eq);
   float thr = band_thr(T, E2, lim);
-  double kth = (double)mx;  // of the exact list so far
+  Ord kth = to_ord((double)mx);  // of the exact list so far
   bool sorted = false;
   if (LEAF) {
 #pragma unroll
@@ -1504,26 +1525,36 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
           break;
         }
         const int cnt = g + lane < p.S ? p.logcnt[(size_t)(g + lane) * p.Q + q] : 0;
-        int incl = cnt;
+        if (LEAF) {  // two logs: excl is where the second one starts
+          excl = __shfl_sync(FULL_MASK, cnt, 0);
+          total = excl + __shfl_sync(FULL_MASK, cnt, 1);
+        } else {
+          int incl = cnt;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(FULL_MASK, incl, o);
-          if (lane >= o) incl += v;
+          for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(FULL_MASK, incl, o);
+            if (lane >= o) incl += v;
+          }
+          excl = incl - cnt;
+          total = __shfl_sync(FULL_MASK, incl, 31);
         }
-        excl = incl - cnt;
-        total = __shfl_sync(FULL_MASK, incl, 31);
         base = 0;
         if (p.counters && lane == 0) atomicAdd(&p.counters[5], (unsigned long long)total);
       }
       if (done) break;
       const int e = base + lane;
-      int s = 0;  // the last log that starts at or before e
+      int s = 0, off;  // the last log that starts at or before e, and e's place in it
+      if (LEAF) {
+        s = e >= excl ? 1 : 0;
+        off = e - (s ? excl : 0);
+      } else {
 #pragma unroll
-      for (int st = 16; st; st >>= 1) {
-        const int v = __shfl_sync(FULL_MASK, excl, s + st);
-        if (v <= e) s += st;
+        for (int st = 16; st; st >>= 1) {
+          const int v = __shfl_sync(FULL_MASK, excl, s + st);
+          if (v <= e) s += st;
+        }
+        off = e - __shfl_sync(FULL_MASK, excl, s);
       }
-      const int off = e - __shfl_sync(FULL_MASK, excl, s);
       float dv[4];
       uint32_t pos = 0u;
       {
@@ -1538,6 +1569,10 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
         dv[2] = fmaf(p.qmul, v.z, qn);
         dv[3] = fmaf(p.qmul, v.w, qn);
       }
+      base += 32;
+      if (!__any_sync(FULL_MASK,
+                      e < total && fminf(fmin3(dv[0], dv[1], dv[2]), dv[3]) <= thr))
+        continue;
 #pragma unroll
       for (int u = 0; u < 4; u++) {
         const bool take = e < total && dv[u] <= thr;
@@ -1547,12 +1582,14 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
               make_uint2(__float_as_uint(dv[u]), pos + u);
         n += __popc(m);
       }
-      base += 32;
     }
     __syncwarp();
-    if (n > 32 && n >= k) T = fminf(T, fmaxf(list_bound(sm.list, n, k, lane), 0.0f));
+    // (a full row of the batching form bounds its candidates itself: most of those it admits are in
+    // it already, so that the rest is one short batch)
+    const bool bound = n > 32 && !(LEAF && lim < Num<float>::inf());
+    if (bound && n >= k) T = fminf(T, fmaxf(list_bound(sm.list, n, k, lane), 0.0f));
     thr = band_thr(T, E2, lim);
-    const float split = n > 32 ? T : Num<float>::inf();  // one batch takes a short list whole
+    const float split = bound ? T : Num<float>::inf();  // one batch takes a short list whole
     if (!done) {
       int w = 0;
       for (int b0 = 0; b0 < n; b0 += 32) {
@@ -1567,47 +1604,34 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
       n = w;
       if (n <= CAP / 2) continue;
     }
-    int nb = 0;  // staged positions
+    int nb = 0;  // staged candidates
     const int nblk = (n + 31) / 32;
-    for (int i = 0; i < (n > 32 ? 2 * nblk : nblk); i++) {
+    for (int i = 0; i < (bound ? 2 * nblk : nblk); i++) {
       const bool pass1 = i >= nblk;
       const int e = (pass1 ? i - nblk : i) * 32 + lane;
-      uint2 ent = make_uint2(0u, 0u);
-      bool take = false;
+      uint32_t id = NO_ID;
       if (e < n) {
-        ent = sm.list[e];
+        const uint2 ent = sm.list[e];
         const float dv = __uint_as_float(ent.x);
-        take = dv <= thr && (dv > split) == pass1;
+        if (dv <= thr && (dv > split) == pass1) id = LEAF ? p.cid[ent.y] : ent.y;
       }
-      const unsigned m = __ballot_sync(FULL_MASK, take);
-      if (take) sm.stage[nb + __popc(m & ((1u << lane) - 1u))] = ent.y;
+      // an id already in the incoming row costs no row gather
+      if (LEAF && id_in_row(id, sm.ids, 8 * E)) id = NO_ID;
+      const unsigned m = __ballot_sync(FULL_MASK, id != NO_ID);
+      if (id != NO_ID) sm.stage[nb + __popc(m & ((1u << lane) - 1u))] = id;
       nb += __popc(m);
       __syncwarp();
       const bool end = i == nblk - 1 || i == 2 * nblk - 1;
       while (nb >= 32 || (end && nb > 0)) {
-        const int count = nb < 32 ? nb : 32;
-        const uint32_t pos = sm.stage[lane < count ? lane : 0];
+        // exact distances of these candidates, merged into the list: lane i takes candidate i's
+        // norm, four lanes its dot product
+        const int cnt = nb < 32 ? nb : 32;
+        id = lane < cnt ? (LEAF ? sm.stage[lane] : p.cid[sm.stage[lane]]) : NO_ID;
         const uint32_t rest = sm.stage[32 + lane];
         __syncwarp();
         sm.stage[lane] = rest;
-        nb -= count;
+        nb -= cnt;
         __syncwarp();
-        // exact distances of these positions, merged into the list: lane i takes candidate i's
-        // id and norm, four lanes its dot product
-        uint32_t id = NO_ID;
-        if (lane < count) id = p.cid[pos];
-        // an id already in the incoming row costs no row gather: the others move together
-        int cnt = count;
-        if (LEAF) {
-          const bool fresh = !id_in_row(id, sm.ids, 8 * E) && id != NO_ID;
-          const unsigned m = __ballot_sync(FULL_MASK, fresh);
-          if (m == 0) continue;
-          cnt = __popc(m);
-          if (fresh) sm.fresh[__popc(m & ((1u << lane) - 1u))] = id;
-          __syncwarp();
-          id = lane < cnt ? sm.fresh[lane] : NO_ID;
-          __syncwarp();
-        }
         const double cc = id != NO_ID ? (double)p.Xc2[id] : 0.0;
         double dot = 0.0;
         if constexpr (sizeof(Tab) == 8) {
@@ -1620,7 +1644,7 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
           part = __shfl_sync(FULL_MASK, sum4(part), (lane & 7) * 4);
           if ((lane >> 3) == (r >> 3)) dot = part;
         }
-        const double dist = id != NO_ID ? exact_dist(dot, cc, qq) : Num<double>::inf();
+        const Ord dist = id != NO_ID ? to_ord(exact_dist(dot, cc, qq)) : ORD_INF;
         if (p.counters && lane == 0) atomicAdd(&p.counters[6], (unsigned long long)cnt);
         if (LEAF) {
           // nothing in this batch can enter (ties are settled by the merge itself)
@@ -1630,13 +1654,14 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
             sorted = true;
           }
         }
-        double b1[1] = {dist};
-        uint32_t i1[1] = {id};
-        warp_sort<double, 1>(b1, i1, lane);
-        warp_merge_32<double, E>(ld, li, b1[0], i1[0], lane);
+        Ord bd = dist;
+        uint32_t bi = id;
+        warp_sort_first(bd, bi, cnt, lane);
+        warp_merge_32<Ord, E>(ld, li, bd, bi, lane);
         kth = list_kth<E>(ld, k);
-        if (kth < 1e38) {
-          lim = fminf(lim, __fadd_ru(__double2float_ru(kth), Eq));
+        const double kd = from_ord(kth);
+        if (kd < 1e38) {
+          lim = fminf(lim, __fadd_ru(__double2float_ru(kd), Eq));
           if (lim < thr) thr = lim;
         }
       }
@@ -1672,7 +1697,7 @@ constexpr int RC_LOGS = 512;  // logs (NPART * S) the prefix array holds
 template <typename Tab, int E>
 __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(RerankParams<Tab> p) {
   __shared__ uint2 list[RC_CAP];
-  __shared__ double xd[RC_CAP];
+  __shared__ Ord xd[RC_CAP];
   __shared__ uint32_t xi[RC_CAP];
   __shared__ int pre[RC_LOGS + 1];
   __shared__ float s_T, s_thr;
@@ -1777,25 +1802,25 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
       dot = sum4(dot);
     }
     if (i < n && lane % LPC == 0) {
-      xd[i] = id != NO_ID ? exact_dist(dot, (double)p.Xc2[id], qq) : Num<double>::inf();
+      xd[i] = id != NO_ID ? to_ord(exact_dist(dot, (double)p.Xc2[id], qq)) : ORD_INF;
       xi[i] = id;
       if (p.counters && id != NO_ID) atomicAdd(&p.counters[6], 1ull);
     }
   }
   __syncthreads();
   if (warp != 0) return;
-  double ld[E];
+  Ord ld[E];
   uint32_t li[E];
   load_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
   sort_heap_row<E>(ld, li, lane);
-  double kth = list_kth<E>(ld, k);
+  Ord kth = list_kth<E>(ld, k);
   for (int base = 0; base < n; base += 32) {
     const int i = base + lane;
-    double b1[1] = {i < n ? xd[i] : Num<double>::inf()};
+    Ord b1[1] = {i < n ? xd[i] : ORD_INF};
     uint32_t i1[1] = {i < n ? xi[i] : NO_ID};
-    if (!__any_sync(FULL_MASK, i1[0] != NO_ID && !(b1[0] > kth))) continue;
-    warp_sort<double, 1>(b1, i1, lane);
-    warp_merge_32<double, E>(ld, li, b1[0], i1[0], lane);
+    if (!__any_sync(FULL_MASK, i1[0] != NO_ID && b1[0] <= kth)) continue;
+    warp_sort<Ord, 1>(b1, i1, lane);
+    warp_merge_32<Ord, E>(ld, li, b1[0], i1[0], lane);
     kth = list_kth<E>(ld, k);
   }
   write_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
@@ -1818,7 +1843,7 @@ struct FallbackParams {
 
 template <int E>
 __global__ void __launch_bounds__(256) tc_fallback(FallbackParams p) {
-  __shared__ double sd[8][32 * E];
+  __shared__ Ord sd[8][32 * E];
   __shared__ uint32_t si[8][32 * E];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = *p.count;
@@ -1827,11 +1852,11 @@ __global__ void __launch_bounds__(256) tc_fallback(FallbackParams p) {
     const long long qrow = p.qidx[q];
     const float *qv = p.Xq + qrow * p.d;
     const double qq = (double)p.Xq2[qrow];
-    double ld[E];
+    Ord ld[E];
     uint32_t li[E];
 #pragma unroll
-    for (int e = 0; e < E; e++) { ld[e] = Num<double>::inf(); li[e] = NO_ID; }
-    double kth = Num<double>::inf();
+    for (int e = 0; e < E; e++) { ld[e] = ORD_INF; li[e] = NO_ID; }
+    Ord kth = ORD_INF;
     // each warp scans a strided share of the candidates, one candidate per lane at a time
     for (int base = warp * 32; base < p.nc; base += 256) {
       const int c = base + lane;
@@ -1848,16 +1873,12 @@ __global__ void __launch_bounds__(256) tc_fallback(FallbackParams p) {
           id = (uint32_t)row;
         }
       }
-      if (__any_sync(FULL_MASK, dist <= kth)) {
-        double b1[1] = {dist};
+      Ord b1[1] = {to_ord(dist)};
+      if (__any_sync(FULL_MASK, b1[0] <= kth)) {
         uint32_t i1[1] = {id};
-        warp_sort<double, 1>(b1, i1, lane);
-        warp_merge_32<double, E>(ld, li, b1[0], i1[0], lane);
-        double t = ld[0];
-#pragma unroll
-        for (int e = 0; e < E; e++)
-          if (e == (p.k - 1) / 32) t = ld[e];
-        kth = __shfl_sync(FULL_MASK, t, (p.k - 1) & 31);
+        warp_sort<Ord, 1>(b1, i1, lane);
+        warp_merge_32<Ord, E>(ld, li, b1[0], i1[0], lane);
+        kth = list_kth<E>(ld, p.k);
       }
     }
 #pragma unroll
@@ -1867,19 +1888,19 @@ __global__ void __launch_bounds__(256) tc_fallback(FallbackParams p) {
     }
     __syncthreads();
     if (warp == 0) {
-      double md[E];
+      Ord md[E];
       uint32_t mi[E];
       load_heap_row<float, E>(p.D, p.I, p.ldD, q, p.k, md, mi, lane);
       sort_heap_row<E>(md, mi, lane);
       for (int w2 = 0; w2 < 8; w2++) {
-        double bd[E];
+        Ord bd[E];
         uint32_t bi[E];
 #pragma unroll
         for (int e = 0; e < E; e++) {
           bd[e] = sd[w2][e * 32 + lane];
           bi[e] = si[w2][e * 32 + lane];
         }
-        warp_merge_lists<double, E>(md, mi, bd, bi, lane);
+        warp_merge_lists<Ord, E>(md, mi, bd, bi, lane);
       }
       write_heap_row<float, E>(p.D, p.I, p.ldD, q, p.k, md, mi, lane);
     }
@@ -1915,7 +1936,7 @@ __global__ void __launch_bounds__(256) tc_fallback_leaf(LeafFallbackParams p) {
     const int2 r = p.rtab[q / TC_M];
     const float *qv = p.X + (long long)hr * p.d;
     const double qq = (double)p.X2[hr];
-    double ld[E];
+    Ord ld[E];
     uint32_t li[E];
     load_heap_row<float, E>(p.D, p.I, p.ldD, hr, p.k, ld, li, lane);
     sort_heap_row<E>(ld, li, lane);
@@ -1938,10 +1959,10 @@ __global__ void __launch_bounds__(256) tc_fallback_leaf(LeafFallbackParams p) {
         dist = Num<double>::inf();
         id = NO_ID;
       }
-      double b1[1] = {dist};
+      Ord b1[1] = {to_ord(dist)};
       uint32_t i1[1] = {id};
-      warp_sort<double, 1>(b1, i1, lane);
-      warp_merge_32<double, E>(ld, li, b1[0], i1[0], lane);
+      warp_sort<Ord, 1>(b1, i1, lane);
+      warp_merge_32<Ord, E>(ld, li, b1[0], i1[0], lane);
     }
     write_heap_row<float, E>(p.D, p.I, p.ldD, hr, p.k, ld, li, lane);
   }
@@ -2428,7 +2449,7 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, bool pack_cand, boo
   RerankParams<T> rp{};
   rp.Q = nq; rp.k = k; rp.S = NPART * P.S; rp.logcap = P.logcap; rp.d = d;
   rp.log = tp.log; rp.logpos = tp.logpos; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
-  rp.qn = tp.qn; rp.qmul = tp.fold ? -2.0f : 1.0f;
+  rp.qn = tp.qn; rp.qmx = tp.qmx; rp.qmul = tp.fold ? -2.0f : 1.0f;
   rp.proot = tp.proot;
   rp.Xq = Xq; rp.Xq2 = Xq2; rp.nrows_q = nrows_q;
   rp.Xc = static_cast<const T *>(C.Xc); rp.Xc2 = static_cast<const T *>(C.Xc2);
@@ -2775,7 +2796,7 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   RerankParams<float> rp{};
   rp.Q = rows; rp.k = k; rp.S = NPART; rp.logcap = P.logcap; rp.d = d;
   rp.log = tp.log; rp.logpos = tp.logpos; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
-  rp.qn = tp.qn; rp.qmul = tp.fold ? -2.0f : 1.0f;
+  rp.qn = tp.qn; rp.qmx = tp.qmx; rp.qmul = tp.fold ? -2.0f : 1.0f;
   rp.proot = tp.proot;
   rp.Xq = X; rp.Xq2 = X2; rp.nrows_q = npts; rp.Xc = X; rp.Xc2 = X2; rp.qidx = iota;
   rp.cid = cid;
