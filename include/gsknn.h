@@ -161,15 +161,16 @@ const char *gsknn_last_error_string(void);
  *   GSKNN_MODE_FP32 -- CUDA-core FP32 distances;
  *   GSKNN_MODE_TF32, GSKNN_MODE_BF16 -- tensor-core distances with an FP64 re-rank of every
  *     candidate within the rounding bound of the k-th distance (exact index sets);
- *   GSKNN_MODE_AUTO -- from d = 128, BF16 (queries whose re-rank band overflows its log run
- *     again in split BF16); below d = 128, split BF16 (the narrowest band; plain BF16 overflows
- *     there); TF32 where neither fits in shared memory; else FP32 (default). Each choice was
- *     measured fastest of the exact forms on the d = 64 and d = 256 workloads. */
+ *   GSKNN_MODE_AUTO -- large calls with d > 64 in scaled FP16 (queries whose re-rank band
+ *     overflows its log run again in split BF16); others in split BF16 (the narrowest band); TF32
+ *     where neither fits in shared memory; else FP32 (default). Each choice was measured fastest
+ *     of the exact forms over d = 20 to 256. */
 #define GSKNN_MODE_AUTO 0
 #define GSKNN_MODE_FP32 1
 #define GSKNN_MODE_TF32 2
 #define GSKNN_MODE_BF16 3
 #define GSKNN_MODE_BF16X3 4 /* split BF16: hi*hi + hi*lo + lo*hi, near-FP32 distances */
+#define GSKNN_MODE_FP16 5   /* AUTO's choice alone: reported by gsknn_serve_mode, not settable */
 int gsknn_set_mode(int mode);
 int gsknn_get_mode(void);
 
@@ -311,9 +312,9 @@ void gsknn_batch_forget_tuning(void);
  *
  * gsknn_serve_create prepares the nref x d float reference set R (device pointer, with norms
  * R2) once: packed for the tensor cores (mode AUTO / TF32 / BF16 / BF16X3) and resident until
- * destroy. In BF16 or TF32 the set is also packed in split BF16, where queries whose re-rank
- * band overflows finish. AUTO prepares BF16 with those split panels, times one probe batch of
- * resident points (k = max_k) both in BF16 and in split BF16 alone, and serves in the faster
+ * destroy. In FP16, BF16 or TF32 the set is also packed in split BF16, where queries whose re-rank
+ * band overflows finish. AUTO prepares FP16 with split panels, times one probe batch of
+ * resident points (k = max_k) both in FP16 and in split BF16 alone, and serves in the faster
  * (TF32 where split tiles do not fit); gsknn_serve_mode reports the choice. Each request is m query rows
  * (host memory, copied at submit) and a k <= max_k; its result is the exact FP64 top-k of every
  * query against R (ties to the lower id), as a heap of m rows x k (descending rows) that stays
@@ -352,8 +353,8 @@ int gsknn_serve_set_slice(gsknn_serve_t *eng, int rows);
 /* While paused (nonzero) the dispatcher starts no new batch; requests still queue. Running
  * batches finish. Resuming dispatches everything queued in arrival order. */
 int gsknn_serve_pause(gsknn_serve_t *eng, int paused);
-/* The arithmetic the engine serves in (GSKNN_MODE_TF32 / BF16 / BF16X3) and, after an AUTO
- * choice, the probe batch's milliseconds in BF16 and in split BF16 (0 when not probed). */
+/* The arithmetic the engine serves in (GSKNN_MODE_TF32 / BF16 / BF16X3 / FP16) and, after an AUTO
+ * choice, the probe batch's milliseconds in FP16 and in split BF16 (0 when not probed). */
 int gsknn_serve_mode(gsknn_serve_t *eng, double *probe_bf16_ms, double *probe_bf16x3_ms);
 void gsknn_serve_destroy(gsknn_serve_t *eng);
 

@@ -516,19 +516,27 @@ static int knn_device_tc(int mode, int nq, int nc, int d, int k, const float *Xq
 
 // The tensor-core mode AUTO takes for a shape (GSKNN_MODE_FP32: none fits).
 static int auto_mode(int nq, int nc, int d, int k) {
-  // Split BF16 keeps the re-rank band narrowest (input error ~u^2): at d = 64 plain BF16's band
-  // overflows the logs and most queries run again. From d = 128 one BF16 MMA per product was
-  // measured fastest (d = 256: 10.8 ms against 13.9 ms in split BF16 for 32,768 x 262,144,
-  // k = 64); the few queries whose log overflows run again in split BF16.
-  if (d >= 128 && tc_plan(nq, nc, d, k, GSKNN_TC_BF16, sm_count()).ok) return GSKNN_TC_BF16;
+  // Split BF16 (three MMAs per product) keeps the re-rank band narrowest. One FP16 MMA per product
+  // (and half the panel bytes) pays from two K chunks (d > 64) where the contraction bounds the
+  // call, about 1.3e10 (pair, padded dimension) products, or the packing does, 2.5e7 (candidate,
+  // padded dimension) entries; beyond d = 256, where split tiles are narrow, 9e6. B200, us, split
+  // -> FP16: 16,384 x 60,000, d = 80 804 -> 539, d = 256 1,532 -> 795; 4,096 x 65,536, d = 128
+  // 318 -> 260; 16 x 250,000, d = 200 613 -> 397; 16 x 30,000, d = 300 208 -> 169; but 2,000 x
+  // 30,000, d = 128 167 -> 175, 16 x 30,000, d = 128 127 -> 164 and 16 x 4,096 96 -> 108 (the
+  // escalation's launches). At d <= 64 it gains 18% on uniform points and nothing on the Gaussian
+  // mixture, whose band is wider.
+  const double d_pad = (d + 63) / 64 * 64, entries = nc * d_pad, products = nq * entries;
+  const bool f16 = tc_plan(nq, nc, d, k, GSKNN_TC_FP16, sm_count()).ok;
+  if (f16 && d > 64 && (products >= 1.3e10 || entries >= (d > 256 ? 9e6 : 2.5e7)))
+    return GSKNN_TC_FP16;
   if (tc_plan(nq, nc, d, k, GSKNN_TC_BF16X3, sm_count()).ok) return GSKNN_TC_BF16X3;
+  if (f16) return GSKNN_TC_FP16;
   if (tc_plan(nq, nc, d, k, GSKNN_TC_TF32, sm_count()).ok) return GSKNN_TC_TF32;
   return GSKNN_MODE_FP32;
 }
 
 // The arithmetic used for a float call: explicit modes are honoured; AUTO takes the
-// tensor-core form with the exact FP64 re-rank where it fits (split BF16 below d = 128, BF16
-// from there, TF32 where neither fits), else the CUDA-core FP32 kernel.
+// tensor-core form with the exact FP64 re-rank where it fits, else the CUDA-core FP32 kernel.
 static int pick_mode(int nq, int nc, int d, int k) {
   return g_mode != GSKNN_MODE_AUTO ? g_mode : auto_mode(nq, nc, d, k);
 }

@@ -101,6 +101,7 @@ cudaError_t block_run(const LargePlan &P, int nq, int nc, int d, const T *Xq, co
 #define GSKNN_TC_TF32 2
 #define GSKNN_TC_BF16 3
 #define GSKNN_TC_BF16X3 4
+#define GSKNN_TC_FP16 5  // taken by AUTO; not a public mode
 
 // Kernel-launch bracket used by the library's tracer (begin/end around a group of launches);
 // `nkernels` (read at the end) counts the library's own kernels launched inside the bracket.
@@ -143,14 +144,14 @@ struct TcPlan {
 };
 
 // Candidates packed once in the MMA input format, with everything a query batch needs from
-// them: shift mu, |mu|^2, bound statistics (maxima over the candidates), packed panels
+// them: shift mu, bound statistics (maxima over the candidates), packed panels
 // [r_pad][d_pad] (r_pad a multiple of 256), effective norms, ids,
 // and the caller's table for the FP64 re-rank. A resident reference set is prepared once and
 // serves any number of query batches.
 struct TcCand {
   int fmt, elem, d, d_pad, nc, r_pad;
   float *mu;
-  double *mu2;
+  float *fscale;  // scale of the FP16 format
   double *part;  // tc_center's partial sums and row counts
   int *part_n;
   unsigned *stats, *estats;  // bound statistics of the main and of the escalation format
@@ -210,7 +211,7 @@ struct TcLeafPlan {
   bool ok;
   TcPlan P;        // the split-BF16 tile plan (one split), per-query area for rows_cap rows
   int rows_cap;    // panel rows one tree may need
-  size_t o_mu, o_mu2, o_cpart, o_stats, o_pb, o_pb_lo, o_pn, o_cn, o_cid, o_iota, bytes;
+  size_t o_mu, o_fscale, o_cpart, o_stats, o_pb, o_pb_lo, o_pn, o_cn, o_cid, o_iota, bytes;
 };
 // npts: points of the table; rows_cap: panel rows one tree may use (a multiple of 128).
 TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms);

@@ -202,7 +202,7 @@ struct Engine {
   // The resident set as batches use it: C itself, or (when the engine measured the escalation
   // format faster) C's escalation panels run as the main format.
   TcCand Crun{};
-  double probe_ms[2] = {0.0, 0.0};  // AUTO: probe batch in BF16 (+escalation) and split BF16
+  double probe_ms[2] = {0.0, 0.0};  // AUTO: probe batch in FP16 (+escalation) and split BF16
   int *cidx = nullptr, *status = nullptr;
   char *arena_mem = nullptr;
   std::unique_ptr<serve::Arena> arena;
@@ -543,16 +543,16 @@ gsknn_serve_t *gsknn_serve_create(const float *R, const float *R2, int nref, int
     serr(GSKNN_ERR_ARG, "gsknn_serve_create: invalid argument");
     return nullptr;
   }
-  // AUTO prepares the resident set in BF16 with split-BF16 escalation panels (queries whose
-  // BF16 band overflows finish in split BF16), then measures a probe batch both ways -- BF16
+  // AUTO prepares the resident set in FP16 with split-BF16 escalation panels (queries whose
+  // FP16 band overflows finish in split BF16), then measures a probe batch both ways -- FP16
   // with escalation, and split BF16 alone on the escalation panels -- and serves with the
   // faster. Where split tiles do not fit, TF32.
   const bool auto_mode = mode == GSKNN_MODE_AUTO;
   if (auto_mode)
     mode = tc_plan(max_batch_queries, nref, d, max_k, GSKNN_TC_BF16X3, 148, false, 148).ok
-               ? GSKNN_MODE_BF16
+               ? GSKNN_MODE_FP16
                : GSKNN_MODE_TF32;
-  if (mode < GSKNN_MODE_TF32 || mode > GSKNN_MODE_BF16X3) {
+  else if (mode < GSKNN_MODE_TF32 || mode > GSKNN_MODE_BF16X3) {
     serr(GSKNN_ERR_ARG, "gsknn_serve_create: mode must be AUTO, TF32, BF16 or BF16X3");
     return nullptr;
   }

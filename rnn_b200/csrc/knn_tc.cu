@@ -44,6 +44,7 @@
 #include "tc_ptx.cuh"
 
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cmath>
@@ -73,19 +74,21 @@ constexpr int CN_SLOTS = 3;
 // The shift is the mean of a strided sample of the candidate rows, summed in a fixed order so that
 // it is the same bits on every run: tc_center, on a grid of (dimension groups of 32, CENTER_SLICES
 // slices of the sample), 16 warps per block, lane = dimension, warps striding over the slice's rows
-// (coalesced row segments), writes one partial sum per (slice, dimension) and one row count per
-// slice; tc_pack adds the partials in slice order. Being the first kernel of a call it also clears
+// (coalesced row segments), writes one partial sum, minimum and maximum per (slice, dimension) and
+// one row count per slice; tc_pack adds the partials in slice order, and takes the scale of the
+// FP16 format from the widest dimension. Being the first kernel of a call it also clears
 // the call's status word and the candidates' bound statistics.
 constexpr int CENTER_SLICES = 16;
 constexpr int CENTER_ROWS = 1024;  // sampled rows (any shift is valid; it only narrows the bound)
 constexpr int CENTER_WARPS = 16;
+constexpr int CENTER_PARTS = 3 * CENTER_SLICES;  // doubles per dimension
 
 template <typename T>
 __global__ void __launch_bounds__(32 * CENTER_WARPS) tc_center(
     const T *__restrict__ X, int d, long long nrows, const int *__restrict__ idx, int count,
     int nsample, double *__restrict__ part, int *__restrict__ part_n, unsigned *stats,
     int nstats, int *clear) {
-  __shared__ double ps[CENTER_WARPS][33];
+  __shared__ double ps[CENTER_WARPS][33], pmn[CENTER_WARPS][33], pmx[CENTER_WARPS][33];
   __shared__ int pc[CENTER_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (blockIdx.x == 0 && blockIdx.y == 0) {
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(32 * CENTER_WARPS) tc_center(
   const int p = blockIdx.x * 32 + lane;
   const int t_lo = (int)((long long)nsample * blockIdx.y / CENTER_SLICES);
   const int t_hi = (int)((long long)nsample * (blockIdx.y + 1) / CENTER_SLICES);
-  double s = 0.0;
+  double s = 0.0, mn = Num<double>::inf(), mx = -Num<double>::inf();
   int used = 0;
   // four sample rows per round: their index and row loads are independent and issue together
   for (int t0 = t_lo + warp; t0 < t_hi; t0 += CENTER_WARPS * 4) {
@@ -112,12 +115,18 @@ __global__ void __launch_bounds__(32 * CENTER_WARPS) tc_center(
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       if (ok[u]) {
-        if (p < d) s += (double)v[u];
+        if (p < d) {
+          s += (double)v[u];
+          mn = fmin(mn, (double)v[u]);
+          mx = fmax(mx, (double)v[u]);
+        }
         used++;
       }
     }
   }
   ps[warp][lane] = s;
+  pmn[warp][lane] = mn;
+  pmx[warp][lane] = mx;
   if (lane == 0) pc[warp] = used;
   __syncthreads();
   if (warp == 0) {
@@ -125,9 +134,15 @@ __global__ void __launch_bounds__(32 * CENTER_WARPS) tc_center(
     int n = 0;
     for (int w = 0; w < CENTER_WARPS; w++) {
       tot += ps[w][lane];
+      mn = fmin(mn, pmn[w][lane]);
+      mx = fmax(mx, pmx[w][lane]);
       n += pc[w];
     }
-    if (p < d) part[(size_t)blockIdx.y * d + p] = tot;
+    if (p < d) {
+      part[(size_t)blockIdx.y * d + p] = tot;
+      part[(size_t)(CENTER_SLICES + blockIdx.y) * d + p] = mn;
+      part[(size_t)(2 * CENTER_SLICES + blockIdx.y) * d + p] = mx;
+    }
     if (blockIdx.x == 0 && lane == 0) part_n[blockIdx.y] = n;
   }
 }
@@ -141,14 +156,21 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
   return r;
 }
 
-// Norm column of candidate row r (32 bytes, the K of one MMA): -cn/2 as the exact sum of three
-// parts in the MMA input format (BF16: 3 x 8 significant bits; TF32: 3 x 11 >= the 24 of the
-// float cn), then zeros. Against an all-ones A column the MMA adds -cn/2 to <q~, c~>, so the
-// accumulator holds w = <q~, c~> - cn/2 = -v/2. A padding row holds -inf (w = -inf, v = +inf:
-// never admitted).
-__device__ __forceinline__ void write_norm_row(int fmt, void *npanel, int r, bool real, float cn) {
+// FP16 rounding with saturation; subnormals become 0 (the residual is measured either way).
+__device__ __forceinline__ __half to_f16(float x) {
+  const __half h = __float2half_rn(fminf(fmaxf(x, -65504.0f), 65504.0f));
+  return fabsf(__half2float(h)) < 6.103515625e-5f ? __ushort_as_half(0) : h;
+}
+
+// Norm column of candidate row r (32 bytes, the K of one MMA): x = -cn/2 as the sum of three parts
+// in the MMA input format, then zeros. Against an A tile whose rows all hold the parts' weights the
+// MMA adds x to <q~, c~>, so the accumulator holds w = <q~, c~> - cn/2 = -v/2. A padding row holds
+// -inf (w = -inf, v = +inf: never admitted). TF32 and BF16: weights 1, and the parts (3 x 11 and
+// 3 x 8 significant bits) are exact for the 24 of the float. FP16: x in the panel's scale, weights
+// 2^14, 2^3, 2^-8 for its narrow exponent; what the parts leave of x is returned.
+__device__ __forceinline__ float write_norm_row(int fmt, void *npanel, int r, bool real, float x) {
   uint4 lo4 = make_uint4(0u, 0u, 0u, 0u), hi4 = make_uint4(0u, 0u, 0u, 0u);
-  const float x = -0.5f * cn;
+  float rest = 0.0f;
   if (fmt == 0) {
     uint32_t h = 0xFF800000u, m = 0u, l = 0u;
     if (real) {
@@ -158,6 +180,20 @@ __device__ __forceinline__ void write_norm_row(int fmt, void *npanel, int r, boo
       l = to_tf32(r1 - __uint_as_float(m));
     }
     lo4 = make_uint4(h, m, l, 0u);
+  } else if (fmt == 3) {
+    uint32_t h = 0xFC00u, m = 0u, l = 0u;
+    if (real) {
+      const __half a = to_f16(x * 6.103515625e-5f);
+      const float r1 = x - __half2float(a) * 16384.0f;
+      const __half b = to_f16(r1 * 0.125f);
+      const float r2 = r1 - __half2float(b) * 8.0f;
+      const __half c = to_f16(r2 * 256.0f);
+      rest = fabsf(r2 - __half2float(c) * 0.00390625f);
+      h = __half_as_ushort(a);
+      m = __half_as_ushort(b);
+      l = __half_as_ushort(c);
+    }
+    lo4 = make_uint4(h | (m << 16), l, 0u, 0u);
   } else {
     uint32_t h = 0xFF80u, m = 0u, l = 0u;
     if (real) {
@@ -174,9 +210,11 @@ __device__ __forceinline__ void write_norm_row(int fmt, void *npanel, int r, boo
   uint4 *dst = reinterpret_cast<uint4 *>(static_cast<char *>(npanel) + (size_t)r * 32);
   dst[0] = lo4;
   dst[1] = hi4;
+  return rest;
 }
 
-// fmt: 0 = TF32 (4-byte panel), 1 = BF16, 2 = split BF16 (hi and lo panels)
+// fmt: 0 = TF32 (4-byte panel), 1 = BF16, 2 = split BF16 (hi and lo panels), 3 = FP16, scaled by a
+// power of two that takes the sampled coordinates to at most 2^12
 //
 // One side of a packing launch: `rows_pad` panel rows, of which the first `count` are points
 // idx[r] (idx[rowmap[r]] with a row map) of table X. `dcount` (device) replaces `count` and limits
@@ -204,20 +242,21 @@ struct PackSide {
 };
 
 // Maxima over the candidates (bits of non-negative floats, which order like unsigned integers):
-// centred norm |c~|, |effective norm|, norm of the rounding residual |c~ - fmt(c~)|, and the scale
-// of the FP64 distance's own rounding.
-enum PackStats { ST_M = 0, ST_CN, ST_RES, ST_SCALE };
+// centred norm |c~|, |effective norm|, norm of the rounding residual |c~ - fmt(c~)|, the scale of
+// the FP64 distance's own rounding, and what the norm column leaves of -cn/2 (FP16).
+enum PackStats { ST_M = 0, ST_CN, ST_RES, ST_SCALE, ST_NRES, ST_COUNT };
+constexpr int STATS_WORDS = 8;
 
 template <typename T>
 struct PackArgs {
   int fmt, d, d_pad;
   PackSide<T> a, b;
-  // the shift: from tc_center's partial sums (and written to mu / mu2 for later launches), or, with
-  // part null, read from mu / mu2
+  // the shift: from tc_center's partial sums (and written to mu for later launches), or, with part
+  // null, read from mu
   const double *part;
   const int *part_n;
   float *mu;
-  double *mu2;
+  float *fscale;     // scale of the FP16 format (written and read as mu)
   float kA, kB, kS;  // bound coefficients (TcPlan)
   int *status;
 };
@@ -250,10 +289,10 @@ __device__ __forceinline__ float up_f(double x) { return __double2float_ru(x); }
 template <typename T>
 __global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
   extern __shared__ double pack_mu[];  // [d] shift, as doubles
-  __shared__ double red[8];
-  __shared__ unsigned bmx[4];
+  __shared__ double red[8], redw[8];
+  __shared__ unsigned bmx[ST_COUNT];
   const int tid = threadIdx.x, lane = tid & 31, sub = lane & 7;
-  if (tid < 4) bmx[tid] = 0u;
+  if (tid < ST_COUNT) bmx[tid] = 0u;
   int a_rows = g.a.rows_pad, b_rows = g.b.rows_pad;
   if (g.a.gate && *g.a.gate == 0) a_rows = 0;
   if (g.b.gate && *g.b.gate == 0) b_rows = 0;
@@ -265,8 +304,9 @@ __global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
   if (blockIdx.x == 0 && tid < 4 && g.b.zero) g.b.zero[tid] = 0;
   if (a_rows + b_rows == 0) return;
   double mu2;
+  float fs = 1.0f;
   {
-    double s2 = 0.0;
+    double s2 = 0.0, wide = 0.0;
     int n = 0;
     if (g.part)
       for (int sl = 0; sl < CENTER_SLICES; sl++) n += g.part_n[sl];
@@ -277,20 +317,47 @@ __global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
         for (int sl = 0; sl < CENTER_SLICES; sl++) tot += g.part[(size_t)sl * g.d + p];
         m = n ? (float)(tot / n) : 0.0f;
         if (blockIdx.x == 0) g.mu[p] = m;
+        if (g.fmt == 3) {
+          double mn = Num<double>::inf(), mxv = -Num<double>::inf();
+          for (int sl = 0; sl < CENTER_SLICES; sl++) {
+            mn = fmin(mn, g.part[(size_t)(CENTER_SLICES + sl) * g.d + p]);
+            mxv = fmax(mxv, g.part[(size_t)(2 * CENTER_SLICES + sl) * g.d + p]);
+          }
+          wide = fmax(wide, mxv - mn);
+        }
       } else {
         m = g.mu[p];
       }
       pack_mu[p] = (double)m;
       s2 += (double)m * (double)m;
     }
-    for (int o = 16; o; o >>= 1) s2 += __shfl_xor_sync(FULL_MASK, s2, o);
-    if (lane == 0) red[tid >> 5] = s2;
+    for (int o = 16; o; o >>= 1) {
+      s2 += __shfl_xor_sync(FULL_MASK, s2, o);
+      wide = fmax(wide, __shfl_xor_sync(FULL_MASK, wide, o));
+    }
+    if (lane == 0) {
+      red[tid >> 5] = s2;
+      redw[tid >> 5] = wide;
+    }
     __syncthreads();
     mu2 = 0.0;
-    for (int w = 0; w < 8; w++) mu2 += red[w];
-    if (g.part && blockIdx.x == 0 && tid == 0) *g.mu2 = mu2;
+    wide = 0.0;
+    for (int w = 0; w < 8; w++) {
+      mu2 += red[w];
+      wide = fmax(wide, redw[w]);
+    }
+    if (g.fmt == 3) {
+      if (g.part) {
+        const int e = wide > 0.0 && wide < 1e300 ? 11 - ilogb(wide) : 0;
+        fs = ldexpf(1.0f, max(-60, min(60, e)));
+        if (blockIdx.x == 0 && tid == 0) *g.fscale = fs;
+      } else {
+        fs = *g.fscale;
+      }
+    }
   }
-  unsigned mx[4] = {0u, 0u, 0u, 0u};
+  const double inv_fs = 1.0 / (double)fs;
+  unsigned mx[ST_COUNT] = {};
   const int step = gridDim.x * 32;
   // (four rows per warp; a side's rows are whole tiles, so a warp's rows lie on one side)
   for (int r4 = blockIdx.x * 32 + (tid >> 5) * 4; r4 < a_rows + b_rows; r4 += step) {
@@ -339,6 +406,18 @@ __global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
         }
         *reinterpret_cast<uint4 *>(reinterpret_cast<uint32_t *>(s.panel) + o) =
             make_uint4(t[0], t[1], t[2], t[3]);
+      } else if (g.fmt == 3) {
+        uint32_t h[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const float ys = y[j] * fs;
+          const __half v16 = to_f16(ys);
+          const double res = (double)(ys - __half2float(v16));
+          r2 = fma(res, res, r2);
+          h[j] = __half_as_ushort(v16);
+        }
+        *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(s.panel) + o) =
+            make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
       } else {
         uint32_t h[4], l[4];
 #pragma unroll
@@ -365,21 +444,24 @@ __global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
     for (int o = 4; o; o >>= 1) {
       s2 += __shfl_xor_sync(FULL_MASK, s2, o);
       smx += __shfl_xor_sync(FULL_MASK, smx, o);
-      if (g.fmt < 2) r2 += __shfl_xor_sync(FULL_MASK, r2, o);
+      if (g.fmt != 2) r2 += __shfl_xor_sync(FULL_MASK, r2, o);
       qmx = fmaxf(qmx, __shfl_xor_sync(FULL_MASK, qmx, o));
     }
     if (sub == 0) {
       // |x - mu|^2 expressed through the caller's norm: X2 - 2 mu.x + mu.mu
       const double x2 = row >= 0 ? (double)s.X2[row] : 0.0;
       const float enf = row >= 0 ? (float)(x2 - 2.0 * smx + mu2) : Num<float>::nan();
-      if (s.npanel) write_norm_row(g.fmt, s.npanel, r, row >= 0, row >= 0 ? enf : 0.0f);
+float nres = 0.0f;
+      if (s.npanel)
+        nres = write_norm_row(g.fmt, s.npanel, r, row >= 0,
+                              row >= 0 ? -0.5f * enf * (fs * fs) : 0.0f);
       // norms of the centred row and of its rounding residual (in split BF16 a bound on it, 3.2 u^2
       // of the norm, that covers the omitted lo x lo product too), rounded up; and the scale of the
       // FP64 distance's own rounding: the caller's norm, and |x|^2 <= 2 (|x - mu|^2 + |mu|^2)
       const float nrm = row >= 0 ? up_f(sqrt(s2) * (1.0 + 1e-6)) : 0.0f;
       const float res = row < 0 ? 0.0f
                         : g.fmt == 2 ? nrm * (3.2f / 65536.0f)
-                                     : up_f(sqrt(r2) * (1.0 + 1e-6));
+                                     : up_f(sqrt(r2) * inv_fs * (1.0 + 1e-6));
       const float scale = row >= 0 ? up_f(fmax(fabs(x2), 2.0 * (s2 + mu2))) : 0.0f;
       if (s.enorm) {
         s.enorm[r] = enf;
@@ -398,6 +480,7 @@ __global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
         mx[ST_CN] = max(mx[ST_CN], __float_as_uint(fabsf(enf) * (1.0f + 1e-6f)));
         mx[ST_RES] = max(mx[ST_RES], __float_as_uint(g.fmt == 2 ? 0.0f : res));
         mx[ST_SCALE] = max(mx[ST_SCALE], __float_as_uint(scale));
+        mx[ST_NRES] = max(mx[ST_NRES], __float_as_uint(up_f((double)nres * inv_fs * inv_fs)));
       }
     }
   }
@@ -406,12 +489,12 @@ __global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
   unsigned *stats = g.a.stats ? g.a.stats : g.b.stats;
   if (!stats) return;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 0; i < ST_COUNT; i++) {
     const unsigned v = __reduce_max_sync(FULL_MASK, mx[i]);
     if (lane == 0 && v) atomicMax(&bmx[i], v);
   }
   __syncthreads();
-  if (tid < 4 && bmx[tid]) atomicMax(&stats[tid], bmx[tid]);
+  if (tid < ST_COUNT && bmx[tid]) atomicMax(&stats[tid], bmx[tid]);
 }
 
 // Blocks of a tc_pack launch over `rows` panel rows: 32 rows a block, up to eight blocks per SM,
@@ -436,6 +519,7 @@ struct TcParams {
   const float *qmx;       // largest incoming distance of each query's heap row (-inf: none)
   const unsigned *stats;  // candidate maxima (PackStats)
   float kC, kS;           // bound coefficients of CN and of the distances' own scale
+  const float *fscale;    // scale of the FP16 panels (null: 1)
   // Band logs: entry e of a log is a quad, four adjacent columns of the accumulator as the epilogue
   // filtered them (v, or w = -v/2 with the norm column), and the packed position of the first.
   float4 *log;
@@ -525,7 +609,9 @@ struct EpiState {
   // root: this part's heap root; o1 <= o2: the two smallest roots among the other partitions
   // the row reads (as last published); pub: what this part last published
   // Tv: the filter bound on v = d' - qn'; Tw = -Tv/2 the same bound on w = -v/2 (norm column)
+  // (FP16: w in the panels' scale s, Tw = -Tv s^2 / 2, v = -2 w / s^2)
   float qn, E2, thr0, root, o1, o2, pub, thr, Tv, Tw;
+  float vw, wv;  // v = vw * w, w = wv * v: powers of two
   int cnt;   // logged quads
   int done;  // of them, already offered to the heap
   int ovf;
@@ -549,7 +635,7 @@ __device__ __forceinline__ void refresh_threshold(EpiState &s) {
   }
   // filter in the v = d' - qn' space with slack for the rounding of the subtraction
   s.Tv = (s.thr - s.qn) + (fabsf(s.thr) + fabsf(s.qn)) * 2.4e-7f + 1e-30f;
-  s.Tw = -0.5f * s.Tv;  // exact: v <= Tv  <=>  w >= Tw
+  s.Tw = s.wv * s.Tv;  // exact: v <= Tv  <=>  w >= Tw
 }
 
 // Partition lists: every row and part keeps its hk smallest values ascending in shared memory,
@@ -591,8 +677,8 @@ __device__ __forceinline__ float quad_extreme(float a, float b, float c, float d
 }
 // approximate distance d' of a filtered value: v + qn, with v = -2w (exact)
 template <bool FOLD>
-__device__ __forceinline__ float epi_dist(float x, float qn) {
-  return FOLD ? fmaf(-2.0f, x, qn) : x + qn;
+__device__ __forceinline__ float epi_dist(const EpiState &s, float x) {
+  return FOLD ? fmaf(s.vw, x, s.qn) : x + s.qn;
 }
 
 // Publish the list's root to the other partitions and tighten the threshold.
@@ -616,7 +702,7 @@ __device__ __forceinline__ void epi_offer(const EpiState &s, float *heap, int ro
   float x[8];
 #pragma unroll
   for (int j = 0; j < 8; j++) {
-    x[j] = epi_dist<FOLD>(g[j], s.qn);
+    x[j] = epi_dist<FOLD>(s, g[j]);
     // padding columns; and padding rows, whose published root would be query 0's
     if (!(x[j] < Num<float>::inf()) || s.thr0 == -Num<float>::inf()) x[j] = Num<float>::inf();
   }
@@ -636,7 +722,7 @@ __device__ __forceinline__ void epi_flush(EpiState &s, float *heap, const float 
     float x[INSERT_BATCH];
 #pragma unroll
     for (int j = 0; j < INSERT_BATCH; j++)
-      x[j] = e + j < np ? epi_dist<FOLD>(ring[(e + j) * TC_M + row], s.qn) : Num<float>::inf();
+      x[j] = e + j < np ? epi_dist<FOLD>(s, ring[(e + j) * TC_M + row]) : Num<float>::inf();
     list_insert(heap, row, hk, x);
   }
   s.done = s.cnt;
@@ -743,9 +829,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (FOLD) {
     // the all-ones A side of the norm column (every 16-byte chunk alike, so any swizzle of it is
     // the same bytes), made visible to the tensor core's operand reads
+    // (FP16: the weights 2^14, 2^3, 2^-8, then zeros)
     const uint32_t one = FMT == 0 ? 0x3F800000u : 0x3F803F80u;
     uint32_t *an = reinterpret_cast<uint32_t *>(sAn);
-    for (int i = threadIdx.x; i < TC_M * NORM_ROW / 4; i += NTHREADS) an[i] = one;
+    for (int i = threadIdx.x; i < TC_M * NORM_ROW / 4; i += NTHREADS)
+      an[i] = FMT != 1 || !p.fscale ? one
+              : (i & 3) == 0        ? 0x48007400u
+              : (i & 3) == 1        ? 0x00001C00u
+                                    : 0u;
     fence_proxy_async_smem();
   }
   tc_fence_before();
@@ -882,6 +973,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     s.n_fl = s.n_sc = 0;
     unsigned *const pslot = p.proot + (size_t)(valid ? gq : 0) * P + NPART * split + part;
     const unsigned *const prow = p.proot + (size_t)(valid ? gq : 0) * P;
+    {
+      const float fs = FMT == 1 && p.fscale ? *p.fscale : 1.0f;
+      s.wv = -0.5f * (fs * fs);
+      s.vw = 1.0f / s.wv;
+    }
     s.root = Num<float>::inf();
     s.qn = 0.0f;
     s.E2 = 0.0f;
@@ -892,7 +988,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const float E = e.x * __uint_as_float(p.stats[ST_M]) +
                       e.y * __uint_as_float(p.stats[ST_RES]) + e.z +
                       p.kC * __uint_as_float(p.stats[ST_CN]) +
-                      p.kS * __uint_as_float(p.stats[ST_SCALE]);
+                      p.kS * __uint_as_float(p.stats[ST_SCALE]) +
+                      (FOLD ? 2.5f * __uint_as_float(p.stats[ST_NRES]) : 0.0f);
       s.E2 = 2.0f * E;
       const float mx = p.qmx[gq];
       if (mx > -Num<float>::inf()) s.thr0 = mx + s.E2;
@@ -920,9 +1017,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         for (int j = 0; j < 8; j++) {
           const float4 c4 = cn4[j];
           float v0, v1, v2, v3;
-          fma2(v0, v1, __uint_as_float(r[4 * j + 0]), __uint_as_float(r[4 * j + 1]), -2.0f, c4.x,
+          fma2(v0, v1, __uint_as_float(r[4 * j + 0]), __uint_as_float(r[4 * j + 1]), s.vw, c4.x,
                c4.y);
-          fma2(v2, v3, __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]), -2.0f, c4.z,
+          fma2(v2, v3, __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]), s.vw, c4.z,
                c4.w);
           r[4 * j + 0] = __float_as_uint(v0);
           r[4 * j + 1] = __float_as_uint(v1);
@@ -944,7 +1041,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     auto dbg_write = [&](const uint32_t (&r)[32], size_t cbase, int c0) {
       for (int i = 0; i < 32; i++) {
         const long long col = (long long)cbase + c0 + i;
-        const float v = FOLD ? -2.0f * __uint_as_float(r[i]) : __uint_as_float(r[i]);
+        const float v = FOLD ? s.vw * __uint_as_float(r[i]) : __uint_as_float(r[i]);
         if (col < p.dbg_ncols) p.dbg[(size_t)gq * p.dbg_ld + col] = v + s.qn;
       }
     };
@@ -1178,12 +1275,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 template <typename T>
 struct RerankParams {
   int Q, k, S, logcap, d;
-  const float4 *log;        // quads as the epilogue filtered them, d' = qmul * value + qn
+  const float4 *log;        // quads as the epilogue filtered them (log_mul)
   const uint32_t *logpos;   // packed position of each quad's first candidate
   const int *logcnt;
   const float *qn;
   const float *qmx;  // largest incoming distance of each query's heap row (tc_pack)
-  float qmul;
+  int fold;             // the logged values are w (in the panels' scale), else v
+  const float *fscale;  // as in TcParams
   const unsigned *proot;  // partition roots of tc_knn ([query][S]; S counts NPART per split)
   const float *margin;
   const T *Xq, *Xq2, *Xc, *Xc2;
@@ -1202,6 +1300,13 @@ struct RerankParams {
   // and overflowed queries go to the fallback list as their own positions q
   int dedup;
 };
+
+// d' of a logged value x: fma(log_mul, x, qn)
+template <typename T>
+__device__ __forceinline__ float log_mul(const RerankParams<T> &p) {
+  const float fs = p.fscale ? *p.fscale : 1.0f;
+  return p.fold ? -2.0f / (fs * fs) : 1.0f;
+}
 
 // (-2 <q,c> + |c|^2) + |q|^2, clamped at zero
 __device__ __forceinline__ double exact_dist(double dot, double cc, double qq) {
@@ -1442,9 +1547,10 @@ __device__ __forceinline__ float band_limit(float mx, float Eq) {
 }
 
 constexpr int RR_WARPS = 8;
-// CTAs per SM the registers are held to: 64 registers up to 64 neighbours
+// CTAs per SM the registers are held to: 64 registers up to 64 neighbours, 80 beyond (10,395 x 377,
+// k = 114: 467 us with 128 registers, 308 with 80, 325 with 64)
 template <int E>
-constexpr int RR_OCC = E <= 2 ? 4 : 2;
+constexpr int RR_OCC = E <= 2 ? 4 : 3;
 template <int E>
 constexpr int rr_cap() { return E == 1 ? 384 : 512; }  // listed entries per warp (k <= 32 E)
 
@@ -1507,6 +1613,7 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
   if (qrow < 0 || qrow >= p.nrows_q) return;  // reported by tc_pack
   const Tab *qv = p.Xq + qrow * p.d;
   const double qq = (double)p.Xq2[qrow];
+  const float qmul = log_mul(p);
   int n = 0;  // listed entries
 
   // The logs, 32 at a time, as one concatenated list: lane s holds where log g + s starts. Entries
@@ -1564,10 +1671,10 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
           v = p.log[at];
           pos = p.logpos[at];
         }
-        dv[0] = fmaf(p.qmul, v.x, qn);
-        dv[1] = fmaf(p.qmul, v.y, qn);
-        dv[2] = fmaf(p.qmul, v.z, qn);
-        dv[3] = fmaf(p.qmul, v.w, qn);
+        dv[0] = fmaf(qmul, v.x, qn);
+        dv[1] = fmaf(qmul, v.y, qn);
+        dv[2] = fmaf(qmul, v.z, qn);
+        dv[3] = fmaf(qmul, v.w, qn);
       }
       base += 32;
       if (!__any_sync(FULL_MASK,
@@ -1751,6 +1858,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
   if (s_state) return;
   const int total = pre[p.S];
   float thr = s_thr;
+  const float qmul = log_mul(p);
   for (int e = tid; e < total; e += 32 * RR_WARPS) {
     int a = 0, b = p.S;  // the last log that starts at or before e
     while (b - a > 1) {
@@ -1764,7 +1872,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
     const float v[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
     for (int u = 0; u < 4; u++) {
-      const float dv = fmaf(p.qmul, v[u], qn);
+      const float dv = fmaf(qmul, v[u], qn);
       if (dv <= thr) {
         const int to = atomicAdd(&s_n, 1);
         if (to < RC_CAP) list[to] = make_uint2(__float_as_uint(dv), pos + u);
@@ -2044,7 +2152,7 @@ static cudaError_t launch_tc_knn(const TcPlan &P, void *npanel, int npanel_rows,
     if (e == cudaSuccess) kern<<<grid, NTHREADS, smem, st>>>(mA, mAlo, mB, mBlo, mBn, tp);
   };
   if (P.fmt == 0) fold ? go(tc_knn<0, true>) : go(tc_knn<0, false>);
-  else if (P.fmt == 1) fold ? go(tc_knn<1, true>) : go(tc_knn<1, false>);
+  else if (P.fmt != 2) fold ? go(tc_knn<1, true>) : go(tc_knn<1, false>);
   else fold ? go(tc_knn<2, true>) : go(tc_knn<2, false>);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e;
@@ -2055,12 +2163,12 @@ static cudaError_t launch_tc_knn(const TcPlan &P, void *npanel, int npanel_rows,
 static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 int tc_format_of_mode(int mode) {
-  return mode == GSKNN_TC_BF16 ? 1 : mode == GSKNN_TC_BF16X3 ? 2 : 0;
+  return mode == GSKNN_TC_BF16 ? 1 : mode == GSKNN_TC_BF16X3 ? 2 : mode == GSKNN_TC_FP16 ? 3 : 0;
 }
 
-// Prepared-candidate area: mu, mu2, stats, panel(s), norms, norm bounds, ids.
+// Prepared-candidate area: shift, FP16 scale, stats, panel(s), norms, ids.
 struct CandLayout {
-  size_t o_mu, o_mu2, o_cpart, o_stats, o_pb, o_pb_lo, o_pn, o_cn, o_cid, bytes;
+  size_t o_mu, o_fscale, o_cpart, o_stats, o_pb, o_pb_lo, o_pn, o_cn, o_cid, bytes;
   int fmt, elem, d_pad, r_pad;
 };
 
@@ -2075,9 +2183,9 @@ static CandLayout cand_layout(int nc, int d, int mode) {
   size_t off = 0;
   auto take = [&](size_t b) { size_t o = off; off = al256(off + b); return o; };
   L.o_mu = take((size_t)d * 4);
-  L.o_mu2 = take(8);
-  L.o_cpart = take((size_t)CENTER_SLICES * d * 8 + CENTER_SLICES * 4);
-  L.o_stats = take(32);
+  L.o_fscale = take(8);
+  L.o_cpart = take((size_t)CENTER_PARTS * d * 8 + CENTER_SLICES * 4);
+  L.o_stats = take(2 * STATS_WORDS * 4);
   L.o_pb = take((size_t)L.r_pad * L.d_pad * L.elem);
   L.o_pb_lo = L.fmt == 2 ? take((size_t)L.r_pad * L.d_pad * L.elem) : 0;
   L.o_pn = take((size_t)L.r_pad * NORM_ROW);
@@ -2088,7 +2196,10 @@ static CandLayout cand_layout(int nc, int d, int mode) {
 }
 
 static int tc_mode_of_format(int fmt) {
-  return fmt == 1 ? GSKNN_TC_BF16 : fmt == 2 ? GSKNN_TC_BF16X3 : GSKNN_TC_TF32;
+  return fmt == 1   ? GSKNN_TC_BF16
+         : fmt == 2 ? GSKNN_TC_BF16X3
+         : fmt == 3 ? GSKNN_TC_FP16
+                    : GSKNN_TC_TF32;
 }
 
 size_t tc_cand_bytes(int nc, int d, int mode) { return cand_layout(nc, d, mode).bytes; }
@@ -2103,11 +2214,11 @@ static cudaError_t cand_begin(TcCand *C, void *mem, int nc, int d, int mode, con
   char *base = static_cast<char *>(mem);
   C->fmt = L.fmt; C->elem = L.elem; C->d = d; C->d_pad = L.d_pad; C->nc = nc; C->r_pad = L.r_pad;
   C->mu = reinterpret_cast<float *>(base + L.o_mu);
-  C->mu2 = reinterpret_cast<double *>(base + L.o_mu2);
   C->part = reinterpret_cast<double *>(base + L.o_cpart);
-  C->part_n = reinterpret_cast<int *>(base + L.o_cpart + (size_t)CENTER_SLICES * d * 8);
+  C->part_n = reinterpret_cast<int *>(base + L.o_cpart + (size_t)CENTER_PARTS * d * 8);
   C->stats = reinterpret_cast<unsigned *>(base + L.o_stats);
-  C->estats = C->stats + 4;
+  C->estats = C->stats + STATS_WORDS;
+  C->fscale = reinterpret_cast<float *>(base + L.o_fscale);
   C->pb = base + L.o_pb;
   C->pb_lo = L.fmt == 2 ? base + L.o_pb_lo : nullptr;
   C->pn = base + L.o_pn;
@@ -2116,7 +2227,8 @@ static cudaError_t cand_begin(TcCand *C, void *mem, int nc, int d, int mode, con
   C->Xc = Xc; C->Xc2 = Xc2; C->nrows_c = nrows_c; C->cidx = cidx;
   C->efmt = -1; C->epb = nullptr; C->epb_lo = nullptr; C->epn = nullptr;
   tc_center<T><<<dim3((d + 31) / 32, CENTER_SLICES), 32 * CENTER_WARPS, 0, st>>>(
-      Xc, d, nrows_c, cidx, nc, std::min(nc, CENTER_ROWS), C->part, C->part_n, C->stats, 8, clear);
+      Xc, d, nrows_c, cidx, nc, std::min(nc, CENTER_ROWS), C->part, C->part_n, C->stats,
+      2 * STATS_WORDS, clear);
   return cudaGetLastError();
 }
 
@@ -2153,7 +2265,7 @@ static cudaError_t launch_tc_pack(const tc::PackSide<T> &a, const tc::PackSide<T
   g.part = sums ? C.part : nullptr;
   g.part_n = C.part_n;
   g.mu = C.mu;
-  g.mu2 = C.mu2;
+  g.fscale = C.fscale;
   g.kA = kA;
   g.kB = kB;
   g.kS = kS;
@@ -2173,10 +2285,12 @@ cudaError_t tc_cand_prepare(TcCand *C, void *mem, int nc, int d, int mode, const
                                true, 0.0f, 0.0f, 0.0f, status, st);
 }
 
-// Quads per log: `want`, or as many as keep all `logs` logs under 16 GB, but not fewer than fit the
-// 8 * want bytes that a log of `want` single candidates takes.
-static int log_entries(int want, size_t logs) {
-  const size_t fit = ((size_t)16 << 30) / (std::max(logs, (size_t)1) * tc::LOG_ENTRY);
+// Quads per log: `want`, or as many as keep all `logs` logs under `budget` bytes, but not fewer than
+// fit the 8 * want bytes that a log of `want` single candidates takes.
+constexpr size_t LOG_BUDGET = (size_t)16 << 30;
+constexpr size_t LOG_BUDGET_SLOT = (size_t)512 << 20;  // a serving slot's (allocated per engine)
+static int log_entries(int want, size_t logs, size_t budget = LOG_BUDGET) {
+  const size_t fit = budget / (std::max(logs, (size_t)1) * tc::LOG_ENTRY);
   if (fit >= (size_t)want) return want;
   return (int)std::max(fit, (size_t)want * 8 / tc::LOG_ENTRY);
 }
@@ -2204,7 +2318,7 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   // are worth less than the norm column's areas.
   const uint32_t smem_max = 227 * 1024;
   const int lists = NPART * list_slots(tc_heap_k(k));
-  bool fold = P.fmt == 2 || (P.fmt == 1 && P.nkc >= 2);
+  bool fold = P.fmt >= 2 || (P.fmt == 1 && P.nkc >= 2);
   if (const char *v = getenv("GSKNN_TC_FOLD"))
     if (atoi(v) == 0) fold = false;
   int best_N = 0, best_NST = 0;
@@ -2252,7 +2366,8 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   P.smem_fold = smem_fold;
   // (no log needs more than the quads its part of a split holds, and the room that a chunk's eight
   // want)
-  P.logcap = std::min(log_entries(std::max(8 * P.kp, 1024), (size_t)NPART * best_s * nq),
+  P.logcap = std::min(log_entries(std::max(8 * P.kp, 1024), (size_t)NPART * best_s * nq,
+                                  max_splits > 0 ? LOG_BUDGET_SLOT : LOG_BUDGET),
                       P.tiles_per_split * (P.N / NPART / 4) + 8);
   // workspace: [prepared candidates | query side]
   P.cand_bytes = with_cand ? al256(tc_cand_bytes(nc, d, mode)) : 0;
@@ -2281,7 +2396,7 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   // rounds once, inside the kB term. The input rounding itself is measured (tc_pack).
   {
     const double D = (double)P.d_pad;
-    const double u = P.fmt == 0 ? std::ldexp(1.0, -11) : std::ldexp(1.0, -8);
+    const double u = P.fmt == 0 || P.fmt == 3 ? std::ldexp(1.0, -11) : std::ldexp(1.0, -8);
     const double n = (P.fmt == 2 ? 3.0 * D : D) + 3.0;
     const double acc = n * std::ldexp(1.0, -23);
     P.kA = (float)(acc * (1 + u) * (1 + u) + std::ldexp(1.0, -22));
@@ -2310,7 +2425,7 @@ int tc_escalation_mode(int nq, int nc, int d, int k, int mode, int sms) {
   const int fmt = tc_format_of_mode(mode);
   if (fmt == 2) return 0;
   if (tc_plan_base(nq, nc, d, k, GSKNN_TC_BF16X3, sms, false, 0).ok) return GSKNN_TC_BF16X3;
-  if (fmt == 1 && tc_plan_base(nq, nc, d, k, GSKNN_TC_TF32, sms, false, 0).ok)
+  if (fmt != 0 && tc_plan_base(nq, nc, d, k, GSKNN_TC_TF32, sms, false, 0).ok)
     return GSKNN_TC_TF32;
   return 0;
 }
@@ -2422,7 +2537,8 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, bool pack_cand, boo
   tp.Q = nq; tp.k = k; tp.nkc = P.nkc; tp.ntiles_r = P.rtiles;
   tp.N = P.N; tp.NST = P.NST; tp.logcap = P.logcap;
   tp.a_terms = P.a_terms; tp.fmt = P.fmt;
-  tp.idesc = idesc_f32acc(P.fmt == 0 ? 2u : 1u, TC_M, P.N);
+  tp.idesc = idesc_f32acc(P.fmt == 0 ? 2u : P.fmt == 3 ? 0u : 1u, TC_M, P.N);
+  tp.fscale = P.fmt == 3 ? C.fscale : nullptr;
   tp.cn = C.cn; tp.cid = C.cid; tp.qn = qn; tp.qe = qs.qe; tp.qmx = qs.qmx; tp.stats = C.stats;
   tp.log = reinterpret_cast<float4 *>(base + P.o_log);
   tp.logpos = reinterpret_cast<uint32_t *>(tp.log + (size_t)NPART * P.S * nq * P.logcap);
@@ -2449,7 +2565,7 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, bool pack_cand, boo
   RerankParams<T> rp{};
   rp.Q = nq; rp.k = k; rp.S = NPART * P.S; rp.logcap = P.logcap; rp.d = d;
   rp.log = tp.log; rp.logpos = tp.logpos; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
-  rp.qn = tp.qn; rp.qmx = tp.qmx; rp.qmul = tp.fold ? -2.0f : 1.0f;
+  rp.qn = tp.qn; rp.qmx = tp.qmx; rp.fold = tp.fold; rp.fscale = tp.fscale;
   rp.proot = tp.proot;
   rp.Xq = Xq; rp.Xq2 = Xq2; rp.nrows_q = nrows_q;
   rp.Xc = static_cast<const T *>(C.Xc); rp.Xc2 = static_cast<const T *>(C.Xc2);
@@ -2666,9 +2782,10 @@ TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms) {
   TcPlan P = tc_plan_base(256, 256, d, k, GSKNN_TC_BF16X3, sms, false, 1);
   if (!P.ok || npts <= 0 || rows_cap <= 0 || rows_cap % TC_M != 0) return L;
   L.rows_cap = rows_cap;
-  // per-query area for rows_cap rows, one split; smaller logs than the per-call path (a leaf
-  // offers at most a few thousand candidates; a full log overflows to the leaf brute force)
-  P.logcap = log_entries(std::max(2 * P.kp, 256), (size_t)NPART * rows_cap);
+  // per-query area for rows_cap rows, one split; smaller logs than the per-call path: a leaf offers
+  // a few thousand candidates, of which a part logs about hk (1 + ln(n / hk)) < 5 hk quads (a full
+  // log overflows to the leaf brute force)
+  P.logcap = log_entries(6 * tc_heap_k(k) + 32, (size_t)NPART * rows_cap);
   P.S = 1;
   P.qtiles = L.rows_cap / TC_M;
   P.q_pad = L.rows_cap;
@@ -2676,9 +2793,9 @@ TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms) {
   auto take = [&](size_t b) { size_t o = off; off = al256(off + b); return o; };
   const size_t R = (size_t)L.rows_cap;
   L.o_mu = take((size_t)d * 4);
-  L.o_mu2 = take(8);
-  L.o_cpart = take((size_t)CENTER_SLICES * d * 8 + CENTER_SLICES * 4);
-  L.o_stats = take(16);
+  L.o_fscale = take(8);
+  L.o_cpart = take((size_t)CENTER_PARTS * d * 8 + CENTER_SLICES * 4);
+  L.o_stats = take(STATS_WORDS * 4);
   L.o_pb = take(R * P.d_pad * 2);
   L.o_pb_lo = take(R * P.d_pad * 2);
   L.o_pn = take(R * NORM_ROW);
@@ -2717,21 +2834,20 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   if (nqt == 0) return cudaSuccess;
   char *base = static_cast<char *>(ws);
   float *mu = reinterpret_cast<float *>(base + L.o_mu);
-  double *mu2 = reinterpret_cast<double *>(base + L.o_mu2);
   unsigned *stats = reinterpret_cast<unsigned *>(base + L.o_stats);
   void *pb = base + L.o_pb, *pb_lo = base + L.o_pb_lo, *pn = base + L.o_pn;
   float *cn = reinterpret_cast<float *>(base + L.o_cn);
   uint32_t *cid = reinterpret_cast<uint32_t *>(base + L.o_cid);
   int *iota = reinterpret_cast<int *>(base + L.o_iota);
   int *fbc = reinterpret_cast<int *>(base + P.o_fbc);
-  cudaError_t e = cudaMemsetAsync(stats, 0, 16, st);
+  cudaError_t e = cudaMemsetAsync(stats, 0, STATS_WORDS * 4, st);
   if (e != cudaSuccess) return e;
   TcCand C{};
   C.d = d;
   C.mu = mu;
-  C.mu2 = mu2;
+  C.fscale = reinterpret_cast<float *>(base + L.o_fscale);
   C.part = reinterpret_cast<double *>(base + L.o_cpart);
-  C.part_n = reinterpret_cast<int *>(base + L.o_cpart + (size_t)CENTER_SLICES * d * 8);
+  C.part_n = reinterpret_cast<int *>(base + L.o_cpart + (size_t)CENTER_PARTS * d * 8);
   if (setup) {
     // once per workspace: the row index map, and the shift (mean of a strided sample of the
     // first panel's rows, padding skipped), which serves every later tree of the same table
@@ -2796,7 +2912,7 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   RerankParams<float> rp{};
   rp.Q = rows; rp.k = k; rp.S = NPART; rp.logcap = P.logcap; rp.d = d;
   rp.log = tp.log; rp.logpos = tp.logpos; rp.logcnt = tp.logcnt; rp.margin = tp.margin;
-  rp.qn = tp.qn; rp.qmx = tp.qmx; rp.qmul = tp.fold ? -2.0f : 1.0f;
+  rp.qn = tp.qn; rp.qmx = tp.qmx; rp.fold = tp.fold; rp.fscale = tp.fscale;
   rp.proot = tp.proot;
   rp.Xq = X; rp.Xq2 = X2; rp.nrows_q = npts; rp.Xc = X; rp.Xc2 = X2; rp.qidx = iota;
   rp.cid = cid;
