@@ -61,7 +61,7 @@ int set_status(int code, const char *fmt, ...) {
 // ------------------------------------------------------------------------------------------
 // scratch cache
 // ------------------------------------------------------------------------------------------
-enum Slot { SLOT_KERNEL = 0, SLOT_STATUS, SLOT_HQTAB, SLOT_HCTAB, SLOT_HQNRM, SLOT_HCNRM,
+enum Slot { SLOT_KERNEL = 0, SLOT_HQTAB, SLOT_HCTAB, SLOT_HQNRM, SLOT_HCNRM,
             SLOT_HQIDX, SLOT_HCIDX, SLOT_HD, SLOT_HI, SLOT_AUX, SLOT_HGATHER };
 
 struct Buf {
@@ -97,8 +97,51 @@ static cudaError_t scratch(int slot, size_t bytes, cudaStream_t st, void **out) 
   return cudaSuccess;
 }
 
+// Status of the calls of one stream: the device word the kernels report to, and its host-visible
+// mirror (pinned), which the last kernel of a call writes, so that reading the status is one
+// synchronisation and no copy. Kept like the scratch buffers.
+struct StatusWords {
+  int *dev, *mirror_dev, *mirror_host;
+};
+static std::map<std::pair<int, uintptr_t>, StatusWords> g_status;
+
+static cudaError_t status_words(cudaStream_t st, StatusWords *out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(g_mu);
+  const auto key = std::make_pair(dev, (uintptr_t)st);
+  auto it = g_status.find(key);
+  if (it == g_status.end()) {
+    StatusWords w{};
+    e = cudaMalloc((void **)&w.dev, 256);
+    if (e == cudaSuccess) e = cudaHostAlloc((void **)&w.mirror_host, 64, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&w.mirror_dev, w.mirror_host, 0);
+    if (e != cudaSuccess) {
+      if (w.mirror_host) cudaFreeHost(w.mirror_host);
+      if (w.dev) cudaFree(w.dev);
+      (void)cudaGetLastError();
+      return e;
+    }
+    *w.mirror_host = 0;
+    it = g_status.emplace(key, w).first;
+  }
+  *out = it->second;
+  return cudaSuccess;
+}
+
 static void release_all_for_device(int dev) {
   std::lock_guard<std::mutex> lk(g_mu);
+  for (auto it = g_status.begin(); it != g_status.end();) {
+    if (it->first.first == dev) {
+      cudaStreamSynchronize((cudaStream_t)it->first.second);
+      cudaFree(it->second.dev);
+      cudaFreeHost(it->second.mirror_host);
+      it = g_status.erase(it);
+    } else {
+      ++it;
+    }
+  }
   for (auto it = g_bufs.begin(); it != g_bufs.end();) {
     if (std::get<0>(it->first) == dev) {
       cudaStreamSynchronize((cudaStream_t)std::get<1>(it->first));
@@ -297,10 +340,15 @@ static cudaStream_t host_stream() {
 }
 
 static int sm_count() {
+  static std::atomic<int> known[64];
   int dev = 0, n = 148;
   cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && known[dev].load(std::memory_order_relaxed) > 0)
+    return known[dev].load(std::memory_order_relaxed);
   cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n > 0 ? n : 148;
+  if (n <= 0) n = 148;
+  if (dev >= 0 && dev < 64) known[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -383,8 +431,9 @@ template <typename T>
 static int simt_run(const SimtPlan &P, int nq, int nc, int d, int k, const T *Xq, const T *Xq2,
                     long long nrows_q, const int *qidx, const T *Xc, const T *Xc2,
                     long long nrows_c, const int *cidx, T *D, int *I, int ldD, char *base,
-                    int *status, cudaStream_t st, int metric, const int *rows = nullptr,
-                    const int *nrows = nullptr) {
+                    const StatusWords &sw, cudaStream_t st, int metric,
+                    const int *rows = nullptr, const int *nrows = nullptr) {
+  int *status = sw.dev;
   const SimtGeom &g = P.g;
   T *Apack = reinterpret_cast<T *>(base + P.oA);
   T *Bpack = reinterpret_cast<T *>(base + P.oB);
@@ -419,6 +468,8 @@ static int simt_run(const SimtPlan &P, int nq, int nc, int d, int k, const T *Xq
   fa.partD = partD; fa.partI = partI; fa.Dout = D; fa.Iout = I;
   fa.dQ = nrows;
   fa.rowmap = rows;
+  fa.status = status;
+  fa.mirror = sw.mirror_dev;
   {
     TraceScope ts(rows ? "tc_fallback" : "finalize_heap", st);
     CU(launch_finalize<T>(fa, g.kp, st));
@@ -442,13 +493,14 @@ int knn_device_simt(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, lon
   const SimtPlan P = simt_plan<T>(nq, nc, d, k);
   if (P.g.kp == 0)
     return set_status(GSKNN_ERR_UNSUPPORTED, "k=%d exceeds the fused kernel's list size", k);
-  void *ws = nullptr, *stv = nullptr;
+  void *ws = nullptr;
+  StatusWords sw;
   CU(scratch(SLOT_KERNEL, P.bytes, st, &ws));
-  CU(scratch(SLOT_STATUS, 256, st, &stv));
-  int *status = static_cast<int *>(stv);
+  CU(status_words(st, &sw));
+  int *status = sw.dev;
   CU(cudaMemsetAsync(status, 0, sizeof(int), st));
   return simt_run<T>(P, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I, ldD,
-                     static_cast<char *>(ws), status, st, metric);
+                     static_cast<char *>(ws), sw, st, metric);
 }
 
 static int g_mode = GSKNN_MODE_AUTO;
@@ -456,7 +508,7 @@ static int g_mode = GSKNN_MODE_AUTO;
 // Tensor-core approximate pass + FP64 re-rank (float inputs). `dbg`, when set, also receives
 // the approximate distance of every (query, candidate) pair (row stride dbg_ld) and `margin`
 // the per-query band width 2E.
-static int knn_device_tc(int mode, int nq, int nc, int d, int k, const float *Xq,
+static int knn_device_tc(int mode, const TcPlan *plan, int nq, int nc, int d, int k, const float *Xq,
                          const float *Xq2, long long nrows_q, const int *qidx, const float *Xc,
                          const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,
                          int ldD, cudaStream_t st, float *dbg = nullptr, long long dbg_ld = 0,
@@ -468,15 +520,16 @@ static int knn_device_tc(int mode, int nq, int nc, int d, int k, const float *Xq
                       k, ldD);
   if (!Xq || !Xq2 || !qidx || !Xc || !Xc2 || !cidx || !D || !I)
     return set_status(GSKNN_ERR_ARG, "null pointer argument");
-  const TcPlan P = tc_plan(nq, nc, d, k, mode, sm_count());
+  const TcPlan P = plan ? *plan : tc_plan(nq, nc, d, k, mode, sm_count());
   if (!P.ok)
     return set_status(GSKNN_ERR_UNSUPPORTED,
                       "tensor-core mode %d does not support d=%d k=%d (shared memory)", mode, d,
                       k);
-  void *ws = nullptr, *stv = nullptr;
+  void *ws = nullptr;
+  StatusWords sw;
   CU(scratch(SLOT_KERNEL, P.bytes, st, &ws));
-  CU(scratch(SLOT_STATUS, 256, st, &stv));
-  int *status = static_cast<int *>(stv);  // cleared by the first kernel
+  CU(status_words(st, &sw));
+  int *status = sw.dev;  // cleared by the first kernel
   // GSKNN_TC_COUNTERS=1: per-call diagnostics of the tensor-core epilogue on stderr
   static const bool want_counters = std::getenv("GSKNN_TC_COUNTERS") != nullptr;
   unsigned long long *counters = nullptr;
@@ -487,7 +540,7 @@ static int knn_device_tc(int mode, int nq, int nc, int d, int k, const float *Xq
     CU(cudaMemsetAsync(counters, 0, 128, st));
   }
   CU(tc_run(P, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I, ldD, ws,
-            status, dbg, dbg_ld, counters, st, trace_hook, nullptr));
+            status, dbg, dbg_ld, counters, st, trace_hook, nullptr, sw.mirror_dev));
   if (counters) {
     unsigned long long h[16] = {};
     int nfb = 0;
@@ -514,8 +567,8 @@ static int knn_device_tc(int mode, int nq, int nc, int d, int k, const float *Xq
   return set_status(GSKNN_OK, nullptr);
 }
 
-// The tensor-core mode AUTO takes for a shape (GSKNN_MODE_FP32: none fits).
-static int auto_mode(int nq, int nc, int d, int k) {
+// The tensor-core mode AUTO takes for a shape (GSKNN_MODE_FP32: none fits), and its plan.
+static int auto_mode(int nq, int nc, int d, int k, TcPlan *P) {
   // Split BF16 (three MMAs per product) keeps the re-rank band narrowest. One FP16 MMA per product
   // (and half the panel bytes) pays from two K chunks (d > 64) where the contraction bounds the
   // call, about 1.3e10 (pair, padded dimension) products, or the packing does, 2.5e7 (candidate,
@@ -526,19 +579,14 @@ static int auto_mode(int nq, int nc, int d, int k) {
   // escalation's launches). At d <= 64 it gains 18% on uniform points and nothing on the Gaussian
   // mixture, whose band is wider.
   const double d_pad = (d + 63) / 64 * 64, entries = nc * d_pad, products = nq * entries;
-  const bool f16 = tc_plan(nq, nc, d, k, GSKNN_TC_FP16, sm_count()).ok;
-  if (f16 && d > 64 && (products >= 1.3e10 || entries >= (d > 256 ? 9e6 : 2.5e7)))
-    return GSKNN_TC_FP16;
-  if (tc_plan(nq, nc, d, k, GSKNN_TC_BF16X3, sm_count()).ok) return GSKNN_TC_BF16X3;
-  if (f16) return GSKNN_TC_FP16;
-  if (tc_plan(nq, nc, d, k, GSKNN_TC_TF32, sm_count()).ok) return GSKNN_TC_TF32;
+  const bool big = d > 64 && (products >= 1.3e10 || entries >= (d > 256 ? 9e6 : 2.5e7));
+  const int order[4] = {big ? GSKNN_TC_FP16 : GSKNN_TC_BF16X3,
+                        big ? GSKNN_TC_BF16X3 : GSKNN_TC_FP16, GSKNN_TC_TF32, GSKNN_MODE_FP32};
+  for (int i = 0; i < 3; i++) {
+    *P = tc_plan(nq, nc, d, k, order[i], sm_count());
+    if (P->ok) return order[i];
+  }
   return GSKNN_MODE_FP32;
-}
-
-// The arithmetic used for a float call: explicit modes are honoured; AUTO takes the
-// tensor-core form with the exact FP64 re-rank where it fits, else the CUDA-core FP32 kernel.
-static int pick_mode(int nq, int nc, int d, int k) {
-  return g_mode != GSKNN_MODE_AUTO ? g_mode : auto_mode(nq, nc, d, k);
 }
 
 // A double call through the tensor cores: approximate distances with a rigorous bound, exact FP64
@@ -554,23 +602,23 @@ static int knn_device_tc_double(int nq, int nc, int d, int k, const double *Xq, 
   if (nq <= 0 || nc <= 0 || d <= 0 || k <= 0 || ldD < k || !Xq || !Xq2 || !qidx || !Xc || !Xc2 ||
       !cidx || !D || !I)
     return -1;  // (the CUDA-core path reports)
-  const int mode = auto_mode(nq, nc, d, k);
-  if (mode == GSKNN_MODE_FP32) return -1;
-  const TcPlan P = tc_plan(nq, nc, d, k, mode, sm_count());
+  TcPlan P;
+  if (auto_mode(nq, nc, d, k, &P) == GSKNN_MODE_FP32) return -1;
   const SimtPlan F = simt_plan<double>(nq, nc, d, k);
   if (!P.ok || F.g.kp == 0) return -1;
-  void *ws = nullptr, *stv = nullptr;
+  void *ws = nullptr;
+  StatusWords sw;
   const size_t simt_off = align256(P.bytes);
   const cudaError_t se = scratch(SLOT_KERNEL, simt_off + F.bytes, st, &ws);
   if (se == cudaErrorMemoryAllocation) return -1;
   CU(se);
-  CU(scratch(SLOT_STATUS, 256, st, &stv));
-  int *status = static_cast<int *>(stv);  // cleared by the first kernel
+  CU(status_words(st, &sw));
+  int *status = sw.dev;  // cleared by the first kernel
   const int *left = nullptr, *nleft = nullptr;
   CU(tc_run_double(P, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I, ldD, ws,
                    status, &left, &nleft, st, trace_hook, nullptr));
   return simt_run<double>(F, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I,
-                          ldD, static_cast<char *>(ws) + simt_off, status, st, 0, left, nleft);
+                          ldD, static_cast<char *>(ws) + simt_off, sw, st, 0, left, nleft);
 }
 
 template <typename T>
@@ -590,10 +638,11 @@ int knn_device_large(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, lo
     return set_status(GSKNN_ERR_UNSUPPORTED, "k=%d exceeds the selection kernel (k <= %d)", k,
                       sizeof(T) == 8 ? 16384 : 16384);
   const LargePlan P = large_plan<T>(nq, nc, d, k, (size_t)1 << 30);
-  void *ws = nullptr, *stv = nullptr;
+  void *ws = nullptr;
+  StatusWords sw;
   CU(scratch(SLOT_KERNEL, P.bytes, st, &ws));
-  CU(scratch(SLOT_STATUS, 256, st, &stv));
-  int *status = static_cast<int *>(stv);
+  CU(status_words(st, &sw));
+  int *status = sw.dev;
   CU(cudaMemsetAsync(status, 0, sizeof(int), st));
   {
     // two packing launches, then a distance block and a selection per chunk of query rows
@@ -601,6 +650,7 @@ int knn_device_large(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, lo
     CU(large_run<T>(P, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I, ldD,
                     four_ary, ws, status, st, metric));
   }
+  CU(cudaMemcpyAsync(sw.mirror_host, status, sizeof(int), cudaMemcpyDeviceToHost, st));
   return set_status(GSKNN_OK, nullptr);
 }
 
@@ -616,10 +666,16 @@ int knn_device(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, long lon
                               I, ldD, st, metric);
   }
   if constexpr (std::is_same<T, float>::value) {
-    const int mode = pick_mode(nq, nc, d, k);
+    // explicit modes are honoured; AUTO takes the tensor-core form with the exact FP64 re-rank
+    // where it fits, else the CUDA-core FP32 kernel
+    TcPlan P;
+    const int set = g_mode;
+    const int mode = set != GSKNN_MODE_AUTO  ? set
+                     : nq > 0 && nc > 0 && d > 0 && k > 0 ? auto_mode(nq, nc, d, k, &P)
+                                                          : GSKNN_MODE_BF16X3;
     if (mode != GSKNN_MODE_FP32)
-      return knn_device_tc(mode, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx,
-                           D, I, ldD, st);
+      return knn_device_tc(mode, set == GSKNN_MODE_AUTO ? &P : nullptr, nq, nc, d, k, Xq, Xq2,
+                           nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I, ldD, st);
   }
   // lists beyond the fused kernels' capacity: explicit distance block + row selection
   if (simt_geometry<T>(k).kp == 0)
@@ -642,11 +698,10 @@ int knn_device(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, long lon
 
 // Reads back the device status word of `st` (after synchronising it).
 static int device_status(cudaStream_t st) {
-  void *stv = nullptr;
-  CU(scratch(SLOT_STATUS, 256, st, &stv));
+  StatusWords sw;
+  CU(status_words(st, &sw));
   CU(cudaStreamSynchronize(st));
-  int h = 0;
-  CU(cudaMemcpy(&h, stv, sizeof(int), cudaMemcpyDeviceToHost));
+  const int h = *static_cast<volatile int *>(sw.mirror_host);
   if (h == GSKNN_ERR_INDEX)
     return set_status(GSKNN_ERR_INDEX, "an alpha/beta index lies outside its point table");
   if (h == GSKNN_ERR_TIMEOUT)
@@ -819,7 +874,8 @@ int sq2nrm_host(int nq, int nc, int d, const T *Xq, const T *Xq2, const int *qid
     return set_status(GSKNN_ERR_INDEX, "negative point index");
   cudaStream_t st = host_stream();
   const size_t qrows = (size_t)(qhi - qlo + 1), crows = (size_t)(chi - clo + 1);
-  void *pq, *pq2, *pc, *pc2, *pqi, *pci, *pC, *stv, *ws;
+  void *pq, *pq2, *pc, *pc2, *pqi, *pci, *pC, *ws;
+  StatusWords sw;
   CU(scratch(SLOT_HQTAB, qrows * d * sizeof(T), st, &pq));
   CU(scratch(SLOT_HQNRM, qrows * sizeof(T), st, &pq2));
   CU(scratch(SLOT_HCTAB, crows * d * sizeof(T), st, &pc));
@@ -827,14 +883,14 @@ int sq2nrm_host(int nq, int nc, int d, const T *Xq, const T *Xq2, const int *qid
   CU(scratch(SLOT_HQIDX, (size_t)nq * 4, st, &pqi));
   CU(scratch(SLOT_HCIDX, (size_t)nc * 4, st, &pci));
   CU(scratch(SLOT_HD, (size_t)nq * nc * sizeof(T), st, &pC));
-  CU(scratch(SLOT_STATUS, 256, st, &stv));
+  CU(status_words(st, &sw));
   CU(cudaMemcpyAsync(pq, Xq + (size_t)qlo * d, qrows * d * sizeof(T), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(pq2, Xq2 + qlo, qrows * sizeof(T), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(pc, Xc + (size_t)clo * d, crows * d * sizeof(T), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(pc2, Xc2 + clo, crows * sizeof(T), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(pqi, qidx, (size_t)nq * 4, cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(pci, cidx, (size_t)nc * 4, cudaMemcpyHostToDevice, st));
-  int *status = static_cast<int *>(stv);
+  int *status = sw.dev;
   CU(cudaMemsetAsync(status, 0, sizeof(int), st));
   const LargePlan P = large_plan<T>(nq, nc, d, 1, 0);
   CU(scratch(SLOT_KERNEL, P.bytes, st, &ws));
@@ -846,6 +902,7 @@ int sq2nrm_host(int nq, int nc, int d, const T *Xq, const T *Xq2, const int *qid
                     static_cast<const T *>(pc2) - clo, (long long)chi + 1,
                     static_cast<const int *>(pci), static_cast<T *>(pC), nc, ws, status, st));
   }
+  CU(cudaMemcpyAsync(sw.mirror_host, status, sizeof(int), cudaMemcpyDeviceToHost, st));
   int rc = device_status(st);
   if (rc != GSKNN_OK) return rc;
   CU(cudaMemcpy2DAsync(C, (size_t)ldc * sizeof(T), pC, (size_t)nc * sizeof(T),
@@ -917,7 +974,7 @@ int gsknn_tc_distances(int mode, int m, int n, int d, int k, const float *XA, co
   if (mode != GSKNN_MODE_TF32 && mode != GSKNN_MODE_BF16 && mode != GSKNN_MODE_BF16X3)
     return set_status(GSKNN_ERR_ARG, "gsknn_tc_distances: mode must be a tensor-core mode");
   if (C && ldc < m) return set_status(GSKNN_ERR_ARG, "gsknn_tc_distances: ldc < m");
-  return knn_device_tc(mode, n, m, d, k, XB, XB2, nB, beta, XA, XA2, nA, alpha, D, I, ldD,
+  return knn_device_tc(mode, nullptr, n, m, d, k, XB, XB2, nB, beta, XA, XA2, nA, alpha, D, I, ldD,
                        (cudaStream_t)stream, C, ldc, margin);
 }
 

@@ -62,6 +62,8 @@ struct FinalizeArgs {
   int *Iout;
   const int *dQ;         // optional, as in SimtArgs
   const int *rowmap;
+  const int *status;     // the call's status word, copied to the host-visible mirror (may be null):
+  int *mirror;           // this is the call's last kernel
 };
 
 template <typename T>
@@ -192,7 +194,7 @@ cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *X
                    const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,
                    int ldD, void *ws, int *status, float *dbg, long long dbg_ld,
                    unsigned long long *counters, cudaStream_t st, TraceHook hook,
-                   void *hook_ctx);
+                   void *hook_ctx, int *mirror = nullptr);
 // The same for double tables: the approximate pass runs on the centred rows rounded to the MMA
 // format, the re-rank on the double rows, in the CUDA-core kernel's order of operations. Queries
 // that neither it nor the escalation could bound are left: their heap rows at *left, their number

@@ -122,6 +122,7 @@ template <typename T, int E>
 __global__ void __launch_bounds__(256) finalize_heap(FinalizeArgs<T> a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + warp;
+  if (a.mirror && blockIdx.x == 0 && threadIdx.x == 0) *a.mirror = *a.status;
   if (i >= (a.dQ ? *a.dQ : a.Q)) return;
   const int q = a.rowmap ? a.rowmap[i] : i;
   const int k = a.k;

@@ -1947,10 +1947,13 @@ struct FallbackParams {
   int ldD;
   const int *list;
   const int *count;
+  const int *status;  // the call's status word, copied to the host-visible mirror (may be null):
+  int *mirror;        // this is the call's last kernel
 };
 
 template <int E>
 __global__ void __launch_bounds__(256) tc_fallback(FallbackParams p) {
+  if (p.mirror && blockIdx.x == 0 && threadIdx.x == 0) *p.mirror = *p.status;
   __shared__ Ord sd[8][32 * E];
   __shared__ uint32_t si[8][32 * E];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2600,9 +2603,11 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, bool pack_cand, boo
 // Exact FP64 brute force for the queries (heap rows) listed at base + P.o_fbl.
 static cudaError_t tc_brute(const TcPlan &P, const TcCand &C, int d, int k, const float *Xq,
                             const float *Xq2, const int *qidx, float *D, int *I, int ldD,
-                            char *base, cudaStream_t st, TraceHook hook, void *hook_ctx) {
+                            char *base, cudaStream_t st, TraceHook hook, void *hook_ctx,
+                            const int *status = nullptr, int *mirror = nullptr) {
   using namespace tc;
   FallbackParams fp{};
+  fp.status = status; fp.mirror = mirror;
   fp.k = k; fp.d = d; fp.nc = C.nc; fp.Xq = Xq; fp.Xq2 = Xq2;
   fp.Xc = static_cast<const float *>(C.Xc); fp.Xc2 = static_cast<const float *>(C.Xc2);
   fp.qidx = qidx; fp.cidx = C.cidx; fp.nrows_c = C.nrows_c; fp.D = D; fp.I = I; fp.ldD = ldD;
@@ -2690,7 +2695,7 @@ cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *X
                    const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,
                    int ldD, void *ws, int *status, float *dbg, long long dbg_ld,
                    unsigned long long *counters, cudaStream_t st, TraceHook hook,
-                   void *hook_ctx) {
+                   void *hook_ctx, int *mirror) {
   TcCand C{};
   const TcPlan *last;
   char *lbase;
@@ -2699,7 +2704,8 @@ cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *X
                                        nrows_c, cidx, D, I, ldD, ws, status, dbg, dbg_ld, counters,
                                        st, hook, hook_ctx, &last, &lbase, &EP);
   if (e != cudaSuccess) return e;
-  return tc_brute(*last, C, d, k, Xq, Xq2, qidx, D, I, ldD, lbase, st, hook, hook_ctx);
+  return tc_brute(*last, C, d, k, Xq, Xq2, qidx, D, I, ldD, lbase, st, hook, hook_ctx,
+                  status, mirror);
 }
 
 cudaError_t tc_run_double(const TcPlan &P, int nq, int nc, int d, int k, const double *Xq,
