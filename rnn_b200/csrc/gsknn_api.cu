@@ -7,6 +7,7 @@
 #include "gsknn.h"
 #include "knn_internal.h"
 
+#include <cmath>
 #include <algorithm>
 #include <atomic>
 #include <cstdarg>
@@ -353,16 +354,31 @@ static int sm_count() {
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Number of candidate splits per query tile: balances the waves of CTAs over the SMs.
-static int choose_splits(int qtiles, int rtiles, int slots) {
+// Number of candidate splits per query tile of the CUDA-core kernels. A CTA's time is its tiles
+// (about 10 + d/4 us each at 1 or 2 CTAs per SM) plus what its lists take to fill: a split of t
+// candidates inserts about k (1 + ln(t/k)) of them into each query's list, however short it is,
+// so every further split costs the filling again. Splitting to level the waves alone (9, 16, 9,
+// 7 splits) was 1.1 to 2.2 times slower on calls of several waves: 20,000 x 20,000 at d = 32,
+// k = 64 takes 11,630 us in 16 splits and 5,280 in the 2 chosen here; 20,000 x 20,000, k = 16
+// 3,605 and 2,389; 2,000 x 20,000 at d = 100, k = 100 1,780 and 1,352; FP64 4,000 x 8,000 at
+// d = 20, k = 100 2,035 and 1,193 (1-norm calls). Few query tiles take all slots where the lists
+// are short (one query, 1,000,000 candidates, k = 16: 855 us in 64 splits, 576 in about 200);
+// merging lists beyond 64 entries costs more than that gives (8 queries, 46,095 candidates,
+// k = 94: 388 us in 64 splits, 407 in 91).
+static int choose_splits(int qtiles, int rtiles, int slots, int d, int k, int br, int minb,
+                         double merge) {
   int best_s = 1;
   double best = 1e300;
-  const int smax = std::min(rtiles, 64);
+  const int smax = std::min(rtiles, k <= 64 ? std::max(64, slots / qtiles) : 64);
+  const double tile = 10.0 + 0.25 * d, insert = 1.6 * minb * k;  // us, of `minb` CTAs per SM
   for (int s = 1; s <= smax; s++) {
+    const int t = (rtiles + s - 1) / s;
+    if (s > 1 && t == (rtiles + s - 2) / (s - 1)) continue;  // no fewer tiles per CTA
     const long long items = (long long)qtiles * s;
     const double waves = (double)((items + slots - 1) / slots);
-    const double cost = waves / s * (1.0 + 0.004 * s);  // small per-split merge cost
-    if (cost < best - 1e-12) {
+    const double fill = insert * (1.0 + std::log(std::max(1.0, (double)t * br / k)));
+    const double cost = waves * (t * tile + fill) * (1.0 + 0.002 * s) + merge * s;
+    if (cost < best) {
       best = cost;
       best_s = s;
     }
@@ -411,7 +427,10 @@ static SimtPlan simt_plan(int nq, int nc, int d, int k) {
   P.nkc = (d + g.dk - 1) / g.dk;
   P.qtiles = (nq + g.bq - 1) / g.bq;
   P.rtiles = (nc + g.br - 1) / g.br;
-  P.S = choose_splits(P.qtiles, P.rtiles, sm_count() * std::max(1, g.minb));
+  const int minb = std::max(1, g.minb);
+  P.S = choose_splits(std::max(1, P.qtiles), P.rtiles, sm_count() * minb, d, k, g.br, minb,
+                      // us per list that a query merges: a sorting network of kp entries
+                      0.08 * (g.kp / 32) * std::log2((double)g.kp) * (sizeof(T) / 4));
   P.tps = (P.rtiles + P.S - 1) / P.S;
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off = align256(off + bytes); return o; };
