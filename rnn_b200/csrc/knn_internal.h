@@ -137,8 +137,8 @@ struct TcPlan {
   size_t cand_bytes;  // prepared-candidate area at the start of the workspace (0: separate)
   // Escalation: queries whose band log overflowed in this format run again in a narrower one
   // (esc_mode, 0 = none: they go straight to the FP64 brute force). Its query-side workspace
-  // starts at o_esc, over the logs that the re-rank is done with; o_ecand holds its candidate panels when the prepared candidates carry
-  // none (packed only when some query overflowed).
+  // starts at o_esc, over the logs that the re-rank is done with; o_ecand holds its candidate
+  // panels when the prepared candidates carry none (packed only when some query overflowed).
   int esc_mode;
   size_t o_esc, o_ecand, esc_bytes, ecand_bytes;
   int sms, max_splits;  // the plan's arguments, to re-derive the escalation pass's plan

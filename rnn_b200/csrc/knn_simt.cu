@@ -254,7 +254,7 @@ cudaError_t launch_finalize(const FinalizeArgs<T> &a, int kp, cudaStream_t st) {
 #define GSKNN_INST(T)                                                                       \
   template cudaError_t launch_pack<T>(const T *, const T *, int, long long, const int *, int, \
                                       int, int, int, T *, T *, uint32_t *, int *,           \
-                                      cudaStream_t, const int *, const int *);                                        \
+                                      cudaStream_t, const int *, const int *);              \
   template SimtGeom simt_geometry<T>(int);                                                  \
   template cudaError_t launch_simt<T>(const SimtArgs<T> &, int, int, int, cudaStream_t);    \
   template cudaError_t launch_finalize<T>(const FinalizeArgs<T> &, int, cudaStream_t);

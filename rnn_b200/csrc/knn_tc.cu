@@ -1,5 +1,5 @@
 // knn_tc.cu -- the precision form of the fused kNN: tensor-core (tcgen05) distances in TF32,
-// BF16 or split BF16 (hi*hi + hi*lo + lo*hi), with FP32 accumulation in TMEM, followed by an
+// BF16, scaled FP16 or split BF16 (hi*hi + hi*lo + lo*hi), with FP32 accumulation in TMEM, followed by an
 // FP64 re-rank of every candidate whose approximate distance lies within a rigorous rounding
 // bound of the query's k-th approximate distance. The result is the exact FP64 top-k (ties to
 // the lower id) of the caller's inputs, merged into the caller's heaps. Tables are float or double:
@@ -16,9 +16,9 @@
 //                 per TMEM lane quarter, each taking half of every tile's columns) with one
 //                 query row per thread: approximate d' = qn' + cn' - 2<q~,c~> (with the norm
 //                 column, cn' enters through one extra MMA against an all-ones A tile and the
-//                 accumulator holds w = -v/2); per row and epilogue part a max-heap of the
-//                 ceil(k/2) smallest d' of its own columns in shared memory; any two such heaps
-//                 hold k candidates, so the second smallest root a row can see (its own, the
+//                 accumulator holds w = -v/2); per row and epilogue part a sorted
+//                 list of the ceil(k/2) smallest quad minima of its own columns in shared memory;
+//                 any two such lists hold k candidates, so the second smallest root a row can see (its own, the
 //                 other part's, and the roots up to three other splits published) bounds the
 //                 k-th from above (threshold = that + 2E); per-query logs in HBM of every group of
 //                 four adjacent candidates with one under the threshold
@@ -526,8 +526,9 @@ struct TcParams {
   uint32_t *logpos;
   int *logcnt;
   // Partition bound. A query's candidates fall into P = NPART * S partitions (split, part). Each
-  // keeps a heap of the hk = ceil(k / NPART) smallest approximate distances among the quad minima
-  // of its own candidates seen so far (each a real candidate of its own), and publishes its root at proot[query * P + split * NPART + part]
+  // keeps a list of the hk = ceil(k / NPART) smallest approximate distances among the quad minima
+  // of its own candidates seen so far (each a real candidate of its own), and publishes its root
+  // (the list's largest) at proot[query * P + split * NPART + part]
   // (bits of max(root, 0); all bits set while the heap is not full). Any NPART heaps hold at
   // least k real candidates, so the NPART-th smallest root among any partitions of the query --
   // those of its own CTA, and of up to W - 1 other splits as far as they have run -- bounds the
@@ -825,7 +826,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
   // the per-row heaps start at +inf before any epilogue warp reads a root (each part of a lane
   // quarter reads the other's root as part of its bound)
-  for (int i = threadIdx.x; i < NPART * list_slots(p.hk) * TC_M; i += NTHREADS) heap[i] = Num<float>::inf();
+  for (int i = threadIdx.x; i < NPART * list_slots(p.hk) * TC_M; i += NTHREADS)
+    heap[i] = Num<float>::inf();
   if (FOLD) {
     // the all-ones A side of the norm column (every 16-byte chunk alike, so any swizzle of it is
     // the same bytes), made visible to the tensor core's operand reads
@@ -1259,9 +1261,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // ------------------------------------------------------------------------------------------
 // FP64 re-rank of the logged band
 // ------------------------------------------------------------------------------------------
-// What bounds it: latency and, in the batching form, issue. A query's band sits in NPART * S short logs, so a warp that walks them
-// one after another waits for a count, then for a few entries, then for the next count. Here the
-// counts are read at once and scanned, and the logs are read as one concatenated list.
+// What bounds it: latency and, in the batching form, issue. A query's band sits in NPART * S short
+// logs, so a warp that walks them one after another waits for a count, then for a few entries,
+// then for the next count. Here the counts are read at once and scanned, and the logs are read as one concatenated list.
 //   1. entries at or under the partition bound + 2E go into a list in shared memory;
 //   2. a bisection over the listed d' gives a bound on the approximate k-th close to it;
 //   3. exact FP64 distances of the entries at or under that bound (about k of them), merged into
@@ -2316,8 +2318,9 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   while (P.kp < k) P.kp <<= 1;
   if (k > 256) return P;
   // Candidate tile width and pipeline depth that fit in shared memory, and whether the norm column
-  // fits beside them: in split BF16, and in BF16 from two K chunks (measured: config 2 split BF16
-  // -4% in tc_knn, BF16 at d = 256 -1.6%, but BF16 at d = 64 +5%). Three stages of the pipeline
+  // fits beside them: in split BF16 and FP16, and in BF16 from two K chunks (measured in tc_knn:
+  // split BF16 at d = 64 -4%, BF16 at d = 256 -1.6%, but BF16 at d = 64 +5%; split BF16 at d = 64
+  // with five stages in place of the norm column 6,320 us against 5,931). Three stages of the pipeline
   // are worth less than the norm column's areas.
   const uint32_t smem_max = 227 * 1024;
   const int lists = NPART * list_slots(tc_heap_k(k));
