@@ -130,6 +130,7 @@ struct TcPlan {
   // shared memory of the form with the norm column (the candidate norms enter through the MMA; 0:
   // it does not fit)
   unsigned smem_fold;
+  bool ringed;  // without the norm column: the list ring fits shared memory
   // query-side workspace offsets (absolute within the workspace; they start after the
   // prepared-candidate area when the plan includes it)
   size_t o_pa, o_pa_lo, o_qn, o_qe, o_qmx, o_log, o_logcnt, o_proot, o_margin, o_fbl, o_fbc;

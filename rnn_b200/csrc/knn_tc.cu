@@ -571,14 +571,21 @@ constexpr int LIST_BLOCK = 8;
 constexpr int FLUSH_AT = 6;
 constexpr int RING = FLUSH_AT - 1 + 8;
 constexpr int INSERT_BATCH = (RING + 1) / 2;
+// Where shared memory is short (long query panels, long lists) the tiles may only fit without the
+// ring's 13 KB: a flush then reads the quads back from their log, a round trip to L2 for
+// INSERT_BATCH of them. Where both fit the ring is up to a quarter faster, also with a stage fewer
+// (16,384 x 131,072, d = 64, k = 32 in BF16 2,595 us, without 3,319; 4,000 x 60,000, d = 100, k =
+// 100 in split BF16 663 with two stages, without and three 755). Calls that fit only without it
+// would else go to the CUDA cores: 4,096 x 60,000, d = 700, k = 32 8,660 us there, 1,068 here.
 __host__ __device__ inline int list_slots(int hk) {
   return (hk + LIST_BLOCK - 1) / LIST_BLOCK * LIST_BLOCK;
 }
 __host__ __device__ inline int tc_window(int S) { return S < 4 ? S : 4; }
 
-// heap_row: heap entries per row over all epilogue parts; fold: the norm column areas
+// heap_row: heap entries per row over all epilogue parts; ringed: with the ring; fold: the norm
+// column areas
 __host__ __device__ inline SmemLayout tc_smem_layout(int nkc, int a_terms, int N, int NST,
-                                                     int heap_row, bool fold = false) {
+                                                     int heap_row, bool ringed, bool fold) {
   SmemLayout L;
   uint32_t off = 0;
   L.a_off = off;
@@ -592,7 +599,7 @@ __host__ __device__ inline SmemLayout tc_smem_layout(int nkc, int a_terms, int N
   L.heap_off = off;
   off += (uint32_t)heap_row * TC_M * 4;
   L.ring_off = off;
-  off += (uint32_t)NPART * RING * TC_M * 4;
+  off += ringed ? (uint32_t)NPART * RING * TC_M * 4 : 0u;
   off = (off + 15) & ~15u;
   L.cn_off = off;  // candidate norms of the tiles in flight, copied by the MMA warp
   off += fold ? 0u : (uint32_t)CN_SLOTS * N * 4;
@@ -712,18 +719,26 @@ __device__ __forceinline__ void epi_offer(const EpiState &s, float *heap, int ro
 
 // Offer the quads logged since the last flush to the row's list, by their extreme values in the
 // ring (all lanes of the warp together), publish the new root to the other partitions and tighten
-// the threshold. (Reading the quads back from their log instead costs a round trip to L2 per
-// flush.)
-template <bool FOLD>
-__device__ __forceinline__ void epi_flush(EpiState &s, float *heap, const float *ring, int row,
-                                          int hk, unsigned *pslot) {
+// the threshold. Without a ring the quads are read back from their log, `lg`.
+template <bool FOLD, bool RINGED>
+__device__ __forceinline__ void epi_flush(EpiState &s, float *heap, const float *ring,
+                                          const float4 *lg, int row, int hk, unsigned *pslot) {
   s.n_fl++;
   const int np = s.cnt - s.done;
   for (int e = 0; __any_sync(FULL_MASK, e < np); e += INSERT_BATCH) {
     float x[INSERT_BATCH];
 #pragma unroll
-    for (int j = 0; j < INSERT_BATCH; j++)
-      x[j] = e + j < np ? epi_dist<FOLD>(s, ring[(e + j) * TC_M + row]) : Num<float>::inf();
+    for (int j = 0; j < INSERT_BATCH; j++) {
+      x[j] = Num<float>::inf();
+      if (e + j < np) {
+        if constexpr (RINGED) {
+          x[j] = epi_dist<FOLD>(s, ring[(e + j) * TC_M + row]);
+        } else {
+          const float4 v = __ldcg(lg + s.done + e + j);
+          x[j] = epi_dist<FOLD>(s, quad_extreme<FOLD>(v.x, v.y, v.z, v.w));
+        }
+      }
+    }
     list_insert(heap, row, hk, x);
   }
   s.done = s.cnt;
@@ -749,7 +764,7 @@ __device__ __noinline__ int log_compact(float4 *lg, uint32_t *lp, int cnt, const
 // FOLD: the candidate norms enter through the MMA (the norm column, write_norm_row), so the
 // accumulator holds w = -v/2 and the epilogue filters it directly; else the epilogue forms
 // v = cn - 2<q~, c~> from the norms it reads into shared memory.
-template <int FMT, bool FOLD>
+template <int FMT, bool FOLD, bool RINGED>
 __global__ void __launch_bounds__(NTHREADS, 1)
     tc_knn(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tAlo,
            const __grid_constant__ CUtensorMap tB, const __grid_constant__ CUtensorMap tBlo,
@@ -766,7 +781,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const uint32_t raw = su32(smem_raw);
   unsigned char *smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   const SmemLayout L =
-      tc_smem_layout(p.nkc, p.a_terms, p.N, p.NST, NPART * list_slots(p.hk), FOLD);
+      tc_smem_layout(p.nkc, p.a_terms, p.N, p.NST, NPART * list_slots(p.hk), RINGED,
+                     FOLD);
   unsigned char *sA = smem + L.a_off;
   unsigned char *sB = smem + L.b_off;
   unsigned char *sAn = smem + L.an_off;
@@ -1061,7 +1077,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // (a compaction that frees less than half of the log marks it overflowed: repeated
       // compactions that each free a few entries would cost a full read of the log per chunk)
       if (__any_sync(FULL_MASK, s.cnt > p.logcap - 8)) {
-        epi_flush<FOLD>(s, myheap, myring, row, p.hk, pslot);
+        epi_flush<FOLD, RINGED>(s, myheap, myring, lg, row, p.hk, pslot);
         if (s.cnt > p.logcap - 8 && !s.ovf) {
           if (!p.no_compact) s.cnt = s.done = log_compact<FOLD>(lg, lp, s.cnt, s);
           if (s.cnt > p.logcap / 2) {
@@ -1089,7 +1105,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
               : "f"(g[j]), "f"(s.Tw), "l"(at), "r"(r[4 * j]), "r"(r[4 * j + 1]),
                 "r"(r[4 * j + 2]), "r"(r[4 * j + 3]), "l"(pt), "r"(pos + 4 * j), "r"(rp)
               : "memory");
-        else
+        else if constexpr (RINGED)
           asm volatile(
               "{\n\t.reg .pred p;\n\t"
               "setp.le.f32 p, %1, %2;\n\t"
@@ -1101,10 +1117,21 @@ __global__ void __launch_bounds__(NTHREADS, 1)
               : "f"(g[j]), "f"(s.Tv), "l"(at), "r"(r[4 * j]), "r"(r[4 * j + 1]),
                 "r"(r[4 * j + 2]), "r"(r[4 * j + 3]), "l"(pt), "r"(pos + 4 * j), "r"(rp)
               : "memory");
+        else
+          asm volatile(
+              "{\n\t.reg .pred p;\n\t"
+              "setp.le.f32 p, %1, %2;\n\t"
+              "@p st.global.v4.b32 [%3], {%4, %5, %6, %7};\n\t"
+              "@p st.global.b32 [%8], %9;\n\t"
+              "@p add.s32 %0, %0, 1;\n\t}\n"
+              : "+r"(s.cnt)
+              : "f"(g[j]), "f"(s.Tv), "l"(at), "r"(r[4 * j]), "r"(r[4 * j + 1]),
+                "r"(r[4 * j + 2]), "r"(r[4 * j + 3]), "l"(pt), "r"(pos + 4 * j)
+              : "memory");
       }
       if (offered) s.done = s.cnt;  // the lists have these already
       if (__any_sync(FULL_MASK, s.cnt - s.done >= FLUSH_AT))
-        epi_flush<FOLD>(s, myheap, myring, row, p.hk, pslot);
+        epi_flush<FOLD, RINGED>(s, myheap, myring, lg, row, p.hk, pslot);
     };
     // the roots up to three other splits have published (all bits set, which orders last: a list
     // not full yet). The loads for the next tile are issued a tile ahead and their values are
@@ -1238,7 +1265,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (__any_sync(FULL_MASK, hit(mb))) slow(rb, gb, (uint32_t)(cbase + c0 + 32), warm);
       }
     }
-    epi_flush<FOLD>(s, myheap, myring, row, p.hk, pslot);
+    epi_flush<FOLD, RINGED>(s, myheap, myring, lg, row, p.hk, pslot);
     if (valid) p.logcnt[(size_t)lslot * p.Q + gq] = s.cnt | (s.ovf ? (int)LOG_OVF : 0);
     if (p.counters) {
       atomicAdd(&p.counters[0], (unsigned long long)s.cnt);
@@ -2156,9 +2183,15 @@ static cudaError_t launch_tc_knn(const TcPlan &P, void *npanel, int npanel_rows,
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) kern<<<grid, NTHREADS, smem, st>>>(mA, mAlo, mB, mBlo, mBn, tp);
   };
-  if (P.fmt == 0) fold ? go(tc_knn<0, true>) : go(tc_knn<0, false>);
-  else if (P.fmt != 2) fold ? go(tc_knn<1, true>) : go(tc_knn<1, false>);
-  else fold ? go(tc_knn<2, true>) : go(tc_knn<2, false>);
+  if (P.fmt == 0)
+    fold ? go(tc_knn<0, true, true>) : P.ringed ? go(tc_knn<0, false, true>)
+                                                : go(tc_knn<0, false, false>);
+  else if (P.fmt != 2)
+    fold ? go(tc_knn<1, true, true>) : P.ringed ? go(tc_knn<1, false, true>)
+                                                : go(tc_knn<1, false, false>);
+  else
+    fold ? go(tc_knn<2, true, true>) : P.ringed ? go(tc_knn<2, false, true>)
+                                                : go(tc_knn<2, false, false>);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e;
 }
@@ -2320,13 +2353,16 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   // Candidate tile width and pipeline depth that fit in shared memory, and whether the norm column
   // fits beside them: in split BF16 and FP16, and in BF16 from two K chunks (measured in tc_knn:
   // split BF16 at d = 64 -4%, BF16 at d = 256 -1.6%, but BF16 at d = 64 +5%; split BF16 at d = 64
-  // with five stages in place of the norm column 6,320 us against 5,931). Three stages of the pipeline
-  // are worth less than the norm column's areas.
+  // with five stages in place of the norm column 6,320 us against 5,931). Three stages of the
+  // pipeline are worth less than the norm column's areas.
   const uint32_t smem_max = 227 * 1024;
   const int lists = NPART * list_slots(tc_heap_k(k));
   bool fold = P.fmt >= 2 || (P.fmt == 1 && P.nkc >= 2);
   if (const char *v = getenv("GSKNN_TC_FOLD"))
     if (atoi(v) == 0) fold = false;
+  // The limit of the format: two chunks of every term in flight, at the narrow tile.
+  const int least = 2 * P.a_terms;
+  if (tc_smem_layout(P.nkc, P.a_terms, 128, least, lists, false, false).total > smem_max) return P;
   int best_N = 0, best_NST = 0;
   uint32_t smem_fold = 0;
   const int Ns[2] = {256, 128};
@@ -2334,7 +2370,7 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
     const int N = Ns[ni];
     if (P.fmt == 0 && N == 256 && P.nkc > 4) continue;  // keep the TF32 A tile room
     for (int NST = 6; NST >= 2 && !best_N; NST--) {
-      const uint32_t with = tc_smem_layout(P.nkc, P.a_terms, N, NST, lists, true).total;
+      const uint32_t with = tc_smem_layout(P.nkc, P.a_terms, N, NST, lists, true, true).total;
       if (fold && with <= smem_max && NST >= 3) {
         best_N = N;
         best_NST = NST;
@@ -2342,10 +2378,16 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
       }
     }
     for (int NST = 6; NST >= 2 && !best_N; NST--) {
-      if (tc_smem_layout(P.nkc, P.a_terms, N, NST, lists).total <= smem_max) {
+      if (tc_smem_layout(P.nkc, P.a_terms, N, NST, lists, true, false).total <= smem_max) {
         best_N = N;
         best_NST = NST;
       }
+    }
+  }
+  for (int NST = 6; NST >= least && !best_N; NST--) {  // without the ring
+    if (tc_smem_layout(P.nkc, P.a_terms, 128, NST, lists, false, false).total <= smem_max) {
+      best_N = 128;
+      best_NST = NST;
     }
   }
   if (!best_N) return P;
@@ -2368,7 +2410,10 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   P.S = best_s;
   P.tiles_per_split = (P.rtiles + P.S - 1) / P.S;
   P.hk = tc_heap_k(k);
-  P.smem = tc_smem_layout(P.nkc, P.a_terms, P.N, P.NST, lists).total;
+  P.smem = tc_smem_layout(P.nkc, P.a_terms, P.N, P.NST, lists, true, false).total;
+  P.ringed = P.smem <= smem_max;
+  if (!P.ringed)
+    P.smem = tc_smem_layout(P.nkc, P.a_terms, P.N, P.NST, lists, false, false).total;
   P.smem_fold = smem_fold;
   // (no log needs more than the quads its part of a split holds, and the room that a chunk's eight
   // want)
