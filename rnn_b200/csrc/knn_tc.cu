@@ -875,7 +875,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (FMT == 2)
           tma_load_2d(sA + (p.nkc + kc) * A_CHUNK, &tAlo, kc * celems, qt * TC_M, afull);
       }
-      int it = 0;
+      int stage = 0;
+      uint32_t round = 0;  // parity of the stage's use
       if (FOLD) prefetch_tmap(&tBn);
       for (int lt = 0; lt < ntile && !failed; lt++) {
         const int tile = t_begin + lt;
@@ -888,10 +889,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
         // a stage is one K chunk of one term: in split BF16 the hi and lo tiles take stages in
         // turn, which the pipeline refills one by one
-        for (int i = 0; i < TERMS * p.nkc; i++, it++) {
-          const int s = it % p.NST;
-          const uint32_t round = (uint32_t)(it / p.NST);
-          if (!mbar_wait(&empty[s], (round & 1u) ^ 1u)) { failed = true; break; }
+        for (int i = 0; i < TERMS * p.nkc; i++) {
+          const int s = stage;
+          if (!mbar_wait(&empty[s], round ^ 1u)) { failed = true; break; }
+          if (++stage == p.NST) { stage = 0; round ^= 1u; }
           mbar_expect_tx(&full[s], b_stage_bytes);
           tma_load_2d(sB + (uint32_t)s * b_stage_bytes, i % TERMS ? &tBlo : &tB,
                       i / TERMS * celems, tile * N, &full[s]);
@@ -906,7 +907,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (!mbar_wait(afull, 0)) failed = true;
       tc_fence_after();
       const uint32_t a_base = su32(sA), b_base = su32(sB);
-      int it = 0;
+      int stage = 0;
+      uint32_t round = 0;  // parity of the stage's use
       for (int lt = 0; lt < ntile && !failed; lt++) {
         const int b = lt & 1;
         const uint32_t use = (uint32_t)(lt >> 1);
@@ -931,30 +933,38 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                    &cnfull[c]);
           tc_fence_after();
         }
-        for (int i = 0; i < TERMS * p.nkc; i++, it++) {
-          const int s = it % p.NST, kc = i / TERMS;
+        for (int i = 0; i < TERMS * p.nkc; i++) {
+          const int s = stage, kc = i / TERMS;
           const bool lo = i % TERMS != 0;
-          const uint32_t round = (uint32_t)(it / p.NST);
           t0 = p.counters ? clock64() : 0;
-          if (!mbar_wait(&full[s], round & 1u)) { failed = true; break; }
+          if (!mbar_wait(&full[s], round)) { failed = true; break; }
+          if (++stage == p.NST) { stage = 0; round ^= 1u; }
           if (p.counters) w_full += clock64() - t0;
           tc_fence_after();
-          const uint32_t a_chunk = a_base + (uint32_t)kc * A_CHUNK;
-          const uint32_t b_chunk = b_base + (uint32_t)s * b_stage_bytes;
+          // One thread issues all of a CTA's MMAs and, with short ones, its own instructions set the
+          // pace: a division for the stage and descriptors built from scratch for each MMA took
+          // 4.17 M cycles a CTA on 32,768 x 262,144, d = 256, k = 64 in split BF16 (128-column
+          // tiles) and 16.95 ms a call, this 13.58 ms; TF32 there 14.2 -> 11.4 ms; 65,536 x
+          // 262,144, d = 64, k = 32 6.40 -> 5.93 ms. K steps of 32 bytes: two more in a
+          // descriptor's address field (16-byte units).
+          const uint64_t ad = sdesc_k_sw128(a_base + (uint32_t)kc * A_CHUNK);
+          const uint64_t bd = sdesc_k_sw128(b_base + (uint32_t)s * b_stage_bytes);
+          const uint32_t first = FOLD || i != 0 ? 1u : 0u;
+          if (FMT == 2 && !lo) {
+            // hi stage: the query's lo part too
+            const uint64_t ld = sdesc_k_sw128(a_base + (uint32_t)(p.nkc + kc) * A_CHUNK);
 #pragma unroll
-          for (int ks = 0; ks < 4; ks++) {
-            const uint32_t off = (uint32_t)ks * 32u;
-            const uint64_t ad = sdesc_k_sw128(a_chunk + off);
-            const uint64_t bd = sdesc_k_sw128(b_chunk + off);
-            const uint32_t first = (!FOLD && i == 0 && ks == 0) ? 0u : 1u;
-            if (FMT == 0) {
-              mma_tf32(tmem_d, ad, bd, p.idesc, first);
-            } else {
-              mma_f16(tmem_d, ad, bd, p.idesc, first);
-              // hi stage: the query's lo part too; lo stage: the query's hi part alone
-              if (FMT == 2 && !lo)
-                mma_f16(tmem_d, sdesc_k_sw128(a_chunk + (uint32_t)p.nkc * A_CHUNK + off), bd,
-                        p.idesc, 1u);
+            for (int ks = 0; ks < 4; ks++) {
+              mma_f16(tmem_d, ad + 2u * ks, bd + 2u * ks, p.idesc, ks == 0 ? first : 1u);
+              mma_f16(tmem_d, ld + 2u * ks, bd + 2u * ks, p.idesc, 1u);
+            }
+          } else {
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++) {
+              if (FMT == 0)
+                mma_tf32(tmem_d, ad + 2u * ks, bd + 2u * ks, p.idesc, ks == 0 ? first : 1u);
+              else
+                mma_f16(tmem_d, ad + 2u * ks, bd + 2u * ks, p.idesc, ks == 0 ? first : 1u);
             }
           }
           mma_commit(&empty[s]);
