@@ -350,6 +350,14 @@ int gsknn_serve_release(gsknn_serve_t *eng, long long id);
 /* Sets the rows per batch (rounded up to a multiple of 128, at most max_batch_queries; rows <= 0
  * restores the default) and returns the value in effect; applies to batches formed afterwards. */
 int gsknn_serve_set_slice(gsknn_serve_t *eng, int rows);
+/* Device bytes of one slot's workspace under these limits on a device of `sms` SMs (0: d or k
+ * outside the tensor-core form), and the bytes a batch of `rows` rows at `k` takes of it. Host
+ * arithmetic, no GPU. An engine that cannot have the workspaces takes smaller ones (more queries
+ * then finish in the escalation; results are the same). */
+size_t gsknn_serve_workspace_bytes(int nref, int d, int mode, int max_batch_queries, int max_k,
+                                   int sms);
+size_t gsknn_serve_batch_bytes(int nref, int d, int mode, int max_batch_queries, int max_k,
+                               int rows, int k, int sms);
 /* While paused (nonzero) the dispatcher starts no new batch; requests still queue. Running
  * batches finish. Resuming dispatches everything queued in arrival order. */
 int gsknn_serve_pause(gsknn_serve_t *eng, int paused);

@@ -143,6 +143,7 @@ struct TcPlan {
   int esc_mode;
   size_t o_esc, o_ecand, esc_bytes, ecand_bytes;
   int sms, max_splits;  // the plan's arguments, to re-derive the escalation pass's plan
+  bool tight;
   size_t bytes;       // whole workspace
 };
 
@@ -187,9 +188,11 @@ cudaError_t tc_cand_prepare(TcCand *C, void *mem, int nc, int d, int mode, const
 
 // with_cand: the workspace starts with the prepared-candidate area (tc_run); otherwise the
 // plan covers the query side only (tc_run_prepared with separately prepared candidates).
-// max_splits caps the candidate splits per query tile (0: the default, 16).
+// max_splits caps the candidate splits per query tile (0: the default, 16). tight: logs of two
+// fifths of the entries, for when the workspace of the full ones cannot be had. A plan's bytes do
+// not fall as nq grows within a query tile (128 rows).
 TcPlan tc_plan(int nq, int nc, int d, int k, int mode, int sms, bool with_cand = true,
-               int max_splits = 0);
+               int max_splits = 0, bool tight = false);
 cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *Xq,
                    const float *Xq2, long long nrows_q, const int *qidx, const float *Xc,
                    const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,

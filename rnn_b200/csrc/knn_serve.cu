@@ -207,6 +207,7 @@ struct Engine {
   char *arena_mem = nullptr;
   std::unique_ptr<serve::Arena> arena;
   size_t ws_bytes = 0;
+  bool tight = false;  // plans with the smaller logs (tc_plan)
   std::vector<serve::Slot> slots;
   std::mutex mu;
   std::condition_variable cv;     // dispatcher: work or a free slot
@@ -290,7 +291,7 @@ static cudaError_t launch_batch(Engine *E, gs::Slot &s) {
     rows += pc.rows;
     kb = std::max(kb, r.k);
   }
-  const TcPlan P = tc_plan(rows, E->nref, E->d, kb, E->mode, E->sms, false, E->sms);
+  const TcPlan P = tc_plan(rows, E->nref, E->d, kb, E->mode, E->sms, false, E->sms, E->tight);
   if (!P.ok || P.bytes > E->ws_bytes) return cudaErrorInvalidValue;
   cudaStream_t st = s.st;
   cudaError_t e = cudaMemcpyAsync(s.Xq, s.h_q, (size_t)rows * E->d * 4, cudaMemcpyHostToDevice, st);
@@ -501,7 +502,7 @@ static bool probe_modes(Engine *E, int esc) {
   if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess) return false;
   bool ok = cudaMemsetAsync(s.status, 0, sizeof(int), s.st) == cudaSuccess;
   for (int m = 0; m < 2 && ok; m++) {
-    const TcPlan P = tc_plan(rows, E->nref, E->d, kb, modes[m], E->sms, false, E->sms);
+    const TcPlan P = tc_plan(rows, E->nref, E->d, kb, modes[m], E->sms, false, E->sms, E->tight);
     if (!P.ok || P.bytes > E->ws_bytes) {
       E->probe_ms[m] = 1e30;
       continue;
@@ -532,8 +533,101 @@ static bool probe_modes(Engine *E, int esc) {
   return ok;
 }
 
+// The arithmetic an engine prepares its reference set in (AUTO: FP16 where split tiles fit), and
+// the format in which queries whose band overflows finish (0: none).
+static void serve_form(int nref, int d, int max_q, int max_k, int sms, int *mode, int *esc) {
+  using namespace gsknn;
+  if (*mode == GSKNN_MODE_AUTO)
+    *mode = tc_plan(max_q, nref, d, max_k, GSKNN_TC_BF16X3, sms, false, sms).ok ? GSKNN_MODE_FP16
+                                                                               : GSKNN_MODE_TF32;
+  *esc = tc_escalation_mode(max_q, nref, d, max_k, *mode, sms);
+}
+
+// Query-side workspace of a slot: the largest plan over batch sizes and k, in the prepared mode and
+// (AUTO) in the escalation mode run alone; 0 when some plan does not exist. A plan's bytes do not
+// fall with the rows of its last query tile, so whole tiles (and max_q) are the largest batches.
+static size_t serve_workspace(int nref, int d, bool auto_mode, int mode, int esc, int max_q,
+                              int max_k, int sms, bool tight) {
+  using namespace gsknn;
+  size_t bytes = 0;
+  for (int kk = 1; kk <= max_k; kk++)
+    for (int q = 128; q < max_q + 128; q += 128) {
+      const int rows = std::min(q, max_q);
+      const TcPlan P = tc_plan(rows, nref, d, kk, mode, sms, false, sms, tight);
+      if (!P.ok) return 0;
+      bytes = std::max(bytes, P.bytes);
+      if (auto_mode && esc) {
+        const TcPlan P2 = tc_plan(rows, nref, d, kk, esc, sms, false, sms, tight);
+        if (P2.ok) bytes = std::max(bytes, P2.bytes);
+      }
+    }
+  return bytes;
+}
+
+static void free_slots(Engine *E) {
+  for (auto &s : E->slots) {
+    if (s.st) cudaStreamSynchronize(s.st);
+    if (s.done_ev) cudaEventDestroy(s.done_ev);
+    cudaFree(s.Xq); cudaFree(s.Xq2); cudaFree(s.Db); cudaFree(s.Ib); cudaFree(s.qidx);
+    cudaFree(s.status); cudaFree(s.reqs_d); cudaFree(s.ws);
+    if (s.h_q) cudaFreeHost(s.h_q);
+    if (s.h_reqs) cudaFreeHost(s.h_reqs);
+    if (s.st) cudaStreamDestroy(s.st);
+  }
+  E->slots.clear();
+}
+
+static bool make_slots(Engine *E) {
+  E->slots.resize(E->nslots);
+  for (int i = 0; i < E->nslots; i++) {
+    gs::Slot &s = E->slots[i];
+    s.eng = E;
+    s.index = i;
+    const size_t q = (size_t)E->max_q, d = (size_t)E->d;
+    if (cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMalloc((void **)&s.Xq, q * d * 4) != cudaSuccess ||
+        cudaMalloc((void **)&s.Xq2, q * 4) != cudaSuccess ||
+        cudaMalloc((void **)&s.Db, q * E->kp_max * 4) != cudaSuccess ||
+        cudaMalloc((void **)&s.Ib, q * E->kp_max * 4) != cudaSuccess ||
+        cudaMalloc((void **)&s.qidx, q * 4) != cudaSuccess ||
+        cudaMalloc((void **)&s.status, 64) != cudaSuccess ||
+        cudaMalloc((void **)&s.reqs_d, (q + 1) * sizeof(gs::ReqDesc)) != cudaSuccess ||
+        cudaMalloc(&s.ws, E->ws_bytes) != cudaSuccess ||
+        cudaHostAlloc((void **)&s.h_q, q * d * 4, cudaHostAllocDefault) != cudaSuccess ||
+        cudaHostAlloc((void **)&s.h_reqs, (q + 2) * sizeof(gs::ReqDesc), cudaHostAllocDefault) !=
+            cudaSuccess)
+      return false;
+    gs::iota<<<(E->max_q + 255) / 256, 256, 0, s.st>>>(s.qidx, E->max_q);
+    if (cudaStreamSynchronize(s.st) != cudaSuccess) return false;
+  }
+  return true;
+}
 
 extern "C" {
+
+size_t gsknn_serve_workspace_bytes(int nref, int d, int mode, int max_batch_queries, int max_k,
+                                   int sms) {
+  if (nref <= 0 || d <= 0 || max_batch_queries <= 0 || max_k <= 0 || max_k > 256 || sms <= 0)
+    return 0;
+  int main = mode, esc = 0;
+  serve_form(nref, d, max_batch_queries, max_k, sms, &main, &esc);
+  return serve_workspace(nref, d, mode == GSKNN_MODE_AUTO, main, esc, max_batch_queries, max_k,
+                         sms, false);
+}
+
+size_t gsknn_serve_batch_bytes(int nref, int d, int mode, int max_batch_queries, int max_k,
+                               int rows, int k, int sms) {
+  using namespace gsknn;
+  if (nref <= 0 || d <= 0 || rows <= 0 || rows > max_batch_queries || k <= 0 || k > max_k ||
+      max_k > 256 || sms <= 0)
+    return 0;
+  int main = mode, esc = 0;
+  serve_form(nref, d, max_batch_queries, max_k, sms, &main, &esc);
+  size_t bytes = tc_plan(rows, nref, d, k, main, sms, false, sms).bytes;
+  if (mode == GSKNN_MODE_AUTO && esc)
+    bytes = std::max(bytes, tc_plan(rows, nref, d, k, esc, sms, false, sms).bytes);
+  return bytes;
+}
 
 gsknn_serve_t *gsknn_serve_create(const float *R, const float *R2, int nref, int d, int mode,
                                   int max_batch_queries, int max_k, size_t heap_budget,
@@ -549,16 +643,12 @@ gsknn_serve_t *gsknn_serve_create(const float *R, const float *R2, int nref, int
   // with escalation, and split BF16 alone on the escalation panels -- and serves with the
   // faster. Where split tiles do not fit, TF32.
   const bool auto_mode = mode == GSKNN_MODE_AUTO;
-  if (auto_mode)
-    mode = tc_plan(max_batch_queries, nref, d, max_k, GSKNN_TC_BF16X3, 148, false, 148).ok
-               ? GSKNN_MODE_FP16
-               : GSKNN_MODE_TF32;
-  else if (mode < GSKNN_MODE_TF32 || mode > GSKNN_MODE_BF16X3) {
+  if (!auto_mode && (mode < GSKNN_MODE_TF32 || mode > GSKNN_MODE_BF16X3)) {
     serr(GSKNN_ERR_ARG, "gsknn_serve_create: mode must be AUTO, TF32, BF16 or BF16X3");
     return nullptr;
   }
   auto E = std::make_unique<Engine>();
-  E->nref = nref; E->d = d; E->mode = mode; E->max_q = max_batch_queries; E->max_k = max_k;
+  E->nref = nref; E->d = d; E->max_q = max_batch_queries; E->max_k = max_k;
   E->heap_budget = heap_budget; E->nslots = slots;
   E->kp_max = 32;
   while (E->kp_max < max_k) E->kp_max <<= 1;
@@ -566,22 +656,14 @@ gsknn_serve_t *gsknn_serve_create(const float *R, const float *R2, int nref, int
   cudaGetDevice(&dev);
   E->device = dev;
   cudaDeviceGetAttribute(&E->sms, cudaDevAttrMultiProcessorCount, dev);
-  // query-side workspace: the largest plan over batch sizes (whole query tiles) and k, in the
-  // prepared mode and (AUTO) in the escalation mode run alone
-  const int esc = tc_escalation_mode(E->max_q, nref, d, max_k, mode, E->sms);
-  for (int kk = 1; kk <= max_k; kk++)
-    for (int q = 128; q < E->max_q + 128; q += 128) {
-      const TcPlan P = tc_plan(std::min(q, E->max_q), nref, d, kk, mode, E->sms, false, E->sms);
-      if (!P.ok) {
-        serr(GSKNN_ERR_UNSUPPORTED, "gsknn_serve_create: d or k outside the tensor-core form");
-        return nullptr;
-      }
-      E->ws_bytes = std::max(E->ws_bytes, P.bytes);
-      if (auto_mode && esc) {
-        const TcPlan P2 = tc_plan(std::min(q, E->max_q), nref, d, kk, esc, E->sms, false, E->sms);
-        if (P2.ok) E->ws_bytes = std::max(E->ws_bytes, P2.bytes);
-      }
-    }
+  int esc = 0;
+  serve_form(nref, d, E->max_q, max_k, E->sms, &mode, &esc);
+  E->mode = mode;
+  E->ws_bytes = serve_workspace(nref, d, auto_mode, mode, esc, E->max_q, max_k, E->sms, false);
+  if (E->ws_bytes == 0) {
+    serr(GSKNN_ERR_UNSUPPORTED, "gsknn_serve_create: d or k outside the tensor-core form");
+    return nullptr;
+  }
   const size_t cb = tc_cand_bytes(nref, d, mode);
   // queries whose band log overflows in this format run again in a narrower one: its panels of
   // the resident set are prepared once, beside the first
@@ -615,28 +697,13 @@ gsknn_serve_t *gsknn_serve_create(const float *R, const float *R2, int nref, int
     gsknn_serve_destroy(reinterpret_cast<gsknn_serve_t *>(E.release()));
     return nullptr;
   }
-  E->slots.resize(slots);
-  for (int i = 0; i < slots; i++) {
-    gs::Slot &s = E->slots[i];
-    s.eng = E.get();
-    s.index = i;
-    const size_t q = (size_t)E->max_q;
-    ok = cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking) == cudaSuccess &&
-         cudaMalloc((void **)&s.Xq, q * d * 4) == cudaSuccess &&
-         cudaMalloc((void **)&s.Xq2, q * 4) == cudaSuccess &&
-         cudaMalloc((void **)&s.Db, q * E->kp_max * 4) == cudaSuccess &&
-         cudaMalloc((void **)&s.Ib, q * E->kp_max * 4) == cudaSuccess &&
-         cudaMalloc((void **)&s.qidx, q * 4) == cudaSuccess &&
-         cudaMalloc((void **)&s.status, 64) == cudaSuccess &&
-         cudaMalloc((void **)&s.reqs_d, (q + 1) * sizeof(gs::ReqDesc)) == cudaSuccess &&
-         cudaMalloc(&s.ws, E->ws_bytes) == cudaSuccess &&
-         cudaHostAlloc((void **)&s.h_q, q * d * 4, cudaHostAllocDefault) == cudaSuccess &&
-         cudaHostAlloc((void **)&s.h_reqs, (q + 2) * sizeof(gs::ReqDesc),
-                       cudaHostAllocDefault) == cudaSuccess;
-    if (!ok) break;
-    gs::iota<<<(E->max_q + 255) / 256, 256, 0, s.st>>>(s.qidx, E->max_q);
-    ok = cudaStreamSynchronize(s.st) == cudaSuccess;
-    if (!ok) break;
+  ok = make_slots(E.get());
+  if (!ok && cudaGetLastError() == cudaErrorMemoryAllocation) {
+    // smaller logs before giving up: more queries overflow to the escalation, results are the same
+    free_slots(E.get());
+    E->tight = true;
+    E->ws_bytes = serve_workspace(nref, d, auto_mode, mode, esc, E->max_q, max_k, E->sms, true);
+    ok = make_slots(E.get());
   }
   if (!ok) {
     cudaGetLastError();
@@ -826,15 +893,7 @@ void gsknn_serve_destroy(gsknn_serve_t *eng) {
   E->ccv.notify_all();
   if (E->dispatcher.joinable()) E->dispatcher.join();
   if (E->completer.joinable()) E->completer.join();
-  for (auto &s : E->slots) {
-    if (s.st) cudaStreamSynchronize(s.st);
-    if (s.done_ev) cudaEventDestroy(s.done_ev);
-    cudaFree(s.Xq); cudaFree(s.Xq2); cudaFree(s.Db); cudaFree(s.Ib); cudaFree(s.qidx);
-    cudaFree(s.status); cudaFree(s.reqs_d); cudaFree(s.ws);
-    if (s.h_q) cudaFreeHost(s.h_q);
-    if (s.h_reqs) cudaFreeHost(s.h_reqs);
-    if (s.st) cudaStreamDestroy(s.st);
-  }
+  free_slots(E);
   cudaFree(E->cand_mem);
   cudaFree(E->ecand_mem);
   cudaFree(E->cidx);

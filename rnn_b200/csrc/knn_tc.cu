@@ -48,6 +48,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 
 namespace gsknn {
 namespace tc {
@@ -2334,9 +2335,8 @@ cudaError_t tc_cand_prepare(TcCand *C, void *mem, int nc, int d, int mode, const
 }
 
 // Quads per log: `want`, or as many as keep all `logs` logs under `budget` bytes, but not fewer than
-// fit the 8 * want bytes that a log of `want` single candidates takes.
+// fit the 8 * want bytes that a log of `want` single candidates takes (a tight plan's logs).
 constexpr size_t LOG_BUDGET = (size_t)16 << 30;
-constexpr size_t LOG_BUDGET_SLOT = (size_t)512 << 20;  // a serving slot's (allocated per engine)
 static int log_entries(int want, size_t logs, size_t budget = LOG_BUDGET) {
   const size_t fit = budget / (std::max(logs, (size_t)1) * tc::LOG_ENTRY);
   if (fit >= (size_t)want) return want;
@@ -2344,12 +2344,13 @@ static int log_entries(int want, size_t logs, size_t budget = LOG_BUDGET) {
 }
 
 static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool with_cand,
-                          int max_splits) {
+                          int max_splits, bool tight = false) {
   using namespace tc;
   TcPlan P{};
   P.ok = false;
   P.sms = sms;
   P.max_splits = max_splits;
+  P.tight = tight;
   P.fmt = tc_format_of_mode(mode);
   const int elem = P.fmt == 0 ? 4 : 2;
   const int celems = CHUNK_BYTES / elem;
@@ -2426,9 +2427,12 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
     P.smem = tc_smem_layout(P.nkc, P.a_terms, P.N, P.NST, lists, false, false).total;
   P.smem_fold = smem_fold;
   // (no log needs more than the quads its part of a split holds, and the room that a chunk's eight
-  // want)
+  // want; a serving slot's workspace is allocated once, for the largest of its batches, so the
+  // entries there depend on the splits and on k alone)
   P.logcap = std::min(log_entries(std::max(8 * P.kp, 1024), (size_t)NPART * best_s * nq,
-                                  max_splits > 0 ? LOG_BUDGET_SLOT : LOG_BUDGET),
+                                  tight            ? 0
+                                  : max_splits > 0 ? SIZE_MAX
+                                                   : LOG_BUDGET),
                       P.tiles_per_split * (P.N / NPART / 4) + 8);
   // workspace: [prepared candidates | query side]
   P.cand_bytes = with_cand ? al256(tc_cand_bytes(nc, d, mode)) : 0;
@@ -2492,12 +2496,12 @@ int tc_escalation_mode(int nq, int nc, int d, int k, int mode, int sms) {
 }
 
 TcPlan tc_plan(int nq, int nc, int d, int k, int mode, int sms, bool with_cand,
-               int max_splits) {
-  TcPlan P = tc_plan_base(nq, nc, d, k, mode, sms, with_cand, max_splits);
+               int max_splits, bool tight) {
+  TcPlan P = tc_plan_base(nq, nc, d, k, mode, sms, with_cand, max_splits, tight);
   if (!P.ok) return P;
   P.esc_mode = tc_escalation_mode(nq, nc, d, k, mode, sms);
   if (P.esc_mode) {
-    const TcPlan EP = tc_plan_base(nq, nc, d, k, P.esc_mode, sms, false, max_splits);
+    const TcPlan EP = tc_plan_base(nq, nc, d, k, P.esc_mode, sms, false, max_splits, tight);
     P.o_esc = P.o_log;
     P.esc_bytes = EP.bytes;
     size_t off = al256(std::max(P.bytes, P.o_esc + EP.bytes));
@@ -2704,7 +2708,7 @@ static cudaError_t tc_passes(const TcPlan &P, const TcCand &C, bool per_call, in
                              hook_ctx);
   if (e != cudaSuccess || !P.esc_mode) return e;
   TcPlan &EP = *EPout;
-  EP = tc_plan_base(nq, C.nc, d, k, P.esc_mode, P.sms, false, P.max_splits);
+  EP = tc_plan_base(nq, C.nc, d, k, P.esc_mode, P.sms, false, P.max_splits, P.tight);
   void *epb = nullptr, *epb_lo = nullptr, *epn = nullptr;
   bool pack = false;
   if (EP.ok && C.efmt == EP.fmt) {
