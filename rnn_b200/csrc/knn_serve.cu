@@ -486,7 +486,7 @@ static int auto_slice(const Engine *E) {
 }
 
 // Times one probe batch (the first resident points as queries, as many as a batch of requests
-// holds but at most 2,048, k = max_k) in the prepared mode with escalation and in the escalation
+// holds, but at most 2,048 and no more than there are; k = max_k) in the prepared mode with escalation and in the escalation
 // mode alone; keeps the faster (second of two runs each, on slot 0's buffers). Returns false when a
 // probe call fails.
 // (Probes of 1,024 rows took the two forms to be level where batches of 2,176 ran 1.4 times
@@ -494,7 +494,7 @@ static int auto_slice(const Engine *E) {
 static bool probe_modes(Engine *E, int esc) {
   using namespace gsknn;
   gs::Slot &s = E->slots[0];
-  const int rows = std::min(auto_slice(E), 2048), kb = E->max_k;
+  const int rows = std::min(std::min(auto_slice(E), 2048), E->nref), kb = E->max_k;
   const TcCand Cesc = escalation_as_main(E->C, esc);
   const int modes[2] = {E->mode, esc};
   const TcCand *cands[2] = {&E->C, &Cesc};
