@@ -569,6 +569,7 @@ __host__ __device__ inline int tc_heap_k(int k) { return (k + NPART - 1) / NPART
 // of the quads a lane has logged but not yet offered to its list wait in a ring in shared memory:
 // a warp offers them once any lane has FLUSH_AT (a chunk may add eight), INSERT_BATCH at a time.
 constexpr int LIST_BLOCK = 8;
+constexpr int LOG_ROOM = 16;  // quads that two chunks of 32 columns may log
 constexpr int FLUSH_AT = 6;
 constexpr int RING = FLUSH_AT - 1 + 8;
 constexpr int INSERT_BATCH = (RING + 1) / 2;
@@ -746,20 +747,47 @@ __device__ __forceinline__ void epi_flush(EpiState &s, float *heap, const float 
   epi_publish(s, heap, row, hk, pslot);
 }
 
-// Drops log entries above the current threshold (all of them already offered to the heap);
-// returns the new count.
+// Drops the entries above the current threshold (the filter bound Tw or Tv) from the logs of the
+// lanes that `want` it, all of them already offered to the lists; returns the lane's new count. The
+// warp takes one log after the other, 32 entries at a time with coalesced loads. One lane per log, an
+// entry at a time, is a chain of round trips to L2 while the tile's other rows wait: 17.2 M
+// cycles a CTA on 16,384 x 60,000, d = 80, k = 32 in split BF16 on clusters of sigma 0.01, 2.65 M so.
 template <bool FOLD>
-__device__ __noinline__ int log_compact(float4 *lg, uint32_t *lp, int cnt, const EpiState &s) {
-  int w = 0;
-  for (int e = 0; e < cnt; e++) {
-    const float4 v = __ldcg(lg + e);
-    const uint32_t pos = __ldcg(lp + e);
-    if (epi_hit<FOLD>(s, quad_extreme<FOLD>(v.x, v.y, v.z, v.w))) {
-      lg[w] = v;
-      lp[w++] = pos;
+__device__ __noinline__ int log_compact(float4 *lg, uint32_t *lp, int cnt, float bound, bool want) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();  // the logs' stores before the other lanes' loads
+  for (unsigned m = __ballot_sync(FULL_MASK, want); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    float4 *const l = reinterpret_cast<float4 *>(
+        __shfl_sync(FULL_MASK, reinterpret_cast<unsigned long long>(lg), src));
+    uint32_t *const p = reinterpret_cast<uint32_t *>(
+        __shfl_sync(FULL_MASK, reinterpret_cast<unsigned long long>(lp), src));
+    const int n = __shfl_sync(FULL_MASK, cnt, src);
+    const float bnd = __shfl_sync(FULL_MASK, bound, src);
+    int w = 0;
+    for (int e = 0; e < n; e += 32) {
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      uint32_t pos = 0u;
+      const bool in = e + lane < n;
+      if (in) {
+        v = __ldcg(l + e + lane);
+        pos = __ldcg(p + e + lane);
+      }
+      const float x = quad_extreme<FOLD>(v.x, v.y, v.z, v.w);
+      const bool keep = in && (FOLD ? x >= bnd : x <= bnd);
+      const unsigned k = __ballot_sync(FULL_MASK, keep);
+      __syncwarp();  // all of the step's loads before its stores, which may reach their places
+      if (keep) {
+        const int at = w + __popc(k & ((1u << lane) - 1u));
+        l[at] = v;
+        p[at] = pos;
+      }
+      w += __popc(k);
     }
+    if (lane == src) cnt = w;
   }
-  return w;
+  __syncwarp();
+  return cnt;
 }
 
 // FOLD: the candidate norms enter through the MMA (the norm column, write_norm_row), so the
@@ -1085,18 +1113,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // 2,003 x 30,011, d = 20 105 -> 64 us; 16 x 4,096 42 -> 10 us; 8 trees over 262,144 points
     // 6.1 -> 3.1 ms.
     auto slow = [&](const uint32_t (&r)[32], const float (&g)[8], uint32_t pos, bool offered) {
-      // (a compaction that frees less than half of the log marks it overflowed: repeated
-      // compactions that each free a few entries would cost a full read of the log per chunk)
-      if (__any_sync(FULL_MASK, s.cnt > p.logcap - 8)) {
-        epi_flush<FOLD, RINGED>(s, myheap, myring, lg, row, p.hk, pslot);
-        if (s.cnt > p.logcap - 8 && !s.ovf) {
-          if (!p.no_compact) s.cnt = s.done = log_compact<FOLD>(lg, lp, s.cnt, s);
-          if (s.cnt > p.logcap / 2) {
-            s.ovf = 1;
-            refresh_threshold(s);
-          }
-        }
-      }
       s.n_sc++;
       const uint32_t rbase = su32(myring + row);
 #pragma unroll
@@ -1143,6 +1159,24 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (offered) s.done = s.cnt;  // the lists have these already
       if (__any_sync(FULL_MASK, s.cnt - s.done >= FLUSH_AT))
         epi_flush<FOLD, RINGED>(s, myheap, myring, lg, row, p.hk, pslot);
+    };
+    // Logs without room for another two chunks drop what has left the band. Called between chunks,
+    // when no accumulator values are held: the call's registers would else be spilled around it,
+    // 1.2 times the ordinary pass's time. (A compaction that frees less than half of the log marks
+    // it overflowed: repeated compactions that each free a few entries would cost a full read of the
+    // log per chunk.)
+    auto make_room = [&]() {
+      if (!__any_sync(FULL_MASK, s.cnt > p.logcap - LOG_ROOM)) return;
+      epi_flush<FOLD, RINGED>(s, myheap, myring, lg, row, p.hk, pslot);
+      const bool full = s.cnt > p.logcap - LOG_ROOM && !s.ovf;
+      if (!p.no_compact) {
+        const int left = log_compact<FOLD>(lg, lp, s.cnt, FOLD ? s.Tw : s.Tv, full);
+        if (full) s.cnt = s.done = left;
+      }
+      if (full && s.cnt > p.logcap / 2) {
+        s.ovf = 1;
+        refresh_threshold(s);
+      }
     };
     // the roots up to three other splits have published (all bits set, which orders last: a list
     // not full yet). The loads for the next tile are issued a tile ahead and their values are
@@ -1272,8 +1306,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           dbg_write(ra, cbase, c0);
           dbg_write(rb, cbase, c0 + 32);
         }
-        if (__any_sync(FULL_MASK, hit(ma))) slow(ra, ga, (uint32_t)(cbase + c0), warm);
-        if (__any_sync(FULL_MASK, hit(mb))) slow(rb, gb, (uint32_t)(cbase + c0 + 32), warm);
+        const bool ha = __any_sync(FULL_MASK, hit(ma));
+        if (ha) slow(ra, ga, (uint32_t)(cbase + c0), warm);
+        const bool hb = __any_sync(FULL_MASK, hit(mb));
+        if (hb) slow(rb, gb, (uint32_t)(cbase + c0 + 32), warm);
+        if (ha || hb) make_room();
       }
     }
     epi_flush<FOLD, RINGED>(s, myheap, myring, lg, row, p.hk, pslot);
@@ -2335,12 +2372,13 @@ cudaError_t tc_cand_prepare(TcCand *C, void *mem, int nc, int d, int mode, const
 }
 
 // Quads per log: `want`, or as many as keep all `logs` logs under `budget` bytes, but not fewer than
-// fit the 8 * want bytes that a log of `want` single candidates takes (a tight plan's logs).
+// fit the 8 * want bytes that a log of `want` single candidates takes (a tight plan's logs), nor than
+// leave half a log for the room that two chunks want.
 constexpr size_t LOG_BUDGET = (size_t)16 << 30;
 static int log_entries(int want, size_t logs, size_t budget = LOG_BUDGET) {
   const size_t fit = budget / (std::max(logs, (size_t)1) * tc::LOG_ENTRY);
   if (fit >= (size_t)want) return want;
-  return (int)std::max(fit, (size_t)want * 8 / tc::LOG_ENTRY);
+  return (int)std::max({fit, (size_t)want * 8 / tc::LOG_ENTRY, (size_t)(2 * tc::LOG_ROOM)});
 }
 
 static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool with_cand,
@@ -2426,14 +2464,13 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   if (!P.ringed)
     P.smem = tc_smem_layout(P.nkc, P.a_terms, P.N, P.NST, lists, false, false).total;
   P.smem_fold = smem_fold;
-  // (no log needs more than the quads its part of a split holds, and the room that a chunk's eight
-  // want; a serving slot's workspace is allocated once, for the largest of its batches, so the
+  // (no log needs more than the quads its part of a split holds, and the room that two chunks want; a serving slot's workspace is allocated once, for the largest of its batches, so the
   // entries there depend on the splits and on k alone)
   P.logcap = std::min(log_entries(std::max(8 * P.kp, 1024), (size_t)NPART * best_s * nq,
                                   tight            ? 0
                                   : max_splits > 0 ? SIZE_MAX
                                                    : LOG_BUDGET),
-                      P.tiles_per_split * (P.N / NPART / 4) + 8);
+                      P.tiles_per_split * (P.N / NPART / 4) + LOG_ROOM);
   // workspace: [prepared candidates | query side]
   P.cand_bytes = with_cand ? al256(tc_cand_bytes(nc, d, mode)) : 0;
   size_t off = P.cand_bytes;
