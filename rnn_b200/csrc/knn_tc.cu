@@ -30,13 +30,13 @@
 //
 // Error bound (per query q, all candidates c; r(x) = |x - fmt(x)|, the norm of a row's rounding
 // residual, measured per row; M = max |c~|, R = max r(c~), CN = max |cn'|, D = padded dimension,
-// n = D + 3 accumulated terms, u = unit roundoff of the MMA input format):
+// n = D + NORM_TERMS accumulated terms, u = unit roundoff of the MMA input format):
 //   |d'(q,c) - d(q,c)| <= E_q = 1.25 * [ 2 (r(q~) M + (|q~| + r(q~)) R)          input rounding
 //                                  + 2 (n 2^-23 (1+u)^2 + 2^-22) |q~| M          accumulation
 //                                  + 3 * 2^-24 (CN + |qn'| + 2 |q~| M) ] + noise
 // For the split format r(q~) M + ... is replaced by 3.2 u^2 |q~| M (u = 2^-8; it covers the omitted
-// lo x lo product) and n = 3D + 3. With the norm column E gains 1.25 (n 2^-23 + 2^-24) CN for the
-// norm parts it sums. `noise` covers the rounding of the FP64 distance itself, (4d + 32) 2^-53 of
+// lo x lo product) and n = 3D + NORM_TERMS. With the norm column E gains
+// 1.25 (NORM_TERMS 2^-23 + 2^-24) CN for the norm parts it sums: they are accumulated last. `noise` covers the rounding of the FP64 distance itself, (4d + 32) 2^-53 of
 // the squared norms' scale. Measuring r takes the input term to about 0.4 of its worst case
 // (2u + u^2) |q~| M.
 #include "knn_common.cuh"
@@ -561,6 +561,8 @@ struct SmemLayout {
 
 // Norm column (fold): an all-ones A tile and two slots of candidate norm tiles, 32-byte rows.
 constexpr int NORM_ROW = 32;
+// Additions of the norm column's MMA (K = 16 in 16-bit formats, 8 in TF32, and the accumulator).
+constexpr int NORM_TERMS = 17;
 
 // Partition bound (see TcParams::proot): heap entries per row and part, and the splits whose
 // published roots a row reads (its own and up to three more).
@@ -947,21 +949,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // every epilogue warp has released tile lt - 2, so all of them are done with tile lt - 3
         // and its norm slot: fetch this tile's candidate norms there
         const uint32_t tmem_d = tmem_base + (uint32_t)(b * N);
-        if (FOLD) {
-          // the norm column first: w = -cn/2, then the products accumulate onto it
-          if (!mbar_wait(&nfull[b], use & 1u)) { failed = true; break; }
-          tc_fence_after();
-          const uint64_t ad = sdesc_k_sw32(su32(sAn));
-          const uint64_t bd = sdesc_k_sw32(su32(sBn) + (uint32_t)b * N * NORM_ROW);
-          if (FMT == 0) mma_tf32(tmem_d, ad, bd, p.idesc, 0u);
-          else mma_f16(tmem_d, ad, bd, p.idesc, 0u);
-        } else {
+        if (!FOLD) {
           const int c = lt % CN_SLOTS;
           mbar_expect_tx(&cnfull[c], (uint32_t)(N * 4));
           bulk_g2s(cn_s + c * N, p.cn + (size_t)(t_begin + lt) * N, (uint32_t)(N * 4),
                    &cnfull[c]);
-          tc_fence_after();
         }
+        tc_fence_after();
         for (int i = 0; i < TERMS * p.nkc; i++) {
           const int s = stage, kc = i / TERMS;
           const bool lo = i % TERMS != 0;
@@ -978,7 +972,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           // descriptor's address field (16-byte units).
           const uint64_t ad = sdesc_k_sw128(a_base + (uint32_t)kc * A_CHUNK);
           const uint64_t bd = sdesc_k_sw128(b_base + (uint32_t)s * b_stage_bytes);
-          const uint32_t first = FOLD || i != 0 ? 1u : 0u;
+          const uint32_t first = i != 0 ? 1u : 0u;
           if (FMT == 2 && !lo) {
             // hi stage: the query's lo part too
             const uint64_t ld = sdesc_k_sw128(a_base + (uint32_t)(p.nkc + kc) * A_CHUNK);
@@ -997,6 +991,19 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             }
           }
           mma_commit(&empty[s]);
+        }
+        if (FOLD && !failed) {
+          // the norm column last: every later addition would add a rounding of |cn|/2 to the bound
+          // (first, E at d = 80 and 128 in split BF16 was 1.27 times what it is without it)
+          if (mbar_wait(&nfull[b], use & 1u)) {
+            tc_fence_after();
+            const uint64_t ad = sdesc_k_sw32(su32(sAn));
+            const uint64_t bd = sdesc_k_sw32(su32(sBn) + (uint32_t)b * N * NORM_ROW);
+            if (FMT == 0) mma_tf32(tmem_d, ad, bd, p.idesc, 1u);
+            else mma_f16(tmem_d, ad, bd, p.idesc, 1u);
+          } else {
+            failed = true;
+          }
         }
         if (!failed) {
           if (FOLD) mma_commit(&nempty[b]);
@@ -2490,20 +2497,20 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   P.o_log = take((size_t)NPART * P.S * nq * P.logcap * LOG_ENTRY);
   P.bytes = off;
   // Error-bound coefficients. kA: accumulation, charged as truncation on the sum of the products'
-  // magnitudes, |q~| |c~| (1 + u)^2 (the rounded factors), over the products and the three parts
-  // of the norm column, and the FP32 rounding of both centred factors. kB: FP32 rounding of the
+  // magnitudes, |q~| |c~| (1 + u)^2 (the rounded factors), over the products and the norm column's
+  // MMA, and the FP32 rounding of both centred factors. kB: FP32 rounding of the
   // norm terms. kS: the FP64 distance's own rounding (and the effective norms'). With the norm
-  // column the accumulation also adds the three parts of -cn/2 (exact in the input format), whose
+  // column the last MMA also adds the three parts of -cn/2 (exact in the input format), whose
   // magnitudes sum to CN / 2; in v = -2w that is twice as much: kC_fold. The final d' = v + qn'
   // rounds once, inside the kB term. The input rounding itself is measured (tc_pack).
   {
     const double D = (double)P.d_pad;
     const double u = P.fmt == 0 || P.fmt == 3 ? std::ldexp(1.0, -11) : std::ldexp(1.0, -8);
-    const double n = (P.fmt == 2 ? 3.0 * D : D) + 3.0;
-    const double acc = n * std::ldexp(1.0, -23);
+    const double n = (P.fmt == 2 ? 3.0 * D : D) + NORM_TERMS;
+    const double acc = n * std::ldexp(1.0, -23), last = NORM_TERMS * std::ldexp(1.0, -23);
     P.kA = (float)(acc * (1 + u) * (1 + u) + std::ldexp(1.0, -22));
     P.kB = (float)(1.25 * 3.0 * std::ldexp(1.0, -24) + 1e-12);
-    P.kC_fold = (float)(1.25 * (acc + std::ldexp(1.0, -24)) + 1e-12);
+    P.kC_fold = (float)(1.25 * (last + std::ldexp(1.0, -24)) + 1e-12);
     P.kS = (float)(1.25 * (4.0 * d + 32.0) * std::ldexp(1.0, -53));
   }
   P.ok = true;
