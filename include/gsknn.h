@@ -161,7 +161,7 @@ const char *gsknn_last_error_string(void);
  *   GSKNN_MODE_FP32 -- CUDA-core FP32 distances;
  *   GSKNN_MODE_TF32, GSKNN_MODE_BF16 -- tensor-core distances with an FP64 re-rank of every
  *     candidate within the rounding bound of the k-th distance (exact index sets);
- *   GSKNN_MODE_AUTO -- large calls with d > 64 in scaled FP16 (queries whose re-rank band
+ *   GSKNN_MODE_AUTO -- large calls from d = 128 in scaled FP16 (queries whose re-rank band
  *     overflows its log run again in split BF16); others in split BF16 (the narrowest band); TF32
  *     where neither fits in shared memory; else FP32 (default). Each choice was measured fastest
  *     of the exact forms over d = 20 to 256. */

@@ -589,16 +589,18 @@ static int knn_device_tc(int mode, const TcPlan *plan, int nq, int nc, int d, in
 // The tensor-core mode AUTO takes for a shape (GSKNN_MODE_FP32: none fits), and its plan.
 static int auto_mode(int nq, int nc, int d, int k, TcPlan *P) {
   // Split BF16 (three MMAs per product) keeps the re-rank band narrowest. One FP16 MMA per product
-  // (and half the panel bytes) pays from two K chunks (d > 64) where the contraction bounds the
-  // call, about 1.3e10 (pair, padded dimension) products, or the packing does, 2.5e7 (candidate,
-  // padded dimension) entries; beyond d = 256, where split tiles are narrow, 9e6. B200, us, split
-  // -> FP16: 16,384 x 60,000, d = 80 804 -> 539, d = 256 1,532 -> 795; 4,096 x 65,536, d = 128
-  // 318 -> 260; 16 x 250,000, d = 200 613 -> 397; 16 x 30,000, d = 300 208 -> 169; but 2,000 x
-  // 30,000, d = 128 167 -> 175, 16 x 30,000, d = 128 127 -> 164 and 16 x 4,096 96 -> 108 (the
-  // escalation's launches). At d <= 64 it gains 18% on uniform points and nothing on the Gaussian
-  // mixture, whose band is wider.
+  // (and half the panel bytes) pays from d = 128 where the contraction bounds the call, about
+  // 1.3e10 (pair, padded dimension) products, or the packing does, 2.5e7 (candidate, padded
+  // dimension) entries; beyond d = 256, where split tiles are narrow, 9e6. B200, us, split -> FP16:
+  // 16,384 x 60,000, d = 256 1,532 -> 795; 4,096 x 65,536, d = 128 318 -> 260; 16 x 250,000,
+  // d = 200 613 -> 397; 16 x 30,000, d = 300 208 -> 169; but 2,000 x 30,000, d = 128 167 -> 175,
+  // 16 x 30,000, d = 128 127 -> 164 and 16 x 4,096 96 -> 108 (the escalation's launches). Below
+  // d = 128 its band overflows the logs on clusters, and all that it gains on other points is less
+  // than what those lose: 16,384 x 60,000, d = 100, k = 32 uniform 785 -> 625, mixture of sigma 0.05
+  // 795 -> 734, 0.02 868 -> 2,625, 0.014 1,145 -> 2,160, 0.01 4,173 -> 190,959; doubles 5,003 x
+  // 50,021, d = 100, k = 50, sigma 0.05 531 -> 593, 0.02 608 -> 1,748.
   const double d_pad = (d + 63) / 64 * 64, entries = nc * d_pad, products = nq * entries;
-  const bool big = d > 64 && (products >= 1.3e10 || entries >= (d > 256 ? 9e6 : 2.5e7));
+  const bool big = d >= 128 && (products >= 1.3e10 || entries >= (d > 256 ? 9e6 : 2.5e7));
   const int order[4] = {big ? GSKNN_TC_FP16 : GSKNN_TC_BF16X3,
                         big ? GSKNN_TC_BF16X3 : GSKNN_TC_FP16, GSKNN_TC_TF32, GSKNN_MODE_FP32};
   for (int i = 0; i < 3; i++) {
