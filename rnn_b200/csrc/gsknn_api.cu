@@ -524,6 +524,44 @@ int knn_device_simt(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, lon
 
 static int g_mode = GSKNN_MODE_AUTO;
 
+// A tensor-core call runs in chunks of heap rows (they are independent) where the logs of all rows
+// together would take more than LOG_BUDGET, or where its workspace cannot be had: all chunks but the
+// last have `rows` rows, whole waves of query tiles where they are that many (1,000,000 x 131,072,
+// d = 32, k = 64: 58.9 ms, in equal chunks 61.8), and every chunk packs the candidates again (80 us for 262,144 x 64).
+constexpr size_t LOG_BUDGET = (size_t)16 << 30;
+constexpr int MIN_CHUNK = 1024;
+struct RowChunks {
+  int rows, tail;  // tail: rows of the last chunk
+  TcPlan P, T;     // plans of the whole chunks and of the last
+};
+
+// Plans the call and gets its workspace; `whole`, when set, is the plan of all rows, and `extra(rows)`
+// the bytes that a chunk takes behind its plan's. cudaErrorInvalidValue: no plan.
+template <typename Extra>
+static cudaError_t tc_workspace(int mode, const TcPlan *whole, int nq, int nc, int d, int k,
+                                cudaStream_t st, Extra extra, RowChunks *c, void **ws) {
+  const int wave = 128 * sm_count();
+  c->rows = nq;
+  for (;;) {
+    const int rows = c->rows;
+    c->tail = nq - (nq - 1) / rows * rows;
+    c->P = whole && rows == nq ? *whole : tc_plan(rows, nc, d, k, mode, sm_count());
+    if (!c->P.ok) return cudaErrorInvalidValue;
+    c->T = c->tail == rows ? c->P : tc_plan(c->tail, nc, d, k, mode, sm_count());
+    double part = 0.5;
+    if (c->P.log_bytes > LOG_BUDGET && rows > MIN_CHUNK) {
+      part = std::min(0.99, (double)LOG_BUDGET / (double)c->P.log_bytes);
+    } else {
+      const cudaError_t e =
+          scratch(SLOT_KERNEL, std::max(align256(c->P.bytes) + extra(rows),
+                                        align256(c->T.bytes) + extra(c->tail)), st, ws);
+      if (e != cudaErrorMemoryAllocation || rows <= MIN_CHUNK) return e;
+    }
+    const int fewer = (int)(rows * part), unit = fewer >= wave ? wave : 128;
+    c->rows = std::max(fewer / unit * unit, MIN_CHUNK);
+  }
+}
+
 // Tensor-core approximate pass + FP64 re-rank (float inputs). `dbg`, when set, also receives
 // the approximate distance of every (query, candidate) pair (row stride dbg_ld) and `margin`
 // the per-query band width 2E.
@@ -539,14 +577,16 @@ static int knn_device_tc(int mode, const TcPlan *plan, int nq, int nc, int d, in
                       k, ldD);
   if (!Xq || !Xq2 || !qidx || !Xc || !Xc2 || !cidx || !D || !I)
     return set_status(GSKNN_ERR_ARG, "null pointer argument");
-  const TcPlan P = plan ? *plan : tc_plan(nq, nc, d, k, mode, sm_count());
-  if (!P.ok)
+  RowChunks ch;
+  void *ws = nullptr;
+  StatusWords sw;
+  const cudaError_t we =
+      tc_workspace(mode, plan, nq, nc, d, k, st, [](int) { return (size_t)0; }, &ch, &ws);
+  if (!ch.P.ok)
     return set_status(GSKNN_ERR_UNSUPPORTED,
                       "tensor-core mode %d does not support d=%d k=%d (shared memory)", mode, d,
                       k);
-  void *ws = nullptr;
-  StatusWords sw;
-  CU(scratch(SLOT_KERNEL, P.bytes, st, &ws));
+  CU(we);
   CU(status_words(st, &sw));
   int *status = sw.dev;  // cleared by the first kernel
   // GSKNN_TC_COUNTERS=1: per-call diagnostics of the tensor-core epilogue on stderr
@@ -556,33 +596,39 @@ static int knn_device_tc(int mode, const TcPlan *plan, int nq, int nc, int d, in
     void *cv = nullptr;
     CU(scratch(SLOT_AUX, 128, st, &cv));
     counters = static_cast<unsigned long long *>(cv);
-    CU(cudaMemsetAsync(counters, 0, 128, st));
   }
-  CU(tc_run(P, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I, ldD, ws,
-            status, dbg, dbg_ld, counters, st, trace_hook, nullptr, sw.mirror_dev));
-  if (counters) {
-    unsigned long long h[16] = {};
-    int nfb = 0;
-    CU(cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, st));
-    CU(cudaMemcpyAsync(&nfb, static_cast<char *>(ws) + P.o_fbc, sizeof(int),
-                       cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
-    const double ctas = (double)P.qtiles * P.S, warps = ctas * TC_EPI_WARPS;
-    std::fprintf(stderr,
-                 "gsknn tc: mode=%d n=%d m=%d d=%d k=%d S=%d N=%d NST=%d: logged/query=%.1f "
-                 "flushes/warp=%.1f slow-chunks/warp=%.1f "
-                 "chunks/warp=%.1f rerank-scanned/query=%.1f exact/query=%.1f fallback=%d | "
-                 "cycles/CTA: mma-loop=%.0f mma-wait-tma=%.0f mma-wait-epilogue=%.0f | "
-                 "cycles/warp: epi-loop=%.0f epi-wait-mma=%.0f\n",
-                 mode, nq, nc, d, k, P.S, P.N, P.NST, (double)h[0] / nq,
-                 (double)h[2] / warps, (double)h[3] / warps, (double)h[4] / warps,
-                 (double)h[5] / nq, (double)h[6] / nq, nfb, (double)h[10] / ctas,
-                 (double)h[7] / ctas, (double)h[8] / ctas, (double)h[11] / warps,
-                 (double)h[9] / warps);
+  for (int q0 = 0; q0 < nq; q0 += ch.rows) {
+    const int n = std::min(ch.rows, nq - q0);
+    const TcPlan &P = n == ch.rows ? ch.P : ch.T;
+    if (counters) CU(cudaMemsetAsync(counters, 0, 128, st));
+    CU(tc_run(P, n, nc, d, k, Xq, Xq2, nrows_q, qidx + q0, Xc, Xc2, nrows_c, cidx,
+              D + (size_t)q0 * ldD, I + (size_t)q0 * ldD, ldD, ws, status,
+              dbg ? dbg + (size_t)q0 * dbg_ld : nullptr, dbg_ld, counters, st, trace_hook, nullptr,
+              sw.mirror_dev, q0 == 0));
+    if (counters) {
+      unsigned long long h[16] = {};
+      int nfb = 0;
+      CU(cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, st));
+      CU(cudaMemcpyAsync(&nfb, static_cast<char *>(ws) + P.o_fbc, sizeof(int),
+                         cudaMemcpyDeviceToHost, st));
+      CU(cudaStreamSynchronize(st));
+      const double ctas = (double)P.qtiles * P.S, warps = ctas * TC_EPI_WARPS;
+      std::fprintf(stderr,
+                   "gsknn tc: mode=%d n=%d m=%d d=%d k=%d S=%d N=%d NST=%d: logged/query=%.1f "
+                   "flushes/warp=%.1f slow-chunks/warp=%.1f "
+                   "chunks/warp=%.1f rerank-scanned/query=%.1f exact/query=%.1f fallback=%d | "
+                   "cycles/CTA: mma-loop=%.0f mma-wait-tma=%.0f mma-wait-epilogue=%.0f | "
+                   "cycles/warp: epi-loop=%.0f epi-wait-mma=%.0f\n",
+                   mode, n, nc, d, k, P.S, P.N, P.NST, (double)h[0] / n,
+                   (double)h[2] / warps, (double)h[3] / warps, (double)h[4] / warps,
+                   (double)h[5] / n, (double)h[6] / n, nfb, (double)h[10] / ctas,
+                   (double)h[7] / ctas, (double)h[8] / ctas, (double)h[11] / warps,
+                   (double)h[9] / warps);
+    }
+    if (margin)
+      CU(cudaMemcpyAsync(margin + q0, static_cast<char *>(ws) + P.o_margin, (size_t)n * 4,
+                         cudaMemcpyDeviceToDevice, st));
   }
-  if (margin)
-    CU(cudaMemcpyAsync(margin, static_cast<char *>(ws) + P.o_margin, (size_t)nq * 4,
-                       cudaMemcpyDeviceToDevice, st));
   return set_status(GSKNN_OK, nullptr);
 }
 
@@ -624,22 +670,34 @@ static int knn_device_tc_double(int nq, int nc, int d, int k, const double *Xq, 
       !cidx || !D || !I)
     return -1;  // (the CUDA-core path reports)
   TcPlan P;
-  if (auto_mode(nq, nc, d, k, &P) == GSKNN_MODE_FP32) return -1;
-  const SimtPlan F = simt_plan<double>(nq, nc, d, k);
-  if (!P.ok || F.g.kp == 0) return -1;
+  const int mode = auto_mode(nq, nc, d, k, &P);
+  if (mode == GSKNN_MODE_FP32) return -1;
+  if (simt_geometry<double>(k).kp == 0) return -1;
+  RowChunks ch;
   void *ws = nullptr;
   StatusWords sw;
-  const size_t simt_off = align256(P.bytes);
-  const cudaError_t se = scratch(SLOT_KERNEL, simt_off + F.bytes, st, &ws);
+  const cudaError_t se = tc_workspace(
+      mode, &P, nq, nc, d, k, st,
+      [&](int rows) { return simt_plan<double>(rows, nc, d, k).bytes; }, &ch, &ws);
   if (se == cudaErrorMemoryAllocation) return -1;
   CU(se);
   CU(status_words(st, &sw));
   int *status = sw.dev;  // cleared by the first kernel
-  const int *left = nullptr, *nleft = nullptr;
-  CU(tc_run_double(P, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I, ldD, ws,
-                   status, &left, &nleft, st, trace_hook, nullptr));
-  return simt_run<double>(F, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c, cidx, D, I,
-                          ldD, static_cast<char *>(ws) + simt_off, sw, st, 0, left, nleft);
+  for (int q0 = 0; q0 < nq; q0 += ch.rows) {
+    const int n = std::min(ch.rows, nq - q0);
+    const TcPlan &R = n == ch.rows ? ch.P : ch.T;
+    const SimtPlan F = simt_plan<double>(n, nc, d, k);
+    const int *left = nullptr, *nleft = nullptr;
+    double *Dq = D + (size_t)q0 * ldD;
+    int *Iq = I + (size_t)q0 * ldD;
+    CU(tc_run_double(R, n, nc, d, k, Xq, Xq2, nrows_q, qidx + q0, Xc, Xc2, nrows_c, cidx, Dq, Iq,
+                     ldD, ws, status, &left, &nleft, st, trace_hook, nullptr, q0 == 0));
+    const int rc = simt_run<double>(F, n, nc, d, k, Xq, Xq2, nrows_q, qidx + q0, Xc, Xc2, nrows_c,
+                                    cidx, Dq, Iq, ldD, static_cast<char *>(ws) + align256(R.bytes),
+                                    sw, st, 0, left, nleft);
+    if (rc != GSKNN_OK) return rc;
+  }
+  return set_status(GSKNN_OK, nullptr);
 }
 
 template <typename T>

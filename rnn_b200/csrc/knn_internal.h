@@ -144,6 +144,7 @@ struct TcPlan {
   size_t o_esc, o_ecand, esc_bytes, ecand_bytes;
   int sms, max_splits;  // the plan's arguments, to re-derive the escalation pass's plan
   bool tight;
+  size_t log_bytes;  // of the main format's logs
   size_t bytes;       // whole workspace
 };
 
@@ -198,7 +199,7 @@ cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *X
                    const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,
                    int ldD, void *ws, int *status, float *dbg, long long dbg_ld,
                    unsigned long long *counters, cudaStream_t st, TraceHook hook,
-                   void *hook_ctx, int *mirror = nullptr);
+                   void *hook_ctx, int *mirror = nullptr, bool clear_status = true);
 // The same for double tables: the approximate pass runs on the centred rows rounded to the MMA
 // format, the re-rank on the double rows, in the CUDA-core kernel's order of operations. Queries
 // that neither it nor the escalation could bound are left: their heap rows at *left, their number
@@ -208,7 +209,7 @@ cudaError_t tc_run_double(const TcPlan &P, int nq, int nc, int d, int k, const d
                           const double *Xc, const double *Xc2, long long nrows_c,
                           const int *cidx, double *D, int *I, int ldD, void *ws, int *status,
                           const int **left, const int **nleft, cudaStream_t st, TraceHook hook,
-                          void *hook_ctx);
+                          void *hook_ctx, bool clear_status = true);
 // Tensor-core form of the batching pass (all-NN within randomized-tree leaves): one tree's
 // leaves laid out in a panel, each leaf padded to whole candidate tiles; every query tile runs
 // against its own leaf's tiles only, and the exact re-rank merges into the heap rows in place,

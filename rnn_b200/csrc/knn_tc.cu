@@ -2389,14 +2389,10 @@ cudaError_t tc_cand_prepare(TcCand *C, void *mem, int nc, int d, int mode, const
                                true, 0.0f, 0.0f, 0.0f, status, st);
 }
 
-// Quads per log: `want`, or as many as keep all `logs` logs under `budget` bytes, but not fewer than
-// fit the 8 * want bytes that a log of `want` single candidates takes (a tight plan's logs), nor than
-// twice the room that two chunks want.
-constexpr size_t LOG_BUDGET = (size_t)16 << 30;
-static int log_entries(int want, size_t logs, size_t budget = LOG_BUDGET) {
-  const size_t fit = budget / (std::max(logs, (size_t)1) * tc::LOG_ENTRY);
-  if (fit >= (size_t)want) return want;
-  return (int)std::max({fit, (size_t)want * 8 / tc::LOG_ENTRY, (size_t)(2 * tc::LOG_ROOM)});
+// Quads per log: `want`, or in a tight plan those that fit the 8 * want bytes of as many single
+// candidates, but not fewer than twice the room that two chunks want.
+static int log_entries(int want, bool tight) {
+  return tight ? std::max((int)(want * 8 / tc::LOG_ENTRY), 2 * tc::LOG_ROOM) : want;
 }
 
 static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool with_cand,
@@ -2482,12 +2478,12 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   if (!P.ringed)
     P.smem = tc_smem_layout(P.nkc, P.a_terms, P.N, P.NST, lists, false, false).total;
   P.smem_fold = smem_fold;
-  // (no log needs more than the quads its part of a split holds, and the room that two chunks want; a serving slot's workspace is allocated once, for the largest of its batches, so the
-  // entries there depend on the splits and on k alone)
-  P.logcap = std::min(log_entries(std::max(8 * P.kp, 1024), (size_t)NPART * best_s * nq,
-                                  tight            ? 0
-                                  : max_splits > 0 ? SIZE_MAX
-                                                   : LOG_BUDGET),
+  // (no log needs more than the quads its part of a split holds, and the room that two chunks want.
+  // The entries depend on the splits and on k alone: a serving slot's workspace is allocated once,
+  // for the largest of its batches, and short logs end in the brute force: cut to 16 GB in all,
+  // 1,000,000 x 131,072, d = 128, k = 128 took 866 ms, and 34.7 s on clusters of sigma 0.02; calls
+  // whose logs would take more run in chunks of rows instead)
+  P.logcap = std::min(log_entries(std::max(8 * P.kp, 1024), tight),
                       P.tiles_per_split * (P.N / NPART / 4) + LOG_ROOM);
   // workspace: [prepared candidates | query side]
   P.cand_bytes = with_cand ? al256(tc_cand_bytes(nc, d, mode)) : 0;
@@ -2505,7 +2501,8 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   P.o_fbl = take((size_t)nq * 4);
   P.o_fbc = take(16);
   // last: once the re-rank has read the logs, the escalation pass takes their place
-  P.o_log = take((size_t)NPART * P.S * nq * P.logcap * LOG_ENTRY);
+  P.log_bytes = (size_t)NPART * P.S * nq * P.logcap * LOG_ENTRY;
+  P.o_log = take(P.log_bytes);
   P.bytes = off;
   // Error-bound coefficients. kA: accumulation, charged as truncation on the sum of the products'
   // magnitudes, |q~| |c~| (1 + u)^2 (the rounded factors), over the products and the norm column's
@@ -2795,11 +2792,12 @@ static cudaError_t tc_call(const TcPlan &P, TcCand *C, int nq, int nc, int d, in
                            const T *Xc2, long long nrows_c, const int *cidx, T *D, int *I, int ldD,
                            void *ws, int *status, float *dbg, long long dbg_ld,
                            unsigned long long *counters, cudaStream_t st, TraceHook hook,
-                           void *hook_ctx, const TcPlan **last, char **last_base, TcPlan *EP) {
+                           void *hook_ctx, const TcPlan **last, char **last_base, TcPlan *EP,
+                           bool clear_status) {
   if (P.cand_bytes == 0) return cudaErrorInvalidValue;
   if (hook) hook(hook_ctx, "tc_pack", true, st, 0);
   const cudaError_t e = cand_begin<T>(C, ws, nc, d, tc_mode_of_format(P.fmt), Xc, Xc2, nrows_c,
-                                      cidx, status, st);
+                                      cidx, clear_status ? status : nullptr, st);
   if (hook) hook(hook_ctx, "tc_pack", false, st, 1);
   if (e != cudaSuccess) return e;
   return tc_passes<T>(P, *C, true, nq, d, k, Xq, Xq2, nrows_q, qidx, D, I, ldD,
@@ -2812,14 +2810,14 @@ cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *X
                    const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,
                    int ldD, void *ws, int *status, float *dbg, long long dbg_ld,
                    unsigned long long *counters, cudaStream_t st, TraceHook hook,
-                   void *hook_ctx, int *mirror) {
+                   void *hook_ctx, int *mirror, bool clear_status) {
   TcCand C{};
   const TcPlan *last;
   char *lbase;
   TcPlan EP;
   const cudaError_t e = tc_call<float>(P, &C, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2,
                                        nrows_c, cidx, D, I, ldD, ws, status, dbg, dbg_ld, counters,
-                                       st, hook, hook_ctx, &last, &lbase, &EP);
+                                       st, hook, hook_ctx, &last, &lbase, &EP, clear_status);
   if (e != cudaSuccess) return e;
   return tc_brute(*last, C, d, k, Xq, Xq2, qidx, D, I, ldD, lbase, st, hook, hook_ctx,
                   status, mirror);
@@ -2830,14 +2828,14 @@ cudaError_t tc_run_double(const TcPlan &P, int nq, int nc, int d, int k, const d
                           const double *Xc, const double *Xc2, long long nrows_c,
                           const int *cidx, double *D, int *I, int ldD, void *ws, int *status,
                           const int **left, const int **nleft, cudaStream_t st, TraceHook hook,
-                          void *hook_ctx) {
+                          void *hook_ctx, bool clear_status) {
   TcCand C{};
   const TcPlan *last;
   char *lbase;
   TcPlan EP;
   const cudaError_t e = tc_call<double>(P, &C, nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2,
                                         nrows_c, cidx, D, I, ldD, ws, status, nullptr, 0, nullptr,
-                                        st, hook, hook_ctx, &last, &lbase, &EP);
+                                        st, hook, hook_ctx, &last, &lbase, &EP, clear_status);
   if (e != cudaSuccess) return e;
   *left = reinterpret_cast<const int *>(lbase + last->o_fbl);
   *nleft = reinterpret_cast<const int *>(lbase + last->o_fbc);
@@ -2908,7 +2906,7 @@ TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms) {
   // per-query area for rows_cap rows, one split; smaller logs than the per-call path: a leaf offers
   // a few thousand candidates, of which a part logs about hk (1 + ln(n / hk)) < 5 hk quads (a full
   // log overflows to the leaf brute force)
-  P.logcap = log_entries(6 * tc_heap_k(k) + 32, (size_t)NPART * rows_cap);
+  P.logcap = 6 * tc_heap_k(k) + 32;
   P.S = 1;
   P.qtiles = L.rows_cap / TC_M;
   P.q_pad = L.rows_cap;
