@@ -1431,40 +1431,52 @@ __device__ __forceinline__ double sum4(double acc) {
   return acc;
 }
 
-// FP64 dot product by one thread, summed in dimension order: the brute-force passes, which compute
-// all of a query's distances themselves, and double tables, whose distances come out of the
-// CUDA-core kernel's order of operations bit for bit.
+// The same dot product by one thread, in the same order (four sums over every fourth group of four
+// dimensions, added as a tree): the brute-force passes. A query's distances are then the same bits
+// whether its band fitted the logs or not. Summed in dimension order, as the brute force was when the
+// re-rank did so too, about one neighbour in 10^8 came out another float.
 __device__ __forceinline__ double dot_lane(const float *q, const float *c, int d) {
-  double acc = 0.0;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
   const uintptr_t qc = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(c);
   if ((d & 3) == 0 && (qc & 15) == 0) {
     const float4 *q4 = reinterpret_cast<const float4 *>(q);
     const float4 *c4 = reinterpret_cast<const float4 *>(c);
-    for (int i = 0; i < (d >> 2); i++) {
-      const float4 a = __ldg(q4 + i), b = __ldg(c4 + i);
-      acc = fma((double)a.x, (double)b.x, acc);
-      acc = fma((double)a.y, (double)b.y, acc);
-      acc = fma((double)a.z, (double)b.z, acc);
-      acc = fma((double)a.w, (double)b.w, acc);
+    for (int i = 0; i < (d >> 2); i += 4) {
+#pragma unroll
+      for (int s = 0; s < 4; s++) {
+        if (i + s < (d >> 2)) {
+          const float4 a = __ldg(q4 + i + s), b = __ldg(c4 + i + s);
+          acc[s] = fma((double)a.x, (double)b.x, acc[s]);
+          acc[s] = fma((double)a.y, (double)b.y, acc[s]);
+          acc[s] = fma((double)a.z, (double)b.z, acc[s]);
+          acc[s] = fma((double)a.w, (double)b.w, acc[s]);
+        }
+      }
     }
   } else {
-    // four loads of each row in flight: left to the compiler, the brute force's loop took 631 ms on
-    // 16,384 x 60,000, d = 127, 355 so (rows of whole quads: d = 128 472 ms a value at a time, 188)
-    int pp = 0;
-    for (; pp + 4 <= d; pp += 4) {
-      float a[4], b[4];
+    // sixteen loads of each row in flight: left to the compiler, the brute force's loop took 631 ms
+    // on 16,384 x 60,000, d = 127, 196 so (rows of whole quads, d = 128: 472 ms a value at a time, 192)
+    int p = 0;
+    for (; p + 16 <= d; p += 16) {
+      float a[16], b[16];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        a[j] = __ldg(q + pp + j);
-        b[j] = __ldg(c + pp + j);
+      for (int j = 0; j < 16; j++) {
+        a[j] = __ldg(q + p + j);
+        b[j] = __ldg(c + p + j);
       }
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc = fma((double)a[j], (double)b[j], acc);
+      for (int j = 0; j < 16; j++) acc[j >> 2] = fma((double)a[j], (double)b[j], acc[j >> 2]);
     }
-    for (; pp < d; pp++) acc = fma((double)__ldg(q + pp), (double)__ldg(c + pp), acc);
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+      if (p + j < d)
+        acc[j >> 2] = fma((double)__ldg(q + p + j), (double)__ldg(c + p + j), acc[j >> 2]);
   }
-  return acc;
+  return (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
+
+// FP64 dot product of two double rows by one thread, summed in dimension order: double tables, whose
+// distances come out of the CUDA-core kernel's order of operations bit for bit.
 __device__ __forceinline__ double dot_lane(const double *q, const double *c, int d) {
   double acc = 0.0;
   const uintptr_t qc = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(c);
