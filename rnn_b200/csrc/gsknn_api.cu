@@ -527,7 +527,8 @@ static int g_mode = GSKNN_MODE_AUTO;
 // A tensor-core call runs in chunks of heap rows (they are independent) where the logs of all rows
 // together would take more than LOG_BUDGET, or where its workspace cannot be had: all chunks but the
 // last have `rows` rows, whole waves of query tiles where they are that many (1,000,000 x 131,072,
-// d = 32, k = 64: 58.9 ms, in equal chunks 61.8), and every chunk packs the candidates again (80 us for 262,144 x 64).
+// d = 32, k = 64: 58.9 ms, in equal chunks 61.8), and every chunk packs the candidates again (80 us
+// for 262,144 x 64).
 constexpr size_t LOG_BUDGET = (size_t)16 << 30;
 constexpr int MIN_CHUNK = 1024;
 struct RowChunks {

@@ -580,12 +580,19 @@ static int ensure_tc(BatchJob *b, long long rows, int tree_rows) {
   free_tc(b);
   const long long cap = (rows + rows / 8 + 128 * b->T + 127) / 128 * 128;
   const long long tcap = ((long long)tree_rows + tree_rows / 8 + 127) / 128 * 128;
-  b->tcl = gsknn::tc_leaf_plan(b->N, (int)std::min<long long>(tcap, 1LL << 30), b->d, b->k,
-                               b->sms);
+  const int tc = (int)std::min<long long>(tcap, 1LL << 30);
+  b->tcl = gsknn::tc_leaf_plan(b->N, tc, b->d, b->k, b->sms);
   if (!b->tcl.ok) return set_err(GSKNN_ERR_UNSUPPORTED, "tensor-core shape: no tile plan");
+  if (cudaMalloc(&b->tc_ws, b->tcl.bytes) != cudaSuccess) {
+    // smaller logs before giving up
+    cudaGetLastError();
+    b->tc_ws = nullptr;
+    b->tcl = gsknn::tc_leaf_plan(b->N, tc, b->d, b->k, b->sms, true);
+    if (cudaMalloc(&b->tc_ws, b->tcl.bytes) != cudaSuccess) b->tc_ws = nullptr;
+  }
   const size_t pb = (size_t)cap * 4, qb = (size_t)(cap / 128) * sizeof(int4),
                rb = (size_t)(cap / 128) * sizeof(int2);
-  if (cudaMalloc(&b->tc_ws, b->tcl.bytes) != cudaSuccess ||
+  if (!b->tc_ws ||
       cudaMalloc((void **)&b->tc_pidx, pb + qb + rb + 512) != cudaSuccess ||
       cudaHostAlloc((void **)&b->h_tc_pidx, pb, cudaHostAllocDefault) != cudaSuccess ||
       cudaHostAlloc((void **)&b->h_tc_qtab, qb, cudaHostAllocDefault) != cudaSuccess ||

@@ -220,8 +220,10 @@ struct TcLeafPlan {
   int rows_cap;    // panel rows one tree may need
   size_t o_mu, o_fscale, o_cpart, o_stats, o_pb, o_pb_lo, o_pn, o_cn, o_cid, o_iota, bytes;
 };
-// npts: points of the table; rows_cap: panel rows one tree may use (a multiple of 128).
-TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms);
+// npts: points of the table; rows_cap: panel rows one tree may use (a multiple of 128); tight: the
+// bytes of max(2 kp, 256) single candidates per log, for when the workspace of the full logs cannot
+// be had (a query whose log overflows ends in a brute force over its leaf).
+TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms, bool tight = false);
 // Candidate tile width of the leaf panels: every leaf starts at a multiple of it (0: no plan).
 int tc_leaf_tile(int d, int k, int sms);
 // One tree: pidx (rows entries: point or -1), qtab (nqt entries), rtab (rows / 128 entries);

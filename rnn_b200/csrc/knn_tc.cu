@@ -2907,7 +2907,7 @@ int tc_leaf_tile(int d, int k, int sms) {
   return P.ok ? P.N : 0;
 }
 
-TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms) {
+TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms, bool tight) {
   using namespace tc;
   TcLeafPlan L{};
   L.ok = false;
@@ -2919,6 +2919,7 @@ TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms) {
   // a few thousand candidates, of which a part logs about hk (1 + ln(n / hk)) < 5 hk quads (a full
   // log overflows to the leaf brute force)
   P.logcap = 6 * tc_heap_k(k) + 32;
+  if (tight) P.logcap = std::min(P.logcap, log_entries(std::max(2 * P.kp, 256), true));
   P.S = 1;
   P.qtiles = L.rows_cap / TC_M;
   P.q_pad = L.rows_cap;
