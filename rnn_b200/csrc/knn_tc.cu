@@ -1506,8 +1506,11 @@ __device__ __forceinline__ double exact_dist_lane(const float *q, const float *c
 typedef unsigned long long Ord;
 constexpr Ord ORD_INF = 0xFFF0000000000000ull;  // image of +inf
 __device__ __forceinline__ Ord to_ord(double x) {
-  const Ord b = (Ord)__double_as_longlong(x + 0.0);
-  return (b >> 63) ? (x != x ? ~0ull : ~b) : b | 0x8000000000000000ull;
+  const Ord b = (Ord)__double_as_longlong(x), mag = b << 1;
+  // (on the bits alone: tested as x != x in the branch of negative numbers, a NaN came out just below
+  // 0 here, since the compiler may take either sign for it)
+  if (mag > ORD_INF << 1 || mag == 0) return mag == 0 ? 0x8000000000000000ull : ~0ull;
+  return (b >> 63) ? ~b : b | 0x8000000000000000ull;
 }
 __device__ __forceinline__ double from_ord(Ord o) {
   return __longlong_as_double((long long)((o >> 63) ? o & 0x7FFFFFFFFFFFFFFFull : ~o));
@@ -1680,7 +1683,8 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
   constexpr int CAP = rr_cap<E>();
   const int lane = threadIdx.x & 31;
   const int hr = p.rowmap ? p.rowmap[q] : q;  // heap row and query position
-  if (hr < 0) return;                          // a padding row of a leaf panel
+  // a padding row of a leaf panel, or a point outside the table (reported by tc_pack)
+  if (hr < 0 || (LEAF && hr >= p.nrows_q)) return;
   const int k = p.k;
   Ord ld[E];
   uint32_t li[E];
@@ -1695,8 +1699,9 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
   }
   const float E2 = p.margin[q], Eq = 0.5f * E2, qn = p.qn[q];
   // overflowed logs: the query goes to the next pass (a narrower format, or brute force); so does a
-  // double query whose bound left the floats' range
-  if (sizeof(Tab) == 8 && !(E2 < 1e38f)) ovf = true;
+  // query whose bound left the floats' range or is NaN (the bound holds the maxima over all
+  // candidates: one NaN coordinate makes every query's NaN, and nothing is logged)
+  if (!(E2 < 1e38f)) ovf = true;
   if (__any_sync(FULL_MASK, ovf)) {
     if (lane == 0) p.fallback_list[atomicAdd(p.fallback_count, 1)] = LEAF ? q : hr;
     return;
@@ -1951,7 +1956,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
       if (g + lane < p.S) pre[g + lane + 1] = carry + incl;
       carry += __shfl_sync(FULL_MASK, incl, 31);
     }
-    ovf = __any_sync(FULL_MASK, ovf) || (sizeof(Tab) == 8 && !(E2 < 1e38f));
+    ovf = __any_sync(FULL_MASK, ovf) || !(E2 < 1e38f);
     two_smallest(m1, m2);
     const float T = m2 == 0xFFFFFFFFu ? Num<float>::inf() : __uint_as_float(m2);
     const float lim = band_limit(row_max(p.D + (size_t)hr * p.ldD, k, lane), Eq);
@@ -2052,7 +2057,7 @@ struct FallbackParams {
   int k, d, nc;
   const float *Xq, *Xq2, *Xc, *Xc2;
   const int *qidx, *cidx;
-  long long nrows_c;
+  long long nrows_q, nrows_c;
   float *D;
   int *I;
   int ldD;
@@ -2072,6 +2077,7 @@ __global__ void __launch_bounds__(256) tc_fallback(FallbackParams p) {
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
     const int q = p.list[w];
     const long long qrow = p.qidx[q];
+    if (qrow < 0 || qrow >= p.nrows_q) continue;  // reported by tc_pack
     const float *qv = p.Xq + qrow * p.d;
     const double qq = (double)p.Xq2[qrow];
     Ord ld[E];
@@ -2728,15 +2734,16 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, bool pack_cand, boo
 
 // Exact FP64 brute force for the queries (heap rows) listed at base + P.o_fbl.
 static cudaError_t tc_brute(const TcPlan &P, const TcCand &C, int d, int k, const float *Xq,
-                            const float *Xq2, const int *qidx, float *D, int *I, int ldD,
-                            char *base, cudaStream_t st, TraceHook hook, void *hook_ctx,
+                            const float *Xq2, long long nrows_q, const int *qidx, float *D,
+                            int *I, int ldD, char *base, cudaStream_t st, TraceHook hook,
+                            void *hook_ctx,
                             const int *status = nullptr, int *mirror = nullptr) {
   using namespace tc;
   FallbackParams fp{};
   fp.status = status; fp.mirror = mirror;
   fp.k = k; fp.d = d; fp.nc = C.nc; fp.Xq = Xq; fp.Xq2 = Xq2;
   fp.Xc = static_cast<const float *>(C.Xc); fp.Xc2 = static_cast<const float *>(C.Xc2);
-  fp.qidx = qidx; fp.cidx = C.cidx; fp.nrows_c = C.nrows_c; fp.D = D; fp.I = I; fp.ldD = ldD;
+  fp.qidx = qidx; fp.cidx = C.cidx; fp.nrows_q = nrows_q; fp.nrows_c = C.nrows_c; fp.D = D; fp.I = I; fp.ldD = ldD;
   fp.list = reinterpret_cast<const int *>(base + P.o_fbl);
   fp.count = reinterpret_cast<const int *>(base + P.o_fbc);
   if (hook) hook(hook_ctx, "tc_fallback", true, st, 0);
@@ -2831,7 +2838,7 @@ cudaError_t tc_run(const TcPlan &P, int nq, int nc, int d, int k, const float *X
                                        nrows_c, cidx, D, I, ldD, ws, status, dbg, dbg_ld, counters,
                                        st, hook, hook_ctx, &last, &lbase, &EP, clear_status);
   if (e != cudaSuccess) return e;
-  return tc_brute(*last, C, d, k, Xq, Xq2, qidx, D, I, ldD, lbase, st, hook, hook_ctx,
+  return tc_brute(*last, C, d, k, Xq, Xq2, nrows_q, qidx, D, I, ldD, lbase, st, hook, hook_ctx,
                   status, mirror);
 }
 
@@ -2866,7 +2873,7 @@ cudaError_t tc_run_prepared(const TcPlan &P, const TcCand &C, int nq, int d, int
                                          static_cast<char *>(ws), status, dbg, dbg_ld, counters,
                                          st, hook, hook_ctx, &last, &lbase, &EP);
   if (e != cudaSuccess) return e;
-  return tc_brute(*last, C, d, k, Xq, Xq2, qidx, D, I, ldD, lbase, st, hook, hook_ctx);
+  return tc_brute(*last, C, d, k, Xq, Xq2, nrows_q, qidx, D, I, ldD, lbase, st, hook, hook_ctx);
 }
 
 // Escalation panels of a prepared candidate set (kept with it, e.g. a serving engine's
