@@ -1368,6 +1368,7 @@ struct RerankParams {
   const float *qmx;  // largest incoming distance of each query's heap row (tc_pack)
   int fold;             // the logged values are w (in the panels' scale), else v
   const float *fscale;  // as in TcParams
+  int limit;  // double tables: a query with more candidates in its band goes to the next pass
   const unsigned *proot;  // partition roots of tc_knn ([query][S]; S counts NPART per split)
   const float *margin;
   const T *Xq, *Xq2, *Xc, *Xc2;
@@ -1731,6 +1732,7 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
   const double qq = (double)p.Xq2[qrow];
   const float qmul = log_mul(p);
   int n = 0;  // listed entries
+  [[maybe_unused]] bool counted = false;
 
   // The logs, 32 at a time, as one concatenated list: lane s holds where log g + s starts. Entries
   // under the threshold fill the list; a full list is first cut down to what the bound from its
@@ -1826,6 +1828,28 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
       }
       n = w;
       if (n <= CAP / 2) continue;
+      // A band that fills the list: a double query whose band is a large part of the candidates
+      // (points closer than the rounding of their own distances) leaves before its first exact
+      // distance, not with its whole band's (band_limit_of).
+      if constexpr (sizeof(Tab) == 8) {
+        if (!counted) {
+          counted = true;
+          int c = 0;
+          for (int s = 0; s < p.S; s++) {
+            const int cnt = p.logcnt[(size_t)s * p.Q + q];
+            const float4 *const lg = p.log + ((size_t)s * p.Q + q) * p.logcap;
+            for (int e = lane; e < cnt; e += 32) {
+              const float4 v = lg[e];
+              c += (fmaf(qmul, v.x, qn) <= thr) + (fmaf(qmul, v.y, qn) <= thr) +
+                   (fmaf(qmul, v.z, qn) <= thr) + (fmaf(qmul, v.w, qn) <= thr);
+            }
+          }
+          if (__reduce_add_sync(FULL_MASK, c) > p.limit) {
+            if (lane == 0) p.fallback_list[atomicAdd(p.fallback_count, 1)] = hr;
+            return;
+          }
+        }
+      }
     }
     int nb = 0;  // staged candidates
     const int nblk = (n + 31) / 32;
@@ -1913,7 +1937,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_leaf(Reran
 }
 
 // One query by one CTA: all warps read the logs into one list and share the exact distances; warp
-// 0 merges. A query whose list does not fit is left to warp 0 alone (rerank_warp).
+// 0 merges.
 constexpr int RC_CAP = 1024;  // listed entries per CTA
 constexpr int RC_LOGS = 512;  // logs (NPART * S) the prefix array holds
 
@@ -1925,7 +1949,6 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
   __shared__ int pre[RC_LOGS + 1];
   __shared__ float s_T, s_thr;
   __shared__ int s_n, s_state;
-  __shared__ RerankSmem<E> sm;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int q = blockIdx.x;
   if (q >= (p.dQ ? *p.dQ : p.Q)) return;
@@ -1972,36 +1995,49 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
   }
   __syncthreads();
   if (s_state) return;
+  const long long qrow = p.qidx[hr];
+  if (qrow < 0 || qrow >= p.nrows_q) return;  // reported by tc_pack
+  const Tab *qv = p.Xq + qrow * p.d;
+  const double qq = (double)p.Xq2[qrow];
   const int total = pre[p.S];
   float thr = s_thr;
   const float qmul = log_mul(p);
-  for (int e = tid; e < total; e += 32 * RR_WARPS) {
-    int a = 0, b = p.S;  // the last log that starts at or before e
-    while (b - a > 1) {
-      const int m = (a + b) >> 1;
-      if (pre[m] <= e) a = m;
-      else b = m;
-    }
-    const size_t at = ((size_t)a * p.Q + q) * p.logcap + (e - pre[a]);
-    const float4 v4 = p.log[at];
-    const uint32_t pos = p.logpos[at];
-    const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+  // lists the entries under thr of the quads e0 .. e1; s_n counts them all
+  auto gather = [&](int e0, int e1) {
+    for (int e = e0 + tid; e < e1; e += 32 * RR_WARPS) {
+      int a = 0, b = p.S;  // the last log that starts at or before e
+      while (b - a > 1) {
+        const int m = (a + b) >> 1;
+        if (pre[m] <= e) a = m;
+        else b = m;
+      }
+      const size_t at = ((size_t)a * p.Q + q) * p.logcap + (e - pre[a]);
+      const float4 v4 = p.log[at];
+      const uint32_t pos = p.logpos[at];
+      const float v[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const float dv = fmaf(qmul, v[u], qn);
-      if (dv <= thr) {
-        const int to = atomicAdd(&s_n, 1);
-        if (to < RC_CAP) list[to] = make_uint2(__float_as_uint(dv), pos + u);
+      for (int u = 0; u < 4; u++) {
+        const float dv = fmaf(qmul, v[u], qn);
+        if (dv <= thr) {
+          const int to = atomicAdd(&s_n, 1);
+          if (to < RC_CAP) list[to] = make_uint2(__float_as_uint(dv), pos + u);
+        }
       }
     }
-  }
-  __syncthreads();
-  const int n = s_n;
-  if (n > RC_CAP) {
-    if (warp == 0) rerank_warp<Tab, E, false>(p, q, sm);
+    __syncthreads();
+  };
+  gather(0, total);
+  int n = s_n;
+  // A band that does not fit the list is taken a quarter of the list's quads at a time (by one warp
+  // alone, as a list it fills again and again, 0.25 us an exact distance: 500 double queries x 50,021,
+  // d = 32, k = 50, clusters of 3,100 965 us, 646 so); of a double query, only if it is a small
+  // part of the candidates (band_limit_of).
+  const bool whole = n <= RC_CAP;
+  if (!whole && sizeof(Tab) == 8 && n > p.limit) {
+    if (tid == 0) p.fallback_list[atomicAdd(p.fallback_count, 1)] = hr;
     return;
   }
-  if (n > 32 && n >= k) {
+  if (whole && n > 32 && n >= k) {
     if (warp == 0) {
       const float T = fminf(s_T, fmaxf(list_bound(list, n, k, lane), 0.0f));
       if (lane == 0) s_thr = band_thr(T, E2, thr);
@@ -2009,45 +2045,59 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
     __syncthreads();
     thr = s_thr;
   }
-  const long long qrow = p.qidx[hr];
-  if (qrow < 0 || qrow >= p.nrows_q) return;  // reported by tc_pack
-  const Tab *qv = p.Xq + qrow * p.d;
-  const double qq = (double)p.Xq2[qrow];
-  constexpr int LPC = sizeof(Tab) == 8 ? 1 : 4;  // lanes per candidate
-  for (int base = warp * (32 / LPC); base < n; base += 32 / LPC * RR_WARPS) {
-    const int i = base + lane / LPC;
-    uint32_t id = NO_ID;
-    if (i < n && __uint_as_float(list[i].x) <= thr) id = p.cid[list[i].y];
-    double dot = 0.0;
-    if constexpr (LPC == 1) {
-      if (id != NO_ID) dot = dot_lane(qv, p.Xc + (long long)id * p.d, p.d);
-    } else {
-      if (id != NO_ID) dot = exact_dot4(qv, p.Xc + (long long)id * p.d, p.d, lane & 3);
-      dot = sum4(dot);
-    }
-    if (i < n && lane % LPC == 0) {
-      xd[i] = id != NO_ID ? to_ord(exact_dist(dot, (double)p.Xc2[id], qq)) : ORD_INF;
-      xi[i] = id;
-      if (p.counters && id != NO_ID) atomicAdd(&p.counters[6], 1ull);
-    }
-  }
-  __syncthreads();
-  if (warp != 0) return;
   Ord ld[E];
   uint32_t li[E];
-  load_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
-  sort_heap_row<E>(ld, li, lane);
-  Ord kth = list_kth<E>(ld, k);
-  for (int base = 0; base < n; base += 32) {
-    const int i = base + lane;
-    Ord b1[1] = {i < n ? xd[i] : ORD_INF};
-    uint32_t i1[1] = {i < n ? xi[i] : NO_ID};
-    if (!__any_sync(FULL_MASK, i1[0] != NO_ID && b1[0] <= kth)) continue;
-    warp_sort<Ord, 1>(b1, i1, lane);
-    warp_merge_32<Ord, E>(ld, li, b1[0], i1[0], lane);
+  Ord kth = 0;
+  if (warp == 0) {
+    load_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+    sort_heap_row<E>(ld, li, lane);
     kth = list_kth<E>(ld, k);
   }
-  write_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+  constexpr int LPC = sizeof(Tab) == 8 ? 1 : 4;  // lanes per candidate
+  constexpr int STEP = RC_CAP / 4;
+  for (int e0 = 0; e0 < (whole ? 1 : total); e0 += STEP) {
+    if (!whole) {
+      __syncthreads();  // warp 0 is done with the last round
+      if (tid == 0) s_n = 0;
+      thr = s_thr;
+      __syncthreads();
+      gather(e0, min(total, e0 + STEP));
+      n = s_n;
+    }
+    for (int base = warp * (32 / LPC); base < n; base += 32 / LPC * RR_WARPS) {
+      const int i = base + lane / LPC;
+      uint32_t id = NO_ID;
+      if (i < n && __uint_as_float(list[i].x) <= thr) id = p.cid[list[i].y];
+      double dot = 0.0;
+      if constexpr (LPC == 1) {
+        if (id != NO_ID) dot = dot_lane(qv, p.Xc + (long long)id * p.d, p.d);
+      } else {
+        if (id != NO_ID) dot = exact_dot4(qv, p.Xc + (long long)id * p.d, p.d, lane & 3);
+        dot = sum4(dot);
+      }
+      if (i < n && lane % LPC == 0) {
+        xd[i] = id != NO_ID ? to_ord(exact_dist(dot, (double)p.Xc2[id], qq)) : ORD_INF;
+        xi[i] = id;
+        if (p.counters && id != NO_ID) atomicAdd(&p.counters[6], 1ull);
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      for (int base = 0; base < n; base += 32) {
+        const int i = base + lane;
+        Ord b1[1] = {i < n ? xd[i] : ORD_INF};
+        uint32_t i1[1] = {i < n ? xi[i] : NO_ID};
+        if (!__any_sync(FULL_MASK, i1[0] != NO_ID && b1[0] <= kth)) continue;
+        warp_sort<Ord, 1>(b1, i1, lane);
+        warp_merge_32<Ord, E>(ld, li, b1[0], i1[0], lane);
+        kth = list_kth<E>(ld, k);
+      }
+      const double kd = from_ord(kth);
+      if (!whole && lane == 0 && kd < 1e38)
+        s_thr = fminf(s_thr, __fadd_ru(__double2float_ru(kd), Eq));
+    }
+  }
+  if (warp == 0) write_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2598,6 +2648,18 @@ static TcCand escalation_cand(const TcCand &C, const TcPlan &EP, void *pb, void 
   return E;
 }
 
+// Candidates in a double query's band beyond which the CUDA-core kernel is the cheaper way to its
+// list. An exact distance of the re-rank costs 5 to 13 pairs of that kernel (B200, ps, d = 8, 32, 100,
+// 256: 86, 84, 285, 670 against 16, 12, 31, 53), so a twelfth of the candidates; less where the
+// queries are too few to fill the chip (a warp each, or a CTA each). Bands of the whole set, us, CUDA
+// cores alone / without the limit / with it: 4,096 x 20,000, d = 32, k = 16, points of scale 1e-20 998
+// / 8,061 / 1,304; 5,000 x 50,000, d = 100, unit cube at 1e6 6,037 / 68,192 / 6,963; 16 x 100,000,
+// d = 100 650 / 35,158 / 770; 40 x 200,000, d = 32, k = 50 in clusters of 12,500 657 / 3,769 / 1,125.
+static int band_limit_of(int nq, int nc, int k, bool cta) {
+  const double part = cta ? 0.5 + 0.5 * std::min(1.0, nq / 500.0) : std::min(1.0, nq / 1000.0);
+  return (int)std::max(4.0 * k + 256.0, nc / 12.0 * part);
+}
+
 // One approximate pass + re-rank: pack the queries (all of them, or on an escalation pass the
 // `dQ` queries listed in `rowmap`) and, with `pack_cand`, the candidates C (for the escalation pass
 // only if some query is listed); tc_knn in the plan's format; tc_rerank. Queries whose log
@@ -2714,7 +2776,8 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, bool pack_cand, boo
   const int rb = (nq + RR_WARPS - 1) / RR_WARPS;
   // one CTA per query up to four waves of one CTA per SM: 16 queries x 4,096 took 21 us against
   // 40 us with a warp each; at 2,003 queries the warps fill the chip (37 us against 67 us)
-  const bool cta = nq <= 4 * 148 && rp.S <= RC_LOGS;
+  const bool cta = nq <= 4 * P.sms && rp.S <= RC_LOGS;
+  rp.limit = band_limit_of(nq, C.nc, k, cta);
   mark(n_rr, true);
   switch (P.kp) {
     case 32: cta ? tc_rerank_cta<T, 1><<<nq, 32 * RR_WARPS, 0, st>>>(rp)
