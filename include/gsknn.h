@@ -170,11 +170,13 @@ const char *gsknn_last_error_string(void);
 #define GSKNN_MODE_TF32 2
 #define GSKNN_MODE_BF16 3
 #define GSKNN_MODE_BF16X3 4 /* split BF16: hi*hi + hi*lo + lo*hi, near-FP32 distances */
-#define GSKNN_MODE_FP16 5   /* AUTO's choice alone: reported by gsknn_serve_mode, not settable */
+#define GSKNN_MODE_FP16 5   /* AUTO's choice alone: reported by gsknn_serve_mode and measured by
+                             * gsknn_tc_distances, not taken by gsknn_set_mode / _serve_create */
 int gsknn_set_mode(int mode);
 int gsknn_get_mode(void);
 
-/* The tensor-core form on device pointers (roles and heaps as gsknn_s_device) in a given mode,
+/* The tensor-core form on device pointers (roles and heaps as gsknn_s_device) in a given mode (TF32,
+ * BF16, BF16X3 or FP16),
  * which additionally writes the approximate distance of every (query j, candidate i) pair to
  * C[j*ldc + i] (when C is not NULL) and each query's re-rank band 2E to margin[j] (when not
  * NULL): every approximate distance lies within E of the exact FP64 distance. For tests and

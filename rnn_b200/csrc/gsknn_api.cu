@@ -1051,7 +1051,7 @@ int gsknn_tc_distances(int mode, int m, int n, int d, int k, const float *XA, co
                        long long nA, const int *alpha, const float *XB, const float *XB2,
                        long long nB, const int *beta, float *D, int *I, int ldD, float *C,
                        long long ldc, float *margin, void *stream) {
-  if (mode != GSKNN_MODE_TF32 && mode != GSKNN_MODE_BF16 && mode != GSKNN_MODE_BF16X3)
+  if (mode < GSKNN_MODE_TF32 || mode > GSKNN_MODE_FP16)
     return set_status(GSKNN_ERR_ARG, "gsknn_tc_distances: mode must be a tensor-core mode");
   if (C && ldc < m) return set_status(GSKNN_ERR_ARG, "gsknn_tc_distances: ldc < m");
   return knn_device_tc(mode, nullptr, n, m, d, k, XB, XB2, nB, beta, XA, XA2, nA, alpha, D, I, ldD,
