@@ -156,6 +156,8 @@ const char *gsknn_last_error_string(void);
 /* Double calls return FP64 distances in any mode. From 32,768 (query, candidate) pairs on, with
  * k <= 256 and the 2-norm, a tensor-core pass with a rigorous error bound first narrows the
  * candidates whose FP64 distances are formed; the results are the CUDA-core kernel's bit for bit.
+ * GSKNN_MODE_FP32 keeps double calls on that kernel alone (the faster way where most distances are
+ * closer than their own rounding: points far from the origin or in very tight clusters).
  *
  * Arithmetic of the float path of sgsknn / sgsknn_var1 / gsknn_s_device:
  *   GSKNN_MODE_FP32 -- CUDA-core FP32 distances;

@@ -766,7 +766,8 @@ int knn_device(int nq, int nc, int d, int k, const T *Xq, const T *Xq2, long lon
     // cores: 1 x 300, d = 3 91 -> 103; 16 x 4,096, d = 32 136 -> 113; 4,096 x 4,096, d = 32
     // 426 -> 130; 1,000 x 20,000, k = 200 1,928 -> 476; 5,003 x 50,021, d = 100, k = 50
     // 7,853 -> 565; 8,192 x 65,536, d = 3 2,584 -> 357).
-    if ((long long)nq * nc >= 32768) {
+    // GSKNN_MODE_FP32 asks for the CUDA cores, here too.
+    if (g_mode != GSKNN_MODE_FP32 && (long long)nq * nc >= 32768) {
       const int rc = knn_device_tc_double(nq, nc, d, k, Xq, Xq2, nrows_q, qidx, Xc, Xc2, nrows_c,
                                           cidx, D, I, ldD, st);
       if (rc != -1) return rc;

@@ -44,3 +44,10 @@ def test_large_calls_take_fp16_from_d_128(d, escalates, dtype):
     assert ("tc_escalate" in auto) == escalates
     if dtype == "float32" and not escalates:
         assert auto == _kernels(4, d, dtype)
+
+
+def test_the_cuda_core_mode_holds_for_doubles():
+    """GSKNN_MODE_FP32 keeps double calls on the CUDA-core kernels, with the same results."""
+    auto, cores = _kernels(0, 20, "float64"), _kernels(1, 20, "float64")
+    assert "tc_knn" in auto
+    assert "fused_knn_simt" in cores and not any(name.startswith("tc_") for name in cores)
