@@ -1036,7 +1036,7 @@ def serving_form(L, G, W, dev, args):
     n_light = max(1, n // 2)
     lat_l, queue_l, rows_l, first_l, wall_l = run_stream(n_light, args.serve_rate / 3.0, 57)
     srv_mode, srv_probe = srv.mode, {k: round(v, 3) for k, v in srv.probe_ms.items()}
-    srv_name = "fp16" if srv_mode == 5 else MODE_NAMES.get(srv_mode, srv_mode)  # 5: AUTO's own
+    srv_name = "fp16" if srv_mode == G.MODE_FP16 else MODE_NAMES.get(srv_mode, srv_mode)
     srv.close()
     evals = float(ms.sum()) * nref
     res = {

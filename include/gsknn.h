@@ -366,8 +366,9 @@ size_t gsknn_serve_batch_bytes(int nref, int d, int mode, int max_batch_queries,
  * batches finish. Resuming dispatches everything queued in arrival order. */
 int gsknn_serve_pause(gsknn_serve_t *eng, int paused);
 /* The arithmetic the engine serves in (GSKNN_MODE_TF32 / BF16 / BF16X3 / FP16) and, after an AUTO
- * choice, the probe batch's milliseconds in FP16 and in split BF16 (0 when not probed). */
-int gsknn_serve_mode(gsknn_serve_t *eng, double *probe_bf16_ms, double *probe_bf16x3_ms);
+ * choice, the probe batch's milliseconds in the main format (FP16) and in split BF16 (0 when not
+ * probed). FP16 is AUTO's alone: gsknn_serve_create does not take it as its mode. */
+int gsknn_serve_mode(gsknn_serve_t *eng, double *probe_main_ms, double *probe_bf16x3_ms);
 void gsknn_serve_destroy(gsknn_serve_t *eng);
 
 /* ---- Streaming form: the batching form for point sets beyond HBM ---------------------------

@@ -141,7 +141,7 @@ struct TcPlan {
   // starts at o_esc, over the logs that the re-rank is done with; o_ecand holds its candidate
   // panels when the prepared candidates carry none (packed only when some query overflowed).
   int esc_mode;
-  size_t o_esc, o_ecand, esc_bytes, ecand_bytes;
+  size_t o_esc, o_ecand, ecand_bytes;
   int sms, max_splits;  // the plan's arguments, to re-derive the escalation pass's plan
   bool tight;
   size_t log_bytes;  // of the main format's logs

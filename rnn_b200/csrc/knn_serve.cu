@@ -461,9 +461,9 @@ static void completion_loop(Engine *E) {
 }
 
 // The resident set's escalation panels as a main-format candidate set of their own.
-static gsknn::TcCand escalation_as_main(const gsknn::TcCand &C, int esc_mode) {
+static gsknn::TcCand escalation_as_main(const gsknn::TcCand &C, int esc_mode, int sms) {
   gsknn::TcCand S = C;
-  const gsknn::TcPlan P = gsknn::tc_plan(128, C.nc, C.d, 1, esc_mode, 148, false, 148);
+  const gsknn::TcPlan P = gsknn::tc_plan(128, C.nc, C.d, 1, esc_mode, sms, false, sms);
   S.fmt = C.efmt;
   S.elem = C.efmt == 0 ? 4 : 2;
   S.d_pad = P.d_pad;
@@ -495,7 +495,7 @@ static bool probe_modes(Engine *E, int esc) {
   using namespace gsknn;
   gs::Slot &s = E->slots[0];
   const int rows = std::min(std::min(auto_slice(E), 2048), E->nref), kb = E->max_k;
-  const TcCand Cesc = escalation_as_main(E->C, esc);
+  const TcCand Cesc = escalation_as_main(E->C, esc, E->sms);
   const int modes[2] = {E->mode, esc};
   const TcCand *cands[2] = {&E->C, &Cesc};
   cudaEvent_t a = nullptr, b = nullptr;
@@ -732,10 +732,10 @@ gsknn_serve_t *gsknn_serve_create(const float *R, const float *R2, int nref, int
   return reinterpret_cast<gsknn_serve_t *>(raw);
 }
 
-int gsknn_serve_mode(gsknn_serve_t *eng, double *probe_bf16_ms, double *probe_bf16x3_ms) {
+int gsknn_serve_mode(gsknn_serve_t *eng, double *probe_main_ms, double *probe_bf16x3_ms) {
   Engine *E = reinterpret_cast<Engine *>(eng);
   if (!E) return -GSKNN_ERR_ARG;
-  if (probe_bf16_ms) *probe_bf16_ms = E->probe_ms[0];
+  if (probe_main_ms) *probe_main_ms = E->probe_ms[0];
   if (probe_bf16x3_ms) *probe_bf16x3_ms = E->probe_ms[1];
   return E->mode;
 }

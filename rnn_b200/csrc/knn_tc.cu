@@ -54,6 +54,7 @@ namespace gsknn {
 namespace tc {
 
 constexpr int TC_M = 128;            // queries per CTA (TMEM lanes)
+constexpr int CHIP_SMS = 148;        // B200: grids of the grid-stride kernels
 constexpr int CHUNK_BYTES = 128;     // K bytes per TMA box / swizzle atom row
 constexpr int A_CHUNK = TC_M * CHUNK_BYTES;  // 16 KB
 // Warp 0 TMA producer, warp 1 MMA issuer, then NEPI epilogue warps: NPART per TMEM lane quarter,
@@ -214,9 +215,6 @@ __device__ __forceinline__ float write_norm_row(int fmt, void *npanel, int r, bo
   return rest;
 }
 
-// fmt: 0 = TF32 (4-byte panel), 1 = BF16, 2 = split BF16 (hi and lo panels), 3 = FP16, scaled by a
-// power of two that takes the sampled coordinates to at most 2^12
-//
 // One side of a packing launch: `rows_pad` panel rows, of which the first `count` are points
 // idx[r] (idx[rowmap[r]] with a row map) of table X. `dcount` (device) replaces `count` and limits
 // the panel to the tiles it needs; `gate` (device) skips the side when it reads 0; `pad_ok` packs
@@ -250,7 +248,10 @@ constexpr int STATS_WORDS = 8;
 
 template <typename T>
 struct PackArgs {
-  int fmt, d, d_pad;
+  // 0 = TF32 (4-byte panel), 1 = BF16, 2 = split BF16 (hi and lo panels), 3 = FP16, scaled by a
+  // power of two that takes the sampled coordinates to at most 2^12
+  int fmt;
+  int d, d_pad;
   PackSide<T> a, b;
   // the shift: from tc_center's partial sums (and written to mu for later launches), or, with part
   // null, read from mu
@@ -452,7 +453,7 @@ __global__ void __launch_bounds__(256) tc_pack(const PackArgs<T> g) {
       // |x - mu|^2 expressed through the caller's norm: X2 - 2 mu.x + mu.mu
       const double x2 = row >= 0 ? (double)s.X2[row] : 0.0;
       const float enf = row >= 0 ? (float)(x2 - 2.0 * smx + mu2) : Num<float>::nan();
-float nres = 0.0f;
+      float nres = 0.0f;
       if (s.npanel)
         nres = write_norm_row(g.fmt, s.npanel, r, row >= 0,
                               row >= 0 ? -0.5f * enf * (fs * fs) : 0.0f);
@@ -502,19 +503,18 @@ float nres = 0.0f;
 // grid-stride beyond.
 static inline unsigned tc_pack_grid(long long rows) {
   const long long want = (rows + 31) / 32;
-  return (unsigned)std::max(1LL, std::min(want, 148LL * 8));
+  return (unsigned)std::max(1LL, std::min(want, CHIP_SMS * 8LL));
 }
 
 // ------------------------------------------------------------------------------------------
 // the tensor-core kernel
 // ------------------------------------------------------------------------------------------
 struct TcParams {
-  int Q, k, nkc, ntiles_r, N, NST, logcap;
-  int a_terms, fmt;
+  int Q, nkc, ntiles_r, N, NST, logcap;
+  int a_terms;
   int fold;  // norm column in use (set by launch_tc_knn)
   uint32_t idesc;
   const float *cn;
-  const uint32_t *cid;
   const float *qn;
   const float4 *qe;       // per-query terms of the error bound (tc_pack)
   const float *qmx;       // largest incoming distance of each query's heap row (-inf: none)
@@ -1383,9 +1383,6 @@ struct RerankParams {
   unsigned long long *counters;  // optional: [5] entries scanned, [6] exact distances
   const int *dQ;      // optional: query count on the device (Q is then the stride)
   const int *rowmap;  // optional: heap row (and query position in qidx) of each query; -1: none
-  // batching form: candidates already in the incoming heap row (by id) are not entered twice,
-  // and overflowed queries go to the fallback list as their own positions q
-  int dedup;
 };
 
 // d' of a logged value x: fma(log_mul, x, qn)
@@ -1677,7 +1674,7 @@ struct RerankSmem {
 };
 
 // One query by one warp. LEAF (the batching form): ids already in the row are not entered again,
-// the incoming row stays unsorted until a candidate can enter it, and a row nothing entered is
+// overflowed queries are listed by their panel rows, the incoming row stays unsorted until a candidate can enter it, and a row nothing entered is
 // not written back.
 template <typename Tab, int E, bool LEAF>
 __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, RerankSmem<E> &sm) {
@@ -2623,7 +2620,6 @@ TcPlan tc_plan(int nq, int nc, int d, int k, int mode, int sms, bool with_cand,
   if (P.esc_mode) {
     const TcPlan EP = tc_plan_base(nq, nc, d, k, P.esc_mode, sms, false, max_splits, tight);
     P.o_esc = P.o_log;
-    P.esc_bytes = EP.bytes;
     size_t off = al256(std::max(P.bytes, P.o_esc + EP.bytes));
     if (with_cand) {  // per-call candidates: their escalation panels live in the workspace
       P.o_ecand = off;
@@ -2731,12 +2727,12 @@ static cudaError_t tc_pass(const TcPlan &P, const TcCand &C, bool pack_cand, boo
     if (e != cudaSuccess) return e;
   }
   TcParams tp{};
-  tp.Q = nq; tp.k = k; tp.nkc = P.nkc; tp.ntiles_r = P.rtiles;
+  tp.Q = nq; tp.nkc = P.nkc; tp.ntiles_r = P.rtiles;
   tp.N = P.N; tp.NST = P.NST; tp.logcap = P.logcap;
-  tp.a_terms = P.a_terms; tp.fmt = P.fmt;
+  tp.a_terms = P.a_terms;
   tp.idesc = idesc_f32acc(P.fmt == 0 ? 2u : P.fmt == 3 ? 0u : 1u, TC_M, P.N);
   tp.fscale = P.fmt == 3 ? C.fscale : nullptr;
-  tp.cn = C.cn; tp.cid = C.cid; tp.qn = qn; tp.qe = qs.qe; tp.qmx = qs.qmx; tp.stats = C.stats;
+  tp.cn = C.cn; tp.qn = qn; tp.qe = qs.qe; tp.qmx = qs.qmx; tp.stats = C.stats;
   tp.log = reinterpret_cast<float4 *>(base + P.o_log);
   tp.logpos = reinterpret_cast<uint32_t *>(tp.log + (size_t)NPART * P.S * nq * P.logcap);
   tp.logcnt = reinterpret_cast<int *>(base + P.o_logcnt);
@@ -2811,10 +2807,10 @@ static cudaError_t tc_brute(const TcPlan &P, const TcCand &C, int d, int k, cons
   fp.count = reinterpret_cast<const int *>(base + P.o_fbc);
   if (hook) hook(hook_ctx, "tc_fallback", true, st, 0);
   switch (P.kp) {
-    case 32: tc_fallback<1><<<148, 256, 0, st>>>(fp); break;
-    case 64: tc_fallback<2><<<148, 256, 0, st>>>(fp); break;
-    case 128: tc_fallback<4><<<148, 256, 0, st>>>(fp); break;
-    case 256: tc_fallback<8><<<148, 256, 0, st>>>(fp); break;
+    case 32: tc_fallback<1><<<CHIP_SMS, 256, 0, st>>>(fp); break;
+    case 64: tc_fallback<2><<<CHIP_SMS, 256, 0, st>>>(fp); break;
+    case 128: tc_fallback<4><<<CHIP_SMS, 256, 0, st>>>(fp); break;
+    case 256: tc_fallback<8><<<CHIP_SMS, 256, 0, st>>>(fp); break;
     default: return cudaErrorInvalidValue;
   }
   cudaError_t e = cudaGetLastError();
@@ -3094,11 +3090,11 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   if (e == cudaSuccess) e = make_panel_map(&mBlo, pb_lo, P.elem, P.d_pad, rows, P.N);
   if (e != cudaSuccess) return e;
   TcParams tp{};
-  tp.Q = rows; tp.k = k; tp.nkc = P.nkc; tp.ntiles_r = rows / P.N;
+  tp.Q = rows; tp.nkc = P.nkc; tp.ntiles_r = rows / P.N;
   tp.N = P.N; tp.NST = P.NST; tp.logcap = P.logcap;
-  tp.a_terms = P.a_terms; tp.fmt = P.fmt;
+  tp.a_terms = P.a_terms;
   tp.idesc = idesc_f32acc(1u, TC_M, P.N);
-  tp.cn = cn; tp.cid = cid; tp.qn = cn; tp.qe = ps.qe; tp.qmx = ps.qmx; tp.stats = stats;
+  tp.cn = cn; tp.qn = cn; tp.qe = ps.qe; tp.qmx = ps.qmx; tp.stats = stats;
   tp.log = reinterpret_cast<float4 *>(base + P.o_log);
   tp.logpos = reinterpret_cast<uint32_t *>(tp.log + (size_t)NPART * P.S * rows * P.logcap);
   tp.logcnt = reinterpret_cast<int *>(base + P.o_logcnt);
@@ -3124,7 +3120,6 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   rp.fallback_list = reinterpret_cast<int *>(base + P.o_fbl);
   rp.fallback_count = fbc;
   rp.rowmap = pidx;
-  rp.dedup = 1;
   rp.counters = counters;
   LeafFallbackParams fp{};
   fp.k = k; fp.d = d; fp.N = P.N; fp.X = X; fp.X2 = X2; fp.rowmap = pidx; fp.ids = cid;
@@ -3134,19 +3129,19 @@ cudaError_t tc_leaf_pass(const TcLeafPlan &L, void *ws, const float *X, const fl
   switch (P.kp) {
     case 32:
       tc_rerank_leaf<1><<<rb, 256, 0, st>>>(rp);
-      tc_fallback_leaf<1><<<148, 256, 0, st>>>(fp);
+      tc_fallback_leaf<1><<<CHIP_SMS, 256, 0, st>>>(fp);
       break;
     case 64:
       tc_rerank_leaf<2><<<rb, 256, 0, st>>>(rp);
-      tc_fallback_leaf<2><<<148, 256, 0, st>>>(fp);
+      tc_fallback_leaf<2><<<CHIP_SMS, 256, 0, st>>>(fp);
       break;
     case 128:
       tc_rerank_leaf<4><<<rb, 256, 0, st>>>(rp);
-      tc_fallback_leaf<4><<<148, 256, 0, st>>>(fp);
+      tc_fallback_leaf<4><<<CHIP_SMS, 256, 0, st>>>(fp);
       break;
     case 256:
       tc_rerank_leaf<8><<<rb, 256, 0, st>>>(rp);
-      tc_fallback_leaf<8><<<148, 256, 0, st>>>(fp);
+      tc_fallback_leaf<8><<<CHIP_SMS, 256, 0, st>>>(fp);
       break;
     default: return cudaErrorInvalidValue;
   }

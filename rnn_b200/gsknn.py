@@ -31,7 +31,8 @@ LIB_PATH = os.path.join(HERE, "libgsknn.so")
 _lib = None
 _lock = threading.Lock()
 
-MODE_AUTO, MODE_FP32, MODE_TF32, MODE_BF16 = 0, 1, 2, 3
+MODE_AUTO, MODE_FP32, MODE_TF32, MODE_BF16, MODE_BF16X3 = 0, 1, 2, 3, 4
+MODE_FP16 = 5  # AUTO's own: what Server.mode may report, not a mode to set
 EARLY_RETURN = 1
 KNN_2NORM, KNN_1NORM = 0, 1  # knn_type (include/gsknn.h)
 

@@ -47,7 +47,8 @@ class Server:
         L.gsknn_serve_mode.argtypes = [vp, vp, vp]
         a, b = ctypes.c_double(0.0), ctypes.c_double(0.0)
         self.mode = L.gsknn_serve_mode(h, ctypes.byref(a), ctypes.byref(b))
-        self.probe_ms = {"bf16": a.value, "bf16x3": b.value}
+        # "main": the format AUTO prepares (FP16); "bf16" is its former name
+        self.probe_ms = {"main": a.value, "bf16": a.value, "bf16x3": b.value}
         self.slice_rows = self.set_slice(slice_rows)
 
     def submit(self, Q: np.ndarray, k: int) -> int:
