@@ -35,8 +35,9 @@
 //                                  + 2 (n 2^-23 (1+u)^2 + 2^-22) |q~| M          accumulation
 //                                  + 3 * 2^-24 (CN + |qn'| + 2 |q~| M) ] + noise
 // For the split format r(q~) M + ... is replaced by 3.2 u^2 |q~| M (u = 2^-8; it covers the omitted
-// lo x lo product) and n = 3D + NORM_TERMS. With the norm column E gains
-// 1.25 (NORM_TERMS 2^-23 + 2^-24) CN for the norm parts it sums: they are accumulated last. `noise` covers the rounding of the FP64 distance itself, (4d + 32) 2^-53 of
+// lo x lo product) and n = 3D + NORM_TERMS. With the norm column E gains 1.25 (t 2^-23 + 2^-24) CN
+// for the norm parts it sums, t = NORM_TERMS in the split format, which accumulates them last, and n
+// in the others. `noise` covers the rounding of the FP64 distance itself, (4d + 32) 2^-53 of
 // the squared norms' scale. Measuring r takes the input term to about 0.4 of its worst case
 // (2u + u^2) |q~| M.
 #include "knn_common.cuh"
@@ -956,6 +957,24 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                    &cnfull[c]);
         }
         tc_fence_after();
+        // The norm column's MMA. In split BF16 it goes last: first, every later addition would add a
+        // rounding of |cn|/2 to the bound (E at d = 80 and 128 was 1.27 times what it is without the
+        // column, and clusters overflowed their logs). The single-term formats' bound is their input
+        // rounding, and last it stands behind the tile's final stage: 32,768 x 262,144, d = 256, k = 64
+        // in FP16 5,502 us, first 5,424.
+        auto norm_mma = [&](uint32_t accumulate) {
+          if (!mbar_wait(&nfull[b], use & 1u)) { failed = true; return; }
+          tc_fence_after();
+          const uint64_t ad = sdesc_k_sw32(su32(sAn));
+          const uint64_t bd = sdesc_k_sw32(su32(sBn) + (uint32_t)b * N * NORM_ROW);
+          if (FMT == 0) mma_tf32(tmem_d, ad, bd, p.idesc, accumulate);
+          else mma_f16(tmem_d, ad, bd, p.idesc, accumulate);
+        };
+        constexpr bool NORM_FIRST = FOLD && FMT != 2;
+        if (NORM_FIRST) {
+          norm_mma(0u);
+          if (failed) break;
+        }
         for (int i = 0; i < TERMS * p.nkc; i++) {
           const int s = stage, kc = i / TERMS;
           const bool lo = i % TERMS != 0;
@@ -972,7 +991,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           // descriptor's address field (16-byte units).
           const uint64_t ad = sdesc_k_sw128(a_base + (uint32_t)kc * A_CHUNK);
           const uint64_t bd = sdesc_k_sw128(b_base + (uint32_t)s * b_stage_bytes);
-          const uint32_t first = i != 0 ? 1u : 0u;
+          const uint32_t first = NORM_FIRST || i != 0 ? 1u : 0u;
           if (FMT == 2 && !lo) {
             // hi stage: the query's lo part too
             const uint64_t ld = sdesc_k_sw128(a_base + (uint32_t)(p.nkc + kc) * A_CHUNK);
@@ -992,19 +1011,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           }
           mma_commit(&empty[s]);
         }
-        if (FOLD && !failed) {
-          // the norm column last: every later addition would add a rounding of |cn|/2 to the bound
-          // (first, E at d = 80 and 128 in split BF16 was 1.27 times what it is without it)
-          if (mbar_wait(&nfull[b], use & 1u)) {
-            tc_fence_after();
-            const uint64_t ad = sdesc_k_sw32(su32(sAn));
-            const uint64_t bd = sdesc_k_sw32(su32(sBn) + (uint32_t)b * N * NORM_ROW);
-            if (FMT == 0) mma_tf32(tmem_d, ad, bd, p.idesc, 1u);
-            else mma_f16(tmem_d, ad, bd, p.idesc, 1u);
-          } else {
-            failed = true;
-          }
-        }
+        if (FOLD && !NORM_FIRST && !failed) norm_mma(1u);
         if (!failed) {
           if (FOLD) mma_commit(&nempty[b]);
           mma_commit(&tfull[b]);
@@ -2573,8 +2580,9 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
   // magnitudes, |q~| |c~| (1 + u)^2 (the rounded factors), over the products and the norm column's
   // MMA, and the FP32 rounding of both centred factors. kB: FP32 rounding of the
   // norm terms. kS: the FP64 distance's own rounding (and the effective norms'). With the norm
-  // column the last MMA also adds the three parts of -cn/2 (exact in the input format), whose
-  // magnitudes sum to CN / 2; in v = -2w that is twice as much: kC_fold. The final d' = v + qn'
+  // column its MMA, the last in split BF16 and the first in the others, also adds the three parts of
+  // -cn/2 (exact in the input format), whose magnitudes sum to CN / 2; in v = -2w that is twice as
+  // much: kC_fold. The final d' = v + qn'
   // rounds once, inside the kB term. The input rounding itself is measured (tc_pack).
   {
     const double D = (double)P.d_pad;
@@ -2583,7 +2591,7 @@ static TcPlan tc_plan_base(int nq, int nc, int d, int k, int mode, int sms, bool
     const double acc = n * std::ldexp(1.0, -23), last = NORM_TERMS * std::ldexp(1.0, -23);
     P.kA = (float)(acc * (1 + u) * (1 + u) + std::ldexp(1.0, -22));
     P.kB = (float)(1.25 * 3.0 * std::ldexp(1.0, -24) + 1e-12);
-    P.kC_fold = (float)(1.25 * (last + std::ldexp(1.0, -24)) + 1e-12);
+    P.kC_fold = (float)(1.25 * ((P.fmt == 2 ? last : acc) + std::ldexp(1.0, -24)) + 1e-12);
     P.kS = (float)(1.25 * (4.0 * d + 32.0) * std::ldexp(1.0, -53));
   }
   P.ok = true;
