@@ -536,8 +536,8 @@ struct RowChunks {
   TcPlan P, T;     // plans of the whole chunks and of the last
 };
 
-// Plans the call and gets its workspace; `whole`, when set, is the plan of all rows, and `extra(rows)`
-// the bytes that a chunk takes behind its plan's. cudaErrorInvalidValue: no plan.
+// Plans the call and gets its workspace; `whole`, when set, is the plan of all rows, and
+// `extra(rows, tail)` the bytes that a chunk takes behind its plan's. cudaErrorInvalidValue: no plan.
 template <typename Extra>
 static cudaError_t tc_workspace(int mode, const TcPlan *whole, int nq, int nc, int d, int k,
                                 cudaStream_t st, Extra extra, RowChunks *c, void **ws) {
@@ -554,8 +554,10 @@ static cudaError_t tc_workspace(int mode, const TcPlan *whole, int nq, int nc, i
       part = std::min(0.99, (double)LOG_BUDGET / (double)c->P.log_bytes);
     } else {
       const cudaError_t e =
-          scratch(SLOT_KERNEL, std::max(align256(c->P.bytes) + extra(rows),
-                                        align256(c->T.bytes) + extra(c->tail)), st, ws);
+          scratch(SLOT_KERNEL,
+                  std::max(align256(c->P.bytes) + extra(rows, false),
+                           c->tail == rows ? 0 : align256(c->T.bytes) + extra(c->tail, true)),
+                  st, ws);
       if (e != cudaErrorMemoryAllocation || rows <= MIN_CHUNK) return e;
     }
     const int fewer = (int)(rows * part), unit = fewer >= wave ? wave : 128;
@@ -582,7 +584,7 @@ static int knn_device_tc(int mode, const TcPlan *plan, int nq, int nc, int d, in
   void *ws = nullptr;
   StatusWords sw;
   const cudaError_t we =
-      tc_workspace(mode, plan, nq, nc, d, k, st, [](int) { return (size_t)0; }, &ch, &ws);
+      tc_workspace(mode, plan, nq, nc, d, k, st, [](int, bool) { return (size_t)0; }, &ch, &ws);
   if (!ch.P.ok)
     return set_status(GSKNN_ERR_UNSUPPORTED,
                       "tensor-core mode %d does not support d=%d k=%d (shared memory)", mode, d,
@@ -677,9 +679,11 @@ static int knn_device_tc_double(int nq, int nc, int d, int k, const double *Xq, 
   RowChunks ch;
   void *ws = nullptr;
   StatusWords sw;
+  SimtPlan F[2];  // of the whole chunks and of the last
   const cudaError_t se = tc_workspace(
       mode, &P, nq, nc, d, k, st,
-      [&](int rows) { return simt_plan<double>(rows, nc, d, k).bytes; }, &ch, &ws);
+      [&](int rows, bool tail) { return (F[tail] = simt_plan<double>(rows, nc, d, k)).bytes; }, &ch,
+      &ws);
   if (se == cudaErrorMemoryAllocation) return -1;
   CU(se);
   CU(status_words(st, &sw));
@@ -687,13 +691,12 @@ static int knn_device_tc_double(int nq, int nc, int d, int k, const double *Xq, 
   for (int q0 = 0; q0 < nq; q0 += ch.rows) {
     const int n = std::min(ch.rows, nq - q0);
     const TcPlan &R = n == ch.rows ? ch.P : ch.T;
-    const SimtPlan F = simt_plan<double>(n, nc, d, k);
     const int *left = nullptr, *nleft = nullptr;
     double *Dq = D + (size_t)q0 * ldD;
     int *Iq = I + (size_t)q0 * ldD;
     CU(tc_run_double(R, n, nc, d, k, Xq, Xq2, nrows_q, qidx + q0, Xc, Xc2, nrows_c, cidx, Dq, Iq,
                      ldD, ws, status, &left, &nleft, st, trace_hook, nullptr, q0 == 0));
-    const int rc = simt_run<double>(F, n, nc, d, k, Xq, Xq2, nrows_q, qidx + q0, Xc, Xc2, nrows_c,
+    const int rc = simt_run<double>(F[n != ch.rows], n, nc, d, k, Xq, Xq2, nrows_q, qidx + q0, Xc, Xc2, nrows_c,
                                     cidx, Dq, Iq, ldD, static_cast<char *>(ws) + align256(R.bytes),
                                     sw, st, 0, left, nleft);
     if (rc != GSKNN_OK) return rc;

@@ -1834,19 +1834,28 @@ __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, R
       if (n <= CAP / 2) continue;
       // A band that fills the list: a double query whose band is a large part of the candidates
       // (points closer than the rounding of their own distances) leaves before its first exact
-      // distance, not with its whole band's (band_limit_of).
+      // distance, not with its whole band's (band_limit_of). Counted are the candidates within 2E
+      // of the nearest one, which are in the band whatever the k-th turns out to be.
       if constexpr (sizeof(Tab) == 8) {
         if (!counted) {
           counted = true;
+          float lo = Num<float>::inf();
           int c = 0;
-          for (int s = 0; s < p.S; s++) {
-            const int cnt = p.logcnt[(size_t)s * p.Q + q];
-            const float4 *const lg = p.log + ((size_t)s * p.Q + q) * p.logcap;
-            for (int e = lane; e < cnt; e += 32) {
-              const float4 v = lg[e];
-              c += (fmaf(qmul, v.x, qn) <= thr) + (fmaf(qmul, v.y, qn) <= thr) +
-                   (fmaf(qmul, v.z, qn) <= thr) + (fmaf(qmul, v.w, qn) <= thr);
+          for (int sweep = 0; sweep < 2; sweep++) {
+            const float t = __fadd_rd(fmaxf(lo, 0.0f), E2);
+            for (int s = 0; s < p.S; s++) {
+              const int cnt = p.logcnt[(size_t)s * p.Q + q];
+              const float4 *const lg = p.log + ((size_t)s * p.Q + q) * p.logcap;
+              for (int e = lane; e < cnt; e += 32) {
+                const float4 v = lg[e];
+                const float d0 = fmaf(qmul, v.x, qn), d1 = fmaf(qmul, v.y, qn),
+                            d2 = fmaf(qmul, v.z, qn), d3 = fmaf(qmul, v.w, qn);
+                if (sweep == 0) lo = fminf(lo, fminf(fmin3(d0, d1, d2), d3));
+                else c += (d0 <= t) + (d1 <= t) + (d2 <= t) + (d3 <= t);
+              }
             }
+            if (sweep == 0)
+              for (int o = 16; o; o >>= 1) lo = fminf(lo, __shfl_xor_sync(FULL_MASK, lo, o));
           }
           if (__reduce_add_sync(FULL_MASK, c) > p.limit) {
             if (lane == 0) p.fallback_list[atomicAdd(p.fallback_count, 1)] = hr;
@@ -1950,6 +1959,8 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
   __shared__ uint2 list[RC_CAP];
   __shared__ Ord xd[RC_CAP];
   __shared__ uint32_t xi[RC_CAP];
+  __shared__ Ord hold_d[32 * E];  // the list between the rounds of a wide band
+  __shared__ uint32_t hold_i[32 * E];
   __shared__ int pre[RC_LOGS + 1];
   __shared__ float s_T, s_thr;
   __shared__ int s_n, s_state;
@@ -2032,6 +2043,28 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
   };
   gather(0, total);
   int n = s_n;
+  // The partition bound is loose where long lists meet many short splits: entries that fill the list
+  // bound the k-th far better, and what is left under their bound mostly fits (2 x 13,650, d = 141,
+  // k = 100 321 us without this, 186).
+  for (int pass = 0; n > RC_CAP && pass < 3; pass++) {
+    if (warp == 0) {
+      const float T = fminf(s_T, fmaxf(list_bound(list, RC_CAP, k, lane), 0.0f));
+      if (lane == 0) {
+        s_T = T;
+        s_thr = band_thr(T, E2, thr);
+        s_n = 0;
+      }
+    }
+    __syncthreads();
+    if (!(s_thr < thr)) {
+      if (tid == 0) s_n = n;
+      __syncthreads();
+      break;
+    }
+    thr = s_thr;
+    gather(0, total);
+    n = s_n;
+  }
   // A band that does not fit the list is taken a quarter of the list's quads at a time (by one warp
   // alone, as a list it fills again and again, 0.25 us an exact distance: 500 double queries x 50,021,
   // d = 32, k = 50, clusters of 3,100 965 us, 646 so); of a double query, only if it is a small
@@ -2049,25 +2082,9 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
     __syncthreads();
     thr = s_thr;
   }
-  Ord ld[E];
-  uint32_t li[E];
-  Ord kth = 0;
-  if (warp == 0) {
-    load_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
-    sort_heap_row<E>(ld, li, lane);
-    kth = list_kth<E>(ld, k);
-  }
   constexpr int LPC = sizeof(Tab) == 8 ? 1 : 4;  // lanes per candidate
-  constexpr int STEP = RC_CAP / 4;
-  for (int e0 = 0; e0 < (whole ? 1 : total); e0 += STEP) {
-    if (!whole) {
-      __syncthreads();  // warp 0 is done with the last round
-      if (tid == 0) s_n = 0;
-      thr = s_thr;
-      __syncthreads();
-      gather(e0, min(total, e0 + STEP));
-      n = s_n;
-    }
+  // exact distances of the listed entries under thr, by all warps
+  auto exact = [&]() {
     for (int base = warp * (32 / LPC); base < n; base += 32 / LPC * RR_WARPS) {
       const int i = base + lane / LPC;
       uint32_t id = NO_ID;
@@ -2086,22 +2103,75 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
       }
     }
     __syncthreads();
-    if (warp == 0) {
-      for (int base = 0; base < n; base += 32) {
-        const int i = base + lane;
-        Ord b1[1] = {i < n ? xd[i] : ORD_INF};
-        uint32_t i1[1] = {i < n ? xi[i] : NO_ID};
-        if (!__any_sync(FULL_MASK, i1[0] != NO_ID && b1[0] <= kth)) continue;
-        warp_sort<Ord, 1>(b1, i1, lane);
-        warp_merge_32<Ord, E>(ld, li, b1[0], i1[0], lane);
-        kth = list_kth<E>(ld, k);
-      }
-      const double kd = from_ord(kth);
-      if (!whole && lane == 0 && kd < 1e38)
-        s_thr = fminf(s_thr, __fadd_ru(__double2float_ru(kd), Eq));
+  };
+  Ord ld[E];
+  uint32_t li[E];
+  // merges them into the list, by warp 0
+  auto merge = [&](Ord kth) {
+    for (int base = 0; base < n; base += 32) {
+      const int i = base + lane;
+      Ord b1[1] = {i < n ? xd[i] : ORD_INF};
+      uint32_t i1[1] = {i < n ? xi[i] : NO_ID};
+      if (!__any_sync(FULL_MASK, i1[0] != NO_ID && b1[0] <= kth)) continue;
+      warp_sort<Ord, 1>(b1, i1, lane);
+      warp_merge_32<Ord, E>(ld, li, b1[0], i1[0], lane);
+      kth = list_kth<E>(ld, k);
+    }
+    return kth;
+  };
+  if (whole) {
+    exact();
+    if (warp != 0) return;
+    load_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+    sort_heap_row<E>(ld, li, lane);
+    merge(list_kth<E>(ld, k));
+    write_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+    return;
+  }
+  // The list waits in shared memory between the rounds (kept in registers across them, the exact
+  // distances of every other call were a third slower).
+  constexpr int STEP = RC_CAP / 4;
+  if (warp == 0) {
+    load_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+    sort_heap_row<E>(ld, li, lane);
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      hold_d[e * 32 + lane] = ld[e];
+      hold_i[e * 32 + lane] = li[e];
     }
   }
-  if (warp == 0) write_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+  for (int e0 = 0; e0 < total; e0 += STEP) {
+    __syncthreads();  // warp 0 is done with the last round
+    if (tid == 0) s_n = 0;
+    thr = s_thr;
+    __syncthreads();
+    gather(e0, min(total, e0 + STEP));
+    n = s_n;
+    if (n == 0) continue;
+    exact();
+    if (warp == 0) {
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        ld[e] = hold_d[e * 32 + lane];
+        li[e] = hold_i[e * 32 + lane];
+      }
+      const double kd = from_ord(merge(list_kth<E>(ld, k)));
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        hold_d[e * 32 + lane] = ld[e];
+        hold_i[e * 32 + lane] = li[e];
+      }
+      if (lane == 0 && kd < 1e38) s_thr = fminf(s_thr, __fadd_ru(__double2float_ru(kd), Eq));
+    }
+  }
+  if (warp == 0) {
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      ld[e] = hold_d[e * 32 + lane];
+      li[e] = hold_i[e * 32 + lane];
+    }
+    write_heap_row<Tab, E>(p.D, p.I, p.ldD, hr, k, ld, li, lane);
+  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2657,8 +2727,8 @@ static TcCand escalation_cand(const TcCand &C, const TcPlan &EP, void *pb, void 
 // 256: 86, 84, 285, 670 against 16, 12, 31, 53), so a twelfth of the candidates; less where the
 // queries are too few to fill the chip (a warp each, or a CTA each). Bands of the whole set, us, CUDA
 // cores alone / without the limit / with it: 4,096 x 20,000, d = 32, k = 16, points of scale 1e-20 998
-// / 8,061 / 1,304; 5,000 x 50,000, d = 100, unit cube at 1e6 6,037 / 68,192 / 6,963; 16 x 100,000,
-// d = 100 650 / 35,158 / 770; 40 x 200,000, d = 32, k = 50 in clusters of 12,500 657 / 3,769 / 1,125.
+// / 8,061 / 1,376; 5,000 x 50,000, d = 100, unit cube at 1e6 6,037 / 68,192 / 7,060; 16 x 100,000,
+// d = 100 650 / 35,158 / 773; 40 x 200,000, d = 32, k = 50 in clusters of 12,500 657 / 3,769 / 1,171.
 static int band_limit_of(int nq, int nc, int k, bool cta) {
   const double part = cta ? 0.5 + 0.5 * std::min(1.0, nq / 500.0) : std::min(1.0, nq / 1000.0);
   return (int)std::max(4.0 * k + 256.0, nc / 12.0 * part);
