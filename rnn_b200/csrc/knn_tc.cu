@@ -3061,8 +3061,8 @@ TcLeafPlan tc_leaf_plan(long long npts, int rows_cap, int d, int k, int sms, boo
   L.rows_cap = rows_cap;
   // per-query area for rows_cap rows, one split; smaller logs than the per-call path: a leaf offers
   // a few thousand candidates, of which a part logs about hk (1 + ln(n / hk)) < 5 hk quads (a full
-  // log overflows to the leaf brute force)
-  P.logcap = 6 * tc_heap_k(k) + 32;
+  // log overflows to the leaf brute force), and the room that two chunks want
+  P.logcap = 6 * tc_heap_k(k) + 24 + LOG_ROOM;
   if (tight) P.logcap = std::min(P.logcap, log_entries(std::max(2 * P.kp, 256), true));
   P.S = 1;
   P.qtiles = L.rows_cap / TC_M;
