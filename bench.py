@@ -1155,6 +1155,9 @@ def kernel_case(name: str) -> dict:
       config1     dgsknn FP64 (pack_panels, fused_knn_simt<double>, finalize_heap)
       large_k     k = 600 float (dist_block, select_rows)
       tc_q8192    split BF16 on 8,192 headline queries (tc_pack, tc_knn, tc_rerank)
+      fp16_q8192  scaled FP16 on 8,192 queries of the precision workload (the same kernels)
+      few_q       100 headline queries (tc_rerank_cta)
+      l1_q8192    the 1-norm on 8,192 headline queries (fused_knn_simt<float>, 1-norm)
       fp32_q8192  plain FP32 on 8,192 headline queries (fused_knn_simt<float>)
       batch_small one pass of 8 trees over 262,144 mixture points (batch_pack, batch_knn_simt,
                   batch_merge); batch_small_tc the same in the tensor-core shape
@@ -1169,7 +1172,7 @@ def kernel_case(name: str) -> dict:
     # device time of the last (profiled) call or pass
     ev = [torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)]
 
-    def dev_call(X, X2, alpha, beta, k, mode=0, reps=2):
+    def dev_call(X, X2, alpha, beta, k, mode=0, reps=2, metric=0):
         Xd, X2d = torch.from_numpy(X).to(dev), torch.from_numpy(X2).to(dev)
         a, b = torch.from_numpy(alpha).to(dev), torch.from_numpy(beta).to(dev)
         D = torch.empty((beta.size, k), dtype=Xd.dtype, device=dev)
@@ -1179,7 +1182,7 @@ def kernel_case(name: str) -> dict:
             D.fill_(float("inf"))
             I.fill_(-1)
             ev[0].record()
-            G.knn_device(Xd, X2d, a, Xd, X2d, b, D, I)
+            G.knn_device(Xd, X2d, a, Xd, X2d, b, D, I, metric=metric)
             ev[1].record()
         torch.cuda.synchronize()
         G.set_mode(0)
@@ -1190,10 +1193,11 @@ def kernel_case(name: str) -> dict:
     elif name == "large_k":
         p = W.config2(n_queries=2048, n_refs=65536, k=600)
         dev_call(p.X, p.X2, p.alpha, p.beta, p.k)
-    elif name in ("tc_q8192", "fp32_q8192"):
-        p = W.config2()
-        beta = np.ascontiguousarray(p.beta[:8192])
-        dev_call(p.X, p.X2, p.alpha, beta, p.k, mode=1 if name == "fp32_q8192" else 0)
+    elif name in ("tc_q8192", "fp32_q8192", "l1_q8192", "few_q", "fp16_q8192"):
+        p = W.config3() if name == "fp16_q8192" else W.config2()
+        beta = np.ascontiguousarray(p.beta[:100 if name == "few_q" else 8192])
+        dev_call(p.X, p.X2, p.alpha, beta, p.k, mode=1 if name == "fp32_q8192" else 0,
+                 metric=G.KNN_1NORM if name == "l1_q8192" else G.KNN_2NORM)
     elif name in ("batch_small", "batch_small_tc"):
         from rnn_b200 import batch as B
         p = W.config4(n_points=1 << 18, passes=1)

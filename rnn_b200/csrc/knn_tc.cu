@@ -1182,9 +1182,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // lasted: 8,192 x 250,000, d = 32, k = 128 on clusters of sigma 0.01 3,121 brute-forced queries
     // and 118 ms, now 246 and 16 ms.)
     auto make_room = [&]() {
-      if (!__any_sync(FULL_MASK, s.cnt > p.logcap - LOG_ROOM)) return;
-      epi_flush<FOLD, RINGED>(s, myheap, myring, lg, row, p.hk, pslot);
       const bool full = s.cnt > p.logcap - LOG_ROOM && !s.ovf;
+      if (!__any_sync(FULL_MASK, full)) return;
+      epi_flush<FOLD, RINGED>(s, myheap, myring, lg, row, p.hk, pslot);
       if (!p.no_compact) {
         const int left = log_compact<FOLD>(lg, lp, s.cnt, FOLD ? s.Tw : s.Tv, full);
         if (full) s.cnt = s.done = left;
