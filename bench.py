@@ -108,7 +108,7 @@ def parse():
                     help="mean request arrival rate (requests/s, Poisson)")
     ap.add_argument("--kernel-case", default=None,
                     choices=["config1", "large_k", "tc_q8192", "batch_small", "serve_one",
-                             "fp32_q8192", "batch_small_tc"],
+                             "fp32_q8192", "batch_small_tc", "fp16_q8192", "few_q", "l1_q8192"],
                     help="one small run of one path, for per-kernel profiling: warm-up call, "
                          "then the profiled call")
     ap.add_argument("--cpu-worker", default=None, help=argparse.SUPPRESS)
@@ -486,7 +486,7 @@ def timed(L, G, prob, mode, steps, warmup, barrier=None, clocks=None):
 
 # DRAM bytes per launch of the dominant kernel, from one ncu capture of this same workload
 # (dram__bytes_read.sum + dram__bytes_write.sum; profiles/launch_list_headline_config2.md)
-TRAFFIC = {("tc_knn", "bf16x3", N_Q): 319163392 + 489858560}
+TRAFFIC = {("tc_knn", "bf16x3", N_Q): 319327744 + 483496192}
 
 
 def roofline(mode_name, prob, trace, peaks, clk):
