@@ -79,6 +79,11 @@ static cudaError_t scratch(int slot, size_t bytes, cudaStream_t st, void **out) 
   std::lock_guard<std::mutex> lk(g_mu);
   Buf &b = g_bufs[std::make_tuple(dev, (uintptr_t)st, slot)];
   if (b.n < bytes) {
+    // what cannot be had is refused before the present buffer is given up: a call that then takes
+    // fewer rows at a time runs in it, call after call
+    size_t left = 0, all = 0;
+    if (cudaMemGetInfo(&left, &all) == cudaSuccess && bytes > left + b.n)
+      return cudaErrorMemoryAllocation;
     if (b.p) {
       e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) return e;
@@ -537,7 +542,8 @@ struct RowChunks {
 };
 
 // Plans the call and gets its workspace; `whole`, when set, is the plan of all rows, and
-// `extra(rows, tail)` the bytes that a chunk takes behind its plan's. cudaErrorInvalidValue: no plan.
+// `extra(rows, tail)` the bytes that a chunk takes behind its plan's. cudaErrorInvalidValue: no
+// plan.
 template <typename Extra>
 static cudaError_t tc_workspace(int mode, const TcPlan *whole, int nq, int nc, int d, int k,
                                 cudaStream_t st, Extra extra, RowChunks *c, void **ws) {
@@ -568,8 +574,8 @@ static cudaError_t tc_workspace(int mode, const TcPlan *whole, int nq, int nc, i
 // Tensor-core approximate pass + FP64 re-rank (float inputs). `dbg`, when set, also receives
 // the approximate distance of every (query, candidate) pair (row stride dbg_ld) and `margin`
 // the per-query band width 2E.
-static int knn_device_tc(int mode, const TcPlan *plan, int nq, int nc, int d, int k, const float *Xq,
-                         const float *Xq2, long long nrows_q, const int *qidx, const float *Xc,
+static int knn_device_tc(int mode, const TcPlan *plan, int nq, int nc, int d, int k,
+                         const float *Xq, const float *Xq2, long long nrows_q, const int *qidx, const float *Xc,
                          const float *Xc2, long long nrows_c, const int *cidx, float *D, int *I,
                          int ldD, cudaStream_t st, float *dbg = nullptr, long long dbg_ld = 0,
                          float *margin = nullptr) {
@@ -696,9 +702,10 @@ static int knn_device_tc_double(int nq, int nc, int d, int k, const double *Xq, 
     int *Iq = I + (size_t)q0 * ldD;
     CU(tc_run_double(R, n, nc, d, k, Xq, Xq2, nrows_q, qidx + q0, Xc, Xc2, nrows_c, cidx, Dq, Iq,
                      ldD, ws, status, &left, &nleft, st, trace_hook, nullptr, q0 == 0));
-    const int rc = simt_run<double>(F[n != ch.rows], n, nc, d, k, Xq, Xq2, nrows_q, qidx + q0, Xc, Xc2, nrows_c,
-                                    cidx, Dq, Iq, ldD, static_cast<char *>(ws) + align256(R.bytes),
-                                    sw, st, 0, left, nleft);
+    const int rc = simt_run<double>(F[n != ch.rows], n, nc, d, k, Xq, Xq2, nrows_q, qidx + q0, Xc,
+                                    Xc2, nrows_c, cidx, Dq, Iq, ldD,
+                                    static_cast<char *>(ws) + align256(R.bytes), sw, st, 0, left,
+                                    nleft);
     if (rc != GSKNN_OK) return rc;
   }
   return set_status(GSKNN_OK, nullptr);

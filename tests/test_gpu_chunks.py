@@ -90,6 +90,12 @@ def test_a_workspace_that_does_not_fit(dtype):
     try:
         G.knn_device(X, X2, alpha, X, X2, beta, D, I)  # logs of all rows: 6 GB
         torch.cuda.synchronize()
+        held = torch.cuda.mem_get_info()[0]
+        D.fill_(float("inf"))
+        I.fill_(-1)
+        G.knn_device(X, X2, alpha, X, X2, beta, D, I)  # in the same workspace
+        torch.cuda.synchronize()
+        assert torch.cuda.mem_get_info()[0] == held
     finally:
         del keep
         torch.cuda.empty_cache()
