@@ -486,9 +486,9 @@ static int auto_slice(const Engine *E) {
 }
 
 // Times one probe batch (the first resident points as queries, as many as a batch of requests
-// holds, but at most 2,048 and no more than there are; k = max_k) in the prepared mode with escalation and in the escalation
-// mode alone; keeps the faster (second of two runs each, on slot 0's buffers). Returns false when a
-// probe call fails.
+// holds, but at most 2,048 and no more than there are; k = max_k) in the prepared mode with
+// escalation and in the escalation mode alone; keeps the faster (second of two runs each, on slot 0's
+// buffers). Returns false when a probe call fails.
 // (Probes of 1,024 rows took the two forms to be level where batches of 2,176 ran 1.4 times
 // faster in BF16: 1,048,576 x 128, 5.4 against 7.7 ms for 9,753 mixed rows.)
 static bool probe_modes(Engine *E, int esc) {

@@ -1681,8 +1681,8 @@ struct RerankSmem {
 };
 
 // One query by one warp. LEAF (the batching form): ids already in the row are not entered again,
-// overflowed queries are listed by their panel rows, the incoming row stays unsorted until a candidate can enter it, and a row nothing entered is
-// not written back.
+// overflowed queries are listed by their panel rows, the incoming row stays unsorted until a
+// candidate can enter it, and a row nothing entered is not written back.
 template <typename Tab, int E, bool LEAF>
 __device__ __forceinline__ void rerank_warp(const RerankParams<Tab> &p, int q, RerankSmem<E> &sm) {
   constexpr int CAP = rr_cap<E>();
@@ -2047,6 +2047,7 @@ __global__ void __launch_bounds__(32 * RR_WARPS, RR_OCC<E>) tc_rerank_cta(Rerank
   // bound the k-th far better, and what is left under their bound mostly fits (2 x 13,650, d = 141,
   // k = 100 321 us without this, 186).
   for (int pass = 0; n > RC_CAP && pass < 3; pass++) {
+    __syncthreads();  // every thread has read the count that warp 0 resets
     if (warp == 0) {
       const float T = fminf(s_T, fmaxf(list_bound(list, RC_CAP, k, lane), 0.0f));
       if (lane == 0) {
@@ -2880,7 +2881,8 @@ static cudaError_t tc_brute(const TcPlan &P, const TcCand &C, int d, int k, cons
   fp.status = status; fp.mirror = mirror;
   fp.k = k; fp.d = d; fp.nc = C.nc; fp.Xq = Xq; fp.Xq2 = Xq2;
   fp.Xc = static_cast<const float *>(C.Xc); fp.Xc2 = static_cast<const float *>(C.Xc2);
-  fp.qidx = qidx; fp.cidx = C.cidx; fp.nrows_q = nrows_q; fp.nrows_c = C.nrows_c; fp.D = D; fp.I = I; fp.ldD = ldD;
+  fp.qidx = qidx; fp.cidx = C.cidx; fp.nrows_q = nrows_q; fp.nrows_c = C.nrows_c;
+  fp.D = D; fp.I = I; fp.ldD = ldD;
   fp.list = reinterpret_cast<const int *>(base + P.o_fbl);
   fp.count = reinterpret_cast<const int *>(base + P.o_fbc);
   if (hook) hook(hook_ctx, "tc_fallback", true, st, 0);
